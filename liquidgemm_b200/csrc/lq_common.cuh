@@ -173,6 +173,174 @@ __device__ __forceinline__ void epi_stage_cols(uint16_t* col, int out_mode, cons
   }
 }
 
+// ---------------------------------------------------------------------------------------------
+// quantisers
+// ---------------------------------------------------------------------------------------------
+template <typename T> __device__ __forceinline__ float to_f32(T v);
+template <> __device__ __forceinline__ float to_f32<float>(float v) { return v; }
+template <> __device__ __forceinline__ float to_f32<__half>(__half v) { return __half2float(v); }
+template <> __device__ __forceinline__ float to_f32<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
+
+__device__ __forceinline__ float block_max(float v, float* red) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (lane == 0) red[warp] = v;
+  __syncthreads();
+  float r = lane < (blockDim.x >> 5) ? red[lane] : 0.f;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) r = fmaxf(r, __shfl_xor_sync(0xffffffffu, r, o));
+  return r;
+}
+
+// Nearest-integer quotients without a division.  Both quantisers need x / scale only to the nearest integer, with
+// |x / scale| < 127.5.  With inv = fl(1 / scale) the product x * inv differs from x / scale by a relative 2^-24, and
+// the IEEE quotient by another 2^-24: together less than 2^-15 here.  So wherever x * inv lies further than 2^-14
+// from every half-integer its nearest integer is rint(x / scale) bit for bit; elements closer than that (about one in
+// 4000), infinities and NaN take the division.
+constexpr float kRoundMagic = 12582912.0f;   // 1.5 * 2^23: x + kRoundMagic has rint(x) in its low bits
+constexpr float kSafeDist = 0.5f - 0x1p-14f;
+
+// max(a, |b|, |c|); unlike fmaxf, a NaN operand gives NaN.
+__device__ __forceinline__ float max_abs_nan(float a, float b, float c) {
+  float d;
+  asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+// Two float32 operations in one instruction (the quantisers are bound by instruction issue, not by the FMA pipe).
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmov.b64 rc, {%6, %7};\n\t"
+      "fma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 ra, rb, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tadd.rn.f32x2 rd, ra, rb;\n\t"
+      "mov.b64 {%0, %1}, rd;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
+
+// t[i] = kRoundMagic + (nearest integer of x[i] * inv); false when one of them needs the division.
+template <int N>
+__device__ __forceinline__ bool round_quotients(const float2 (&x)[N], float inv, float2 (&t)[N]) {
+  float far = 0.f;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    t[i] = fma2(x[i], both(inv), both(kRoundMagic));
+    const float2 r = add2(t[i], both(-kRoundMagic));     // the nearest integer, exactly
+    const float2 d = fma2(x[i], both(-inv), r);          // its distance from x * inv
+    far = max_abs_nan(far, d.x, d.y);
+  }
+  return far < kSafeDist;
+}
+
+// Two elements of a 32-bit word (16-bit types), low half first.
+template <typename T> __device__ __forceinline__ float2 unpack2(uint32_t w);
+template <> __device__ __forceinline__ float2 unpack2<__half>(uint32_t w) {
+  return __half22float2(*reinterpret_cast<const __half2*>(&w));
+}
+template <> __device__ __forceinline__ float2 unpack2<__nv_bfloat16>(uint32_t w) {
+  return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+}
+
+// Running |max| of a row, two 16-bit elements (or one float) at a time; NaN is ignored like fmaxf ignores it.
+template <typename T> struct RowMax;
+template <> struct RowMax<float> {
+  float m = 0.f;
+  __device__ __forceinline__ void take(const uint4& v) {
+    const float* e = reinterpret_cast<const float*>(&v);
+    m = fmaxf(fmaxf(m, fmaxf(fabsf(e[0]), fabsf(e[1]))), fmaxf(fabsf(e[2]), fabsf(e[3])));
+  }
+  __device__ __forceinline__ float value() const { return m; }
+};
+// (max.xorsign.abs: the larger magnitude in one instruction; its sign is dropped at the end)
+template <> struct RowMax<__half> {
+  uint32_t m = 0u;
+  static __device__ __forceinline__ uint32_t mx(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("max.xorsign.abs.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+  }
+  __device__ __forceinline__ void take(const uint4& v) { m = mx(m, mx(mx(v.x, v.y), mx(v.z, v.w))); }
+  __device__ __forceinline__ float value() const {
+    const __half2 h = __habs2(*reinterpret_cast<const __half2*>(&m));
+    return fmaxf(__low2float(h), __high2float(h));
+  }
+};
+template <> struct RowMax<__nv_bfloat16> {
+  uint32_t m = 0u;
+  static __device__ __forceinline__ uint32_t mx(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("max.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+  }
+  __device__ __forceinline__ void take(const uint4& v) { m = mx(m, mx(mx(v.x, v.y), mx(v.z, v.w))); }
+  __device__ __forceinline__ float value() const {
+    return fmaxf(fabsf(__uint_as_float(m << 16)), fabsf(__uint_as_float(m & 0xffff0000u)));
+  }
+};
+
+// The elements of one 16-byte vector, in pairs.
+template <typename T>
+__device__ __forceinline__ void vec_floats(const uint4& raw, float2 (&x)[8 / sizeof(T)]) {
+  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+  for (int i = 0; i < 8 / (int)sizeof(T); ++i) {
+    if constexpr (sizeof(T) == 4) x[i] = make_float2(__uint_as_float(w[2 * i]), __uint_as_float(w[2 * i + 1]));
+    else x[i] = unpack2<T>(w[i]);
+  }
+}
+
+// ---- activations ----
+__device__ __forceinline__ int quant1(float x, float scale) {
+  // IEEE division, round half to even, clamp: liquidgemm/quant.py:140 of the reference.
+  int q = __float2int_rn(__fdiv_rn(x, scale));
+  return max(-127, min(127, q));
+}
+
+// The quantised bytes of one 16-byte vector: VEC int8 in VEC / 4 words.
+template <typename T>
+__device__ __forceinline__ void quant_vec(const uint4& raw, float scale, float inv, uint32_t (&out)[4 / sizeof(T)]) {
+  constexpr int VEC = 16 / sizeof(T);
+  float2 x[VEC / 2], t[VEC / 2];
+  vec_floats<T>(raw, x);
+  uint32_t q[VEC];
+  const bool safe = round_quotients(x, inv, t);
+#pragma unroll
+  for (int i = 0; i < VEC / 2; ++i) {
+    q[2 * i] = __float_as_uint(t[i].x);
+    q[2 * i + 1] = __float_as_uint(t[i].y);
+  }
+  if (!safe) {
+#pragma unroll
+    for (int i = 0; i < VEC / 2; ++i) {
+      q[2 * i] = (uint32_t)quant1(x[i].x, scale);
+      q[2 * i + 1] = (uint32_t)quant1(x[i].y, scale);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < VEC / 4; ++i)
+    out[i] = __byte_perm(__byte_perm(q[4 * i], q[4 * i + 1], 0x0040), __byte_perm(q[4 * i + 2], q[4 * i + 3], 0x0040), 0x5410);
+}
+
+// The register-held row kernels: how many units (a power of two, at most nv_max) of a row of `n` a thread holds, and the
+// CTA's threads.  Few rows spread wide, so that a row's latency is short; many rows use small CTAs (down to
+// `few_threads`), whose load, reduction and store phases overlap each other's.  0: the row does not fit.
+inline int row_units_per_thread(long rows, long n, int nv_max, int few_threads, int max_threads, int* threads) {
+  for (int nv = 1; nv <= nv_max; nv *= 2) {
+    *threads = (int)((n + nv - 1) / nv + 31) / 32 * 32;
+    if (*threads <= max_threads && (nv == nv_max || *threads <= few_threads || rows * *threads <= (long)sm_count() * 1280))
+      return nv;
+  }
+  return 0;
+}
+
 // Where a kernel's outputs go: the same [M, N] block is written into up to 8 row-major matrices with
 // row stride `ld` elements at column offset `col0`.  One destination with ld = N, col0 = 0 is the
 // ordinary output; several destinations (this GPU's and its peers' full-width output, mapped into this
