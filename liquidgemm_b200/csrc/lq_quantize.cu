@@ -24,10 +24,144 @@ namespace quantw {
 
 constexpr int kTileBytes = 8704;
 
-template <typename T> __device__ __forceinline__ float to_f32(T v);
-template <> __device__ __forceinline__ float to_f32<float>(float v) { return v; }
-template <> __device__ __forceinline__ float to_f32<__half>(__half v) { return __half2float(v); }
-template <> __device__ __forceinline__ float to_f32<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
+// ---- one pass: a CTA per row, the row in registers ------------------------------------------------------------
+// Thread t holds the 32-element units t, t + threads, ... (NV of them): the row is read once and the row scale needs
+// one block reduction.  A unit is one 16-byte chunk of the blob, and a group of 64 (128) elements is the units of two
+// (four) neighbouring lanes, so a group's range takes one (two) shuffles and its step is worked out once per 32 elements.
+// Bound by instruction issue (the two IEEE divisions an element that this replaces, and the group arithmetic once per
+// eight elements of a first version, were most of the time).
+
+// 32 bytes in one load (32-byte aligned).
+__device__ __forceinline__ void ldg_stream_v8(const void* p, uint4& a, uint4& b) {
+  asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
+               : "l"(p));
+}
+
+template <typename T, int NV>
+__global__ void __launch_bounds__(NV * sizeof(T) >= 16 ? 256 : 512)
+quantise_rows_kernel(const T* __restrict__ w, float* __restrict__ s1, uint8_t* __restrict__ s_u8,
+                     uint8_t* __restrict__ offset_a, uint8_t* __restrict__ codes, uint8_t* __restrict__ blob,
+                     int* __restrict__ status, int N, int K, int group) {
+  __shared__ float red[32];
+  constexpr int VU = 2 * sizeof(T);   // 16-byte vectors of a unit
+  const int row = blockIdx.x;
+  const int units = K >> 5;
+  const int lane = threadIdx.x & 31;
+  uint8_t* tile = blob + (size_t)(row >> 7) * (K >> 7) * kTileBytes;   // of k-tile 0
+  const int r = row & 127;
+  if (row >= N) {   // padding rows of the last tile: code 0, step 1, offset 128 reconstructs to 0
+    for (int u = threadIdx.x; u < units; u += blockDim.x) {
+      uint8_t* t = tile + (size_t)(u >> 2) * kTileBytes;
+      *reinterpret_cast<uint4*>(t + ((u & 3) * 128 + r) * 16) = make_uint4(0u, 0u, 0u, 0u);
+      if ((u & 1) == 0) *reinterpret_cast<uint16_t*>(t + 8192 + r * 4 + (u & 2)) = 0x8001;
+    }
+    return;
+  }
+  const T* src = w + (size_t)row * K;
+  uint4 raw[NV][VU];
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int u = threadIdx.x + i * blockDim.x;
+#pragma unroll
+    for (int v = 0; v < VU; v += 2) {
+      raw[i][v] = raw[i][v + 1] = make_uint4(0u, 0u, 0u, 0u);
+      if (u < units) ldg_stream_v8(src + (size_t)u * 32 + v * (32 / VU), raw[i][v], raw[i][v + 1]);
+    }
+  }
+  RowMax<T> rm;
+#pragma unroll
+  for (int i = 0; i < NV; ++i)
+#pragma unroll
+    for (int v = 0; v < VU; ++v) rm.take(raw[i][v]);
+  const float amax = block_max(rm.value(), red);
+  const float scale = __fdiv_rn(fmaxf(amax, 1e-12f), 119.0f);
+  const float inv = __fdiv_rn(1.0f, scale);
+  if (threadIdx.x == 0) s1[row] = scale;
+  const float inv_of_lane = __fdiv_rn(1.0f, (float)max(lane, 1));   // 1 / step, fetched by shuffle
+  constexpr int kMagicBits = 0x4B400000;                            // kRoundMagic
+  const int lanes = group >> 5;                                     // units of a group
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int u = threadIdx.x + i * blockDim.x;
+    // level 1: q = clamp(rint(w / s1), -119, 119), kept as kRoundMagic + q (|w| <= amax: the fast side needs no clamp)
+    float2 t[4][4];
+    float mx = kRoundMagic - 128.0f, mn = kRoundMagic + 128.0f;
+#pragma unroll
+    for (int o = 0; o < 4; ++o) {   // octets: one 32-bit word of the blob each
+      float2 x[4];
+#pragma unroll
+      for (int v = 0; v < VU / 4; ++v) {
+        float2 e[8 / sizeof(T)];
+        vec_floats<T>(raw[i][o * (VU / 4) + v], e);
+#pragma unroll
+        for (int j = 0; j < 8 / (int)sizeof(T); ++j) x[v * (8 / sizeof(T)) + j] = e[j];
+      }
+      if (!round_quotients(x, inv, t[o])) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          t[o][j].x = kRoundMagic + (float)max(-119, min(119, __float2int_rn(__fdiv_rn(x[j].x, scale))));
+          t[o][j].y = kRoundMagic + (float)max(-119, min(119, __float2int_rn(__fdiv_rn(x[j].y, scale))));
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        mx = fmaxf(fmaxf(mx, t[o][j].x), t[o][j].y);
+        mn = fminf(fminf(mn, t[o][j].x), t[o][j].y);
+      }
+    }
+    // (max, -min) of the group as two 16-bit halves
+    uint32_t pk = ((uint32_t)(__float_as_int(mx) - kMagicBits) & 0xffffu) |
+                  ((uint32_t)(kMagicBits - __float_as_int(mn)) << 16);
+    pk = __vmaxs2(pk, __shfl_xor_sync(0xffffffffu, pk, 1));
+    if (group == 128) pk = __vmaxs2(pk, __shfl_xor_sync(0xffffffffu, pk, 2));
+    const int neg_lo = (int)pk >> 16;
+    const int range = (int)(short)(pk & 0xffffu) + neg_lo;
+    const int step = max(1, (range + 14) / 15);   // ceil(range / 15): 0 <= range <= 238, so at most 16
+    const int off = 128 - neg_lo;
+    // level 2: code = rint((q - lo) / step).  The product with fl(1 / step) is within 15 * 2^-24 of the quotient, the
+    // nearest quotient that is not a half-integer is 1/32 away from one, and adding 1.5 * 2^13 first rounds the
+    // product to a multiple of 2^-10: half-integers come out exact and the second addition resolves them to even,
+    // like the division would.  No clamp: (q - lo) / step <= range / ceil(range / 15) <= 15.
+    const float inv_step = __shfl_sync(0xffffffffu, inv_of_lane, step);
+    const float2 minus_lo = both((float)neg_lo - kRoundMagic);
+    if (u >= units) continue;
+    uint32_t words[4];   // byte b of word o = code[8 o + b] | code[8 o + 4 + b] << 4
+    uint32_t bytes[8];
+#pragma unroll
+    for (int o = 0; o < 4; ++o) {
+      uint32_t c[8];   // kMagicBits + code
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 e = add2(fma2(add2(t[o][j], minus_lo), both(inv_step), both(12288.0f)), both(kRoundMagic - 12288.0f));
+        c[2 * j] = __float_as_uint(e.x);
+        c[2 * j + 1] = __float_as_uint(e.y);
+      }
+      bytes[2 * o] = __byte_perm(__byte_perm(c[0], c[1], 0x0040), __byte_perm(c[2], c[3], 0x0040), 0x5410);
+      bytes[2 * o + 1] = __byte_perm(__byte_perm(c[4], c[5], 0x0040), __byte_perm(c[6], c[7], 0x0040), 0x5410);
+      words[o] = bytes[2 * o] | (bytes[2 * o + 1] << 4);
+    }
+    if (blob) {
+      uint8_t* tk = tile + (size_t)(u >> 2) * kTileBytes;
+      *reinterpret_cast<uint4*>(tk + ((u & 3) * 128 + r) * 16) = make_uint4(words[0], words[1], words[2], words[3]);
+      if ((u & 1) == 0) *reinterpret_cast<uint16_t*>(tk + 8192 + r * 4 + (u & 2)) = (uint16_t)(step | (off << 8));
+    }
+    if ((u & (lanes - 1)) == 0) {
+      const size_t g = (size_t)row * (units / lanes) + u / lanes;
+      s_u8[g] = (uint8_t)step;
+      offset_a[g] = (uint8_t)off;
+      // The packed dequant's invariant, once per group: code * step + offset grows with q, so its largest value
+      // belongs to the group's largest q (and its smallest is the offset).
+      const int top = __float2int_rn(__fmul_rn((float)range, inv_step));
+      if (step > 16 || off < 0 || top * step + off > 255) atomicExch(status, 501);
+    }
+    if (codes) {
+      uint4* dst = reinterpret_cast<uint4*>(codes + (size_t)row * K + (size_t)u * 32);
+      dst[0] = make_uint4(bytes[0], bytes[1], bytes[2], bytes[3]);
+      dst[1] = make_uint4(bytes[4], bytes[5], bytes[6], bytes[7]);
+    }
+  }
+}
 
 template <typename T>
 __global__ void __launch_bounds__(256) row_amax_kernel(const T* __restrict__ w, float* __restrict__ s1, int N, long K) {
@@ -160,6 +294,20 @@ static int run(const void* w, int N, long K, int group, float* s1, uint8_t* s_u8
                uint8_t* blob, cudaStream_t st) {
   int* status = status_word();
   if (!status) return LQ_ERR_CUDA;
+  // One pass wherever the rows are 32-byte vectors and a CTA holds one.
+  int threads = 0;
+  const int nv = (reinterpret_cast<uintptr_t>(w) & 31) == 0
+                     ? row_units_per_thread(N, K >> 5, 4, 256, sizeof(T) == 2 ? 512 : 256, &threads) : 0;
+  if (nv) {
+    const int rows = blob ? (N + 127) / 128 * 128 : N;
+    auto launch = [&](auto kern) {
+      kern<<<rows, threads, 0, st>>>(static_cast<const T*>(w), s1, s_u8, offset_a, codes, blob, status, N, (int)K, group);
+    };
+    if (nv == 1) launch(quantise_rows_kernel<T, 1>);
+    else if (nv == 2) launch(quantise_rows_kernel<T, 2>);
+    else launch(quantise_rows_kernel<T, 4>);
+    return check_launch("quantise_rows_kernel");
+  }
   row_amax_kernel<T><<<(N + 7) / 8, 256, 0, st>>>(static_cast<const T*>(w), s1, N, K);
   if (int rc = check_launch("row_amax_kernel")) return rc;
   dim3 grid((unsigned)(K >> 7), (unsigned)((N + 127) / 128));

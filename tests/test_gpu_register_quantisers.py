@@ -71,3 +71,24 @@ def test_tokens_of_every_kind_match_the_general_kernel(ops, dtype, K):
     x = _specials(_ragged(6, K, dtype, K, 127)).cuda()
     a, b = torch.ops.liquidgemm.quant_per_token(x), torch.ops.liquidgemm.quant_per_token(_unaligned(x))
     assert torch.equal(a[0], b[0]) and torch.equal(a[1].view(torch.int32), b[1].view(torch.int32))
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("group", [64, 128])
+@pytest.mark.parametrize("N,K", [(6, 128), (130, 384), (6, 4096), (6, 4224), (6, 14336), (6, 32768), (6, 32896)])
+def test_weights_of_every_kind_match_the_general_kernels(ops, dtype, group, N, K):
+    w = _ragged(N, K, dtype, N + K, 119)
+    for v in (w, _specials(w)):
+        v = v.cuda()
+        a, ab = ops.quantize_weight_cuda(v, group, want_codes=True, want_blob=True)
+        b, bb = ops.quantize_weight_cuda(_unaligned(v), group, want_codes=True, want_blob=True)
+        assert torch.equal(a.s1.view(torch.int32), b.s1.view(torch.int32))
+        assert torch.equal(a.s_u8, b.s_u8) and torch.equal(a.offset_a, b.offset_a)
+        assert torch.equal(a.qweight_u4, b.qweight_u4) and torch.equal(ab, bb)
+        only, none = ops.quantize_weight_cuda(v, group, want_codes=True, want_blob=False)
+        assert none is None and torch.equal(only.qweight_u4, a.qweight_u4)
+    want = O.quantize_weight(w.float().numpy(), group)
+    got, _ = ops.quantize_weight_cuda(w.cuda(), group)
+    assert np.array_equal(got.qweight_u4.cpu().numpy(), want.qweight_u4)
+    assert np.array_equal(got.s_u8.cpu().numpy(), want.s_u8) and np.array_equal(got.offset_a.cpu().numpy(), want.offset_a)
+    ops.poll_status()
