@@ -211,7 +211,7 @@ LQ_API int lq_quantize_weight(const void* w, int w_dtype, int N, int K, int grou
  *              (scaled outputs only): streaming dp4a GEMV over the tile blob;
  *     up to 16 tokens on matrices up to 32 M weights: the streaming tensor-core kernel, ONE launch:
  *              stream-K over two CTAs per SM, one 64-bit atomic per element joins cut tiles;
- *     3072 tokens and more (5120 on matrices above 32 M weights) on layers with K < 8192, whole 256-channel
+ *     3072 tokens and more (2048 on matrices above 32 M weights) on layers with K < 8192, whole 256-channel
  *              blocks and at most 256 M weights, one destination: the blob is unpacked to INT8 in the workspace
  *              (scratch, N x K bytes) and the INT8 x INT8 CTA-pair kernel does the GEMM, TWO launches
  *              (LQ_UNPACK_I8_MIN_M in the environment moves the limit, 0 switches the route off);
@@ -260,6 +260,16 @@ LQ_API int lq_w4a8_linear_bias(const int8_t* x_i8, const uint8_t* blob, const fl
                         const float* s1, const void* bias, void* y, int out_dtype, int M, int N, int K,
                         void* workspace, size_t workspace_bytes, void* stream);
 
+/* One W4A8 linear from activations to outputs: lq_quant_per_token followed by lq_w4a8_gemm_fused (with `bias`, or null:
+ * lq_w4a8_linear_bias), bit for bit.  For a few tokens it is ONE kernel, which quantises the tokens itself; otherwise
+ * the quantised tokens go through `scratch`.
+ * lq_linear_plan() fills plan[0] = scratch bytes (any content, 16-byte aligned), plan[1] = workspace bytes and
+ * plan[2] = workspace kind (as lq_gemm_workspace_kind) for the same x (its alignment matters), M, N, K and splitk. */
+LQ_API int lq_linear_plan(const void* x, int M, int N, int K, int splitk, size_t* plan);
+LQ_API int lq_w4a8_linear(const void* x, int x_dtype, const uint8_t* blob, const float* s1, const void* bias, void* y,
+                   int out_dtype, int M, int N, int K, int splitk, void* scratch, size_t scratch_bytes,
+                   void* workspace, size_t workspace_bytes, void* stream);
+
 /* Plain INT8 x INT8 -> INT32 tensor-core GEMM c[M,N] = a[M,K] @ b[N,K]^T.
  * Replaces torch.ops.liquidgemm.wgmma_i8_gemm (reference csrc/liquid_gemm/w4a8_wgmma.cu:648-694).
  * K % 128 == 0; M and N are arbitrary here (the reference needs multiples of 128).
@@ -275,6 +285,7 @@ LQ_API int lq_i8_gemm_i32(const int8_t* a, const int8_t* b, int32_t* c, int M, i
 LQ_API int lq_i8_gemm_scaled(const int8_t* a, const int8_t* b, const float* a_scale,
                       const float* b_scale, void* y, int out_dtype, int M, int N, int K,
                       void* stream);
+
 
 #ifdef __cplusplus
 }

@@ -54,6 +54,8 @@ _SIGNATURES = {
     "lq_gemm_workspace_kind": (c_int, [c_int, c_int, c_int, c_int]),
     "lq_gemm_launches": (c_int, [c_int, c_int, c_int, c_int]),
     "lq_w4a8_linear_bias": (c_int, [P, P, P, P, P, P, c_int, c_int, c_int, c_int, P, c_size_t, P]),
+    "lq_linear_plan": (c_int, [P, c_int, c_int, c_int, c_int, P]),
+    "lq_w4a8_linear": (c_int, [P, c_int, P, P, P, P, c_int, c_int, c_int, c_int, c_int, P, c_size_t, P, c_size_t, P]),
     "lq_quantize_weight": (c_int, [P, c_int, c_int, c_int, c_int, P, P, P, P, P, P]),
     "lq_w4a8_gemm_i32": (c_int, [P, P, P, c_int, c_int, c_int, c_int, P, c_size_t, P]),
     "lq_w4a8_gemm_fused": (c_int, [P, P, P, P, P, c_int, c_int, c_int, c_int, c_int, P, c_size_t, P]),

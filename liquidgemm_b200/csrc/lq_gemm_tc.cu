@@ -66,6 +66,9 @@ size_t gemv_blob_workspace_bytes(int N, int K);                              // 
 int run_gemv_blob_ws(const int8_t* x, const uint8_t* blob, const float* ascale, const float* s1, const void* bias,
                      const OutSpec& out, const PeerSync* sync, int out_dtype, int M, int N, int K, void* ws,
                      size_t ws_bytes, cudaStream_t st);  // lq_gemv_blob.cu
+bool gemv_quant_serves(int M, int N, int K);                                 // lq_gemv_blob.cu
+int run_gemv_quant(const void* x, int x_dtype, const uint8_t* blob, const float* s1, const void* bias, void* out,
+                   int out_dtype, int M, int N, int K, void* ws, size_t ws_bytes, cudaStream_t st);   // lq_gemv_blob.cu
 int decode_tc_grid(int N, int K);                                            // lq_decode_tc.cu
 bool pair_serves(int M, int N, int K);                                       // lq_gemm_pair.cu
 bool i8_pair_serves(int M, int N, int K);                                    // lq_i8_pair.cu
@@ -841,6 +844,65 @@ int lq_w4a8_linear_bias(const int8_t* x_i8, const uint8_t* blob, const float* as
   if (bias && (reinterpret_cast<uintptr_t>(bias) % (out_dtype == LQ_DT_F32 ? 4 : 2))) return LQ_ERR_BAD_ARG;
   return blob_gemm(x_i8, blob, ascale, s1, bias, y, out_dtype, M, N, K, 0, workspace, workspace_bytes,
                    as_stream(stream));
+}
+
+// ---- one call from activations to outputs -------------------------------------------------------------------------
+static bool quantises_in_gemv(const void* x, int M, int N, int K, int splitk) {
+  return splitk == 0 && gemv_quant_serves(M, N, K) && reinterpret_cast<uintptr_t>(x) % 16 == 0;
+}
+
+static size_t token_scratch_bytes(int M, int K) { return (((size_t)M * K + 255) & ~(size_t)255) + (size_t)M * 4; }
+
+int lq_linear_plan(const void* x, int M, int N, int K, int splitk, size_t* plan) {
+  if (!plan || M <= 0 || N <= 0) return LQ_ERR_BAD_ARG;
+  if (K < 128 || K % 128) return LQ_ERR_SHAPE;
+  if (quantises_in_gemv(x, M, N, K, splitk)) {
+    plan[0] = 0;
+    plan[1] = gemv_blob_workspace_bytes(N, K);
+    plan[2] = 2;
+  } else {
+    plan[0] = token_scratch_bytes(M, K);
+    plan[1] = lq_gemm_workspace_bytes(M, N, K, splitk);
+    plan[2] = (size_t)lq_gemm_workspace_kind(M, N, K, splitk);
+  }
+  return LQ_OK;
+}
+
+static int linear_impl(const void* x, int x_dtype, const uint8_t* blob, const float* s1, const void* bias, void* y,
+                       int out_dtype, int M, int N, int K, int splitk, bool one_kernel, void* scratch, size_t scratch_bytes,
+                       void* workspace, size_t workspace_bytes, void* stream) {
+  if (one_kernel) {
+    if (int rc = lq_check_device()) return rc;
+    return run_gemv_quant(x, x_dtype, blob, s1, bias, y, out_dtype, M, N, K, workspace, workspace_bytes, as_stream(stream));
+  }
+  if (!scratch || reinterpret_cast<uintptr_t>(scratch) % 16 || scratch_bytes < token_scratch_bytes(M, K)) return LQ_ERR_WORKSPACE;
+  int8_t* xq = static_cast<int8_t*>(scratch);
+  float* ascale = reinterpret_cast<float*>(xq + (((size_t)M * K + 255) & ~(size_t)255));
+  if (int rc = lq_quant_per_token(x, x_dtype, xq, ascale, M, K, stream)) return rc;
+  return blob_gemm(xq, blob, ascale, s1, bias, y, out_dtype, M, N, K, splitk, workspace, workspace_bytes, as_stream(stream));
+}
+
+int lq_w4a8_linear(const void* x, int x_dtype, const uint8_t* blob, const float* s1, const void* bias, void* y,
+                   int out_dtype, int M, int N, int K, int splitk, void* scratch, size_t scratch_bytes, void* workspace,
+                   size_t workspace_bytes, void* stream) {
+  if (!x || !blob || !s1 || !y || M < 0 || N <= 0 || K <= 0) return LQ_ERR_BAD_ARG;
+  if (x_dtype < LQ_DT_BF16 || x_dtype > LQ_DT_F32 || out_dtype < LQ_DT_BF16 || out_dtype > LQ_DT_F32) return LQ_ERR_BAD_ARG;
+  if (bias && (reinterpret_cast<uintptr_t>(bias) % (out_dtype == LQ_DT_F32 ? 4 : 2))) return LQ_ERR_BAD_ARG;
+  if (K % 128) return LQ_ERR_SHAPE;
+  if (reinterpret_cast<uintptr_t>(blob) % 16) return LQ_ERR_BAD_ARG;
+  if (M == 0) return LQ_OK;
+  return linear_impl(x, x_dtype, blob, s1, bias, y, out_dtype, M, N, K, splitk, quantises_in_gemv(x, M, N, K, splitk), scratch,
+                     scratch_bytes, workspace, workspace_bytes, stream);
+}
+
+// The same for lq_w4a8_linear_host, whose callers size the workspace with lq_gemm_workspace_bytes() and _kind(): one
+// kernel where that contract already hands it the all-zero buffer.
+int linear_for_host(const void* x, int x_dtype, const uint8_t* blob, const float* s1, void* y, int out_dtype, int M, int N,
+                    int K, void* scratch, size_t scratch_bytes, void* workspace, size_t workspace_bytes, void* stream) {
+  const bool one = quantises_in_gemv(x, M, N, K, 0) && lq_gemm_workspace_kind(M, N, K, 0) == 2 &&
+                   workspace_bytes >= gemv_blob_workspace_bytes(N, K);
+  return linear_impl(x, x_dtype, blob, s1, nullptr, y, out_dtype, M, N, K, 0, one, scratch, scratch_bytes, workspace,
+                     workspace_bytes, stream);
 }
 
 int lq_w4a8_gemm_fused_scatter_sync(const int8_t* x_i8, const uint8_t* blob, const float* ascale, const float* s1,

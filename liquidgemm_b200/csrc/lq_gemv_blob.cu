@@ -41,10 +41,12 @@ constexpr uint64_t kWaitLimitNs = 2000000000ull;
 // finishes its reduction and leaves the workspace clean.
 constexpr uint64_t kPeerWaitLimitNs = 1000000000ull;
 
+constexpr int kMaxQuantSmem = 112 * 1024;   // quantising form: two CTAs per SM
+
 struct Args {
   const uint8_t* blob;
-  const int8_t* x;       // [M, K]
-  const float* ascale;   // [M]
+  const void* x;         // [M, K]: int8 tokens, or the activations themselves (kernels that quantise)
+  const float* ascale;   // [M]; null with activations
   const float* s1;       // [N]
   void* out;             // [M, N] (single-destination kernels; the others get a MultiOut parameter)
   unsigned long long* slots;   // [grid][MT][128] packed (k-tile count, biased partial sum), zero between launches
@@ -54,12 +56,12 @@ struct Args {
   const void* bias;      // [N] in the output dtype, or null
 };
 
-template <int MT, int NS>
+template <int MT, int NS, bool QUANT = false>
 struct Cfg {
-  static constexpr int kXStage = MT * 128;
+  static constexpr int kXStage = QUANT ? 0 : MT * 128;
   static constexpr int kStage = kTileBytes + kXStage;
   static constexpr int kRedBytes = MT * 128 * 4;
-  static constexpr int kUsedBytes = 128 + NS * kStage + 2 * NS * 8 + kRedBytes + 16;
+  static constexpr int kUsedBytes = 128 + NS * kStage + 2 * NS * 8 + kRedBytes + 16;   // QUANT: and the quantised tokens behind it
   // Never three CTAs on one SM: with programmatic dependent launch the next kernel's CTAs fill whatever
   // fits, and an SM that holds three streams while its neighbour holds one makes the slowest CTA
   // (hence the kernel) much later than the average one.  Asking for more than a third of the SM's
@@ -78,11 +80,69 @@ __device__ __forceinline__ int dp4a_s8(uint32_t w, uint32_t x, int acc) {
   return d;
 }
 
-template <int MT, int NS, bool MULTI>
+// The quantising form (XT an activation type): tokens of the k-tiles a CTA works on, in the order it meets them.
+struct TokenTiles {
+  int first, count;   // k-tile of the CTA's first unit; k-tiles it needs (all of K when its range is longer)
+};
+__device__ __forceinline__ TokenTiles token_tiles(const SegmentWalk& walk) {
+  SegmentWalk w = walk;
+  Segment s;
+  TokenTiles t = {0, 0};
+  if (w.split == 0) {
+    t.first = (int)(w.u % (unsigned)w.kt);
+    t.count = min((int)(w.u_end - w.u), w.kt);
+  } else if (w.next(s)) {   // a fixed split gives every CTA one segment
+    t.first = s.kb;
+    t.count = s.ke - s.kb;
+  }
+  return t;
+}
+
+// amax of the CTA's token rows over the whole of K, in registers of all consumer threads; eight loads in flight each.
+template <int MT, typename XT>
+__device__ __forceinline__ void token_amax(const XT* x, int M, int K, int c, float (&amax)[MT], float* red) {
+  constexpr int VEC = 16 / sizeof(XT);
+  constexpr int U = MT >= 8 ? 1 : 8 / MT;
+  const int nvec = K / VEC;
+  RowMax<XT> rm[MT];
+#pragma unroll 1
+  for (int v0 = c; v0 < nvec; v0 += U * kConsumers) {
+    uint4 raw[MT][U];
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int v = v0 + u * kConsumers;
+        raw[m][u] = (m < M && v < nvec) ? *reinterpret_cast<const uint4*>(x + (size_t)m * K + (size_t)v * VEC)
+                                        : make_uint4(0u, 0u, 0u, 0u);
+      }
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+      for (int u = 0; u < U; ++u) rm[m].take(raw[m][u]);
+  }
+#pragma unroll
+  for (int m = 0; m < MT; ++m) {
+    amax[m] = rm[m].value();
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) amax[m] = fmaxf(amax[m], __shfl_xor_sync(0xffffffffu, amax[m], o));
+    if ((c & 31) == 0) red[m * 8 + (c >> 5)] = amax[m];
+  }
+  consumer_barrier();
+#pragma unroll
+  for (int m = 0; m < MT; ++m) {
+    const float4 a = *reinterpret_cast<const float4*>(red + m * 8), b = *reinterpret_cast<const float4*>(red + m * 8 + 4);
+    amax[m] = fmaxf(fmaxf(fmaxf(a.x, a.y), fmaxf(a.z, a.w)), fmaxf(fmaxf(b.x, b.y), fmaxf(b.z, b.w)));
+  }
+}
+
+template <int MT, int NS, bool MULTI, typename XT>
 __global__ void __launch_bounds__(kThreads, 2)
 gemv_blob_kernel(const Args args, const std::conditional_t<MULTI, MultiOut, NoMultiOut> multi) {
+  constexpr bool QUANT = !std::is_same_v<XT, int8_t>;
+  static_assert(!(QUANT && MULTI), "the quantising form has one destination");
   const int kt_total = args.K >> 7;
-  using C = Cfg<MT, NS>;
+  using C = Cfg<MT, NS, QUANT>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 127u) & ~127u;
@@ -93,6 +153,7 @@ gemv_blob_kernel(const Args args, const std::conditional_t<MULTI, MultiOut, NoMu
   const uint32_t bar_full = xs + NS * C::kXStage;
   const uint32_t bar_empty = bar_full + NS * 8;
   int32_t* red = reinterpret_cast<int32_t*>(smem + (bar_empty + NS * 8 - base));   // [MT][128]
+  uint8_t* xq = smem + (bar_empty + NS * 8 - base) + C::kRedBytes;                 // QUANT: [k-tiles][MT][128]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int M = args.M;
@@ -121,7 +182,7 @@ gemv_blob_kernel(const Args args, const std::conditional_t<MULTI, MultiOut, NoMu
     if (lane == 0) {
       // One plain 128-byte copy per token and k-tile.  (A single tensor-map box of MT rows x 128 bytes per
       // k-tile instead was measured: equal at two tokens, 10-15 % slower at four.)
-      const uint32_t tx = (uint32_t)(kTileBytes + M * 128);
+      const uint32_t tx = (uint32_t)(kTileBytes + (QUANT ? 0 : M * 128));   // QUANT: the consumers fetch the tokens
       Ring<NS> ring;
       int issued = 0;
       bool ok = true;
@@ -131,6 +192,10 @@ gemv_blob_kernel(const Args args, const std::conditional_t<MULTI, MultiOut, NoMu
       int early_kt[NS];
       bool dependency_met = false;
       auto meet_dependency = [&]() {
+        if constexpr (QUANT) {
+          dependency_met = true;
+          return;
+        }
         dependency_wait();
         if constexpr (MULTI) {
           if (!peer_wait(multi.sync, kPeerWaitLimitNs)) atomicExch(args.status, 303);   // tokens gathered from peers
@@ -138,7 +203,7 @@ gemv_blob_kernel(const Args args, const std::conditional_t<MULTI, MultiOut, NoMu
         dependency_met = true;
         const int n = issued < NS ? issued : NS;
         for (int j = 0; j < n; ++j) {
-          const int8_t* xsrc = args.x + (size_t)early_kt[j] * 128;
+          const int8_t* xsrc = static_cast<const int8_t*>(args.x) + (size_t)early_kt[j] * 128;
           for (int m = 0; m < M; ++m)
             ptx::bulk_load(xs + j * C::kXStage + m * 128, xsrc + (size_t)m * args.K, 128, bar_full + 8 * j);
         }
@@ -158,10 +223,11 @@ gemv_blob_kernel(const Args args, const std::conditional_t<MULTI, MultiOut, NoMu
           const uint32_t full = bar_full + 8 * ring.s;
           ptx::mbar_expect_tx(full, tx);
           ptx::bulk_load(ws + ring.s * kTileBytes, src, kTileBytes, full);
-          if (issued < NS) {
+          if (QUANT) {
+          } else if (issued < NS) {
             early_kt[issued] = kt;
           } else {
-            const int8_t* xsrc = args.x + (size_t)kt * 128;
+            const int8_t* xsrc = static_cast<const int8_t*>(args.x) + (size_t)kt * 128;
             for (int m = 0; m < M; ++m)
               ptx::bulk_load(xs + ring.s * C::kXStage + m * 128, xsrc + (size_t)m * args.K, 128, full);
           }
@@ -194,8 +260,40 @@ gemv_blob_kernel(const Args args, const std::conditional_t<MULTI, MultiOut, NoMu
       else store_out_bias(args.out, (size_t)m * args.N + n, v, bias, has_bias, args.out_dtype);
     };
     float a_scale[MT];   // token scales: read once, they are needed right after the last tile
+    [[maybe_unused]] int x_tile = 0, x_tiles = 0;   // QUANT: position in, and number of, the CTA's token tiles
+    if constexpr (!QUANT) {
 #pragma unroll
-    for (int m = 0; m < MT; ++m) a_scale[m] = (m < M) ? __ldg(args.ascale + m) : 0.f;
+      for (int m = 0; m < MT; ++m) a_scale[m] = (m < M) ? __ldg(args.ascale + m) : 0.f;
+    } else {
+      const XT* x = static_cast<const XT*>(args.x);
+      float inv[MT];
+      token_amax<MT, XT>(x, M, args.K, c, a_scale, reinterpret_cast<float*>(red));
+#pragma unroll
+      for (int m = 0; m < MT; ++m) {
+        a_scale[m] = __fdiv_rn(fmaxf(a_scale[m], 1e-12f), 127.0f);
+        inv[m] = __fdiv_rn(1.0f, a_scale[m]);
+      }
+      const TokenTiles tt = token_tiles(walk);
+      x_tiles = tt.count;
+      constexpr int VEC = 16 / sizeof(XT), VPT = 128 / VEC;   // vectors of a token's 128-element slice
+      for (int i = c; i < tt.count * VPT; i += kConsumers) {
+        const int j = i / VPT, q = i % VPT;
+        int kt = tt.first + j;
+        if (kt >= kt_total) kt -= kt_total;
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+          if (m < M) {
+            uint32_t w[4 / sizeof(XT)];
+            quant_vec<XT>(*reinterpret_cast<const uint4*>(x + (size_t)m * args.K + (size_t)kt * 128 + q * VEC), a_scale[m],
+                          inv[m], w);
+            uint8_t* dst = xq + (j * MT + m) * 128 + q * VEC;
+            if constexpr (sizeof(XT) == 4) *reinterpret_cast<uint32_t*>(dst) = w[0];
+            else *reinterpret_cast<uint2*>(dst) = make_uint2(w[0], w[1]);
+          }
+        }
+      }
+      consumer_barrier();   // also: `red` has been read
+    }
 
     // A partial segment whose atomics are in flight while the CTA streams its next segment.
     bool pend = false;
@@ -247,7 +345,8 @@ gemv_blob_kernel(const Args args, const std::conditional_t<MULTI, MultiOut, NoMu
           v[2 * j] = lqq_dequant4(pk[j] & 0x0F0F0F0Fu, step, ab);
           v[2 * j + 1] = lqq_dequant4((pk[j] >> 4) & 0x0F0F0F0Fu, step, ab);
         }
-        const uint8_t* xst = smem + (xs - base) + ring.s * C::kXStage + 64 * h;
+        const uint8_t* xst = (QUANT ? xq + x_tile * (MT * 128) : smem + (xs - base) + ring.s * C::kXStage) + 64 * h;
+        if (QUANT && ++x_tile == x_tiles) x_tile = 0;   // a range longer than K wraps
 #pragma unroll
         for (int m = 0; m < MT; ++m) {
           const uint4* xp = reinterpret_cast<const uint4*>(xst + m * 128);
@@ -330,23 +429,27 @@ gemv_blob_kernel(const Args args, const std::conditional_t<MULTI, MultiOut, NoMu
   __syncthreads();
 }
 
-template <int MT, int NS, bool MULTI>
-static int launch(const Args& a, const MultiOut* multi, int grid, cudaStream_t st) {
-  using C = Cfg<MT, NS>;
-  auto kern = &gemv_blob_kernel<MT, NS, MULTI>;
+// `tokens`: bytes of quantised tokens behind the fixed part (quantising form).
+template <int MT, int NS, bool MULTI, typename XT = int8_t>
+static int launch(const Args& a, const MultiOut* multi, int grid, cudaStream_t st, int tokens = 0) {
+  using C = Cfg<MT, NS, !std::is_same_v<XT, int8_t>>;
+  constexpr int kMaxSmem = std::is_same_v<XT, int8_t> ? C::kSmemBytes : kMaxQuantSmem;
+  const int smem = C::kUsedBytes + tokens > C::kSmemBytes ? C::kUsedBytes + tokens : C::kSmemBytes;
+  if (smem > kMaxSmem) return LQ_ERR_SHAPE;
+  auto kern = &gemv_blob_kernel<MT, NS, MULTI, XT>;
   static std::once_flag once[64];
   int dev = 0;
   cudaGetDevice(&dev);
   cudaError_t e = cudaSuccess;
   std::call_once(once[dev & 63], [&]() {
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
   });
   if (e != cudaSuccess) {
     record_cuda_error(e, "cudaFuncSetAttribute(gemv_blob_kernel)");
     return LQ_ERR_CUDA;
   }
-  if constexpr (MULTI) e = launch_overlapped(kern, dim3(grid), dim3(kThreads), (size_t)C::kSmemBytes, st, a, *multi);
-  else e = launch_overlapped(kern, dim3(grid), dim3(kThreads), (size_t)C::kSmemBytes, st, a, NoMultiOut{});
+  if constexpr (MULTI) e = launch_overlapped(kern, dim3(grid), dim3(kThreads), (size_t)smem, st, a, *multi);
+  else e = launch_overlapped(kern, dim3(grid), dim3(kThreads), (size_t)smem, st, a, NoMultiOut{});
   if (e != cudaSuccess) {
     record_cuda_error(e, "gemv_blob_kernel launch");
     return LQ_ERR_CUDA;
@@ -410,6 +513,62 @@ int run_gemv_blob(const int8_t* x, const uint8_t* blob, const float* ascale, con
   if (M <= 2) return launch<2, 8, true>(a, &mo, grid, st);
   if (M <= 4) return launch<4, 8, true>(a, &mo, grid, st);
   return launch<8, 7, true>(a, &mo, grid, st);
+}
+
+// ---- the quantising form: activations in, no token quantiser before it -------------------------------------------
+namespace gblob {
+// k-tiles of tokens a CTA may need: its whole range, at most all of K.
+static int token_tiles_max(int N, int K) {
+  const DecodePlan p = plan_for(N, K);
+  const int kt = K / 128;
+  const long units = (long)((N + 127) / 128) * kt;
+  const long per = p.fixed_split ? (kt + p.fixed_split - 1) / p.fixed_split : (units + p.grid - 1) / p.grid;
+  return (int)(per < kt ? per : kt);
+}
+
+template <typename XT>
+static int launch_quant(const Args& a, int grid, cudaStream_t st) {
+  const int tokens = token_tiles_max(a.N, a.K) * 128;
+  if (a.M == 1) return launch<1, 8, false, XT>(a, nullptr, grid, st, tokens);
+  return launch<2, 8, false, XT>(a, nullptr, grid, st, 2 * tokens);
+}
+}  // namespace gblob
+
+// Whether one kernel quantises and multiplies.  Every CTA reads all of the tokens for their scales, which costs less than
+// the second kernel and its place in the stream (2 us) for one token (6144 x 4096 6.3 -> 5.6 us, 28672 x 4096 15.3 -> 13.5,
+// 4096 x 14336 9.7 -> 8.8, 1280 x 8192 5.0 -> 4.3) and for two (6.7 -> 6.7, 15.5 -> 15.4, 10.7 -> 10.2, 5.5 -> 5.0); with
+// three and four the dp4a arithmetic is behind the tensor-core kernels (6144 x 4096 at four: 7.7 -> 9.9, 28672 x 4096 15.7 ->
+// 24.2).  The quantised tokens have to fit beside the weight ring of two CTAs per SM.
+bool gemv_quant_serves(int M, int N, int K) {
+  if (M < 1 || M > 2 || N < 1 || K < 128 || K % 128) return false;
+  return gblob::token_tiles_max(N, K) * M * 128 + gblob::Cfg<2, 8, true>::kUsedBytes <= gblob::kMaxQuantSmem;
+}
+
+// x: [M, K] activations of type x_dtype, 16-byte aligned.  `ws` as for run_gemv_blob_ws.
+int run_gemv_quant(const void* x, int x_dtype, const uint8_t* blob, const float* s1, const void* bias, void* out,
+                   int out_dtype, int M, int N, int K, void* ws, size_t ws_bytes, cudaStream_t st) {
+  using namespace gblob;
+  if (!gemv_quant_serves(M, N, K)) return LQ_ERR_SHAPE;
+  const DecodePlan p = plan_for(N, K);
+  if (!ws || ws_bytes < gemv_blob_ws_bytes(p.grid)) return LQ_ERR_WORKSPACE;
+  Args a;
+  a.blob = blob;
+  a.x = x;
+  a.ascale = nullptr;
+  a.s1 = s1;
+  a.out = out;
+  a.slots = static_cast<unsigned long long*>(ws);
+  a.status = status_word();
+  a.out_dtype = out_dtype;
+  a.M = M;
+  a.N = N;
+  a.K = K;
+  a.fixed_split = p.fixed_split;
+  a.bias = bias;
+  if (!a.status) return LQ_ERR_CUDA;
+  if (x_dtype == LQ_DT_BF16) return launch_quant<__nv_bfloat16>(a, p.grid, st);
+  if (x_dtype == LQ_DT_F16) return launch_quant<__half>(a, p.grid, st);
+  return launch_quant<float>(a, p.grid, st);
 }
 
 int run_gemv_blob_ws(const int8_t* x, const uint8_t* blob, const float* ascale, const float* s1, const void* bias,

@@ -31,6 +31,9 @@ Scratch layout(int M, int N, int K, int x_dtype, int out_dtype) {
 
 extern "C" {
 
+int linear_for_host(const void* x, int x_dtype, const uint8_t* blob, const float* s1, void* y, int out_dtype, int M, int N,
+                    int K, void* scratch, size_t scratch_bytes, void* workspace, size_t workspace_bytes, void* stream);   // lq_gemm_tc.cu
+
 LQ_API size_t lq_linear_host_scratch_bytes(int M, int N, int K, int x_dtype, int out_dtype) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   return layout(M, N, K, x_dtype, out_dtype).total;
@@ -53,12 +56,8 @@ LQ_API int lq_w4a8_linear_host(const void* x_host, int x_dtype, const void* blob
     lq::record_cuda_error(e, "lq_w4a8_linear_host upload");
     return LQ_ERR_CUDA;
   }
-  int rc = lq_quant_per_token(base + s.x, x_dtype, reinterpret_cast<int8_t*>(base + s.xq),
-                              reinterpret_cast<float*>(base + s.ascale), M, K, stream);
-  if (rc) return rc;
-  rc = lq_w4a8_gemm_fused(reinterpret_cast<const int8_t*>(base + s.xq), static_cast<const uint8_t*>(blob),
-                          reinterpret_cast<const float*>(base + s.ascale), static_cast<const float*>(s1), base + s.y,
-                          out_dtype, M, N, K, 0, workspace, workspace_bytes, stream);
+  const int rc = linear_for_host(base + s.x, x_dtype, static_cast<const uint8_t*>(blob), static_cast<const float*>(s1), base + s.y,
+                                 out_dtype, M, N, K, base + s.xq, s.y - s.xq, workspace, workspace_bytes, stream);
   if (rc) return rc;
   e = cudaMemcpyAsync(y_host, base + s.y, (size_t)M * N * dtype_bytes(out_dtype), cudaMemcpyDeviceToHost, st);
   if (e != cudaSuccess) {

@@ -59,6 +59,9 @@ _SCHEMAS = {
 _libdef = torch.library.Library("liquidgemm", "DEF")
 for _name, _sig in _SCHEMAS.items():
     _libdef.define(_name + _sig)
+# one linear from activations to outputs: token quantiser and fused GEMM, in one kernel where that serves
+_libdef.define("w4a8_linear(Tensor x, Tensor w, Tensor s_u8, Tensor off_a, Tensor s1, Tensor? bias, int N, int K, "
+               "int group_size, int out_dtype) -> Tensor")
 _impl = torch.library.Library("liquidgemm", "IMPL", "CUDA")
 
 
@@ -113,6 +116,11 @@ def _f_i8s(a, b, a_scale, b_scale, out_dtype):
 @torch.library.register_fake("liquidgemm::w4a8_linear_bias")
 def _f_lb(x_i8, w, ascale, s1, bias, N, K, out_dtype):
     return x_i8.new_empty((x_i8.shape[0], N), dtype=_OUT_DTYPES[int(out_dtype)])
+
+
+@torch.library.register_fake("liquidgemm::w4a8_linear")
+def _f_lin(x, w, s_u8, off_a, s1, bias, N, K, group_size, out_dtype):
+    return x.new_empty((x.shape[0], N), dtype=_OUT_DTYPES[int(out_dtype)])
 
 
 @torch.library.register_fake("liquidgemm::w4a8_wgmma")
@@ -235,10 +243,10 @@ _WORKSPACES: dict = {}
 _RETIRED: list = []
 
 
-def _workspace(nbytes: int, device: torch.device):
+def _workspace(nbytes: int, device: torch.device, stream=None):
     if nbytes == 0:
         return None
-    key = (device.index, _stream())
+    key = (device.index, _stream() if stream is None else stream)
     ws = _WORKSPACES.get(key)
     if ws is None or ws.numel() < nbytes:
         if ws is not None:
@@ -346,6 +354,61 @@ def linear_bias(x_i8, blob, ascale, s1, bias, N, K, out_dtype):
                                                                  _ptr(bias) if bias is not None else None, _ptr(y),
                                                                  int(out_dtype), M, N, K, ws, nb, st))
     return y
+
+
+def _linear(x, w, s_u8, off_a, s1, bias, N, K, group_size, out_dtype):
+    """Token quantiser and fused linear in one native call: the same checks, bits and workspaces as
+    ``quant_per_token`` followed by ``w4a8_wgmma_rs_fused`` (with ``bias``: ``w4a8_linear_bias``)."""
+    _req(x.is_cuda and x.dim() == 2, "x must be 2D CUDA")
+    code = _DTYPE_CODES.get(x.dtype)
+    _req(code is not None, "x must be bfloat16, float16 or float32")
+    _req(w.dtype == torch.uint8 and group_size == 64, "w must be uint8 and group_size 64")
+    # like the operators it stands for: N % 64 only where there is no bias
+    _req((N % 64 == 0 or bias is not None) and K % 128 == 0, "N%64==0 and K%128==0 required")
+    x = x.contiguous()
+    M = x.shape[0]
+    _req(x.shape[1] == K, "K%128==0 required and x_i8 must be [M,K]")
+    odt = _OUT_DTYPES.get(int(out_dtype))
+    _req(odt is not None, "out_dtype must be 0 (bf16), 1 (fp16) or 2 (fp32)")
+    _req(w.is_cuda and w.numel() == ((N + 127) // 128) * (K // 128) * TILE_BYTES and w.numel() > 0,
+         f"w must be the tile blob of repack_rs_weight for N={N}, K={K} ({w.numel()} bytes)")
+    w = w.contiguous()
+    s1 = _f32(s1, "s1")
+    _req(s1.numel() == N, "ascale must be [M] and s1 [N]")
+    if bias is not None:
+        _req(bias.is_cuda and bias.dtype == odt and bias.numel() == N, "bias must be a CUDA [N] tensor of the output dtype")
+        bias = bias.contiguous()
+    dev = x.device
+    y = torch.empty((M, N), dtype=odt, device=dev)
+    if M == 0:
+        return y
+    if dev.index == torch.cuda.current_device():
+        _linear_call(x, code, w, s1, bias, y, int(out_dtype), M, N, K, dev)
+    else:
+        with torch.cuda.device(dev):
+            _linear_call(x, code, w, s1, bias, y, int(out_dtype), M, N, K, dev)
+    return y
+
+
+def _linear_call(x, code, w, s1, bias, y, out_dtype, M, N, K, dev):
+    S = _splitk_for(M, N, K) if _SPLITK_ENV else 0
+    px = x.data_ptr()
+    plan = (ctypes.c_size_t * 3)()
+    check(lib.lq_linear_plan(px, M, N, K, S, plan), "w4a8_linear")
+    nscratch, nws, kind = plan
+    stream = _stream()
+    scratch = torch.empty((nscratch,), dtype=torch.uint8, device=dev) if nscratch else None
+    if kind == 1:
+        ws = torch.empty((nws,), dtype=torch.uint8, device=dev)
+    else:
+        ws = _workspace(nws, dev, stream)
+    rc = lib.lq_w4a8_linear(px, code, w.data_ptr(), s1.data_ptr(), None if bias is None else bias.data_ptr(),
+                            y.data_ptr(), out_dtype, M, N, K, S, None if scratch is None else scratch.data_ptr(),
+                            nscratch, None if ws is None else ws.data_ptr(), 0 if ws is None else ws.numel(), stream)
+    if rc != 0:
+        if ws is not None and kind == 2:
+            ws.zero_()
+        check(rc, "w4a8_linear")
 
 
 def quantize_weight_cuda(W: torch.Tensor, group_size: int = 64, want_codes: bool = True, want_blob: bool = False):
@@ -557,6 +620,7 @@ _impl.impl("w4a8_wgmma_rs_fused", _wgmma_rs_fused)
 _impl.impl("w4a8_wgmma", _wgmma_ss)
 _impl.impl("wgmma_i8_gemm", _wgmma_i8)
 _impl.impl("i8_gemm_scaled", _i8_gemm_scaled)
+_impl.impl("w4a8_linear", _linear)
 _impl.impl("w4a8_linear_bias", linear_bias)
 _impl.impl("w4a8_gemm", _gemm_v1)
 _libdef.impl("wgmma_rs_a_coords", _coords, "CompositeExplicitAutograd")
@@ -653,12 +717,12 @@ def w4a8_linear(x: torch.Tensor, qw_dev: dict, out_dtype: torch.dtype = None) ->
     ``qw_dev`` holds device tensors ``s1, s_u8, offset_a, N, K`` and ``rs`` (tile blob) and/or ``gp``.
     """
     odt = _DTYPE_CODES[out_dtype or x.dtype]
-    x_i8, ascale = torch.ops.liquidgemm.quant_per_token(x)
-    if use_gemv(x_i8.shape[0], qw_dev["N"], qw_dev["K"], qw_dev.get("gp") is not None, qw_dev.get("rs") is not None):
+    if qw_dev.get("rs") is None and use_gemv(x.shape[0], qw_dev["N"], qw_dev["K"], qw_dev.get("gp") is not None, False):
+        x_i8, ascale = torch.ops.liquidgemm.quant_per_token(x)
         return torch.ops.liquidgemm.w4a8_gemv2(x_i8, qw_dev["gp"], qw_dev["s_u8"], qw_dev["offset_a"], ascale,
                                                qw_dev["s1"], qw_dev["N"], qw_dev["K"], 64, odt)
-    return torch.ops.liquidgemm.w4a8_wgmma_rs_fused(x_i8, qw_dev["rs"], qw_dev["s_u8"], qw_dev["offset_a"], ascale,
-                                                    qw_dev["s1"], qw_dev["N"], qw_dev["K"], 64, odt)
+    return torch.ops.liquidgemm.w4a8_linear(x, qw_dev["rs"], qw_dev["s_u8"], qw_dev["offset_a"], qw_dev["s1"], None,
+                                            qw_dev["N"], qw_dev["K"], 64, odt)
 
 
 _HOST_SCRATCH: dict = {}

@@ -157,16 +157,17 @@ def apply_layer(layer: torch.nn.Module, x: torch.Tensor, bias: Optional[torch.Te
     x2 = x.reshape(-1, shape[-1]).contiguous()
     n = layer.lq_N
     odt = _DT.get(x.dtype, 0)
-    x_i8, ascale = torch.ops.liquidgemm.quant_per_token(x2)
     if w4:
         if bias is not None and bias.dtype == x.dtype and x.dtype in _DT:
             # the bias rides in the kernel's epilogue, added to the rounded output exactly like the
             # separate `y + bias` of the reference (liquidgemm/vllm_plugin.py:205-206)
-            y = torch.ops.liquidgemm.w4a8_linear_bias(x_i8, layer.lq_rs, ascale, layer.lq_s1, bias, n, layer.lq_K, odt)
+            y = torch.ops.liquidgemm.w4a8_linear(x2, layer.lq_rs, layer.lq_s_u8, layer.lq_offset_a, layer.lq_s1, bias, n,
+                                                 layer.lq_K, 64, odt)
             return y.reshape(*shape[:-1], n)
-        y = torch.ops.liquidgemm.w4a8_wgmma_rs_fused(x_i8, layer.lq_rs, layer.lq_s_u8, layer.lq_offset_a, ascale,
-                                                     layer.lq_s1, n, layer.lq_K, group_size, odt)
+        y = torch.ops.liquidgemm.w4a8_linear(x2, layer.lq_rs, layer.lq_s_u8, layer.lq_offset_a, layer.lq_s1, None, n,
+                                             layer.lq_K, group_size, odt)
     else:
+        x_i8, ascale = torch.ops.liquidgemm.quant_per_token(x2)
         y = torch.ops.liquidgemm.i8_gemm_scaled(x_i8, layer.lq_w_i8, ascale, layer.lq_s1, odt)
     y = y.reshape(*shape[:-1], n)
     return y if bias is None else y + bias

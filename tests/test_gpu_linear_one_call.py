@@ -1,0 +1,84 @@
+"""``w4a8_linear`` from activations to outputs in one call: the GEMV that quantises its own tokens, and the two-launch
+form behind it, against ``quant_per_token`` followed by the fused operator (both tested against the oracle
+elsewhere).  Tolerance: none."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from liquidgemm_b200 import ops as _ops
+    return _ops
+
+
+def _layer(ops, n, k, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    w = torch.randn(n, k, generator=g, device="cuda") * 0.03
+    qw, blob = ops.quantize_weight_cuda(w, 64, want_codes=False, want_blob=True)
+    return {"s1": qw.s1, "s_u8": qw.s_u8, "offset_a": qw.offset_a, "N": n, "K": k, "rs": blob.reshape(-1)}
+
+
+def _tokens(m, k, dtype, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x = torch.randn(m, k, generator=g, device="cuda")
+    x[:, 5] *= 20
+    x[-1, k - 1] = 30.0      # the largest value of the row in the last k-tile
+    if m > 1:
+        x[0] = 0.0
+    return x.to(dtype)
+
+
+def _two_calls(x, L, bias, code):
+    xq, sc = torch.ops.liquidgemm.quant_per_token(x)
+    if bias is None:
+        return torch.ops.liquidgemm.w4a8_wgmma_rs_fused(xq, L["rs"], L["s_u8"], L["offset_a"], sc, L["s1"], L["N"], L["K"],
+                                                        64, code)
+    return torch.ops.liquidgemm.w4a8_linear_bias(xq, L["rs"], sc, L["s1"], bias, L["N"], L["K"], code)
+
+
+# one k-tile; fewer k-tiles than CTAs; cut tiles; ranges longer than K (stream-K over many n-tiles); ragged N; long K
+SHAPES = [(64, 128), (192, 256), (1280, 8192), (4096, 4096), (40000, 256), (28672, 1024), (19200, 4096), (1024, 28672)]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("N,K", SHAPES)
+def test_one_call_equals_two(ops, dtype, N, K):
+    L = _layer(ops, N, K, N + K)
+    code = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}[dtype]
+    bias = torch.randn(N, device="cuda").to(dtype)
+    for M in (1, 2, 3, 4, 5, 8, 9, 40):
+        x = _tokens(M, K, dtype, M)
+        want = _two_calls(x, L, None, code)
+        assert torch.equal(ops.w4a8_linear(x, L), want), M
+        got = torch.ops.liquidgemm.w4a8_linear(x, L["rs"], L["s_u8"], L["offset_a"], L["s1"], bias, N, K, 64, code)
+        assert torch.equal(got, _two_calls(x, L, bias, code)), M
+        if M <= 4:
+            buf = torch.empty(x.numel() + 1, dtype=dtype, device="cuda")   # unaligned activations: the two-launch form
+            buf[1:] = x.reshape(-1)
+            assert torch.equal(ops.w4a8_linear(buf[1:].view(M, K), L), want), M
+    ops.poll_status()
+
+
+def test_special_activations(ops):
+    L = _layer(ops, 512, 1024, 3)
+    x = _tokens(4, 1024, torch.bfloat16, 1)
+    x[0, 3], x[1, 4], x[2, 5] = float("nan"), float("inf"), torch.finfo(torch.bfloat16).max
+    got, want = ops.w4a8_linear(x, L), _two_calls(x, L, None, 0)
+    assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+
+
+def test_refusals_stay(ops):
+    L = _layer(ops, 128, 256, 0)
+    good = _tokens(2, 256, torch.float16, 0)
+    for bad in (good.cpu(), good[0], good.to(torch.float64), good[:, :128].contiguous()):
+        with pytest.raises((RuntimeError, KeyError, NotImplementedError)):
+            ops.w4a8_linear(bad, L)
+    with pytest.raises(RuntimeError):
+        ops.w4a8_linear(good, {**L, "rs": L["rs"][:-1]})
+    with pytest.raises(RuntimeError):
+        ops.w4a8_linear(good, {**L, "s1": L["s1"][:-1]})
+    assert ops.w4a8_linear(good[:0], L).shape == (0, 128)
+    assert torch.equal(ops.w4a8_linear(good.t().contiguous().t(), L), ops.w4a8_linear(good, L))
