@@ -286,6 +286,15 @@ LQ_API int lq_i8_gemm_scaled(const int8_t* a, const int8_t* b, const float* a_sc
                       const float* b_scale, void* y, int out_dtype, int M, int N, int K,
                       void* stream);
 
+/* The same two with `workspace` (lq_i8_workspace_bytes(M, N, K) of scratch, any content; null and 0 where that is 0):
+ * batches below the CTA-pair kernel's sizes then run on a streaming kernel that may cut the layer's K and add the
+ * parts up through it.  Results are bit-identical. */
+LQ_API size_t lq_i8_workspace_bytes(int M, int N, int K);
+LQ_API int lq_i8_gemm_i32_ws(const int8_t* a, const int8_t* b, int32_t* c, int M, int N, int K, void* workspace,
+                      size_t workspace_bytes, void* stream);
+LQ_API int lq_i8_gemm_scaled_ws(const int8_t* a, const int8_t* b, const float* a_scale, const float* b_scale, void* y,
+                         int out_dtype, int M, int N, int K, void* workspace, size_t workspace_bytes, void* stream);
+
 
 #ifdef __cplusplus
 }

@@ -61,6 +61,9 @@ _SIGNATURES = {
     "lq_w4a8_gemm_fused": (c_int, [P, P, P, P, P, c_int, c_int, c_int, c_int, c_int, P, c_size_t, P]),
     "lq_i8_gemm_i32": (c_int, [P, P, P, c_int, c_int, c_int, P]),
     "lq_i8_gemm_scaled": (c_int, [P, P, P, P, P, c_int, c_int, c_int, c_int, P]),
+    "lq_i8_workspace_bytes": (c_size_t, [c_int, c_int, c_int]),
+    "lq_i8_gemm_i32_ws": (c_int, [P, P, P, c_int, c_int, c_int, P, c_size_t, P]),
+    "lq_i8_gemm_scaled_ws": (c_int, [P, P, P, P, P, c_int, c_int, c_int, c_int, P, c_size_t, P]),
 }
 
 for _name, (_res, _args) in _SIGNATURES.items():

@@ -74,6 +74,10 @@ bool pair_serves(int M, int N, int K);                                       // 
 bool i8_pair_serves(int M, int N, int K);                                    // lq_i8_pair.cu
 int run_i8_pair_gemm(const int8_t* x, const int8_t* w, const float* ascale, const float* s1, const void* bias, void* out,
                      int out_mode, int M, int N, int K, cudaStream_t st);
+bool i8_stream_serves(int M, int N, int K);                                  // lq_i8_stream.cu
+size_t i8_stream_workspace_bytes(int M, int N, int K);
+int run_i8_stream(const int8_t* x, const int8_t* w, const float* ascale, const float* s1, void* out, int out_mode, int M,
+                  int N, int K, void* ws, size_t ws_bytes, cudaStream_t st);
 int run_unpack_blob_i8(const uint8_t* blob, int8_t* w, int N, int K, cudaStream_t st);   // lq_elementwise.cu
 bool pair_prefers(int M, int N, int K);                                      // lq_gemm_pair.cu
 size_t pair_workspace_bytes(int M, int N, int K);                                // lq_gemm_pair.cu
@@ -1008,27 +1012,54 @@ static bool i8_pair_enabled() {
   return !(e && e[0] == '0');
 }
 
+enum I8Route { kI8Pair, kI8Stream, kI8Persistent };
+static I8Route i8_route(int M, int N, int K) {
+  if (i8_pair_serves(M, N, K) && i8_pair_enabled()) return kI8Pair;
+  return i8_stream_serves(M, N, K) ? kI8Stream : kI8Persistent;   // lq_i8_stream.cu
+}
+
+size_t lq_i8_workspace_bytes(int M, int N, int K) {
+  if (M <= 0 || N <= 0 || K < 128 || K % 128 || i8_route(M, N, K) != kI8Stream) return 0;
+  return i8_stream_workspace_bytes(M, N, K);
+}
+
 static int i8_common(const int8_t* a, const int8_t* b, const float* a_scale, const float* b_scale, void* out,
-                     int out_mode, int M, int N, int K, void* stream) {
+                     int out_mode, int M, int N, int K, void* ws, size_t ws_bytes, void* stream) {
   if (!a || !b || !out || M < 0 || N <= 0 || K <= 0) return LQ_ERR_BAD_ARG;
   if (K % 128) return LQ_ERR_SHAPE;
   if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) % 16) return LQ_ERR_BAD_ARG;
   if (M == 0) return LQ_OK;
-  // whole-tile scheduling: the plain INT8 entry points take no workspace
-  if (i8_pair_serves(M, N, K) && i8_pair_enabled())
+  const I8Route r = i8_route(M, N, K);
+  if (r == kI8Pair)
     return run_i8_pair_gemm(a, b, a_scale, b_scale, nullptr, out, out_mode, M, N, K, as_stream(stream));
+  // without the workspace of the split streaming kernel (the plain entry points): whole tiles, one CTA per SM
+  if (r == kI8Stream && ws_bytes >= i8_stream_workspace_bytes(M, N, K)) {
+    if (int rc = lq_check_device()) return rc;
+    return run_i8_stream(a, b, a_scale, b_scale, out, out_mode, M, N, K, ws, ws_bytes, as_stream(stream));
+  }
   return run_gemm<kInt8>(a, b, a_scale, b_scale, out, out_mode, M, N, K, 1, nullptr, 0,
                          as_stream(stream));
 }
 
 int lq_i8_gemm_i32(const int8_t* a, const int8_t* b, int32_t* c, int M, int N, int K, void* stream) {
-  return i8_common(a, b, nullptr, nullptr, c, kOutI32, M, N, K, stream);
+  return i8_common(a, b, nullptr, nullptr, c, kOutI32, M, N, K, nullptr, 0, stream);
 }
 
 int lq_i8_gemm_scaled(const int8_t* a, const int8_t* b, const float* a_scale, const float* b_scale, void* y,
                       int out_dtype, int M, int N, int K, void* stream) {
   if (!a_scale || !b_scale || out_dtype < 0 || out_dtype > 2) return LQ_ERR_BAD_ARG;
-  return i8_common(a, b, a_scale, b_scale, y, out_dtype, M, N, K, stream);
+  return i8_common(a, b, a_scale, b_scale, y, out_dtype, M, N, K, nullptr, 0, stream);
+}
+
+int lq_i8_gemm_i32_ws(const int8_t* a, const int8_t* b, int32_t* c, int M, int N, int K, void* workspace,
+                      size_t workspace_bytes, void* stream) {
+  return i8_common(a, b, nullptr, nullptr, c, kOutI32, M, N, K, workspace, workspace_bytes, stream);
+}
+
+int lq_i8_gemm_scaled_ws(const int8_t* a, const int8_t* b, const float* a_scale, const float* b_scale, void* y,
+                         int out_dtype, int M, int N, int K, void* workspace, size_t workspace_bytes, void* stream) {
+  if (!a_scale || !b_scale || out_dtype < 0 || out_dtype > 2) return LQ_ERR_BAD_ARG;
+  return i8_common(a, b, a_scale, b_scale, y, out_dtype, M, N, K, workspace, workspace_bytes, stream);
 }
 
 }  // extern "C"

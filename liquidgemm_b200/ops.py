@@ -541,6 +541,12 @@ def _wgmma_ss(x_i8, packed, s_u8, off_a, N, K, group_size):
     return gemm_i32(x_i8, blob.reshape(-1), N, K)
 
 
+def _i8_workspace(a, M, N, K):
+    """Scratch of the INT8 streaming kernel (the partial sums of a cut K), or None."""
+    nbytes = lib.lq_i8_workspace_bytes(M, N, K)
+    return torch.empty((nbytes,), dtype=torch.uint8, device=a.device) if nbytes else None
+
+
 def _wgmma_i8(a, b):
     a, b = _i8(a, "a"), _i8(b, "b")
     M, K = a.shape
@@ -550,7 +556,9 @@ def _wgmma_i8(a, b):
     c = torch.empty((M, N), dtype=torch.int32, device=a.device)
     if M:
         with _dev_ctx(a):
-            check(lib.lq_i8_gemm_i32(_ptr(a), _ptr(b), _ptr(c), M, N, K, _stream()), "wgmma_i8_gemm")
+            ws = _i8_workspace(a, M, N, K)
+            check(lib.lq_i8_gemm_i32_ws(_ptr(a), _ptr(b), _ptr(c), M, N, K, _ptr(ws) if ws is not None else None,
+                                        ws.numel() if ws is not None else 0, _stream()), "wgmma_i8_gemm")
     return c
 
 
@@ -565,8 +573,10 @@ def _i8_gemm_scaled(a, b, a_scale, b_scale, out_dtype):
     y = torch.empty((M, N), dtype=_OUT_DTYPES[int(out_dtype)], device=a.device)
     if M:
         with _dev_ctx(a):
-            check(lib.lq_i8_gemm_scaled(_ptr(a), _ptr(b), _ptr(a_scale), _ptr(b_scale), _ptr(y), int(out_dtype), M, N,
-                                        K, _stream()), "i8_gemm_scaled")
+            ws = _i8_workspace(a, M, N, K)
+            check(lib.lq_i8_gemm_scaled_ws(_ptr(a), _ptr(b), _ptr(a_scale), _ptr(b_scale), _ptr(y), int(out_dtype), M, N,
+                                           K, _ptr(ws) if ws is not None else None, ws.numel() if ws is not None else 0,
+                                           _stream()), "i8_gemm_scaled")
     return y
 
 
