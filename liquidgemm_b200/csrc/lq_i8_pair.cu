@@ -10,13 +10,14 @@
 //
 // Per CTA (640 threads), connected by mbarrier rings; rank = CTA's rank in its pair:
 //   warp 0        weight producer: 128 channels x 128 bytes of k per k-step (rows 256 * block + 128 * rank ...)
-//   warp 2        token producer: 128 token rows x 128 bytes of k per k-step (rows 256 * tile + 128 * rank ...)
+//   warp 2        token producer: bn / 2 token rows x 128 bytes of k per k-step (rows bn * tile + bn / 2 * rank ...)
 //   warp 3        relay: when both copies of a stage have landed HERE it tells the leader CTA (whose MMA reads the
 //                 shared memory of both CTAs); one arrival per CTA and stage
 //   warp 1        tensor-memory allocation (both CTAs); on rank 0 the MMA issue: four MMAs per k-step, then one
 //                 commit that frees the stage in both CTAs
 //   warps 4..19   four epilogue groups sharing every tile (16-token chunks g, g + 4, ...)
-// Work: tile = 256 channels x 256 tokens, pair p of P takes tiles p, p + P, ... whole (the INT8 entry points take
+// Work: tile = 256 channels x bn tokens (a multiple of 32, see tile_tokens), pair p of P takes tiles p, p + P, ...
+// whole (the INT8 entry points take
 // no workspace).  Every wait is bounded; the status codes are 141-146.
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -38,18 +39,17 @@ namespace i8pair {
 
 using namespace pairc;
 
-constexpr int kBN = 256;                 // tokens per tile
-constexpr int kHalf = kBN / 2;           // token rows staged by each CTA
+constexpr int kMaxBN = 256;              // tokens per tile: at most (Args::bn)
 constexpr int kNS = 6;                   // shared-memory stages
 constexpr int kGroups = 4;               // epilogue groups of four warps
 constexpr int kThreads = 128 + 128 * kGroups;
 constexpr int kAStage = 128 * 128;       // 128 channels x 128 bytes of k
-constexpr int kXStage = kHalf * 128;
+constexpr int kXStage = kMaxBN / 2 * 128;
 constexpr int kTmemCols = 512;           // two 256-column accumulators
 constexpr int kNumBars = 3 * kNS + 4;
 constexpr int kBarBytes = kNumBars * 8 + 64;
 constexpr int kSmemBytes = 1024 /* alignment slack */ + kNS * (kAStage + kXStage) + ((kBarBytes + 15) & ~15) +
-                           kGroups * 2 * kBN * 4;
+                           kGroups * 2 * kMaxBN * 4;
 constexpr uint64_t kWaitLimitNs = 2000000000ull;
 constexpr int kOutI32 = kEpiI32;
 
@@ -62,7 +62,8 @@ struct Args {
   int out_mode;            // LQ_DT_* or kOutI32
   int M, N, K;
   int kt_total;            // K / 128
-  int n2_tiles, m_tiles;   // 256-channel blocks, 256-token blocks
+  int bn;                  // tokens per tile, a multiple of 32
+  int n2_tiles, m_tiles;   // 256-channel blocks, token tiles
   int pairs;               // CTA pairs of the launch
   int tail_s;              // always 1: whole tiles
 };
@@ -88,7 +89,7 @@ i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
   uint8_t* gen_bars = smem + (bars - base);
   volatile uint32_t* tmem_slot_p = reinterpret_cast<volatile uint32_t*>(gen_bars + kNumBars * 8);
   volatile int* wait_flag = reinterpret_cast<volatile int*>(gen_bars + kNumBars * 8 + 8);   // [group][2]
-  float* tok_scale = reinterpret_cast<float*>(gen_bars + ((kBarBytes + 15) & ~15));          // [group][2][kBN]
+  float* tok_scale = reinterpret_cast<float*>(gen_bars + ((kBarBytes + 15) & ~15));          // [group][2][kMaxBN]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = ptx::cluster_ctarank();
@@ -124,6 +125,7 @@ i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
     // ------------------------------------------------------------------ producers (one thread each)
     if (lane == 0) {
       const bool weights = (warp == 0);
+      const int half = args.bn / 2;   // token rows staged by each CTA
       PairWalk walk(args, pair);
       Segment sg;
       Ring<kNS> ring;
@@ -132,7 +134,7 @@ i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
       while (ok && walk.next(sg)) {
         int n2, mt;
         tile_coords(sg.tile, args.n2_tiles, args.m_tiles, kGroupM, n2, mt);
-        const int row0 = weights ? (2 * n2 + (int)rank) * 128 : mt * kBN + (int)rank * kHalf;
+        const int row0 = weights ? (2 * n2 + (int)rank) * 128 : mt * args.bn + (int)rank * half;
         for (int kt = sg.kb; kt < sg.ke; ++kt) {
           if (!ptx::mbar_wait_bounded(bar_empty + 8 * ring.s, ring.ph ^ 1u, kWaitLimitNs)) {
             atomicExch(args.status, 141);
@@ -144,7 +146,7 @@ i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
             ptx::mbar_expect_tx(full, kAStage);
             ptx::tensor_load_2d(as + ring.s * kAStage, &tmap_w, kt * 128, row0, full);
           } else {
-            ptx::mbar_expect_tx(full, kXStage);
+            ptx::mbar_expect_tx(full, (uint32_t)half * 128u);
             ptx::tensor_load_2d(xs + ring.s * kXStage, &tmap_x, kt * 128, row0, full);
           }
           ring.advance();
@@ -186,7 +188,7 @@ i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
     // The whole warp walks the loop; one elected lane issues (see ptx::elect_one).
     if (rank == 0) {
       const bool leader = ptx::elect_one();
-      constexpr uint32_t idesc = ptx::idesc_i8_pair(kBN);
+      const uint32_t idesc = ptx::idesc_i8_pair(args.bn);
       PairWalk walk(args, pair);
       Segment sg;
       Ring<kNS> ring;
@@ -200,7 +202,7 @@ i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         ptx::tc_fence_after();
-        const uint32_t tmem_acc = tmem_base + accring.s * kBN;
+        const uint32_t tmem_acc = tmem_base + accring.s * kMaxBN;
         for (int kt = sg.kb; kt < sg.ke; ++kt) {
           if (!ptx::mbar_wait_bounded(bar_ready + 8 * ring.s, ring.ph, kWaitLimitNs)) {
             if (leader) atomicExch(args.status, 144);
@@ -254,12 +256,12 @@ i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
       }
       int n2, mt;
       tile_coords(sg.tile, args.n2_tiles, args.m_tiles, kGroupM, n2, mt);
-      const int m0 = mt * kBN;
+      const int m0 = mt * args.bn;
       const long n = (long)(2 * n2 + (int)rank) * 128 + row;
-      const int cols = (args.M - m0) < kBN ? (args.M - m0) : kBN;   // valid token columns of this tile
-      float* tsc = tok_scale + (2 * g + fslot) * kBN;
+      const int cols = (args.M - m0) < args.bn ? (args.M - m0) : args.bn;   // valid token columns of this tile
+      float* tsc = tok_scale + (2 * g + fslot) * kMaxBN;
       if (!raw) {
-        for (int i = et; i < kBN; i += 128) tsc[i] = (i < cols) ? __ldg(args.ascale + m0 + i) : 0.f;
+        for (int i = et; i < kMaxBN; i += 128) tsc[i] = (i < cols) ? __ldg(args.ascale + m0 + i) : 0.f;
       }
       group_bar(g);
       if (wflag[fslot] == 0) {
@@ -267,7 +269,7 @@ i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         break;
       }
       ptx::tc_fence_after();
-      const uint32_t tmem_acc = tmem_base + b * kBN + lane_addr;
+      const uint32_t tmem_acc = tmem_base + b * kMaxBN + lane_addr;
       const float w_scale = raw ? 0.f : __ldg(args.s1 + n);
       const float bias = has_bias ? load_bias(args.bias, n, args.out_mode) : 0.f;
 #pragma unroll 1
@@ -329,6 +331,27 @@ static int max_pairs() {
   return v;
 }
 
+// Tokens per tile: 256, or the width with the smallest (waves of tiles) x (time of a tile, which grows with its width) where
+// that is at least 10 % less.  Measured: 4096 x 4096 at 1500 tokens 25.5 -> 22.4 us with 192 (96 tiles in two waves -> 128 in
+// two), 4096 x 14336 75.3 -> 64.1, 6144 x 4096 at 777 tokens 25.5 -> 22.2 with 160 and at 1024 25.9 -> 23.4 with 192, 28672 x 4096
+// at 777 80.9 -> 76.5 with 224.  Smaller wins on paper do not hold: under the power limit a fuller last wave only lowers the
+// clock (4096 x 4096 at 4096 tokens, 4 % less by this count, 48.7 -> 51.0 us).
+static int tile_tokens(int M, int N) {
+  const int P = max_pairs();
+  int best = kMaxBN;
+  long widest_cost = 0, best_cost = 0;
+  for (int bn = kMaxBN; bn >= 160; bn -= 32) {
+    const long tiles = (long)(N / 256) * ((M + bn - 1) / bn);
+    const long cost = (tiles + P - 1) / P * (bn + 16);
+    if (bn == kMaxBN) widest_cost = best_cost = cost;
+    else if (cost < best_cost && cost * 10 <= widest_cost * 9) {
+      best = bn;
+      best_cost = cost;
+    }
+  }
+  return best;
+}
+
 }  // namespace i8pair
 
 // Shapes the INT8 pair kernel takes: whole 256-channel blocks and at least 60 tiles of 256 x 256 for the 74 pairs.
@@ -337,7 +360,7 @@ static int max_pairs() {
 // 16-48 tiles 0-4 % slower.
 bool i8_pair_serves(int M, int N, int K) {
   if (M < 256 || N < 256 || N % 256 || K < 128 || K % 128) return false;
-  const long tiles = (long)(N / 256) * ((M + i8pair::kBN - 1) / i8pair::kBN);
+  const long tiles = (long)(N / 256) * ((M + i8pair::kMaxBN - 1) / i8pair::kMaxBN);
   return tiles >= 60;
 }
 
@@ -345,8 +368,9 @@ int run_i8_pair_gemm(const int8_t* x, const int8_t* w, const float* ascale, cons
                      int out_mode, int M, int N, int K, cudaStream_t st) {
   using namespace i8pair;
   if (out_mode < 0 || out_mode > kOutI32) return LQ_ERR_BAD_ARG;
+  const int bn = tile_tokens(M, N);
   CUtensorMap tx, tw;
-  if (int rc = make_byte_matrix_map(&tx, x, M, K, kHalf, 128)) return rc;
+  if (int rc = make_byte_matrix_map(&tx, x, M, K, bn / 2, 128)) return rc;
   if (int rc = make_byte_matrix_map(&tw, w, N, K, 128, 128)) return rc;
   Args a;
   a.ascale = ascale;
@@ -360,7 +384,8 @@ int run_i8_pair_gemm(const int8_t* x, const int8_t* w, const float* ascale, cons
   a.K = K;
   a.kt_total = K / 128;
   a.n2_tiles = N / 256;
-  a.m_tiles = (M + kBN - 1) / kBN;
+  a.bn = bn;
+  a.m_tiles = (M + bn - 1) / bn;
   const long tiles = (long)a.n2_tiles * a.m_tiles;
   const int cap = max_pairs();
   a.pairs = (int)(tiles < cap ? tiles : cap);
