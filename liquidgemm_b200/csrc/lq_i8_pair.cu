@@ -120,6 +120,8 @@ i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
   const uint32_t tmem_base = *tmem_slot_p;
   const uint32_t leader_ready = ptx::map_to_cta(bar_ready, 0);
   const uint32_t leader_accfree = ptx::map_to_cta(bar_accfree, 0);
+  allow_dependents();   // every CTA of this launch is resident: the next kernel may be scheduled behind it
+  dependency_wait();    // everything it reads may come from the kernel before it (the weights too: the unpacked blob)
 
   if (warp == 0 || warp == 2) {
     // ------------------------------------------------------------------ producers (one thread each)
@@ -402,7 +404,11 @@ int run_i8_pair_gemm(const int8_t* x, const int8_t* w, const float* ascale, cons
     record_cuda_error(attr_err, "cudaFuncSetAttribute(i8_pair_kernel)");
     return LQ_ERR_CUDA;
   }
-  i8_pair_kernel<<<2 * a.pairs, kThreads, kSmemBytes, st>>>(tx, tw, a);
+  const cudaError_t e = launch_overlapped(i8_pair_kernel, dim3(2 * a.pairs), dim3(kThreads), (size_t)kSmemBytes, st, tx, tw, a);
+  if (e != cudaSuccess) {
+    record_cuda_error(e, "i8_pair_kernel launch");
+    return LQ_ERR_CUDA;
+  }
   return check_launch("i8_pair_kernel");
 }
 
