@@ -720,18 +720,19 @@ static bool gemv_serves(int M, int N, int K) {
 }
 
 // Large token counts on layers the INT8 pair kernel serves: unpacking the whole blob to INT8 once (a pass over
-// N x K bytes of scratch: 38 us for 28672 x 4096) and running the INT8 x INT8 pair kernel, which keeps the tensor
-// pipe 95 % busy, beats unpacking inside the main loop (71 %).  Measured in one process: at 8192 tokens qkv 158.6
-// -> 144.0 us, o 108.9 -> 93.8, gate_up 720.6 -> 660.4; at 5120 tokens 6 / 3 / 2.5 %; at 3072 tokens qkv 6 %, o
-// 2 %, gate_up 5 % slower; at 2048 all slower.  down (K = 14336, where the W4 kernel's epilogues weigh least) is
-// level at every size: layers with K >= 8192 stay on the W4 pair kernel, and so do layers above 256 MB of INT8
-// weights (the scratch would be larger than that).  LQ_UNPACK_I8_MIN_M replaces both limits (0 switches the route
-// off).  Running the two kernels overlapped (the GEMM launched programmatically behind a persistent unpack kernel,
-// waiting per channel block on counts of finished tiles) was measured as well: bit-exact, 3-7 % SLOWER than one after
-// the other (the unpack's memory traffic slows the GEMM it runs beside); not kept.
+// N x K bytes of scratch: about 30 us for 28672 x 4096) and running the INT8 x INT8 pair kernel, which keeps the tensor
+// pipe 95 % busy, beats unpacking inside the main loop (71 %).  Measured in one process, W4 pair kernel -> this route:
+// 28672 x 4096 at 2048 / 2560 / 3072 / 4096 / 8192 tokens 184 -> 179, 232 -> 221, 266 -> 256, 360 -> 327, 704 -> 610 us; at 1500
+// 136 -> 143.  6144 x 4096 at 2048 / 3072 / 8192 44.5 -> 44.7, 62.8 -> 55.1, 151 -> 137; 4096 x 4096 at 2560 / 3072 / 8192 40.2 ->
+// 42.5, 44.6 -> 42.0, 105 -> 90: matrices up to 32 M weights start at 3072.  4096 x 14336 (where the W4 kernel's
+// epilogues weigh least) is level at every size: layers with K >= 8192 stay on the W4 pair kernel, and so do layers above
+// 256 MB of INT8 weights (the scratch would be larger than that).  LQ_UNPACK_I8_MIN_M replaces both limits (0 switches
+// the route off).  Running the two kernels overlapped (the GEMM launched programmatically behind a persistent unpack
+// kernel, waiting per channel block on counts of finished tiles) was measured as well: bit-exact, 3-7 % SLOWER than one
+// after the other (the unpack's memory traffic slows the GEMM it runs beside); not kept.
 static bool unpack_i8_serves(int M, int N, int K) {
   const char* e = getenv("LQ_UNPACK_I8_MIN_M");   // read at every call: a measurement switch
-  const int lim = e ? atoi(e) : ((size_t)N * K <= ((size_t)1 << 25) ? 3072 : 5120);
+  const int lim = e ? atoi(e) : ((size_t)N * K <= ((size_t)1 << 25) ? 3072 : 2048);
   return lim > 0 && M >= lim && K < 8192 && (size_t)N * K <= ((size_t)256 << 20) && i8_pair_serves(M, N, K);
 }
 
