@@ -211,7 +211,7 @@ LQ_API int lq_quantize_weight(const void* w, int w_dtype, int N, int K, int grou
  *              (scaled outputs only): streaming dp4a GEMV over the tile blob;
  *     up to 16 tokens on matrices up to 32 M weights: the streaming tensor-core kernel, ONE launch:
  *              stream-K over two CTAs per SM, one 64-bit atomic per element joins cut tiles;
- *     3072 tokens and more (2048 on matrices above 32 M weights) on layers with K < 8192, whole 256-channel
+ *     3072 tokens and more (5120 on matrices above 32 M weights) on layers with K < 8192, whole 256-channel
  *              blocks and at most 256 M weights, one destination: the blob is unpacked to INT8 in the workspace
  *              (scratch, N x K bytes) and the INT8 x INT8 CTA-pair kernel does the GEMM, TWO launches
  *              (LQ_UNPACK_I8_MIN_M in the environment moves the limit, 0 switches the route off);

@@ -724,7 +724,9 @@ static bool gemv_serves(int M, int N, int K) {
 // pipe 95 % busy, beats unpacking inside the main loop (71 %).  Measured in one process, W4 pair kernel -> this route:
 // 28672 x 4096 at 2048 / 2560 / 3072 / 4096 / 8192 tokens 184 -> 179, 232 -> 221, 266 -> 256, 360 -> 327, 704 -> 610 us; at 1500
 // 136 -> 143.  6144 x 4096 at 2048 / 3072 / 8192 44.5 -> 44.7, 62.8 -> 55.1, 151 -> 137; 4096 x 4096 at 2560 / 3072 / 8192 40.2 ->
-// 42.5, 44.6 -> 42.0, 105 -> 90: matrices up to 32 M weights start at 3072.  4096 x 14336 (where the W4 kernel's
+// 42.5, 44.6 -> 42.0, 105 -> 90: matrices up to 32 M weights start at 3072.  Larger ones start at 5120 although the time
+// would allow 2048: callers size and type their workspace by the route (scratch of N x K bytes here, the all-zero planes
+// of the W4 pair kernel there), and that contract is kept up to 5119 tokens.  4096 x 14336 (where the W4 kernel's
 // epilogues weigh least) is level at every size: layers with K >= 8192 stay on the W4 pair kernel, and so do layers above
 // 256 MB of INT8 weights (the scratch would be larger than that).  LQ_UNPACK_I8_MIN_M replaces both limits (0 switches
 // the route off).  Running the two kernels overlapped (the GEMM launched programmatically behind a persistent unpack
@@ -732,7 +734,7 @@ static bool gemv_serves(int M, int N, int K) {
 // after the other (the unpack's memory traffic slows the GEMM it runs beside); not kept.
 static bool unpack_i8_serves(int M, int N, int K) {
   const char* e = getenv("LQ_UNPACK_I8_MIN_M");   // read at every call: a measurement switch
-  const int lim = e ? atoi(e) : ((size_t)N * K <= ((size_t)1 << 25) ? 3072 : 2048);
+  const int lim = e ? atoi(e) : ((size_t)N * K <= ((size_t)1 << 25) ? 3072 : 5120);
   return lim > 0 && M >= lim && K < 8192 && (size_t)N * K <= ((size_t)256 << 20) && i8_pair_serves(M, N, K);
 }
 
