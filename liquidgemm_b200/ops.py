@@ -71,15 +71,30 @@ def _req(cond: bool, msg: str) -> None:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream of the current device (the raw handle: no Stream object is built for it)."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _ptr(t: torch.Tensor) -> int:
     return t.data_ptr()
 
 
+class _CurrentDevice:
+    """The context of a tensor that already lives on the current device: nothing to switch."""
+
+    def __enter__(self):
+        return None
+
+    def __exit__(self, *exc):
+        return False
+
+
+_CURRENT = _CurrentDevice()
+
+
 def _dev_ctx(t: torch.Tensor):
-    return torch.cuda.device(t.device)
+    dev = t.device
+    return _CURRENT if dev.index == torch.cuda.current_device() else torch.cuda.device(dev)
 
 
 @torch.library.register_fake("liquidgemm::dequant_weight")
@@ -568,7 +583,7 @@ def _i8_gemm_scaled(a, b, a_scale, b_scale, out_dtype):
     N = b.shape[0]
     _req(b.shape[1] == K and K % 128 == 0, "K mismatch or K not a multiple of 128")
     _req(int(out_dtype) in _OUT_DTYPES, "out_dtype must be 0 (bf16), 1 (fp16) or 2 (fp32)")
-    a_scale, b_scale = _f32(a_scale, "a_scale").reshape(-1), _f32(b_scale, "b_scale").reshape(-1)
+    a_scale, b_scale = _f32(a_scale, "a_scale"), _f32(b_scale, "b_scale")   # contiguous: read as flat vectors
     _req(a_scale.numel() == M and b_scale.numel() == N, "a_scale must have M and b_scale N elements")
     y = torch.empty((M, N), dtype=_OUT_DTYPES[int(out_dtype)], device=a.device)
     if M:
