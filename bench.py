@@ -15,7 +15,7 @@ output, and its quantised tokens, are compared bit for bit with the CPU oracle (
 
 The JSON line printed by rank 0 carries
   value     weight GB/s (packed weight bytes N*K/2 per launch / device time), whole job
-  e2e       the same metric from host buffers (ops.HostStepPlan over lq_w4a8_linear_host): per linear a pinned
+  e2e       the same metric from host buffers (ops.HostStepPlan: copies and lq_w4a8_linear): per linear a pinned
             fp16 activation copy to the device, quant_per_token + linear, and the result copied back
   roofline  algorithmic bytes of the sweep / device time, against the measured HBM copy rate
   cpu_baseline  the CPU oracle (C, OpenMP) on the same sweep, timed on this host

@@ -171,6 +171,10 @@ LQ_API int lq_w4a8_linear_host(const void* x_host, int x_dtype, const void* blob
                                size_t scratch_bytes, void* workspace, size_t workspace_bytes,
                                void* stream);
 
+/* Enqueue one host-to-device (to_device != 0) or device-to-host copy of `bytes` bytes. */
+LQ_API int lq_copy_async(void* dst, const void* src, size_t bytes, int to_device, void* stream);
+
+
 /* Same product from the plain pack_nibbles() layout with float32 output, any M.
  * Replaces torch.ops.liquidgemm.w4a8_gemm (reference csrc/liquid_gemm/w4a8_gemm.cu:183-227).
  * M <= 16 runs the GEMV (K % 64 == 0); larger M re-tiles the weights into `workspace`

@@ -67,4 +67,16 @@ LQ_API int lq_w4a8_linear_host(const void* x_host, int x_dtype, const void* blob
   return LQ_OK;
 }
 
+// One leg of the above on its own, for callers that spread a step's uploads, linears and downloads over streams.
+LQ_API int lq_copy_async(void* dst, const void* src, size_t bytes, int to_device, void* stream) {
+  if (!dst || !src) return LQ_ERR_BAD_ARG;
+  const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost,
+                                        lq::as_stream(stream));
+  if (e != cudaSuccess) {
+    lq::record_cuda_error(e, "lq_copy_async");
+    return LQ_ERR_CUDA;
+  }
+  return LQ_OK;
+}
+
 }  // extern "C"

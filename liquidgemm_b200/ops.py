@@ -405,8 +405,8 @@ def _linear(x, w, s_u8, off_a, s1, bias, N, K, group_size, out_dtype):
     return y
 
 
-def _linear_call(x, code, w, s1, bias, y, out_dtype, M, N, K, dev):
-    S = _splitk_for(M, N, K) if _SPLITK_ENV else 0
+def _linear_call(x, code, w, s1, bias, y, out_dtype, M, N, K, dev, splitk=None):
+    S = (_splitk_for(M, N, K) if _SPLITK_ENV else 0) if splitk is None else splitk
     px = x.data_ptr()
     plan = (ctypes.c_size_t * 3)()
     check(lib.lq_linear_plan(px, M, N, K, S, plan), "w4a8_linear")
@@ -830,9 +830,9 @@ class HostStepPlan:
 
     ``requests`` is a list of ``(x_host, layer, y_host)`` as for :func:`w4a8_linear_host`: pinned host
     activations, a layer dict with the tile blob, a pinned host output.  Construction runs every request
-    once (which also sizes the per-stream scratch) and then records the same calls -- host-to-device copy,
-    token quantiser, linear, device-to-host copy, spread round-robin over ``n_streams`` streams so that the
-    copies of one request overlap the kernels of another -- into a CUDA graph.  :meth:`run` replays it: the
+    once (which checks it and sizes the workspaces) and then records the step into a CUDA graph: uploads on a stream of
+    their own, ahead of the linears; the linears spread over ``n_streams`` streams; each stream's downloads on one
+    beside it, so that no copy stands between two linears.  :meth:`run` replays it: the
     host pays for one launch instead of four to five driver calls per linear, which is what a step of 5-20 us
     kernels is otherwise dominated by.  The buffers are read and written in place on every replay; call
     :meth:`synchronize` before reading the outputs.  Plans built on the same ``stream`` replay in order.  (The reference drives every linear from Python, one
@@ -858,18 +858,51 @@ class HostStepPlan:
                 k = min(range(len(self.side)), key=lambda q: load[q])
                 self.assignment[i] = k
                 load[k] += cost[i]
-            # eager pass: allocates scratch and workspaces of every stream outside the capture
+            # eager pass: checks every request and allocates the workspaces of every stream outside the capture
+            self.tokens = [torch.empty(x.shape, dtype=x.dtype, device=dev) for x, _, _ in self.requests]
+            self.outputs = [torch.empty(y.shape, dtype=y.dtype, device=dev) for _, _, y in self.requests]
             for i, (x, L, y) in enumerate(self.requests):
                 w4a8_linear_host(x, L, y, stream=self.side[self.assignment[i]])
             torch.cuda.synchronize()
+            for i in range(len(self.requests)):
+                self._linear(i)
+            torch.cuda.synchronize()
+            # Uploads run ahead of the linears on a stream of their own, in the order the streams need them, and
+            # downloads behind them on one stream beside each: a copy's latency (several times its bytes' time on the
+            # bus at these sizes) is then paid at the two ends of the step and not between the linears.
+            up = torch.cuda.Stream()
+            down = [torch.cuda.Stream() for _ in self.side]
+            place = [sum(1 for j in range(i) if self.assignment[j] == k) for i, k in enumerate(self.assignment)]
             self.graph = torch.cuda.CUDAGraph()
             with torch.cuda.graph(self.graph, stream=self.main):
-                for st in self.side:
+                for st in (up, *self.side):
                     st.wait_stream(self.main)
-                for i, (x, L, y) in enumerate(self.requests):
-                    w4a8_linear_host(x, L, y, stream=self.side[self.assignment[i]])
-                for st in self.side:
+                landed = {}
+                for i in sorted(range(len(self.requests)), key=lambda j: (place[j], -cost[j])):
+                    x = self.requests[i][0]
+                    if x.numel():
+                        check(lib.lq_copy_async(self.tokens[i].data_ptr(), x.data_ptr(), x.numel() * x.element_size(), 1,
+                                                up.cuda_stream), "HostStepPlan upload")
+                    landed[i] = up.record_event()
+                for i, (_, _, y) in enumerate(self.requests):
+                    st, dn = self.side[self.assignment[i]], down[self.assignment[i]]
+                    st.wait_event(landed[i])
+                    self._linear(i)
+                    dn.wait_stream(st)
+                    if y.numel():
+                        check(lib.lq_copy_async(y.data_ptr(), self.outputs[i].data_ptr(), y.numel() * y.element_size(), 0,
+                                                dn.cuda_stream), "HostStepPlan download")
+                for st in (up, *self.side, *(down[k] for k in sorted(set(self.assignment)))):
                     self.main.wait_stream(st)
+
+    def _linear(self, i):
+        """Enqueue request ``i``'s linear on its stream, between the plan's device buffers."""
+        x, y = self.tokens[i], self.outputs[i]
+        L = self.requests[i][1]
+        if x.shape[0]:
+            with torch.cuda.stream(self.side[self.assignment[i]]):
+                _linear_call(x, _DTYPE_CODES[x.dtype], L["rs"], L["s1"], None, y, _DTYPE_CODES[y.dtype], x.shape[0], L["N"],
+                             L["K"], self.device, splitk=0)
 
     def run(self) -> None:
         """Enqueue the whole step (on the plan's own stream)."""
