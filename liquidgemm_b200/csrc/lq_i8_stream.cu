@@ -5,9 +5,9 @@
 // tensor cores attached.  One 128-channel x BN-token tile and one k-range per CTA, two CTAs per SM; `splits` k-ranges
 // per tile so that the grid fills the SMs.  With one k-range the epilogue is fused; with several every CTA writes an
 // int32 plane and the finish pass adds the planes, scales and casts (exact in any order).
-//  * warp 0  producer: one thread keeps NS 128 x 128 weight boxes in flight (tensor map, 128-byte swizzle).  The
-//            weights do not depend on the previous kernel of the stream: the first NS are requested before the wait
-//            for it.
+//  * warp 0  producer: one thread keeps NS 128 x 128 weight boxes in flight (tensor map, 128-byte swizzle).  B may be the
+//            output of the kernel just before (a quantiser, the dequantiser), so it is read after the wait for that
+//            kernel; before it the first NS boxes are only hinted to L2, which changes no result whoever writes them.
 //  * warp 1  tensor memory and MMA issue: four 128 x BN x 32 tcgen05.mma kind::i8 per k-step, both operands from
 //            shared memory; its commit recycles the stage.
 //  * warps 2..9  two sets of 128 threads, k-steps in turn: the set that owns a k-step fetches its BN x 128-byte token
@@ -104,6 +104,8 @@ i8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const Args args) {
   if (warp == 0) {
     // ------------------------------------------------------------------ producer
     if (lane == 0) {
+      for (int j = 0; j < nk && j < NS; ++j) ptx::tensor_prefetch_2d(&tmap_w, (kt_begin + j) * 128, nt * 128);
+      dependency_wait();
       int i = 0;
       bool ok = true;
       for (; i < nk; ++i) {

@@ -113,6 +113,10 @@ __device__ __forceinline__ void tensor_load_2d(uint32_t dst_smem, const void* tm
       "l"(tmap), "r"(bar), "r"(x), "r"(y)
       : "memory");
 }
+// The same box fetched into L2 only: a hint, without effect on what any later access reads.
+__device__ __forceinline__ void tensor_prefetch_2d(const void* tmap, int x, int y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(tmap), "r"(x), "r"(y) : "memory");
+}
 __device__ __forceinline__ void prefetch_tensormap(const void* tmap) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory");
 }

@@ -1,0 +1,44 @@
+"""Operands that the kernel directly before has written: the overlapped launches must wait for them.  Exact sums, so the
+tolerance is none."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _exact(a, b):
+    """a @ b.T in integers: every partial sum is below 2^53."""
+    return (a.double() @ b.double().t()).to(torch.int32)
+
+
+# streaming kernel with K cut, whole tiles in several waves, its widest token tile; the CTA-pair kernel
+@pytest.mark.parametrize("M,N,K", [(8, 4096, 4096), (1, 28672, 2048), (33, 40064, 1024), (200, 1024, 4096), (300, 16384, 512)])
+@pytest.mark.parametrize("between", [False, True])
+def test_int8_weights_quantised_just_before(M, N, K, between):
+    """Both operands from ``quant_per_token``, the weights last, or (a second early-triggering kernel between the
+    writer and the reader) the tokens last.  The weights' buffer is the same in every pass, with other contents."""
+    from liquidgemm_b200 import ops
+    from liquidgemm_b200._lib import lib, check
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    ws = [torch.randn(N, K, device="cuda", generator=g, dtype=torch.bfloat16) for _ in range(2)]
+    x = torch.randn(M, K, device="cuda", generator=g, dtype=torch.bfloat16)
+    w8, sw = torch.zeros(N, K, device="cuda", dtype=torch.int8), torch.zeros(N, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    settled = [torch.ops.liquidgemm.quant_per_token(w) for w in ws]
+    x8, sx = torch.ops.liquidgemm.quant_per_token(x)
+    torch.cuda.synchronize()
+    acc = [_exact(x8, q) for q, _ in settled]
+    want = [((a.float() * sx[:, None]) * s).to(torch.bfloat16) for a, (_, s) in zip(acc, settled)]
+    got = []
+    for i in range(12):
+        check(lib.lq_quant_per_token(ws[i & 1].data_ptr(), 0, w8.data_ptr(), sw.data_ptr(), N, K, st), "quant_per_token")
+        if between:
+            x8, sx = torch.ops.liquidgemm.quant_per_token(x)
+        if i < 6:
+            got.append(torch.ops.liquidgemm.wgmma_i8_gemm(x8, w8))
+        else:
+            got.append(torch.ops.liquidgemm.i8_gemm_scaled(x8, w8, sx, sw, 0))
+    for i, y in enumerate(got):
+        assert torch.equal(y, (acc if i < 6 else want)[i & 1]), i
+    ops.poll_status()
