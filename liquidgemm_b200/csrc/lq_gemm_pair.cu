@@ -168,8 +168,8 @@ w4a8_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const Args args,
   const uint32_t tmem_a = tmem_base + 2 * kBN;   // kNT operand stages behind the two accumulators
   const uint32_t leader_aready = ptx::map_to_cta(bar_aready, 0);
   const uint32_t leader_accfree = ptx::map_to_cta(bar_accfree, 0);
-  allow_dependents();                 // every CTA of this launch is resident: the next kernel may be scheduled behind it
-  if (warp != 0) dependency_wait();   // tokens, scales, outputs and planes belong to earlier kernels until here; weights do not
+  allow_dependents();   // every CTA of this launch is resident: the next kernel may be scheduled behind it
+  dependency_wait();    // everything it reads may come from the kernel before it (the weights too: a blob re-tiled on the spot)
 
   if (warp == 0 || warp == 2) {
     // ------------------------------------------------------------------ producers (one thread each)
@@ -715,7 +715,7 @@ static int launch(const CUtensorMap& tx, const Args& a, const MultiOut* multi, c
     record_cuda_error(attr_err, "cudaFuncSetAttribute(w4a8_pair_kernel)");
     return LQ_ERR_CUDA;
   }
-  // Launched programmatically: set-up and the first weight tiles overlap the end of the token quantiser before it.
+  // Launched programmatically: set-up overlaps the end of the token quantiser before it.
   cudaError_t e;
   if constexpr (MULTI) e = launch_overlapped(kern, dim3(2 * a.pairs), dim3(kThreads), (size_t)kSmemBytes, st, tx, a, *multi);
   else e = launch_overlapped(kern, dim3(2 * a.pairs), dim3(kThreads), (size_t)kSmemBytes, st, tx, a, NoMultiOut{});

@@ -42,3 +42,34 @@ def test_int8_weights_quantised_just_before(M, N, K, between):
     for i, y in enumerate(got):
         assert torch.equal(y, (acc if i < 6 else want)[i & 1]), i
     ops.poll_status()
+
+
+# CTA-pair kernel (where it serves: LQ_PAIR_ALWAYS), whole and cut last waves
+RETILED = [(2048, 4096, 1024), (700, 28672, 512)]
+
+
+@pytest.mark.parametrize("M,N,K", RETILED)
+@pytest.mark.parametrize("op", ["w4a8_wgmma", "w4a8_wgmma_rs"])
+def test_weights_retiled_just_before(monkeypatch, M, N, K, op):
+    """The operators that take ``pack_nibbles`` weights re-tile them into scratch (the same block of the allocator in
+    every pass, with other contents) and multiply at once."""
+    from liquidgemm_b200 import ops
+    from liquidgemm_b200.pack import pack_nibbles
+    monkeypatch.setenv("LQ_PAIR_ALWAYS", "1")
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    layers = []
+    for _ in range(2):
+        qw, _ = ops.quantize_weight_cuda(torch.randn(N, K, device="cuda", generator=g), 64)
+        w8 = torch.ops.liquidgemm.dequant_weight(qw.qweight_u4, qw.s_u8, qw.offset_a, N, K, 64)
+        layers.append((pack_nibbles(qw.qweight_u4).contiguous(), qw.s_u8, qw.offset_a, w8))
+    x = torch.randint(-127, 128, (M, K), device="cuda", dtype=torch.int8, generator=g)
+    torch.cuda.synchronize()
+    acc = [_exact(x, w8) for *_, w8 in layers]
+    for i in range(8):
+        w, s, a, _ = layers[i & 1]
+        if op == "w4a8_wgmma":
+            y = torch.ops.liquidgemm.w4a8_wgmma(x, w, s, a, N, K, 64)
+        else:
+            y = torch.ops.liquidgemm.w4a8_wgmma_rs(x, w, s, s, a, N, K, 64, False)
+        assert torch.equal(y, acc[i & 1]), i
+    ops.poll_status()
