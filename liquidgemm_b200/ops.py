@@ -17,7 +17,6 @@ from __future__ import annotations
 import os
 
 import ctypes
-import weakref
 
 import torch
 
@@ -257,7 +256,6 @@ def _splitk_for(M, N, K):
 # captured graph may still point at them.
 _WORKSPACES: dict = {}
 _RETIRED: list = []
-_PLANS: "weakref.WeakSet" = weakref.WeakSet()   # HostStepPlans: each has zero-filled workspaces of its own
 
 
 def _workspace(nbytes: int, device: torch.device, stream=None):
@@ -277,7 +275,7 @@ def poll_status(device=None) -> None:
     """Read (and clear) the device-side status word of ``device`` (default: the current one) after
     synchronising its current stream.  Kernels never hang: a bounded wait that gives up records a site code
     there and the kernel finishes, possibly with partial sums left in the shared reduction workspaces.  When
-    the word is set this function therefore clears every cached workspace (and every plan's) of the device and raises
+    the word is set this function therefore clears every cached workspace of the device and raises
     :class:`liquidgemm_b200._lib.LiquidGemmError`; call it wherever a wrong result must not go unnoticed
     (after a benchmark, between serving batches, in tests)."""
     dev = torch.cuda.current_device() if device is None else torch.device(device).index
@@ -287,10 +285,6 @@ def poll_status(device=None) -> None:
             for (d, _), ws in list(_WORKSPACES.items()):
                 if d == dev:
                     ws.zero_()
-            for plan in list(_PLANS):
-                if plan.device.index == dev:
-                    for ws in plan.zeroed:
-                        ws.zero_()
             torch.cuda.synchronize()
         check(rc, "poll_status")
 
@@ -413,17 +407,12 @@ def _linear(x, w, s_u8, off_a, s1, bias, N, K, group_size, out_dtype):
     return y
 
 
-def _linear_sizes(px, M, N, K, splitk):
-    """Scratch bytes, workspace bytes and workspace kind of ``lq_w4a8_linear`` for activations at ``px``."""
-    plan = (ctypes.c_size_t * 3)()
-    check(lib.lq_linear_plan(px, M, N, K, splitk, plan), "w4a8_linear")
-    return plan
-
-
-def _linear_call(x, code, w, s1, bias, y, out_dtype, M, N, K, dev):
-    S = _splitk_for(M, N, K) if _SPLITK_ENV else 0
+def _linear_call(x, code, w, s1, bias, y, out_dtype, M, N, K, dev, splitk=None):
+    S = (_splitk_for(M, N, K) if _SPLITK_ENV else 0) if splitk is None else splitk
     px = x.data_ptr()
-    nscratch, nws, kind = _linear_sizes(px, M, N, K, S)
+    plan = (ctypes.c_size_t * 3)()
+    check(lib.lq_linear_plan(px, M, N, K, S, plan), "w4a8_linear")
+    nscratch, nws, kind = plan
     stream = _stream()
     scratch = torch.empty((nscratch,), dtype=torch.uint8, device=dev) if nscratch else None
     if kind == 1:
@@ -768,19 +757,6 @@ _HOST_PLANES: dict = {}
 _HOST_SIZES: dict = {}
 
 
-def _check_host_request(x_host, qw_dev, y_host, odt):
-    if x_host.is_cuda or x_host.dim() != 2 or not x_host.is_contiguous() or x_host.dtype not in _DTYPE_CODES:
-        raise RuntimeError("liquidgemm_b200: x_host must be a contiguous CPU [M,K] tensor of bf16, fp16 or fp32")
-    M, K = x_host.shape
-    N = qw_dev["N"]
-    if K != qw_dev["K"] or K % 128:
-        raise RuntimeError("liquidgemm_b200: K mismatch or K % 128 != 0")
-    if y_host is not None and (y_host.is_cuda or y_host.dtype != odt or y_host.shape[0] != M or y_host.shape[1] != N or
-                               not y_host.is_contiguous()):
-        raise RuntimeError("liquidgemm_b200: y_host must be a contiguous CPU [M,N] tensor of the output dtype")
-    return M, N, K
-
-
 def w4a8_linear_host(x_host: torch.Tensor, qw_dev: dict, y_host: torch.Tensor = None,
                      out_dtype: torch.dtype = None, stream: "torch.cuda.Stream" = None) -> torch.Tensor:
     """The same linear for activations and outputs in HOST memory (pinned for asynchronous copies):
@@ -792,10 +768,18 @@ def w4a8_linear_host(x_host: torch.Tensor, qw_dev: dict, y_host: torch.Tensor = 
 
     The wrapper is on the per-layer critical path of a host-driven decode loop, so it caches what does
     not change between calls (buffer sizes per shape, the scratch per stream) and does no tensor work."""
+    if x_host.is_cuda or x_host.dim() != 2 or not x_host.is_contiguous() or x_host.dtype not in _DTYPE_CODES:
+        raise RuntimeError("liquidgemm_b200: x_host must be a contiguous CPU [M,K] tensor of bf16, fp16 or fp32")
+    M, K = x_host.shape
+    N = qw_dev["N"]
     odt = out_dtype or x_host.dtype
-    M, N, K = _check_host_request(x_host, qw_dev, y_host, odt)
+    if K != qw_dev["K"] or K % 128:
+        raise RuntimeError("liquidgemm_b200: K mismatch or K % 128 != 0")
     if y_host is None:
         y_host = torch.empty((M, N), dtype=odt, pin_memory=True)
+    elif y_host.is_cuda or y_host.dtype != odt or y_host.shape[0] != M or y_host.shape[1] != N or \
+            not y_host.is_contiguous():
+        raise RuntimeError("liquidgemm_b200: y_host must be a contiguous CPU [M,N] tensor of the output dtype")
     if M == 0:
         return y_host
     blob, s1 = qw_dev["rs"], qw_dev["s1"]
@@ -842,36 +826,18 @@ def w4a8_linear_host(x_host: torch.Tensor, qw_dev: dict, y_host: torch.Tensor = 
     return y_host
 
 
-def _overlaps(requests):
-    """Pairs ``(kind, i, j)``, i < j, of requests that share host memory: ``"yx"`` j's input lies in i's output, ``"xy"``
-    j's output in i's input, ``"yy"`` output in output."""
-    spans = sorted((t.data_ptr(), t.data_ptr() + t.numel() * t.element_size(), side, i)
-                   for i, (x, _, y) in enumerate(requests) for side, t in (("x", x), ("y", y)) if t.numel())
-    pairs, live = set(), []
-    for span in spans:
-        live = [o for o in live if o[1] > span[0]]
-        for other in live:
-            (si, i), (sj, j) = sorted((other[2:], span[2:]), key=lambda e: e[1])
-            if i != j and si + sj != "xx":
-                pairs.add((si + sj, i, j))
-        live.append(span)
-    return pairs
-
-
 class HostStepPlan:
     """A fixed set of host-buffer linears (one decode step of a host-driven loop) recorded once and replayed
     with a single call.
 
     ``requests`` is a list of ``(x_host, layer, y_host)`` as for :func:`w4a8_linear_host`: pinned host
-    activations, a layer dict with the tile blob, a pinned host output.  Construction runs the step once and then
-    records it into a CUDA graph: uploads on a stream of their own, ahead of the linears; the linears spread over
-    ``n_streams`` streams; each stream's downloads on one beside it, so that no copy stands between two linears.
-    Requests that share host memory (one's output is a later one's input, say) take effect in the order of the list.
-    :meth:`run` replays the step: the host pays for one launch instead of four to five driver calls per linear,
-    which is what a step of 5-20 us kernels is otherwise dominated by.  The host buffers are read and written in
-    place on every replay; call :meth:`synchronize` before reading the outputs.  Plans built on the same ``stream``
-    replay in order, plans on different streams may replay side by side: every device buffer belongs to one plan, and
-    dropping a plan returns them once its last replay has finished.  (The reference drives every linear from Python, one
+    activations, a layer dict with the tile blob, a pinned host output.  Construction runs every request
+    once (which checks it and sizes the workspaces) and then records the step into a CUDA graph: uploads on a stream of
+    their own, ahead of the linears; the linears spread over ``n_streams`` streams; each stream's downloads on one
+    beside it, so that no copy stands between two linears.  :meth:`run` replays it: the
+    host pays for one launch instead of four to five driver calls per linear, which is what a step of 5-20 us
+    kernels is otherwise dominated by.  The buffers are read and written in place on every replay; call
+    :meth:`synchronize` before reading the outputs.  Plans built on the same ``stream`` replay in order.  (The reference drives every linear from Python, one
     operator call at a time: liquidgemm/vllm_plugin.py:174-206.)"""
 
     def __init__(self, requests, n_streams: int = 3, device=None, stream: "torch.cuda.Stream" = None):
@@ -879,13 +845,7 @@ class HostStepPlan:
             raise RuntimeError("liquidgemm_b200: HostStepPlan needs at least one request")
         self.requests = list(requests)
         dev = torch.device(device) if device is not None else self.requests[0][1]["rs"].device
-        if dev.index is None:
-            dev = torch.device(dev.type, torch.cuda.current_device())
         self.device = dev
-        for x, L, y in self.requests:
-            _check_host_request(x, L, y, x.dtype)
-            if L["rs"].device != dev or L["s1"].device != dev:
-                raise RuntimeError("liquidgemm_b200: every layer of a HostStepPlan must be on its device")
         with torch.cuda.device(dev):
             # replays are ordered on `stream`: plans that share it run one after the other, like the steps
             # of a decode loop
@@ -900,84 +860,51 @@ class HostStepPlan:
                 k = min(range(len(self.side)), key=lambda q: load[q])
                 self.assignment[i] = k
                 load[k] += cost[i]
-            place = [sum(1 for j in range(i) if self.assignment[j] == k) for i, k in enumerate(self.assignment)]
-            self._upload_order = sorted(range(len(self.requests)), key=lambda j: (place[j], -cost[j]))
-            self._after = {"yx": {}, "xy": {}, "yy": {}}   # kind -> request -> earlier requests it waits for
-            for kind, i, j in _overlaps(self.requests):
-                self._after[kind].setdefault(j, []).append(i)
-            # Device buffers of the plan alone: streams are pooled, so buffers kept by stream would be shared by plans
-            # that may replay side by side.  Allocated outside the capture (a graph's private pool costs milliseconds).
+            # eager pass: checks every request and allocates the workspaces of every stream outside the capture
             self.tokens = [torch.empty(x.shape, dtype=x.dtype, device=dev) for x, _, _ in self.requests]
             self.outputs = [torch.empty(y.shape, dtype=y.dtype, device=dev) for _, _, y in self.requests]
-            self._sizes = [tuple(_linear_sizes(t.data_ptr(), t.shape[0], L["N"], L["K"], 0)) if t.shape[0] else (0, 0, 0)
-                           for t, (_, L, _) in zip(self.tokens, self.requests)]
-            nscratch, nzeroed = [0] * len(self.side), [0] * len(self.side)
-            for (ns, nws, kind), k in zip(self._sizes, self.assignment):
-                nscratch[k] = max(nscratch[k], (ns + 255) // 256 * 256 + (nws if kind == 1 else 0))
-                nzeroed[k] = max(nzeroed[k], nws if kind == 2 else 0)
-            self.scratch = [torch.empty((n,), dtype=torch.uint8, device=dev) for n in nscratch]
-            self.zeroed = [torch.zeros((n,), dtype=torch.uint8, device=dev) for n in nzeroed]
-            for t in (*self.tokens, *self.outputs, *self.scratch, *self.zeroed):
-                t.record_stream(self.main)   # freed buffers wait for the replays in flight
-            _PLANS.add(self)
+            for i, (x, L, y) in enumerate(self.requests):
+                w4a8_linear_host(x, L, y, stream=self.side[self.assignment[i]])
             torch.cuda.synchronize()
-            up, down = torch.cuda.Stream(), [torch.cuda.Stream() for _ in self.side]
-            self._step(up, down)             # loads every kernel, so that the capture finds them loaded
+            for i in range(len(self.requests)):
+                self._linear(i)
             torch.cuda.synchronize()
+            # Uploads run ahead of the linears on a stream of their own, in the order the streams need them, and
+            # downloads behind them on one stream beside each: a copy's latency (several times its bytes' time on the
+            # bus at these sizes) is then paid at the two ends of the step and not between the linears.
+            up = torch.cuda.Stream()
+            down = [torch.cuda.Stream() for _ in self.side]
+            place = [sum(1 for j in range(i) if self.assignment[j] == k) for i, k in enumerate(self.assignment)]
             self.graph = torch.cuda.CUDAGraph()
             with torch.cuda.graph(self.graph, stream=self.main):
-                self._step(up, down)
-
-    def _step(self, up, down):
-        """Enqueue one step behind ``self.main``, which then waits for all of it.  Uploads run ahead of the linears on a
-        stream of their own, in the order the streams need them, and downloads behind them on one stream beside each: a
-        copy's latency (several times its bytes' time on the bus at these sizes) is then paid at the two ends of the step
-        and not between the linears.  Requests that share host memory wait for each other's copies."""
-        for st in (up, *self.side):
-            st.wait_stream(self.main)
-        uploaded, downloaded = {}, {}
-
-        def upload(i, st):
-            x = self.requests[i][0]
-            if x.numel():
-                check(lib.lq_copy_async(self.tokens[i].data_ptr(), x.data_ptr(), x.numel() * x.element_size(), 1,
-                                        st.cuda_stream), "HostStepPlan upload")
-            uploaded[i] = st.record_event()
-
-        for i in self._upload_order:
-            if i not in self._after["yx"]:
-                upload(i, up)
-        for i, (_, _, y) in enumerate(self.requests):
-            st, dn = self.side[self.assignment[i]], down[self.assignment[i]]
-            if i in self._after["yx"]:       # its input is an earlier request's output
-                for j in self._after["yx"][i]:
-                    st.wait_event(downloaded[j])
-                upload(i, st)
-            else:
-                st.wait_event(uploaded[i])
-            self._linear(i)
-            dn.wait_stream(st)
-            for j in self._after["xy"].get(i, ()):
-                dn.wait_event(uploaded[j])
-            for j in self._after["yy"].get(i, ()):
-                dn.wait_event(downloaded[j])
-            if y.numel():
-                check(lib.lq_copy_async(y.data_ptr(), self.outputs[i].data_ptr(), y.numel() * y.element_size(), 0,
-                                        dn.cuda_stream), "HostStepPlan download")
-            downloaded[i] = dn.record_event()
-        for st in (up, *self.side, *(down[k] for k in sorted(set(self.assignment)))):
-            self.main.wait_stream(st)
+                for st in (up, *self.side):
+                    st.wait_stream(self.main)
+                landed = {}
+                for i in sorted(range(len(self.requests)), key=lambda j: (place[j], -cost[j])):
+                    x = self.requests[i][0]
+                    if x.numel():
+                        check(lib.lq_copy_async(self.tokens[i].data_ptr(), x.data_ptr(), x.numel() * x.element_size(), 1,
+                                                up.cuda_stream), "HostStepPlan upload")
+                    landed[i] = up.record_event()
+                for i, (_, _, y) in enumerate(self.requests):
+                    st, dn = self.side[self.assignment[i]], down[self.assignment[i]]
+                    st.wait_event(landed[i])
+                    self._linear(i)
+                    dn.wait_stream(st)
+                    if y.numel():
+                        check(lib.lq_copy_async(y.data_ptr(), self.outputs[i].data_ptr(), y.numel() * y.element_size(), 0,
+                                                dn.cuda_stream), "HostStepPlan download")
+                for st in (up, *self.side, *(down[k] for k in sorted(set(self.assignment)))):
+                    self.main.wait_stream(st)
 
     def _linear(self, i):
         """Enqueue request ``i``'s linear on its stream, between the plan's device buffers."""
-        x, y, k = self.tokens[i], self.outputs[i], self.assignment[i]
-        L, (ns, nws, kind) = self.requests[i][1], self._sizes[i]
+        x, y = self.tokens[i], self.outputs[i]
+        L = self.requests[i][1]
         if x.shape[0]:
-            scratch = self.scratch[k].data_ptr()
-            ws = scratch + (ns + 255) // 256 * 256 if kind == 1 else self.zeroed[k].data_ptr()
-            check(lib.lq_w4a8_linear(x.data_ptr(), _DTYPE_CODES[x.dtype], L["rs"].data_ptr(), L["s1"].data_ptr(), None,
-                                     y.data_ptr(), _DTYPE_CODES[y.dtype], x.shape[0], L["N"], L["K"], 0, scratch or None, ns,
-                                     ws or None, nws, self.side[k].cuda_stream), "HostStepPlan")
+            with torch.cuda.stream(self.side[self.assignment[i]]):
+                _linear_call(x, _DTYPE_CODES[x.dtype], L["rs"], L["s1"], None, y, _DTYPE_CODES[y.dtype], x.shape[0], L["N"],
+                             L["K"], self.device, splitk=0)
 
     def run(self) -> None:
         """Enqueue the whole step (on the plan's own stream)."""
