@@ -826,19 +826,35 @@ def w4a8_linear_host(x_host: torch.Tensor, qw_dev: dict, y_host: torch.Tensor = 
     return y_host
 
 
+def _overlaps(requests):
+    """Pairs ``(kind, i, j)``, i < j, of requests that share host memory: ``"yx"`` j's input lies in i's output, ``"xy"``
+    j's output in i's input, ``"yy"`` output in output."""
+    spans = sorted((t.data_ptr(), t.data_ptr() + t.numel() * t.element_size(), side, i)
+                   for i, (x, _, y) in enumerate(requests) for side, t in (("x", x), ("y", y)) if t.numel())
+    pairs, live = set(), []
+    for span in spans:
+        live = [o for o in live if o[1] > span[0]]
+        for other in live:
+            (si, i), (sj, j) = sorted((other[2:], span[2:]), key=lambda e: e[1])
+            if i != j and si + sj != "xx":
+                pairs.add((si + sj, i, j))
+        live.append(span)
+    return pairs
+
+
 class HostStepPlan:
     """A fixed set of host-buffer linears (one decode step of a host-driven loop) recorded once and replayed
     with a single call.
 
     ``requests`` is a list of ``(x_host, layer, y_host)`` as for :func:`w4a8_linear_host`: pinned host
-    activations, a layer dict with the tile blob, a pinned host output.  Construction runs every request
-    once (which checks it and sizes the workspaces) and then records the step into a CUDA graph: uploads on a stream of
-    their own, ahead of the linears; the linears spread over ``n_streams`` streams; each stream's downloads on one
-    beside it, so that no copy stands between two linears.  :meth:`run` replays it: the
-    host pays for one launch instead of four to five driver calls per linear, which is what a step of 5-20 us
-    kernels is otherwise dominated by.  The buffers are read and written in place on every replay; call
-    :meth:`synchronize` before reading the outputs.  Plans built on the same ``stream`` replay in order.  (The reference drives every linear from Python, one
-    operator call at a time: liquidgemm/vllm_plugin.py:174-206.)"""
+    activations, a layer dict with the tile blob, a pinned host output.  Construction runs the step once and then
+    records it into a CUDA graph: uploads on a stream of their own, ahead of the linears; the linears spread over
+    ``n_streams`` streams; each stream's downloads on one beside it, so that no copy stands between two linears.
+    Requests that share host memory (one's output is a later one's input, say) take effect in the order of the list.
+    :meth:`run` replays the step: the host pays for one launch instead of four to five driver calls per linear,
+    which is what a step of 5-20 us kernels is otherwise dominated by.  The host buffers are read and written in
+    place on every replay; call :meth:`synchronize` before reading the outputs.  Plans built on the same ``stream``
+    replay in order.  (The reference drives every linear from Python, one operator call at a time: liquidgemm/vllm_plugin.py:174-206.)"""
 
     def __init__(self, requests, n_streams: int = 3, device=None, stream: "torch.cuda.Stream" = None):
         if not requests:
@@ -860,42 +876,63 @@ class HostStepPlan:
                 k = min(range(len(self.side)), key=lambda q: load[q])
                 self.assignment[i] = k
                 load[k] += cost[i]
-            # eager pass: checks every request and allocates the workspaces of every stream outside the capture
+            place = [sum(1 for j in range(i) if self.assignment[j] == k) for i, k in enumerate(self.assignment)]
+            self._upload_order = sorted(range(len(self.requests)), key=lambda j: (place[j], -cost[j]))
+            self._after = {"yx": {}, "xy": {}, "yy": {}}   # kind -> request -> earlier requests it waits for
+            for kind, i, j in _overlaps(self.requests):
+                self._after[kind].setdefault(j, []).append(i)
             self.tokens = [torch.empty(x.shape, dtype=x.dtype, device=dev) for x, _, _ in self.requests]
             self.outputs = [torch.empty(y.shape, dtype=y.dtype, device=dev) for _, _, y in self.requests]
+            # eager pass: checks every request and allocates the workspaces of every stream outside the capture
             for i, (x, L, y) in enumerate(self.requests):
                 w4a8_linear_host(x, L, y, stream=self.side[self.assignment[i]])
             torch.cuda.synchronize()
-            for i in range(len(self.requests)):
-                self._linear(i)
+            up, down = torch.cuda.Stream(), [torch.cuda.Stream() for _ in self.side]
+            self._step(up, down)             # allocates the workspaces of every stream outside the capture
             torch.cuda.synchronize()
-            # Uploads run ahead of the linears on a stream of their own, in the order the streams need them, and
-            # downloads behind them on one stream beside each: a copy's latency (several times its bytes' time on the
-            # bus at these sizes) is then paid at the two ends of the step and not between the linears.
-            up = torch.cuda.Stream()
-            down = [torch.cuda.Stream() for _ in self.side]
-            place = [sum(1 for j in range(i) if self.assignment[j] == k) for i, k in enumerate(self.assignment)]
             self.graph = torch.cuda.CUDAGraph()
             with torch.cuda.graph(self.graph, stream=self.main):
-                for st in (up, *self.side):
-                    st.wait_stream(self.main)
-                landed = {}
-                for i in sorted(range(len(self.requests)), key=lambda j: (place[j], -cost[j])):
-                    x = self.requests[i][0]
-                    if x.numel():
-                        check(lib.lq_copy_async(self.tokens[i].data_ptr(), x.data_ptr(), x.numel() * x.element_size(), 1,
-                                                up.cuda_stream), "HostStepPlan upload")
-                    landed[i] = up.record_event()
-                for i, (_, _, y) in enumerate(self.requests):
-                    st, dn = self.side[self.assignment[i]], down[self.assignment[i]]
-                    st.wait_event(landed[i])
-                    self._linear(i)
-                    dn.wait_stream(st)
-                    if y.numel():
-                        check(lib.lq_copy_async(y.data_ptr(), self.outputs[i].data_ptr(), y.numel() * y.element_size(), 0,
-                                                dn.cuda_stream), "HostStepPlan download")
-                for st in (up, *self.side, *(down[k] for k in sorted(set(self.assignment)))):
-                    self.main.wait_stream(st)
+                self._step(up, down)
+
+    def _step(self, up, down):
+        """Enqueue one step behind ``self.main``, which then waits for all of it.  Uploads run ahead of the linears on a
+        stream of their own, in the order the streams need them, and downloads behind them on one stream beside each: a
+        copy's latency (several times its bytes' time on the bus at these sizes) is then paid at the two ends of the step
+        and not between the linears.  Requests that share host memory wait for each other's copies."""
+        for st in (up, *self.side):
+            st.wait_stream(self.main)
+        uploaded, downloaded = {}, {}
+
+        def upload(i, st):
+            x = self.requests[i][0]
+            if x.numel():
+                check(lib.lq_copy_async(self.tokens[i].data_ptr(), x.data_ptr(), x.numel() * x.element_size(), 1,
+                                        st.cuda_stream), "HostStepPlan upload")
+            uploaded[i] = st.record_event()
+
+        for i in self._upload_order:
+            if i not in self._after["yx"]:
+                upload(i, up)
+        for i, (_, _, y) in enumerate(self.requests):
+            st, dn = self.side[self.assignment[i]], down[self.assignment[i]]
+            if i in self._after["yx"]:       # its input is an earlier request's output
+                for j in self._after["yx"][i]:
+                    st.wait_event(downloaded[j])
+                upload(i, st)
+            else:
+                st.wait_event(uploaded[i])
+            self._linear(i)
+            dn.wait_stream(st)
+            for j in self._after["xy"].get(i, ()):
+                dn.wait_event(uploaded[j])
+            for j in self._after["yy"].get(i, ()):
+                dn.wait_event(downloaded[j])
+            if y.numel():
+                check(lib.lq_copy_async(y.data_ptr(), self.outputs[i].data_ptr(), y.numel() * y.element_size(), 0,
+                                        dn.cuda_stream), "HostStepPlan download")
+            downloaded[i] = dn.record_event()
+        for st in (up, *self.side, *(down[k] for k in sorted(set(self.assignment)))):
+            self.main.wait_stream(st)
 
     def _linear(self, i):
         """Enqueue request ``i``'s linear on its stream, between the plan's device buffers."""

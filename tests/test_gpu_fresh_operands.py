@@ -74,3 +74,34 @@ def test_weights_retiled_just_before(monkeypatch, M, N, K, op):
             y = torch.ops.liquidgemm.w4a8_wgmma_rs(x, w, s, s, a, N, K, 64, False)
         assert torch.equal(y, acc[i & 1]), i
     ops.poll_status()
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 4096, 4096), (8, 4096, 4096), (8, 28672, 1024), (40, 1024, 4096)])
+@pytest.mark.parametrize("writer", ["quantise", "repack"])
+def test_blob_written_just_before(M, N, K, writer):
+    """The package's own writers of tile blobs, into the same buffer with changing contents, directly before a fused
+    linear that fetches its first tiles ahead of the stream."""
+    from liquidgemm_b200 import ops
+    from liquidgemm_b200._lib import lib, check
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    ws = [torch.randn(N, K, device="cuda", generator=g, dtype=torch.bfloat16) for _ in range(2)]
+    settled = [ops.quantize_weight_cuda(w, 64, want_codes=True, want_blob=True) for w in ws]
+    x8, sx = torch.ops.liquidgemm.quant_per_token(torch.randn(M, K, device="cuda", generator=g))
+    want = []
+    for qw, blob in settled:
+        torch.cuda.synchronize()
+        want.append(ops.gemm_fused(x8, blob.reshape(-1), sx, qw.s1, N, K, 0))
+    blob, (s1, s, a) = torch.zeros_like(settled[0][1]), (torch.empty_like(t) for t in (qw.s1, qw.s_u8, qw.offset_a))
+    st = torch.cuda.current_stream().cuda_stream
+    torch.cuda.synchronize()
+    for i in range(8):
+        qw = settled[i & 1][0]
+        if writer == "quantise":
+            check(lib.lq_quantize_weight(ws[i & 1].data_ptr(), 0, N, K, 64, s1.data_ptr(), s.data_ptr(), a.data_ptr(), None,
+                                         blob.data_ptr(), st), "quantize_weight")
+        else:
+            check(lib.lq_repack_tiles(qw.qweight_u4.data_ptr(), 0, qw.s_u8.data_ptr(), qw.offset_a.data_ptr(),
+                                      blob.data_ptr(), N, K, 64, st), "repack_tiles")
+        y = ops.gemm_fused(x8, blob.reshape(-1), sx, qw.s1, N, K, 0)
+        assert torch.equal(y, want[i & 1]), i
+    ops.poll_status()

@@ -27,3 +27,36 @@ def test_replays_follow_the_inputs(n_streams):
         for (x, _, y), layer in zip(requests, layers):
             assert torch.equal(y, ops.w4a8_linear(x.cuda(), layer).cpu()), tuple(y.shape)
     ops.poll_status()
+
+
+def _layer(n, k, g):
+    from liquidgemm_b200 import ops
+    qw, blob = ops.quantize_weight_cuda(torch.randn(n, k, device="cuda", generator=g) * 0.05, 64, want_codes=False, want_blob=True)
+    return {"s1": qw.s1, "s_u8": qw.s_u8, "offset_a": qw.offset_a, "N": n, "K": k, "rs": blob.reshape(-1)}
+
+
+def _pinned(m, k):
+    return torch.zeros(m, k, dtype=torch.float16).pin_memory()
+
+
+@pytest.mark.parametrize("n_streams", [1, 3])
+def test_requests_that_share_memory_run_in_order(n_streams):
+    """One request's output is the next one's input; an input is overwritten by a later output; two requests write the
+    same output, the later one last.  Every replay starts from new values."""
+    from liquidgemm_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(7)
+    up, down, again = _layer(2048, 512, g), _layer(512, 2048, g), _layer(2048, 512, g)
+    x, mid, end = _pinned(5, 512), _pinned(5, 2048), _pinned(5, 2048)
+    # the second request reads what the first wrote and writes over what the first read, and so on through the chain
+    requests = [(x, up, mid), (mid, down, x), (x, again, end), (x, up, end), (end, down, x)]
+    plan = ops.HostStepPlan(requests, n_streams=n_streams)
+    for _ in range(4):
+        x.copy_(torch.randn(x.shape, device="cuda", generator=g))
+        h = ops.w4a8_linear(x.cuda(), up)
+        d = ops.w4a8_linear(h, down)
+        last = ops.w4a8_linear(d, up)
+        plan.run()
+        plan.synchronize()
+        assert torch.equal(mid, h.cpu()) and torch.equal(end, last.cpu())
+        assert torch.equal(x, ops.w4a8_linear(last, down).cpu())
+    ops.poll_status()
