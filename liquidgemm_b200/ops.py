@@ -757,6 +757,19 @@ _HOST_PLANES: dict = {}
 _HOST_SIZES: dict = {}
 
 
+def _check_host_request(x_host, qw_dev, y_host, odt):
+    if x_host.is_cuda or x_host.dim() != 2 or not x_host.is_contiguous() or x_host.dtype not in _DTYPE_CODES:
+        raise RuntimeError("liquidgemm_b200: x_host must be a contiguous CPU [M,K] tensor of bf16, fp16 or fp32")
+    M, K = x_host.shape
+    N = qw_dev["N"]
+    if K != qw_dev["K"] or K % 128:
+        raise RuntimeError("liquidgemm_b200: K mismatch or K % 128 != 0")
+    if y_host is not None and (y_host.is_cuda or y_host.dtype != odt or y_host.shape[0] != M or y_host.shape[1] != N or
+                               not y_host.is_contiguous()):
+        raise RuntimeError("liquidgemm_b200: y_host must be a contiguous CPU [M,N] tensor of the output dtype")
+    return M, N, K
+
+
 def w4a8_linear_host(x_host: torch.Tensor, qw_dev: dict, y_host: torch.Tensor = None,
                      out_dtype: torch.dtype = None, stream: "torch.cuda.Stream" = None) -> torch.Tensor:
     """The same linear for activations and outputs in HOST memory (pinned for asynchronous copies):
@@ -768,18 +781,10 @@ def w4a8_linear_host(x_host: torch.Tensor, qw_dev: dict, y_host: torch.Tensor = 
 
     The wrapper is on the per-layer critical path of a host-driven decode loop, so it caches what does
     not change between calls (buffer sizes per shape, the scratch per stream) and does no tensor work."""
-    if x_host.is_cuda or x_host.dim() != 2 or not x_host.is_contiguous() or x_host.dtype not in _DTYPE_CODES:
-        raise RuntimeError("liquidgemm_b200: x_host must be a contiguous CPU [M,K] tensor of bf16, fp16 or fp32")
-    M, K = x_host.shape
-    N = qw_dev["N"]
     odt = out_dtype or x_host.dtype
-    if K != qw_dev["K"] or K % 128:
-        raise RuntimeError("liquidgemm_b200: K mismatch or K % 128 != 0")
+    M, N, K = _check_host_request(x_host, qw_dev, y_host, odt)
     if y_host is None:
         y_host = torch.empty((M, N), dtype=odt, pin_memory=True)
-    elif y_host.is_cuda or y_host.dtype != odt or y_host.shape[0] != M or y_host.shape[1] != N or \
-            not y_host.is_contiguous():
-        raise RuntimeError("liquidgemm_b200: y_host must be a contiguous CPU [M,N] tensor of the output dtype")
     if M == 0:
         return y_host
     blob, s1 = qw_dev["rs"], qw_dev["s1"]
@@ -861,7 +866,13 @@ class HostStepPlan:
             raise RuntimeError("liquidgemm_b200: HostStepPlan needs at least one request")
         self.requests = list(requests)
         dev = torch.device(device) if device is not None else self.requests[0][1]["rs"].device
+        if dev.index is None:
+            dev = torch.device(dev.type, torch.cuda.current_device())
         self.device = dev
+        for x, L, y in self.requests:
+            _check_host_request(x, L, y, x.dtype)
+            if L["rs"].device != dev or L["s1"].device != dev:
+                raise RuntimeError("liquidgemm_b200: every layer of a HostStepPlan must be on its device")
         with torch.cuda.device(dev):
             # replays are ordered on `stream`: plans that share it run one after the other, like the steps
             # of a decode loop
@@ -883,9 +894,6 @@ class HostStepPlan:
                 self._after[kind].setdefault(j, []).append(i)
             self.tokens = [torch.empty(x.shape, dtype=x.dtype, device=dev) for x, _, _ in self.requests]
             self.outputs = [torch.empty(y.shape, dtype=y.dtype, device=dev) for _, _, y in self.requests]
-            # eager pass: checks every request and allocates the workspaces of every stream outside the capture
-            for i, (x, L, y) in enumerate(self.requests):
-                w4a8_linear_host(x, L, y, stream=self.side[self.assignment[i]])
             torch.cuda.synchronize()
             up, down = torch.cuda.Stream(), [torch.cuda.Stream() for _ in self.side]
             self._step(up, down)             # allocates the workspaces of every stream outside the capture

@@ -60,3 +60,26 @@ def test_requests_that_share_memory_run_in_order(n_streams):
         assert torch.equal(mid, h.cpu()) and torch.equal(end, last.cpu())
         assert torch.equal(x, ops.w4a8_linear(last, down).cpu())
     ops.poll_status()
+
+
+def test_construction_leaves_no_scratch_by_stream():
+    from liquidgemm_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(19)
+    kept = {k: t.data_ptr() for d in (ops._HOST_SCRATCH, ops._HOST_PLANES) for k, t in d.items()}
+    x, y = torch.randn(40, 2048).half().pin_memory(), _pinned(40, 512)
+    L = _layer(512, 2048, g)
+    plan = ops.HostStepPlan([(x, L, y)], n_streams=5)
+    assert torch.equal(y, ops.w4a8_linear(x.cuda(), L).cpu())     # construction has run the step once
+    assert kept == {k: t.data_ptr() for d in (ops._HOST_SCRATCH, ops._HOST_PLANES) for k, t in d.items()}
+    del plan
+
+
+def test_refused_requests():
+    from liquidgemm_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(17)
+    L = _layer(128, 256, g)
+    good = (_pinned(2, 256), L, _pinned(2, 128))
+    for bad in ((_pinned(2, 128), L, _pinned(2, 128)), (good[0], L, _pinned(3, 128)), (good[0].cuda(), L, good[2]),
+                (good[0], L, good[2].float()), (good[0], {**L, "s1": L["s1"].cpu()}, good[2])):
+        with pytest.raises(RuntimeError):
+            ops.HostStepPlan([good, bad])
