@@ -17,6 +17,7 @@ from __future__ import annotations
 import os
 
 import ctypes
+import weakref
 
 import torch
 
@@ -256,6 +257,7 @@ def _splitk_for(M, N, K):
 # captured graph may still point at them.
 _WORKSPACES: dict = {}
 _RETIRED: list = []
+_PLANS: "weakref.WeakSet" = weakref.WeakSet()   # HostStepPlans: each has zero-filled workspaces of its own
 
 
 def _workspace(nbytes: int, device: torch.device, stream=None):
@@ -275,7 +277,7 @@ def poll_status(device=None) -> None:
     """Read (and clear) the device-side status word of ``device`` (default: the current one) after
     synchronising its current stream.  Kernels never hang: a bounded wait that gives up records a site code
     there and the kernel finishes, possibly with partial sums left in the shared reduction workspaces.  When
-    the word is set this function therefore clears every cached workspace of the device and raises
+    the word is set this function therefore clears every cached workspace (and every plan's) of the device and raises
     :class:`liquidgemm_b200._lib.LiquidGemmError`; call it wherever a wrong result must not go unnoticed
     (after a benchmark, between serving batches, in tests)."""
     dev = torch.cuda.current_device() if device is None else torch.device(device).index
@@ -285,6 +287,10 @@ def poll_status(device=None) -> None:
             for (d, _), ws in list(_WORKSPACES.items()):
                 if d == dev:
                     ws.zero_()
+            for plan in list(_PLANS):
+                if plan.device.index == dev:
+                    for ws in plan.zeroed:
+                        ws.zero_()
             torch.cuda.synchronize()
         check(rc, "poll_status")
 
@@ -407,12 +413,17 @@ def _linear(x, w, s_u8, off_a, s1, bias, N, K, group_size, out_dtype):
     return y
 
 
-def _linear_call(x, code, w, s1, bias, y, out_dtype, M, N, K, dev, splitk=None):
-    S = (_splitk_for(M, N, K) if _SPLITK_ENV else 0) if splitk is None else splitk
-    px = x.data_ptr()
+def _linear_sizes(px, M, N, K, splitk):
+    """Scratch bytes, workspace bytes and workspace kind of ``lq_w4a8_linear`` for activations at ``px``."""
     plan = (ctypes.c_size_t * 3)()
-    check(lib.lq_linear_plan(px, M, N, K, S, plan), "w4a8_linear")
-    nscratch, nws, kind = plan
+    check(lib.lq_linear_plan(px, M, N, K, splitk, plan), "w4a8_linear")
+    return plan
+
+
+def _linear_call(x, code, w, s1, bias, y, out_dtype, M, N, K, dev):
+    S = _splitk_for(M, N, K) if _SPLITK_ENV else 0
+    px = x.data_ptr()
+    nscratch, nws, kind = _linear_sizes(px, M, N, K, S)
     stream = _stream()
     scratch = torch.empty((nscratch,), dtype=torch.uint8, device=dev) if nscratch else None
     if kind == 1:
@@ -859,7 +870,8 @@ class HostStepPlan:
     :meth:`run` replays the step: the host pays for one launch instead of four to five driver calls per linear,
     which is what a step of 5-20 us kernels is otherwise dominated by.  The host buffers are read and written in
     place on every replay; call :meth:`synchronize` before reading the outputs.  Plans built on the same ``stream``
-    replay in order.  (The reference drives every linear from Python, one operator call at a time: liquidgemm/vllm_plugin.py:174-206.)"""
+    replay in order, plans on different streams may replay side by side: every device buffer belongs to one plan.
+    (The reference drives every linear from Python, one operator call at a time: liquidgemm/vllm_plugin.py:174-206.)"""
 
     def __init__(self, requests, n_streams: int = 3, device=None, stream: "torch.cuda.Stream" = None):
         if not requests:
@@ -892,11 +904,22 @@ class HostStepPlan:
             self._after = {"yx": {}, "xy": {}, "yy": {}}   # kind -> request -> earlier requests it waits for
             for kind, i, j in _overlaps(self.requests):
                 self._after[kind].setdefault(j, []).append(i)
+            # Device buffers of the plan alone: streams are pooled, so buffers kept by stream would be shared by plans
+            # that may replay side by side.  Allocated outside the capture (a graph's private pool costs milliseconds).
             self.tokens = [torch.empty(x.shape, dtype=x.dtype, device=dev) for x, _, _ in self.requests]
             self.outputs = [torch.empty(y.shape, dtype=y.dtype, device=dev) for _, _, y in self.requests]
+            self._sizes = [tuple(_linear_sizes(t.data_ptr(), t.shape[0], L["N"], L["K"], 0)) if t.shape[0] else (0, 0, 0)
+                           for t, (_, L, _) in zip(self.tokens, self.requests)]
+            nscratch, nzeroed = [0] * len(self.side), [0] * len(self.side)
+            for (ns, nws, kind), k in zip(self._sizes, self.assignment):
+                nscratch[k] = max(nscratch[k], (ns + 255) // 256 * 256 + (nws if kind == 1 else 0))
+                nzeroed[k] = max(nzeroed[k], nws if kind == 2 else 0)
+            self.scratch = [torch.empty((n,), dtype=torch.uint8, device=dev) for n in nscratch]
+            self.zeroed = [torch.zeros((n,), dtype=torch.uint8, device=dev) for n in nzeroed]
+            _PLANS.add(self)
             torch.cuda.synchronize()
             up, down = torch.cuda.Stream(), [torch.cuda.Stream() for _ in self.side]
-            self._step(up, down)             # allocates the workspaces of every stream outside the capture
+            self._step(up, down)             # loads every kernel, so that the capture finds them loaded
             torch.cuda.synchronize()
             self.graph = torch.cuda.CUDAGraph()
             with torch.cuda.graph(self.graph, stream=self.main):
@@ -944,12 +967,14 @@ class HostStepPlan:
 
     def _linear(self, i):
         """Enqueue request ``i``'s linear on its stream, between the plan's device buffers."""
-        x, y = self.tokens[i], self.outputs[i]
-        L = self.requests[i][1]
+        x, y, k = self.tokens[i], self.outputs[i], self.assignment[i]
+        L, (ns, nws, kind) = self.requests[i][1], self._sizes[i]
         if x.shape[0]:
-            with torch.cuda.stream(self.side[self.assignment[i]]):
-                _linear_call(x, _DTYPE_CODES[x.dtype], L["rs"], L["s1"], None, y, _DTYPE_CODES[y.dtype], x.shape[0], L["N"],
-                             L["K"], self.device, splitk=0)
+            scratch = self.scratch[k].data_ptr()
+            ws = scratch + (ns + 255) // 256 * 256 if kind == 1 else self.zeroed[k].data_ptr()
+            check(lib.lq_w4a8_linear(x.data_ptr(), _DTYPE_CODES[x.dtype], L["rs"].data_ptr(), L["s1"].data_ptr(), None,
+                                     y.data_ptr(), _DTYPE_CODES[y.dtype], x.shape[0], L["N"], L["K"], 0, scratch or None, ns,
+                                     ws or None, nws, self.side[k].cuda_stream), "HostStepPlan")
 
     def run(self) -> None:
         """Enqueue the whole step (on the plan's own stream)."""

@@ -83,3 +83,27 @@ def test_refused_requests():
                 (good[0], L, good[2].float()), (good[0], {**L, "s1": L["s1"].cpu()}, good[2])):
         with pytest.raises(RuntimeError):
             ops.HostStepPlan([good, bad])
+
+
+def test_plans_own_their_buffers():
+    """Plans on streams of their own replay side by side without sharing a reduction workspace, however many there are
+    (stream handles are pooled)."""
+    from liquidgemm_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(11)
+    layers = [_layer(1024, 4096, g) for _ in range(4)]
+    kept = {k: t.data_ptr() for k, t in ops._WORKSPACES.items()}
+    plans = []
+    for _ in range(12):
+        req = [(torch.randn(1, 4096).half().pin_memory(), L, _pinned(1, 1024)) for L in layers]
+        plans.append((ops.HostStepPlan(req), req))
+    assert kept == {k: t.data_ptr() for k, t in ops._WORKSPACES.items()}
+    owned = [t.data_ptr() for p, _ in plans for t in (*p.tokens, *p.outputs, *p.scratch, *p.zeroed) if t.numel()]
+    assert len(set(owned)) == len(owned)
+    want = [[ops.w4a8_linear(x.cuda(), L).cpu() for x, L, _ in req] for _, req in plans]
+    for _ in range(20):
+        for p, _ in plans:
+            p.run()
+    torch.cuda.synchronize()
+    for (_, req), w in zip(plans, want):
+        assert all(torch.equal(y, e) for (_, _, y), e in zip(req, w))
+    ops.poll_status()
