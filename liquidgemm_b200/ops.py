@@ -870,8 +870,9 @@ class HostStepPlan:
     :meth:`run` replays the step: the host pays for one launch instead of four to five driver calls per linear,
     which is what a step of 5-20 us kernels is otherwise dominated by.  The host buffers are read and written in
     place on every replay; call :meth:`synchronize` before reading the outputs.  Plans built on the same ``stream``
-    replay in order, plans on different streams may replay side by side: every device buffer belongs to one plan.
-    (The reference drives every linear from Python, one operator call at a time: liquidgemm/vllm_plugin.py:174-206.)"""
+    replay in order, plans on different streams may replay side by side: every device buffer belongs to one plan, and
+    dropping a plan returns them once its last replay has finished.  (The reference drives every linear from Python, one
+    operator call at a time: liquidgemm/vllm_plugin.py:174-206.)"""
 
     def __init__(self, requests, n_streams: int = 3, device=None, stream: "torch.cuda.Stream" = None):
         if not requests:
@@ -916,6 +917,8 @@ class HostStepPlan:
                 nzeroed[k] = max(nzeroed[k], nws if kind == 2 else 0)
             self.scratch = [torch.empty((n,), dtype=torch.uint8, device=dev) for n in nscratch]
             self.zeroed = [torch.zeros((n,), dtype=torch.uint8, device=dev) for n in nzeroed]
+            for t in (*self.tokens, *self.outputs, *self.scratch, *self.zeroed):
+                t.record_stream(self.main)   # freed buffers wait for the replays in flight
             _PLANS.add(self)
             torch.cuda.synchronize()
             up, down = torch.cuda.Stream(), [torch.cuda.Stream() for _ in self.side]

@@ -107,3 +107,24 @@ def test_plans_own_their_buffers():
     for (_, req), w in zip(plans, want):
         assert all(torch.equal(y, e) for (_, _, y), e in zip(req, w))
     ops.poll_status()
+
+
+def test_a_dropped_plan_keeps_its_buffers_until_its_replays_end():
+    from liquidgemm_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(13)
+    layers = [_layer(4096, 4096, g) for _ in range(6)]
+    req = [(torch.randn(40, 4096).half().pin_memory(), L, _pinned(40, 4096)) for L in layers]
+    want = [ops.w4a8_linear(x.cuda(), L).cpu() for x, L, _ in req]
+    plan = ops.HostStepPlan(req)
+    for _, _, y in req:
+        y.zero_()
+    main = plan.main
+    torch.cuda.synchronize()
+    for _ in range(20):
+        plan.run()
+    del plan
+    # blocks of the plan's sizes, filled on the stream they were allocated from
+    junk = [torch.full((40, 4096), 99.0, dtype=torch.float16, device="cuda") for _ in range(24)]
+    main.synchronize()
+    assert all(torch.equal(y, e) for (_, _, y), e in zip(req, want))
+    del junk
