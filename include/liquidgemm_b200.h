@@ -249,13 +249,6 @@ LQ_API int lq_gemm_launches(int M, int N, int K, int splitk);
 LQ_API int lq_w4a8_gemm_i32(const int8_t* x_i8, const uint8_t* blob, int32_t* acc, int M, int N, int K,
                      int splitk, void* workspace, size_t workspace_bytes, void* stream);
 
-/* The same for a blob that the work directly before on `stream` writes (weights re-tiled for one product).  The other
- * W4A8 calls fetch the first tiles of the blob while the previous kernel of the stream may still run, so their blob has to
- * be settled: written by lq_repack_tiles or lq_quantize_weight (whose kernels publish it before they end), copied, or
- * separated from the call by any kernel launched without programmatic serialisation. */
-LQ_API int lq_w4a8_gemm_i32_ordered(const int8_t* x_i8, const uint8_t* blob, int32_t* acc, int M, int N, int K,
-                     int splitk, void* workspace, size_t workspace_bytes, void* stream);
-
 /* W4A8 tensor-core GEMM with the fused (split-K reduce +) scale + cast epilogue.
  * Replaces torch.ops.liquidgemm.w4a8_wgmma_rs_fused
  * (reference csrc/liquid_gemm/w4a8_wgmma.cu:575-645). */

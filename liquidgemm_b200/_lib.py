@@ -59,7 +59,6 @@ _SIGNATURES = {
     "lq_w4a8_linear": (c_int, [P, c_int, P, P, P, P, c_int, c_int, c_int, c_int, c_int, P, c_size_t, P, c_size_t, P]),
     "lq_quantize_weight": (c_int, [P, c_int, c_int, c_int, c_int, P, P, P, P, P, P]),
     "lq_w4a8_gemm_i32": (c_int, [P, P, P, c_int, c_int, c_int, c_int, P, c_size_t, P]),
-    "lq_w4a8_gemm_i32_ordered": (c_int, [P, P, P, c_int, c_int, c_int, c_int, P, c_size_t, P]),
     "lq_w4a8_gemm_fused": (c_int, [P, P, P, P, P, c_int, c_int, c_int, c_int, c_int, P, c_size_t, P]),
     "lq_i8_gemm_i32": (c_int, [P, P, P, c_int, c_int, c_int, P]),
     "lq_i8_gemm_scaled": (c_int, [P, P, P, P, P, c_int, c_int, c_int, c_int, P]),

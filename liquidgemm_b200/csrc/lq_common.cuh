@@ -20,14 +20,14 @@ int* status_word();                                         // lq_api.cu: device
 
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
-// Launch with programmatic stream serialisation (`overlapped`): the kernel may start while the previous kernel
+// Launch with programmatic stream serialisation: the kernel may start while the previous kernel
 // of the stream is still draining, and must execute griddepcontrol.wait (dependency_wait()) before
 // it touches anything an earlier kernel may have written or may still read-modify-write.  Switched
 // off with LIQUIDGEMM_PDL=0 (then this is an ordinary launch).
 bool pdl_enabled();                                         // lq_api.cu
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_kernel(bool overlapped, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                                 cudaStream_t st, Args... args) {
+inline cudaError_t launch_overlapped(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                     Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -37,13 +37,8 @@ inline cudaError_t launch_kernel(bool overlapped, void (*kern)(KArgs...), dim3 g
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = overlapped && pdl_enabled() ? 1 : 0;
+  cfg.numAttrs = pdl_enabled() ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kern, args...);
-}
-template <typename... KArgs, typename... Args>
-inline cudaError_t launch_overlapped(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                                     Args... args) {
-  return launch_kernel(true, kern, grid, block, smem, st, args...);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -514,7 +514,7 @@ w4a8_decode_tc_kernel(const Args args, const std::conditional_t<MULTI, MultiOut,
 }
 
 template <int BN, int NW, int NT, bool MULTI>
-static int launch(const Args& a, const MultiOut* multi, int grid, bool overlapped, cudaStream_t st) {
+static int launch(const Args& a, const MultiOut* multi, int grid, cudaStream_t st) {
   using C = Cfg<BN, NW, NT>;
   auto kern = &w4a8_decode_tc_kernel<BN, NW, NT, MULTI>;
   static std::once_flag once[64];
@@ -525,8 +525,8 @@ static int launch(const Args& a, const MultiOut* multi, int grid, bool overlappe
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
   });
   if (e == cudaSuccess) {
-    if constexpr (MULTI) e = launch_kernel(overlapped, kern, dim3(grid), dim3(kThreads), (size_t)C::kSmemBytes, st, a, *multi);
-    else e = launch_kernel(overlapped, kern, dim3(grid), dim3(kThreads), (size_t)C::kSmemBytes, st, a, NoMultiOut{});
+    if constexpr (MULTI) e = launch_overlapped(kern, dim3(grid), dim3(kThreads), (size_t)C::kSmemBytes, st, a, *multi);
+    else e = launch_overlapped(kern, dim3(grid), dim3(kThreads), (size_t)C::kSmemBytes, st, a, NoMultiOut{});
   }
   if (e != cudaSuccess) {
     record_cuda_error(e, "w4a8_decode_tc_kernel launch");
@@ -552,10 +552,9 @@ size_t decode_tc_workspace_bytes(int M, int N, int K) {
 }
 
 // out_mode: LQ_DT_* or 3 (raw int32).  M <= 32.  `ws`: decode_tc_workspace_bytes(), all zero, left all zero.
-// `overlapped` as for run_tile_gemm.
 int run_decode_tc(const int8_t* x, const uint8_t* blob, const float* ascale, const float* s1, const void* bias,
                   const OutSpec& out, const PeerSync* sync, int out_mode, int M, int N, int K, void* ws,
-                  size_t ws_bytes, cudaStream_t st, bool overlapped) {
+                  size_t ws_bytes, cudaStream_t st) {
   using namespace dtc;
   if (M < 1 || M > 32) return LQ_ERR_SHAPE;
   if (!ws || ws_bytes < decode_tc_workspace_bytes(M, N, K)) return LQ_ERR_WORKSPACE;
@@ -581,14 +580,14 @@ int run_decode_tc(const int8_t* x, const uint8_t* blob, const float* ascale, con
   a.fixed_split = plan.fixed_split;
   if (!a.status) return LQ_ERR_CUDA;
   if (!multi) {
-    if (bn == 16) return launch<16, 8, 7, false>(a, nullptr, grid, overlapped, st);
-    return launch<32, 8, 6, false>(a, nullptr, grid, overlapped, st);
+    if (bn == 16) return launch<16, 8, 7, false>(a, nullptr, grid, st);
+    return launch<32, 8, 6, false>(a, nullptr, grid, st);
   }
   MultiOut mo;
   mo.out = out;
   mo.sync = sync ? *sync : PeerSync{};
-  if (bn == 16) return launch<16, 8, 7, true>(a, &mo, grid, overlapped, st);
-  return launch<32, 8, 6, true>(a, &mo, grid, overlapped, st);
+  if (bn == 16) return launch<16, 8, 7, true>(a, &mo, grid, st);
+  return launch<32, 8, 6, true>(a, &mo, grid, st);
 }
 
 }  // namespace lq

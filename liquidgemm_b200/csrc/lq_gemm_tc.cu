@@ -56,12 +56,12 @@ int tile_pick_splits(int M, int N, int K);                                   // 
 size_t tile_workspace_bytes(int M, int N, int splits);                       // lq_gemm_tile.cu
 int run_tile_gemm(const int8_t* x, const uint8_t* blob, const float* ascale, const float* s1, const void* bias,
                   const OutSpec& out, const PeerSync* sync, int out_mode, int M, int N, int K, int splits, void* ws,
-                  size_t ws_bytes, cudaStream_t st, bool overlapped = true);  // lq_gemm_tile.cu
+                  size_t ws_bytes, cudaStream_t st);  // lq_gemm_tile.cu
 int tile_output_grid(int M, int N, int K, int splits);                            // lq_gemm_tile.cu
 size_t decode_tc_workspace_bytes(int M, int N, int K);                       // lq_decode_tc.cu
 int run_decode_tc(const int8_t* x, const uint8_t* blob, const float* ascale, const float* s1, const void* bias,
                   const OutSpec& out, const PeerSync* sync, int out_mode, int M, int N, int K, void* ws,
-                  size_t ws_bytes, cudaStream_t st, bool overlapped = true);  // lq_decode_tc.cu
+                  size_t ws_bytes, cudaStream_t st);  // lq_decode_tc.cu
 size_t gemv_blob_workspace_bytes(int N, int K);                              // lq_gemv_blob.cu
 int run_gemv_blob_ws(const int8_t* x, const uint8_t* blob, const float* ascale, const float* s1, const void* bias,
                      const OutSpec& out, const PeerSync* sync, int out_dtype, int M, int N, int K, void* ws,
@@ -797,10 +797,9 @@ int lq_gemm_launches(int M, int N, int K, int splitk) {
   return ((r.kind == kRouteTile && r.splits > 1) || r.kind == kRouteUnpackI8) ? 2 : 1;
 }
 
-// `overlapped` as for run_tile_gemm; the kernels of the other int32 routes read no weight before they have waited.
 static int blob_gemm(const int8_t* x, const uint8_t* blob, const float* ascale, const float* s1, const void* bias,
                      void* out, int out_mode, int M, int N, int K, int splitk, void* ws, size_t ws_bytes,
-                     cudaStream_t st, bool overlapped = true) {
+                     cudaStream_t st) {
   if (!x || !blob || !out || M < 0 || N <= 0 || K <= 0) return LQ_ERR_BAD_ARG;
   if (K % 128) return LQ_ERR_SHAPE;
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(blob)) % 16) return LQ_ERR_BAD_ARG;
@@ -813,11 +812,10 @@ static int blob_gemm(const int8_t* x, const uint8_t* blob, const float* ascale, 
     case kRouteGemv:
       return run_gemv_blob_ws(x, blob, ascale, s1, bias, single_out(out, N), nullptr, out_mode, M, N, K, ws, ws_bytes, st);
     case kRouteDecodeTc:
-      return run_decode_tc(x, blob, ascale, s1, bias, single_out(out, N), nullptr, out_mode, M, N, K, ws, ws_bytes, st,
-                           overlapped);
+      return run_decode_tc(x, blob, ascale, s1, bias, single_out(out, N), nullptr, out_mode, M, N, K, ws, ws_bytes, st);
     case kRouteTile:
       return run_tile_gemm(x, blob, ascale, s1, bias, single_out(out, N), nullptr, out_mode, M, N, K, r.splits, ws,
-                           ws_bytes, st, overlapped);
+                           ws_bytes, st);
     case kRoutePair:
       return run_pair_gemm(x, blob, ascale, s1, bias, single_out(out, N), nullptr, out_mode, M, N, K, ws, ws_bytes, st);
     case kRouteUnpackI8: {
@@ -836,12 +834,6 @@ int lq_w4a8_gemm_i32(const int8_t* x_i8, const uint8_t* blob, int32_t* acc, int 
                      void* workspace, size_t workspace_bytes, void* stream) {
   return blob_gemm(x_i8, blob, nullptr, nullptr, nullptr, acc, kOutI32, M, N, K, splitk, workspace, workspace_bytes,
                    as_stream(stream));
-}
-
-int lq_w4a8_gemm_i32_ordered(const int8_t* x_i8, const uint8_t* blob, int32_t* acc, int M, int N, int K, int splitk,
-                             void* workspace, size_t workspace_bytes, void* stream) {
-  return blob_gemm(x_i8, blob, nullptr, nullptr, nullptr, acc, kOutI32, M, N, K, splitk, workspace, workspace_bytes,
-                   as_stream(stream), false);
 }
 
 int lq_w4a8_gemm_fused(const int8_t* x_i8, const uint8_t* blob, const float* ascale, const float* s1, void* y,

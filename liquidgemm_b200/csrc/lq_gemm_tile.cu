@@ -391,8 +391,7 @@ w4a8_tile_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmArgs args
 }
 
 template <int BN, int NS, int NT, bool W4, bool MULTI>
-static int launch_one(const CUtensorMap& tx, const GemmArgs& a, const MultiOut* multi, int splits, bool overlapped,
-                      cudaStream_t st) {
+static int launch_one(const CUtensorMap& tx, const GemmArgs& a, const MultiOut* multi, int splits, cudaStream_t st) {
   using Cfg = TcCfg<BN, NS, NT, W4>;
   auto kern = &w4a8_tile_kernel<BN, NS, NT, W4, MULTI>;
   static std::once_flag once[64];
@@ -408,8 +407,8 @@ static int launch_one(const CUtensorMap& tx, const GemmArgs& a, const MultiOut* 
   }
   dim3 grid((a.N + 127) / 128, (a.M + BN - 1) / BN, splits);
   cudaError_t le;
-  if constexpr (MULTI) le = launch_kernel(overlapped, kern, grid, dim3(kThreads), (size_t)Cfg::kSmemBytes, st, tx, a, *multi);
-  else le = launch_kernel(overlapped, kern, grid, dim3(kThreads), (size_t)Cfg::kSmemBytes, st, tx, a, NoMultiOut{});
+  if constexpr (MULTI) le = launch_overlapped(kern, grid, dim3(kThreads), (size_t)Cfg::kSmemBytes, st, tx, a, *multi);
+  else le = launch_overlapped(kern, grid, dim3(kThreads), (size_t)Cfg::kSmemBytes, st, tx, a, NoMultiOut{});
   if (le != cudaSuccess) {
     record_cuda_error(le, "w4a8_tile_kernel launch");
     return LQ_ERR_CUDA;
@@ -418,10 +417,9 @@ static int launch_one(const CUtensorMap& tx, const GemmArgs& a, const MultiOut* 
 }
 
 template <int BN, int NS, int NT, bool W4>
-static int launch_cfg(const CUtensorMap& tx, const GemmArgs& a, const MultiOut* multi, int splits, bool overlapped,
-                      cudaStream_t st) {
-  if (multi) return launch_one<BN, NS, NT, W4, true>(tx, a, multi, splits, overlapped, st);
-  return launch_one<BN, NS, NT, W4, false>(tx, a, nullptr, splits, overlapped, st);
+static int launch_cfg(const CUtensorMap& tx, const GemmArgs& a, const MultiOut* multi, int splits, cudaStream_t st) {
+  if (multi) return launch_one<BN, NS, NT, W4, true>(tx, a, multi, splits, st);
+  return launch_one<BN, NS, NT, W4, false>(tx, a, nullptr, splits, st);
 }
 
 // Token-tile widths: the smallest that holds a decode batch, 128 tokens for prefill.  A 192-token
@@ -479,11 +477,10 @@ int tile_output_grid(int M, int N, int K, int splits) {
 }
 
 // out_mode: LQ_DT_* or 3 (raw int32).  Any M.  `ws` holds `splits` int32 planes (need not be zeroed).
-// `out`: one or several destinations (gather by stores); `sync`: optional cross-GPU flags.  `overlapped`: the first weight
-// tiles are read before the previous kernel of the stream is waited for, so not for a blob which that kernel writes.
+// `out`: one or several destinations (gather by stores); `sync`: optional cross-GPU flags.
 int run_tile_gemm(const int8_t* x, const uint8_t* blob, const float* ascale, const float* s1, const void* bias,
                   const OutSpec& out, const PeerSync* sync, int out_mode, int M, int N, int K, int splits, void* ws,
-                  size_t ws_bytes, cudaStream_t st, bool overlapped) {
+                  size_t ws_bytes, cudaStream_t st) {
   using namespace tile;
   if (splits > 1 && (!ws || ws_bytes < tile_workspace_bytes(M, N, splits))) return LQ_ERR_WORKSPACE;
   const int bn = tile_bn(M, N, K);
@@ -527,10 +524,10 @@ int run_tile_gemm(const int8_t* x, const uint8_t* blob, const float* ascale, con
     // 16 tokens: 8 stages, 4 operand stages (95 KB, two CTAs per SM).  Five stages and two operand stages, so
     // that three CTAs fit an SM and the next launch's CTAs can start beside this one's, measured 30 % slower
     // on 28672 x 4096 (19.2 vs 14.8 us) and 9 % slower on 4096 x 14336.
-    case 16: rc = launch_cfg<16, 8, 4, true>(tx, a, mop, splits, overlapped, st); break;
-    case 32: rc = launch_cfg<32, 8, 4, true>(tx, a, mop, splits, overlapped, st); break;
-    case 64: rc = launch_cfg<64, 6, 4, true>(tx, a, mop, splits, overlapped, st); break;
-    default: rc = launch_cfg<128, 4, 4, true>(tx, a, mop, splits, overlapped, st); break;
+    case 16: rc = launch_cfg<16, 8, 4, true>(tx, a, mop, splits, st); break;
+    case 32: rc = launch_cfg<32, 8, 4, true>(tx, a, mop, splits, st); break;
+    case 64: rc = launch_cfg<64, 6, 4, true>(tx, a, mop, splits, st); break;
+    default: rc = launch_cfg<128, 4, 4, true>(tx, a, mop, splits, st); break;
   }
   if (rc || splits <= 1) return rc;
   PeerSync fsync = {};

@@ -322,19 +322,17 @@ def _check_blob(w, N, K):
     return w.contiguous()
 
 
-def gemm_i32(x_i8, blob, N, K, splitk=None, fresh=False):
+def gemm_i32(x_i8, blob, N, K, splitk=None):
     """Exact int32 accumulators from a tile blob.  ``splitk``: None = automatic (stream-K unless
-    LIQUIDGEMM_SPLITK applies), S >= 1 = that split-K factor, -1 = force the persistent stream-K kernel.
-    ``fresh``: the blob was re-tiled for this product, no part of it may be read ahead of the stream."""
+    LIQUIDGEMM_SPLITK applies), S >= 1 = that split-K factor, -1 = force the persistent stream-K kernel."""
     x_i8 = _i8(x_i8, "x_i8")
     _req(K % 128 == 0 and x_i8.shape[1] == K, "K%128==0 required and x_i8 must be [M,K]")
     blob = _check_blob(blob, N, K)
     M = x_i8.shape[0]
     acc = torch.empty((M, N), dtype=torch.int32, device=x_i8.device)
     if M:
-        fn = lib.lq_w4a8_gemm_i32_ordered if fresh else lib.lq_w4a8_gemm_i32
         _gemm_call("w4a8_gemm_i32", x_i8, M, N, K, splitk,
-                   lambda S, ws, nb, st: fn(_ptr(x_i8), _ptr(blob), _ptr(acc), M, N, K, S, ws, nb, st))
+                   lambda S, ws, nb, st: lib.lq_w4a8_gemm_i32(_ptr(x_i8), _ptr(blob), _ptr(acc), M, N, K, S, ws, nb, st))
     return acc
 
 
@@ -553,7 +551,7 @@ def _wgmma_rs(x_i8, w, spack, s_u8, off_a, N, K, group_size, packed):
         # plain pack_nibbles layout: re-tile into scratch first (reference gathers per element,
         # csrc/liquid_gemm/w4a8_wgmma.cu:424-434)
         w = _repack_device(w, 1, s_u8, off_a, N, K, group_size)
-    return gemm_i32(x_i8, w.reshape(-1), N, K, fresh=not packed)
+    return gemm_i32(x_i8, w.reshape(-1), N, K)
 
 
 def _wgmma_rs_fused(x_i8, w, s_u8, off_a, ascale, s1, N, K, group_size, out_dtype):
@@ -566,7 +564,7 @@ def _wgmma_ss(x_i8, packed, s_u8, off_a, N, K, group_size):
     _req(group_size == 64, "group_size must be 64")
     _req(K % 128 == 0, "K must be a multiple of 128")
     blob = _repack_device(packed, 1, s_u8, off_a, N, K, group_size)
-    return gemm_i32(x_i8, blob.reshape(-1), N, K, fresh=True)
+    return gemm_i32(x_i8, blob.reshape(-1), N, K)
 
 
 def _i8_workspace(a, M, N, K):
