@@ -197,6 +197,11 @@ LQ_API size_t lq_tile_blob_bytes(int N, int K);
 LQ_API int lq_repack_tiles(const uint8_t* src, int src_layout, const uint8_t* s_u8,
                     const uint8_t* offset_a, uint8_t* blob, int N, int K, int group_size,
                     void* stream);
+/* The W4A8 calls request the first tiles of their blob while the kernel before them on the stream may still run, so a
+ * blob must be settled by then.  lq_repack_tiles and lq_quantize_weight see to that themselves; a caller whose own
+ * kernel writes a blob and that wants to use it without synchronising calls lq_settle_blob() on the stream in between
+ * (one empty kernel). */
+LQ_API int lq_settle_blob(void* stream);
 
 /* LiquidQuant weight quantiser on the device: w [N, K] (w_dtype: LQ_DT_*) -> s1 [N] float32, s_u8 and
  * offset_a [N, K/group_size], and optionally codes [N, K] (one 4-bit code per byte) and / or the tile blob

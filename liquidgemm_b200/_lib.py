@@ -49,6 +49,7 @@ _SIGNATURES = {
     "lq_gemm_v1_workspace_bytes": (c_size_t, [c_int, c_int, c_int]),
     "lq_w4a8_gemm_v1": (c_int, [P, P, P, P, P, P, P, c_int, c_int, c_int, c_int, P, c_size_t, P]),
     "lq_tile_blob_bytes": (c_size_t, [c_int, c_int]),
+    "lq_settle_blob": (c_int, [P]),
     "lq_repack_tiles": (c_int, [P, c_int, P, P, P, c_int, c_int, c_int, P]),
     "lq_gemm_pick_splitk": (c_int, [c_int, c_int, c_int, c_int]),
     "lq_gemm_workspace_bytes": (c_size_t, [c_int, c_int, c_int, c_int]),

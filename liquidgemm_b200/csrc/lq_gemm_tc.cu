@@ -78,6 +78,8 @@ bool i8_stream_serves(int M, int N, int K);                                  // 
 size_t i8_stream_workspace_bytes(int M, int N, int K);
 int run_i8_stream(const int8_t* x, const int8_t* w, const float* ascale, const float* s1, void* out, int out_mode, int M,
                   int N, int K, void* ws, size_t ws_bytes, cudaStream_t st);
+int repack_tiles(const uint8_t* src, int src_layout, const uint8_t* s_u8, const uint8_t* offset_a, uint8_t* blob, int N,
+                 int K, int group_size, cudaStream_t st);   // lq_elementwise.cu
 int run_unpack_blob_i8(const uint8_t* blob, int8_t* w, int N, int K, cudaStream_t st);   // lq_elementwise.cu
 bool pair_prefers(int M, int N, int K);                                      // lq_gemm_pair.cu
 size_t pair_workspace_bytes(int M, int N, int K);                                // lq_gemm_pair.cu
@@ -1004,7 +1006,7 @@ int lq_w4a8_gemm_v1(const int8_t* x_i8, const uint8_t* nibbles, const uint8_t* s
   if (!workspace || workspace_bytes < lq_gemm_v1_workspace_bytes(M, N, K)) return LQ_ERR_WORKSPACE;
   // scratch = re-tiled weights only; whole-tile scheduling (splitk 1) needs no reduction slots
   uint8_t* blob = static_cast<uint8_t*>(workspace);
-  int rc = lq_repack_tiles(nibbles, LQ_SRC_NIBBLES, s_u8, offset_a, blob, N, K, group_size, stream);
+  int rc = repack_tiles(nibbles, LQ_SRC_NIBBLES, s_u8, offset_a, blob, N, K, group_size, st);
   if (rc) return rc;
   return run_gemm<kBlob>(x_i8, blob, ascale, s1, y, LQ_DT_F32, M, N, K, 1, nullptr, 0, st);
 }

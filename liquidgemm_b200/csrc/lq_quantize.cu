@@ -21,6 +21,9 @@
 #include "lq_common.cuh"
 
 namespace lq {
+
+int settle_blob(cudaStream_t st);   // lq_elementwise.cu
+
 namespace quantw {
 
 constexpr int kTileBytes = 8704;
@@ -307,14 +310,16 @@ static int run(const void* w, int N, long K, int group, float* s1, uint8_t* s_u8
     if (nv == 1) launch(quantise_rows_kernel<T, 1>);
     else if (nv == 2) launch(quantise_rows_kernel<T, 2>);
     else launch(quantise_rows_kernel<T, 4>);
-    return check_launch("quantise_rows_kernel");
+    if (int rc = check_launch("quantise_rows_kernel")) return rc;
+    return blob ? settle_blob(st) : LQ_OK;
   }
   row_amax_kernel<T><<<(N + 7) / 8, 256, 0, st>>>(static_cast<const T*>(w), s1, N, K);
   if (int rc = check_launch("row_amax_kernel")) return rc;
   dim3 grid((unsigned)(K >> 7), (unsigned)((N + 127) / 128));
   quantise_tiles_kernel<T><<<grid, 256, 0, st>>>(static_cast<const T*>(w), s1, s_u8, offset_a, codes, blob, status, N, K,
                                                  group);
-  return check_launch("quantise_tiles_kernel");
+  if (int rc = check_launch("quantise_tiles_kernel")) return rc;
+  return blob ? settle_blob(st) : LQ_OK;
 }
 
 }  // namespace quantw

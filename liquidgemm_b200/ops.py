@@ -319,7 +319,15 @@ def _check_blob(w, N, K):
     need = lib.lq_tile_blob_bytes(N, K)
     _req(need > 0 and w.numel() == need,
          f"w must be the tile blob of repack_rs_weight for N={N}, K={K} ({need} bytes, got {w.numel()})")
-    return w.contiguous()
+    return w if w.is_contiguous() else _compact_blob(w)
+
+
+def _compact_blob(w):
+    """A contiguous copy of a blob: written just now, so it has to settle before a kernel may fetch it early."""
+    with _dev_ctx(w):
+        w = w.contiguous()
+        check(lib.lq_settle_blob(_stream()), "settle_blob")
+    return w
 
 
 def gemm_i32(x_i8, blob, N, K, splitk=None):
@@ -360,7 +368,7 @@ def linear_bias(x_i8, blob, ascale, s1, bias, N, K, out_dtype):
     x_i8 = _i8(x_i8, "x_i8")
     _req(K % 128 == 0 and x_i8.shape[1] == K, "K%128==0 required and x_i8 must be [M,K]")
     _req(int(out_dtype) in _OUT_DTYPES, "out_dtype must be 0 (bf16), 1 (fp16) or 2 (fp32)")
-    blob = _check_blob(blob.reshape(-1), N, K)
+    blob = _check_blob(blob, N, K)
     ascale, s1 = _f32(ascale, "ascale"), _f32(s1, "s1")
     M = x_i8.shape[0]
     _req(ascale.numel() == M and s1.numel() == N, "ascale must be [M] and s1 [N]")
@@ -393,7 +401,8 @@ def _linear(x, w, s_u8, off_a, s1, bias, N, K, group_size, out_dtype):
     _req(odt is not None, "out_dtype must be 0 (bf16), 1 (fp16) or 2 (fp32)")
     _req(w.is_cuda and w.numel() == ((N + 127) // 128) * (K // 128) * TILE_BYTES and w.numel() > 0,
          f"w must be the tile blob of repack_rs_weight for N={N}, K={K} ({w.numel()} bytes)")
-    w = w.contiguous()
+    if not w.is_contiguous():
+        w = _compact_blob(w)
     s1 = _f32(s1, "s1")
     _req(s1.numel() == N, "ascale must be [M] and s1 [N]")
     if bias is not None:
@@ -551,20 +560,20 @@ def _wgmma_rs(x_i8, w, spack, s_u8, off_a, N, K, group_size, packed):
         # plain pack_nibbles layout: re-tile into scratch first (reference gathers per element,
         # csrc/liquid_gemm/w4a8_wgmma.cu:424-434)
         w = _repack_device(w, 1, s_u8, off_a, N, K, group_size)
-    return gemm_i32(x_i8, w.reshape(-1), N, K)
+    return gemm_i32(x_i8, w, N, K)
 
 
 def _wgmma_rs_fused(x_i8, w, s_u8, off_a, ascale, s1, N, K, group_size, out_dtype):
     _req(w.dtype == torch.uint8 and group_size == 64, "w must be uint8 and group_size 64")
     _req(N % 64 == 0 and K % 128 == 0, "N%64==0 and K%128==0 required")
-    return gemm_fused(x_i8, w.reshape(-1), ascale, s1, N, K, out_dtype)
+    return gemm_fused(x_i8, w, ascale, s1, N, K, out_dtype)
 
 
 def _wgmma_ss(x_i8, packed, s_u8, off_a, N, K, group_size):
     _req(group_size == 64, "group_size must be 64")
     _req(K % 128 == 0, "K must be a multiple of 128")
     blob = _repack_device(packed, 1, s_u8, off_a, N, K, group_size)
-    return gemm_i32(x_i8, blob.reshape(-1), N, K)
+    return gemm_i32(x_i8, blob, N, K)
 
 
 def _i8_workspace(a, M, N, K):

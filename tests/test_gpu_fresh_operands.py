@@ -44,8 +44,9 @@ def test_int8_weights_quantised_just_before(M, N, K, between):
     ops.poll_status()
 
 
-# CTA-pair kernel (where it serves: LQ_PAIR_ALWAYS), whole and cut last waves
-RETILED = [(2048, 4096, 1024), (700, 28672, 512)]
+# CTA-pair kernel (where it serves: LQ_PAIR_ALWAYS), whole and cut last waves; decode tensor-core kernel; tile kernel with
+# K cut and with whole tiles in several waves
+RETILED = [(2048, 4096, 1024), (700, 28672, 512), (8, 4096, 4096), (40, 1024, 4096), (100, 40064, 512)]
 
 
 @pytest.mark.parametrize("M,N,K", RETILED)
@@ -76,7 +77,7 @@ def test_weights_retiled_just_before(monkeypatch, M, N, K, op):
 
 
 @pytest.mark.parametrize("M,N,K", [(1, 4096, 4096), (8, 4096, 4096), (8, 28672, 1024), (40, 1024, 4096)])
-@pytest.mark.parametrize("writer", ["quantise", "repack"])
+@pytest.mark.parametrize("writer", ["quantise", "repack", "copy"])
 def test_blob_written_just_before(M, N, K, writer):
     """The package's own writers of tile blobs, into the same buffer with changing contents, directly before a fused
     linear that fetches its first tiles ahead of the stream."""
@@ -98,6 +99,10 @@ def test_blob_written_just_before(M, N, K, writer):
         if writer == "quantise":
             check(lib.lq_quantize_weight(ws[i & 1].data_ptr(), 0, N, K, 64, s1.data_ptr(), s.data_ptr(), a.data_ptr(), None,
                                          blob.data_ptr(), st), "quantize_weight")
+        elif writer == "copy":   # a blob that the operator itself has to make contiguous
+            y = ops.gemm_fused(x8, settled[i & 1][1].reshape(-1).repeat_interleave(2)[::2], sx, qw.s1, N, K, 0)
+            assert torch.equal(y, want[i & 1]), i
+            continue
         else:
             check(lib.lq_repack_tiles(qw.qweight_u4.data_ptr(), 0, qw.s_u8.data_ptr(), qw.offset_a.data_ptr(),
                                       blob.data_ptr(), N, K, 64, st), "repack_tiles")
