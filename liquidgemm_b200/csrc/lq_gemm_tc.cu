@@ -711,12 +711,16 @@ static bool pair_forced() {   // read at every call: a test sets and clears it i
   return e && atoi(e) != 0;
 }
 
-static bool gemv_serves(int M, int N, int K) {
-  static const int cap = []() {   // LQ_GEMV_MAX_M (0..4) lowers the limit for measurements
+static int gemv_max_m() {   // LQ_GEMV_MAX_M (0..4) lowers the limit of both forms of the GEMV for measurements
+  static const int cap = []() {
     const char* e = getenv("LQ_GEMV_MAX_M");
     return e ? atoi(e) : kGemvBlobMaxM;
   }();
-  if (M > cap) return false;
+  return cap;
+}
+
+static bool gemv_serves(int M, int N, int K) {
+  if (M > gemv_max_m()) return false;
   const long w = (long)N * K;
   return M == 1 || (M == 2 && w <= (1L << 26)) || (M <= kGemvBlobMaxM && w <= (1L << 24));
 }
@@ -857,7 +861,7 @@ int lq_w4a8_linear_bias(const int8_t* x_i8, const uint8_t* blob, const float* as
 
 // ---- one call from activations to outputs -------------------------------------------------------------------------
 static bool quantises_in_gemv(const void* x, int M, int N, int K, int splitk) {
-  return splitk == 0 && gemv_quant_serves(M, N, K) && reinterpret_cast<uintptr_t>(x) % 16 == 0;
+  return splitk == 0 && M <= gemv_max_m() && gemv_quant_serves(M, N, K) && reinterpret_cast<uintptr_t>(x) % 16 == 0;
 }
 
 static size_t token_scratch_bytes(int M, int K) { return (((size_t)M * K + 255) & ~(size_t)255) + (size_t)M * 4; }
