@@ -1023,7 +1023,8 @@ static bool i8_pair_enabled() {
 
 enum I8Route { kI8Pair, kI8Stream, kI8Persistent };
 static I8Route i8_route(int M, int N, int K) {
-  if (i8_pair_serves(M, N, K) && i8_pair_enabled()) return kI8Pair;
+  if (!i8_pair_enabled()) return kI8Persistent;
+  if (i8_pair_serves(M, N, K)) return kI8Pair;
   return i8_stream_serves(M, N, K) ? kI8Stream : kI8Persistent;   // lq_i8_stream.cu
 }
 

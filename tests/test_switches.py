@@ -21,3 +21,13 @@ def test_gemv_limit_reaches_the_quantising_form(limit, two_launches):
     out = subprocess.run([sys.executable, "-c", PROBE], env=env, cwd=root, capture_output=True, text=True, timeout=300)
     assert out.returncode == 0, out.stderr
     assert out.stdout.strip() == str(two_launches)
+
+
+@pytest.mark.parametrize("M,N,K", [(8, 4096, 4096), (200, 1024, 4096)])
+def test_i8_pair_switch_keeps_the_persistent_kernel(monkeypatch, M, N, K):
+    """The streaming kernel cuts these layers and needs a workspace for it; the persistent kernel needs none."""
+    from liquidgemm_b200._lib import lib
+    monkeypatch.delenv("LQ_I8_PAIR", raising=False)
+    assert lib.lq_i8_workspace_bytes(M, N, K) > 0
+    monkeypatch.setenv("LQ_I8_PAIR", "0")
+    assert lib.lq_i8_workspace_bytes(M, N, K) == 0
