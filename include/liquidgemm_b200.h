@@ -295,7 +295,8 @@ LQ_API int lq_i8_gemm_scaled(const int8_t* a, const int8_t* b, const float* a_sc
                       const float* b_scale, void* y, int out_dtype, int M, int N, int K,
                       void* stream);
 
-/* The same two with `workspace` (lq_i8_workspace_bytes(M, N, K) of scratch, any content; null and 0 where that is 0):
+/* The same two with `workspace` (lq_i8_workspace_bytes(M, N, K) of 4-byte aligned scratch, any content; null and 0 where
+ * that is 0; below 16-byte alignment the parts are added up more slowly):
  * batches below the CTA-pair kernel's sizes then run on a streaming kernel that may cut the layer's K and add the
  * parts up through it.  Results are bit-identical. */
 LQ_API size_t lq_i8_workspace_bytes(int M, int N, int K);

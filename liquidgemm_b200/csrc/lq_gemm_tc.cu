@@ -1044,6 +1044,7 @@ static int i8_common(const int8_t* a, const int8_t* b, const float* a_scale, con
     return run_i8_pair_gemm(a, b, a_scale, b_scale, nullptr, out, out_mode, M, N, K, as_stream(stream));
   // without the workspace of the split streaming kernel (the plain entry points): whole tiles, one CTA per SM
   if (r == kI8Stream && ws_bytes >= i8_stream_workspace_bytes(M, N, K)) {
+    if (reinterpret_cast<uintptr_t>(ws) & 3) return LQ_ERR_WORKSPACE;   // int32 planes
     if (int rc = lq_check_device()) return rc;
     return run_i8_stream(a, b, a_scale, b_scale, out, out_mode, M, N, K, ws, ws_bytes, as_stream(stream));
   }
