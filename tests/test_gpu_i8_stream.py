@@ -35,8 +35,9 @@ def test_matches_exact_sums(M, N, K):
 
 
 @pytest.mark.parametrize("M", [4, 100])
-def test_more_tiles_than_cta_slots(M):
-    """Whole tiles in more than one wave, and the same bits from the entry point that takes no workspace."""
+def test_more_tiles_than_cta_slots(monkeypatch, M):
+    """Whole tiles in more than one wave (the streaming kernel at 4 tokens, the persistent one at 100), the same bits from
+    the entry point that takes no workspace, and from the persistent kernel at both."""
     from liquidgemm_b200 import ops
     from liquidgemm_b200._lib import lib, check
     N, K = 40000, 384
@@ -47,4 +48,6 @@ def test_more_tiles_than_cta_slots(M):
     c = torch.empty(M, N, dtype=torch.int32, device="cuda")
     check(lib.lq_i8_gemm_i32(at.data_ptr(), bt.data_ptr(), c.data_ptr(), M, N, K, torch.cuda.current_stream().cuda_stream), "i8")
     assert np.array_equal(c.cpu().numpy(), acc)
+    monkeypatch.setenv("LQ_I8_PAIR", "0")
+    assert np.array_equal(torch.ops.liquidgemm.wgmma_i8_gemm(at, bt).cpu().numpy(), acc)
     ops.poll_status()

@@ -39,6 +39,15 @@ def _two_calls(x, L, bias, code):
     return torch.ops.liquidgemm.w4a8_linear_bias(xq, L["rs"], sc, L["s1"], bias, L["N"], L["K"], code)
 
 
+def _one_kernel(x, N, K):
+    """Whether the call quantises its tokens inside the GEMV: it then needs no scratch for them."""
+    import ctypes
+    from liquidgemm_b200._lib import lib, check
+    plan = (ctypes.c_size_t * 3)()
+    check(lib.lq_linear_plan(x.data_ptr(), x.shape[0], N, K, 0, plan), "linear_plan")
+    return plan[0] == 0
+
+
 # one k-tile; fewer k-tiles than CTAs; cut tiles; ranges longer than K (stream-K over many n-tiles); ragged N; long K
 SHAPES = [(64, 128), (192, 256), (1280, 8192), (4096, 4096), (40000, 256), (28672, 1024), (19200, 4096), (1024, 28672)]
 
@@ -55,19 +64,40 @@ def test_one_call_equals_two(ops, dtype, N, K):
         assert torch.equal(ops.w4a8_linear(x, L), want), M
         got = torch.ops.liquidgemm.w4a8_linear(x, L["rs"], L["s_u8"], L["offset_a"], L["s1"], bias, N, K, 64, code)
         assert torch.equal(got, _two_calls(x, L, bias, code)), M
+        assert _one_kernel(x, N, K) == (M <= 2), M
         if M <= 4:
-            buf = torch.empty(x.numel() + 1, dtype=dtype, device="cuda")   # unaligned activations: the two-launch form
+            buf = torch.empty(x.numel() + 1, dtype=dtype, device="cuda")   # unaligned activations: two launches at any M
             buf[1:] = x.reshape(-1)
+            assert not _one_kernel(buf[1:].view(M, K), N, K)
             assert torch.equal(ops.w4a8_linear(buf[1:].view(M, K), L), want), M
     ops.poll_status()
 
 
-def test_special_activations(ops):
-    L = _layer(ops, 512, 1024, 3)
-    x = _tokens(4, 1024, torch.bfloat16, 1)
-    x[0, 3], x[1, 4], x[2, 5] = float("nan"), float("inf"), torch.finfo(torch.bfloat16).max
-    got, want = ops.w4a8_linear(x, L), _two_calls(x, L, None, 0)
-    assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_special_activations(ops, dtype):
+    """One kind of value a row, alone and beside an ordinary row, through the GEMV's own scales and rounding; four such
+    rows through the two launches."""
+    N, K = 512, 1024
+    L = _layer(ops, N, K, 3)
+    code = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}[dtype]
+    bits = torch.int32 if dtype == torch.float32 else torch.int16
+    fi = torch.finfo(dtype)
+    base = _tokens(9, K, dtype, 1)[1:]
+    base[0, 3] = float("nan")
+    base[1, 4] = float("inf")
+    base[2, 5], base[2, 900] = float("-inf"), float("nan")
+    base[3, K - 1] = fi.max
+    base[4] = fi.tiny
+    base[5] = fi.min
+    base[6] = float("nan")
+    base[7] = 0.0
+    plain = _tokens(2, K, dtype, 2)[1:]
+    cases = [row.view(1, K).clone() for row in base] + [torch.cat([row.view(1, K), plain]) for row in base]
+    cases += [torch.cat([plain, row.view(1, K)]) for row in base]
+    assert all(_one_kernel(x, N, K) for x in cases)
+    for x in cases + [base[:4].clone()]:
+        got, want = ops.w4a8_linear(x, L), _two_calls(x, L, None, code)
+        assert torch.equal(got.view(bits), want.view(bits))
 
 
 def test_refusals_stay(ops):
