@@ -205,8 +205,9 @@ LQ_API int lq_settle_blob(void* stream);
 
 /* LiquidQuant weight quantiser on the device: w [N, K] (w_dtype: LQ_DT_*) -> s1 [N] float32, s_u8 and
  * offset_a [N, K/group_size], and optionally codes [N, K] (one 4-bit code per byte) and / or the tile blob
- * of lq_tile_blob_bytes(N, K) bytes (either may be null).  Two kernels, no host read: the overflow
- * invariants are checked on the device (lq_poll_status reports site 501).  Bit-identical to the
+ * of lq_tile_blob_bytes(N, K) bytes (either may be null).  One kernel for 32-byte aligned rows of up to
+ * 65536 elements (float32: 32768), two otherwise, and with a blob the empty one of lq_settle_blob(); no host read: the
+ * overflow invariants are checked on the device (lq_poll_status reports site 501).  Bit-identical to the
  * reference's quantize_weight on the CPU followed by its prepack
  * (liquidgemm/quant.py:61-100, liquidgemm/ops.py:118-150).  K % 128 == 0, group_size 64 or 128;
  * codes and blob 16-byte aligned. */
@@ -283,8 +284,10 @@ LQ_API int lq_w4a8_linear(const void* x, int x_dtype, const uint8_t* blob, const
  * Replaces torch.ops.liquidgemm.wgmma_i8_gemm (reference csrc/liquid_gemm/w4a8_wgmma.cu:648-694).
  * K % 128 == 0; M and N are arbitrary here (the reference needs multiples of 128).
  * Dispatch: from 256 tokens, on layers with whole 256-channel blocks and at least 60 tiles of 256 x 256, a
- * CTA-pair kernel (tcgen05.mma.cta_group::2, both operands from shared memory); otherwise a persistent one-CTA
- * kernel.  LQ_I8_PAIR=0 in the environment keeps every call on the latter (a measurement switch). */
+ * CTA-pair kernel (tcgen05.mma.cta_group::2, both operands from shared memory); up to 64 tokens, and below 256
+ * where the tiles leave at least half of the CTA slots free, a streaming kernel, as long as it need not cut K (for that
+ * it needs a workspace: lq_i8_gemm_i32_ws); otherwise a persistent one-CTA kernel.  LQ_I8_PAIR=0 in the environment
+ * keeps every call on the latter (a measurement switch).  Both operands may be the output of the work directly before. */
 LQ_API int lq_i8_gemm_i32(const int8_t* a, const int8_t* b, int32_t* c, int M, int N, int K,
                    void* stream);
 
@@ -297,8 +300,7 @@ LQ_API int lq_i8_gemm_scaled(const int8_t* a, const int8_t* b, const float* a_sc
 
 /* The same two with `workspace` (lq_i8_workspace_bytes(M, N, K) of 4-byte aligned scratch, any content; null and 0 where
  * that is 0; below 16-byte alignment the parts are added up more slowly):
- * batches below the CTA-pair kernel's sizes then run on a streaming kernel that may cut the layer's K and add the
- * parts up through it.  Results are bit-identical. */
+ * the streaming kernel may then cut the layer's K and add the parts up through it.  Results are bit-identical. */
 LQ_API size_t lq_i8_workspace_bytes(int M, int N, int K);
 LQ_API int lq_i8_gemm_i32_ws(const int8_t* a, const int8_t* b, int32_t* c, int M, int N, int K, void* workspace,
                       size_t workspace_bytes, void* stream);

@@ -731,8 +731,9 @@ static bool gemv_serves(int M, int N, int K) {
 // 28672 x 4096 at 2048 / 2560 / 3072 / 4096 / 8192 tokens 184 -> 179, 232 -> 221, 266 -> 256, 360 -> 327, 704 -> 610 us; at 1500
 // 136 -> 143.  6144 x 4096 at 2048 / 3072 / 8192 44.5 -> 44.7, 62.8 -> 55.1, 151 -> 137; 4096 x 4096 at 2560 / 3072 / 8192 40.2 ->
 // 42.5, 44.6 -> 42.0, 105 -> 90: matrices up to 32 M weights start at 3072.  Larger ones start at 5120 although the time
-// would allow 2048: callers size and type their workspace by the route (scratch of N x K bytes here, the all-zero planes
-// of the W4 pair kernel there), and that contract is kept up to 5119 tokens.  4096 x 14336 (where the W4 kernel's
+// would allow 2048: callers of lq_w4a8_gemm_fused size and type their workspace by the route (scratch of N x K bytes here,
+// the all-zero planes of the W4 pair kernel there), and what they are told up to 5119 tokens is kept.  lq_linear_plan and
+// lq_w4a8_linear, which report sizes of their own, follow the same limits; nothing but that choice holds them to it.  4096 x 14336 (where the W4 kernel's
 // epilogues weigh least) is level at every size: layers with K >= 8192 stay on the W4 pair kernel, and so do layers above
 // 256 MB of INT8 weights (the scratch would be larger than that).  LQ_UNPACK_I8_MIN_M replaces both limits (0 switches
 // the route off).  Running the two kernels overlapped (the GEMM launched programmatically behind a persistent unpack
@@ -1042,7 +1043,8 @@ static int i8_common(const int8_t* a, const int8_t* b, const float* a_scale, con
   const I8Route r = i8_route(M, N, K);
   if (r == kI8Pair)
     return run_i8_pair_gemm(a, b, a_scale, b_scale, nullptr, out, out_mode, M, N, K, as_stream(stream));
-  // without the workspace of the split streaming kernel (the plain entry points): whole tiles, one CTA per SM
+  // Without the workspace that a cut K needs (the plain entry points have none): whole tiles, one CTA per SM.  Where K is
+  // not cut the streaming kernel needs no workspace and serves every entry point.
   if (r == kI8Stream && ws_bytes >= i8_stream_workspace_bytes(M, N, K)) {
     if (reinterpret_cast<uintptr_t>(ws) & 3) return LQ_ERR_WORKSPACE;   // int32 planes
     if (int rc = lq_check_device()) return rc;

@@ -538,7 +538,9 @@ static int launch_quant(const Args& a, int grid, cudaStream_t st) {
 // the second kernel and its place in the stream (2 us) for one token (6144 x 4096 6.3 -> 5.6 us, 28672 x 4096 15.3 -> 13.5,
 // 4096 x 14336 9.7 -> 8.8, 1280 x 8192 5.0 -> 4.3) and for two (6.7 -> 6.7, 15.5 -> 15.4, 10.7 -> 10.2, 5.5 -> 5.0); with
 // three and four the dp4a arithmetic is behind the tensor-core kernels (6144 x 4096 at four: 7.7 -> 9.9, 28672 x 4096 15.7 ->
-// 24.2).  The quantised tokens have to fit beside the weight ring of two CTAs per SM.
+// 24.2).  The exception measured is two tokens on wide layers with a very long K, where every CTA's pass over the tokens
+// shows (bf16): 8192 x 28672 28.2 -> 30.9 (28672 x 14336 46.6 -> 45.4, 57344 x 8192 52.9 -> 50.0).  The quantised tokens
+// have to fit beside the weight ring of two CTAs per SM.
 bool gemv_quant_serves(int M, int N, int K) {
   if (M < 1 || M > 2 || N < 1 || K < 128 || K % 128) return false;
   return gblob::token_tiles_max(N, K) * M * 128 + gblob::Cfg<2, 8, true>::kUsedBytes <= gblob::kMaxQuantSmem;

@@ -7,7 +7,9 @@
 // int32 plane and the finish pass adds the planes, scales and casts (exact in any order).
 //  * warp 0  producer: one thread keeps NS 128 x 128 weight boxes in flight (tensor map, 128-byte swizzle).  B may be the
 //            output of the kernel just before (a quantiser, the dequantiser), so it is read after the wait for that
-//            kernel; before it the first NS boxes are only hinted to L2, which changes no result whoever writes them.
+//            kernel; before it the first NS boxes are only hinted to L2, which changes no result whoever writes them
+//            (eight linears behind quantisers, 8 tokens: 123.2 us without the hint, 122.5 with it, 115 when they were
+//            read without waiting, which was wrong wherever B was fresh).
 //  * warp 1  tensor memory and MMA issue: four 128 x BN x 32 tcgen05.mma kind::i8 per k-step, both operands from
 //            shared memory; its commit recycles the stage.
 //  * warps 2..9  two sets of 128 threads, k-steps in turn: the set that owns a k-step fetches its BN x 128-byte token
@@ -249,9 +251,10 @@ static long i8_stream_tiles(int M, int N) {
 
 // Up to 64 tokens always; up to 255 where the tiles leave at least half of the CTA slots to k-ranges.  Measured against
 // the one-CTA-per-SM persistent kernel, which takes whole tiles (so that a 4096-channel layer kept 32 SMs busy): 8 tokens
-// 6144 x 4096 11.2 -> 8.4 us, 4096 x 4096 10.9 -> 6.8, 28672 x 4096 25.1 -> 22.4, 4096 x 14336 27.7 -> 14.3; 64 tokens 12.6 -> 9.5,
-// 12.3 -> 8.7, 26.8 -> 25.3, 29.4 -> 16.5; 200 tokens 17.4 -> 17.1, 17.0 -> 13.9, 39.5 -> 30.7; but 28672 x 4096 at 128 tokens 29.3 ->
-// 32.1 and at 200 48.5 -> 52.3, and from 256 tokens on the persistent kernel's 192-token tiles win.
+// 6144 x 4096 11.2 -> 8.2 us, 4096 x 4096 10.9 -> 6.7, 28672 x 4096 25.2 -> 22.8, 4096 x 14336 27.7 -> 14.0, 1024 x 28672 50.2 -> 10.6;
+// 64 tokens 12.7 -> 10.1, 12.4 -> 9.4, 26.3 -> 25.1, 29.6 -> 16.6, 52.6 -> 12.4; 200 tokens 17.5 -> 16.8, 16.8 -> 13.6, (wide layers keep
+// the persistent kernel), 39.3 -> 31.0, 66.0 -> 19.9; but 28672 x 4096 at 128 tokens 29.3 -> 32.1 and at 200 48.5 -> 52.3, and from 256
+// tokens on the persistent kernel's 192-token tiles win.
 bool i8_stream_serves(int M, int N, int K) {
   (void)K;
   return M <= 64 || (M < 256 && 2 * i8_stream_tiles(M, N) <= 2L * sm_count());

@@ -447,7 +447,8 @@ def _linear_call(x, code, w, s1, bias, y, out_dtype, M, N, K, dev):
 
 
 def quantize_weight_cuda(W: torch.Tensor, group_size: int = 64, want_codes: bool = True, want_blob: bool = False):
-    """LiquidQuant quantiser as two CUDA kernels (``lq_quantize_weight``): bit-identical to
+    """LiquidQuant quantiser in one pass over the weights (``lq_quantize_weight``; two for unaligned or very long
+    rows): bit-identical to
     :func:`liquidgemm_b200.quant.quantize_weight` and to the reference's CPU result
     (liquidgemm/quant.py:61-100) without its chain of elementwise launches and host reads.
     Returns ``(LiquidQuantWeight, blob)``; ``qweight_u4`` is None without ``want_codes`` and ``blob`` is
