@@ -756,6 +756,9 @@ static Route route_for(int M, int N, int K, int splitk, bool scaled, bool single
       // 4096 x 14336: 10.4 vs 10.8 us; 6144 x 4096: 7.3 vs 7.0 us, 4096 x 4096: 6.6 vs 6.0 us).
       if (M <= decode_tc_max_m() && (long)N * K <= (1L << 25)) return {kRouteDecodeTc, 0};
     }
+    // int32 outputs where the scaled call takes the GEMV: callers are told one kind of workspace for both, the all-zero
+    // buffer, so the tile kernel must not write its planes there.
+    if (splitk == 0 && !scaled && gemv_serves(M, N, K)) return {kRoutePersistent, 0};
     int S = splitk > 0 ? splitk : tile_pick_splits(M, N, K);
     if (S > kt) S = kt;
     return {kRouteTile, S < 1 ? 1 : S};

@@ -1,0 +1,28 @@
+"""int32 accumulators at a token count whose scaled call takes the GEMV: both use the same all-zero reduction buffer, and
+each leaves it all zero."""
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import lqq_oracle as O
+from tests.helpers import assert_bits_equal, random_lqq, random_tokens, to_torch_qw
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 256, 28672), (2, 4096, 14336), (1, 28672, 4096), (4, 200, 5120)])
+def test_buffer_stays_zero(M, N, K):
+    from liquidgemm_b200 import ops
+    qw = random_lqq(N, K, seed=M + N)
+    tq = to_torch_qw(qw)
+    blob = ops._repack_device(tq.qweight_u4, 0, tq.s_u8, tq.offset_a, N, K, 64).reshape(-1)
+    x, sc = random_tokens(M, K, seed=M)
+    xt, st = torch.from_numpy(x).cuda(), torch.from_numpy(sc).cuda()
+    w = (qw.qweight_u4.astype(np.int32) * np.repeat(qw.s_u8, 64, 1) + np.repeat(qw.offset_a, 64, 1).astype(np.int32) - 128)
+    acc = (x.astype(np.float64) @ w.astype(np.float64).T).astype(np.int64).astype(np.int32)   # below 2^53: exact
+    for _ in range(2):
+        assert np.array_equal(ops.gemm_i32(xt, blob, N, K).cpu().numpy(), acc)
+        assert_bits_equal(ops.gemm_fused(xt, blob, st, tq.s1, N, K, 0), O.scale_f32(acc, sc, qw.s1), 0, f"{M}x{N}x{K}")
+    assert all(int(ws.max()) == 0 for ws in ops._WORKSPACES.values())
+    ops.poll_status()
