@@ -241,6 +241,12 @@ __device__ __forceinline__ bool round_quotients(const float2 (&x)[N], float inv,
   return far < kSafeDist;
 }
 
+// The same test for one element.
+__device__ __forceinline__ bool near_integer(float x, float inv) {
+  const float r = __fadd_rn(__fmaf_rn(x, inv, kRoundMagic), -kRoundMagic);
+  return fabsf(__fmaf_rn(x, -inv, r)) < kSafeDist;
+}
+
 // Two elements of a 32-bit word (16-bit types), low half first.
 template <typename T> __device__ __forceinline__ float2 unpack2(uint32_t w);
 template <> __device__ __forceinline__ float2 unpack2<__half>(uint32_t w) {
@@ -305,6 +311,17 @@ __device__ __forceinline__ int quant1(float x, float scale) {
   return max(-127, min(127, q));
 }
 
+// The scale of a token row: max(amax, 1e-12) / 127, correctly rounded.  Markstein's division step (IBM J. Res. Dev. 34,
+// 1990): the exact residual of the quotient by the rounded reciprocal corrects it.  It saves the general division's 100
+// cycles where a row's latency counts; infinities and NaN take the division.
+__device__ __forceinline__ float token_scale(float amax) {
+  const float a = fmaxf(amax, 1e-12f);
+  constexpr float kInv = 1.0f / 127.0f;
+  const float q = __fmul_rn(a, kInv);
+  const float s = __fmaf_rn(__fmaf_rn(-127.0f, q, a), kInv, q);
+  return a < 3e38f ? s : __fdiv_rn(a, 127.0f);
+}
+
 // The quantised bytes of one 16-byte vector: VEC int8 in VEC / 4 words.
 template <typename T>
 __device__ __forceinline__ void quant_vec(const uint4& raw, float scale, float inv, uint32_t (&out)[4 / sizeof(T)]) {
@@ -318,11 +335,11 @@ __device__ __forceinline__ void quant_vec(const uint4& raw, float scale, float i
     q[2 * i] = __float_as_uint(t[i].x);
     q[2 * i + 1] = __float_as_uint(t[i].y);
   }
-  if (!safe) {
+  if (!safe) {   // one element, nearly always
 #pragma unroll
     for (int i = 0; i < VEC / 2; ++i) {
-      q[2 * i] = (uint32_t)quant1(x[i].x, scale);
-      q[2 * i + 1] = (uint32_t)quant1(x[i].y, scale);
+      if (!near_integer(x[i].x, inv)) q[2 * i] = (uint32_t)quant1(x[i].x, scale);
+      if (!near_integer(x[i].y, inv)) q[2 * i + 1] = (uint32_t)quant1(x[i].y, scale);
     }
   }
 #pragma unroll

@@ -1,43 +1,29 @@
-// W4A8 tensor-core linear for decode batches (up to 32 tokens; the dispatch uses it for 3..16 tokens on matrices
-// up to 32 M weights, where its single launch beats the tile kernel's planes + finish pass): HBM-bound, so built like a streaming
-// copy with tensor cores attached, in ONE launch.  Replaces the reference's split-K WGMMA path for small
-// M (csrc/liquid_gemm/w4a8_wgmma.cu:333-503 with the split rule at :523-534 and the finish kernel :39-56).
+// W4A8 tensor-core linear for decode batches (up to 32 tokens): the weights stream from HBM once and everything else is
+// small, so what a launch costs is its chain of latencies.  Replaces the reference's split-K WGMMA path for small M
+// (csrc/liquid_gemm/w4a8_wgmma.cu:333-503 with the split rule at :523-534 and the finish kernel :39-56) in ONE launch.
 //
-//  * Work = the (n-tile, k-tile) grid of 8704-byte blob tiles, cut into equal contiguous ranges, one
-//    per CTA, two CTAs per SM (stream-K; layers with few n-tiles are cut into equal k-ranges per tile):
-//    every SM streams the same number of weight bytes whatever N and K are.
-//  * warp 0  producer: one thread keeps a ring of NW weight tiles in flight, one contiguous bulk copy
-//            each.  The dequant threads release a stage as soon as they hold the tile in registers, so
-//            the ring only has to cover the memory latency.  The tokens do NOT come through the copy
-//            engine: measured on B200, a second (tensor-map) copy per k-tile made the copy engine the
-//            bottleneck -- the producer was never idle, its copy instructions blocked on a full queue, the
-//            MMAs waited for token boxes a third of the time and the stream ran at 60 % of the dp4a GEMV's
-//            rate.  The 128 threads of the dequant set that owns a k-tile fetch its BN x 128-byte token
-//            slice themselves (16 bytes each, an L2 hit issued before the wait for the weights) and store
-//            it into the operand stage in the 128-byte-swizzled layout the MMA's descriptor expects.
-//  * warps 2..9  two dequant sets taking alternate k-tiles; thread r of a set owns weight row r:
-//            64 bytes of nibbles -> 128 INT8 (AND / SHR+AND / IMAD / XOR on 4-lane words) ->
-//            tcgen05.st into tensor-memory lane r (the MMA's A operand, 4 consecutive k per column).
-//  * warp 1  MMA: the warp walks the loop, one elected lane issues four 128 x BN x 32 tcgen05.mma kind::i8 per k-tile (A from tensor
-//            memory, B = tokens through a shared-memory descriptor); its commit recycles the operand
-//            stage (NT stages: 32 tensor-memory columns + the token slice in shared memory).
-//  * Two accumulators in tensor memory, taken in turn by the segments (tile, k-range) of the CTA's
-//    range.  Set p owns accumulator p and runs the epilogue of a segment only when that accumulator is
-//    needed again, or at the very end -- where the two sets finish the CTA's (at most two) partial
-//    segments side by side.  Nothing stalls in the middle of the stream: measured on B200, an epilogue
-//    between two segments (tensor-memory load, atomics, stores: one to two microseconds during which
-//    no operand is produced) cost more than the imbalance stream-K removes.
-//  * Epilogue: tcgen05.ld (lane = channel, column = token); a segment that covers its tile's whole K
-//    is scaled and stored directly; otherwise the partial sums of the CTAs that share the tile meet in
-//    a zeroed workspace word per output element through ONE returning 64-bit atomic add that carries
-//    the k-tile count along with the sum, and whoever completes the count stores the output and
-//    re-zeroes the word.  Integer sums are exact in any order, so results do not depend on the split.
-//    The optional bias is added to the value already rounded to the output type, as PyTorch's
-//    `y + bias` after the reference's operator does (liquidgemm/vllm_plugin.py:205-206).
-//  * Launched with programmatic stream serialisation: weight tiles are requested before the wait for
-//    the previous kernel of the stream, tokens / outputs / workspace are touched only after it.
-// Every wait is bounded; a thread whose wait expires records a site code, stops waiting and still
-// runs the rest of its control flow, so the CTA reaches the exit where tensor memory is released.
+//  * One 128-channel tile and one k-range per CTA; the CTAs that share a tile's K form a thread-block cluster (up to
+//    eight).  320 threads, at most half of an SM, so that the next launch's CTAs become resident beside this launch's.
+//  * Everything that needs only the weights happens BEFORE the wait for the previous kernel: the ring fills and the first
+//    NT k-tiles are unpacked into tensor memory (the MMA's A operand).  After the wait come, one after the other, one
+//    round of token loads, the MMAs, the join, the stores.
+//  * warp 0  producer: one thread keeps a ring of weight tiles in flight, one contiguous 8704-byte bulk copy each.
+//  * warps 2..9  two dequant sets taking alternate k-tiles; thread r of a set owns weight row r: 64 bytes of nibbles ->
+//            128 INT8 (AND / SHR+AND / IMAD / XOR on 4-lane words) -> tcgen05.st into tensor-memory lane r.
+//            After the wait they fetch the tokens of the CTA's whole k-range in one go (16 bytes a thread and load, L2
+//            hits) and store them in the 128-byte-swizzled layout the MMA's descriptor expects.  Tokens do not come
+//            through the copy engine, where they would queue behind the weights.
+//            XT an activation type: the tokens are quantised here, which saves the quantiser's launch and its place in the
+//            stream.  A CTA reads only its k-range of the activations; the row maxima of the cluster's CTAs meet in each
+//            CTA's shared memory (st.async), and what a thread has loaded it quantises out of its registers.
+//  * warp 1  MMA: the warp walks the loop, one elected lane issues four 128 x BN x 32 tcgen05.mma kind::i8 per k-tile (A from
+//            tensor memory, B = tokens through a shared-memory descriptor); its commit recycles the operand stage.
+//  * Join: each CTA of the cluster owns a block of the tile's channels and receives the other CTAs' int32 sums for it in
+//    its shared memory (st.async, counted by an mbarrier); it adds them, scales and stores.  Integer sums are exact in any
+//    order, so results do not depend on the split.  The optional bias is added to the value already rounded to the
+//    output type, as PyTorch's `y + bias` after the reference's operator does (liquidgemm/vllm_plugin.py:205-206).
+// Every wait is bounded; a thread whose wait expires records a site code, stops waiting and still runs the rest of its
+// control flow, so the CTA reaches the exit where tensor memory is released.
 
 #include <stdint.h>
 
@@ -46,98 +32,147 @@
 #include <type_traits>
 
 #include "lq_common.cuh"
-#include "lq_sched.cuh"
 #include "lq_tc_ptx.cuh"
 
 namespace lq {
 
 namespace dtc {
 
-// Pipeline studies (-DLQ_PIPELINE_TRACE, a build of its own): per-CTA cycle counters of every role, read
-// back with lq_debug_read_decode_trace().  The product build compiles none of it.
+// Pipeline studies (-DLQ_PIPELINE_TRACE, a build of its own): %globaltimer stamps of every CTA's milestones, read back with
+// lq_debug_read_decode_trace().  The product build compiles none of it.
 #ifdef LQ_PIPELINE_TRACE
-__device__ long long g_trace[1024 * 16];
-#define TR_NOW() clock64()
-#define TR_ADD(acc, t0) (acc) += clock64() - (t0)
-#define TR_SET(slot, v) g_trace[(blockIdx.x & 1023) * 16 + (slot)] = (long long)(v)
-#define TR_VAR(name) long long name = 0
+__device__ long long g_trace[1024 * 8];
+#define DT_STAMP(slot)                                                                      \
+  do {                                                                                      \
+    if (blockIdx.x < 1024u) g_trace[blockIdx.x * 8 + (slot)] = (long long)ptx::globaltimer_ns(); \
+  } while (0)
 #else
-#define TR_NOW() 0ll
-#define TR_ADD(acc, t0) ((void)(t0))
-#define TR_SET(slot, v) ((void)(v))
-#define TR_VAR(name) const long long name = 0
+#define DT_STAMP(slot) ((void)0)
 #endif
 
 constexpr int kTileBytes = 8704;
-constexpr int kSets = 2;                    // dequant sets of 128 threads; set p also owns accumulator p
+constexpr int kSets = 2;                    // dequant sets of 128 threads
 constexpr int kDequant = 128 * kSets;
 constexpr int kThreads = 64 + kDequant;
 constexpr uint64_t kWaitLimitNs = 2000000000ull;
 // The wait for tokens gathered from peer GPUs gives up well before the barrier waits of the threads that
-// depend on it, so that one late peer is reported once (by the producer) and the rest of the CTA still
-// finishes its reduction and leaves the workspace clean.
+// depend on it, so that one late peer is reported once and the rest of the CTA still finishes.
 constexpr uint64_t kPeerWaitLimitNs = 1000000000ull;
 constexpr int kOutI32 = 3;
+constexpr int kMaxRing = 12;                // weight tiles in flight
+constexpr int kMaxSplits = 8;               // portable cluster size
+constexpr int kTmemCols = 256;              // two CTAs per SM share 512
+constexpr int kSmemLimit = 113 * 1024;      // and the shared memory
 
 struct Args {
   const uint8_t* blob;
-  const int8_t* x;       // [M, K]
-  const float* ascale;   // [M]
+  const void* x;         // [M, K]: int8 tokens, or the activations themselves (kernels that quantise)
+  const float* ascale;   // [M]; null with activations
   const float* s1;       // [N]
   const void* bias;      // [N] in the output dtype, or null
   void* out;             // [M, N] (single-destination kernels; the others get a MultiOut parameter)
-  unsigned long long* slots;   // [grid][BN][128] packed (k-tile count, biased partial sum), zero between launches
   int* status;
   int out_mode;          // LQ_DT_* or kOutI32
-  int M, N, K, fixed_split;
+  int M, N, K, splits;   // CTAs of a cluster = k-ranges of a tile
+  int ring;              // weight tiles in flight
 };
 
-template <int BN, int NW, int NT>
+template <int BN>
 struct Cfg {
   static constexpr int kXStage = BN * 128;
-  static constexpr int kAccCols = 2 * BN;   // two accumulators
-  static constexpr int kACols = 32 * NT;    // one tensor-memory operand stage per token box
-  static constexpr int kColsNeeded = kAccCols + kACols;
-  static constexpr int kTmemCols = kColsNeeded <= 128 ? 128 : 256;
-  static constexpr int kNumBars = 2 * NW + 2 * NT + 4;
-  static constexpr int kUsedBytes = 1024 + NT * kXStage + NW * kTileBytes + kNumBars * 8 + 16 + 2 * BN * 4;
-  // more than a third of the SM's shared memory, so that never three CTAs (of this and of the next
-  // kernel, under programmatic dependent launch) share an SM while another SM holds one
-  static constexpr int kSmemBytes = kUsedBytes > 78 * 1024 ? kUsedBytes : 78 * 1024;
-  static_assert(kColsNeeded <= 256, "two CTAs per SM share 512 tensor-memory columns");
-  static_assert(kSmemBytes <= 113 * 1024, "two CTAs per SM share the shared memory");
+  static constexpr int kACol = BN < 32 ? 32 : BN;             // operand stages behind the accumulator, on whole stages
+  static constexpr int kNT = (kTmemCols - kACol) / 32;
+};
+constexpr int kQuantTokens = 8;              // limit of the quantising form: a warp per row
+constexpr int kMaxParts = 8 * kMaxSplits;    // parts of the row maxima: one per warp and CTA of the cluster
+constexpr int kNumBars = 2 * kMaxRing + 2 * 8 + 4;
+
+// Rows of the tile that each CTA of a cluster joins: blocks of eight rows, as evenly as they go.
+__host__ __device__ inline int join_first_block(int rank, int splits) { return (16 * rank + splits - 1) / splits; }
+__host__ __device__ inline int join_rows_max(int splits) { return (16 + splits - 1) / splits * 8; }
+
+// Shared memory in bytes behind the 1024-byte aligned base.
+struct Layout {
+  int ws, join, bars, small, total;
+};
+__host__ __device__ inline Layout layout(int bn, int nk_max, int ring, int splits) {
+  Layout l;
+  l.ws = nk_max * bn * 128;
+  l.join = l.ws + ring * kTileBytes;
+  l.bars = l.join + (splits > 1 ? splits * join_rows_max(splits) * bn * 4 : 0);
+  l.small = l.bars + kNumBars * 8 + 16;
+  l.total = l.small + (32 + 2 * 128) * 4 + kMaxParts * 16;   // token scales, channel scales, bias, parts of the row maxima
+  return l;
+}
+
+// Sixteen activations: one 16-byte chunk of quantised tokens.
+template <typename XT>
+struct Chunk {
+  uint4 r[sizeof(XT)];
+  __device__ __forceinline__ void load(const XT* p) {
+#pragma unroll
+    for (int i = 0; i < (int)sizeof(XT); ++i) r[i] = __ldg(reinterpret_cast<const uint4*>(p) + i);
+  }
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int i = 0; i < (int)sizeof(XT); ++i) r[i] = make_uint4(0u, 0u, 0u, 0u);
+  }
+  __device__ __forceinline__ uint4 quantised(float scale, float inv) const {
+    uint32_t q[4];
+#pragma unroll
+    for (int i = 0; i < (int)sizeof(XT); ++i) {
+      uint32_t o[4 / sizeof(XT)];
+      quant_vec<XT>(r[i], scale, inv, o);
+#pragma unroll
+      for (int j = 0; j < 4 / (int)sizeof(XT); ++j) q[i * (4 / sizeof(XT)) + j] = o[j];
+    }
+    return make_uint4(q[0], q[1], q[2], q[3]);
+  }
 };
 
-// What the epilogue needs to know about a segment after the walk has moved on.
-struct SegInfo {
-  int tile, nk, slot;
-  bool whole;
-  float w_scale, bias;   // of this thread's output channel: weights, fetched when the segment starts
-};
-
-template <int BN, int NW, int NT, bool MULTI>
+template <int BN, bool MULTI, typename XT>
 __global__ void __launch_bounds__(kThreads, 2)
 w4a8_decode_tc_kernel(const Args args, const std::conditional_t<MULTI, MultiOut, NoMultiOut> multi) {
+  constexpr bool QUANT = !std::is_same_v<XT, int8_t>;
+  constexpr int NT = Cfg<BN>::kNT;
+  constexpr int kXStage = Cfg<BN>::kXStage;
+  const int M = args.M, S = args.splits, NW = args.ring;
   const int kt_total = args.K >> 7;
-  using C = Cfg<BN, NW, NT>;
+  const int rank = (int)(blockIdx.x % (unsigned)S), tile = (int)(blockIdx.x / (unsigned)S);
+  const int kb = rank * kt_total / S;
+  const int nk = (rank + 1) * kt_total / S - kb;
+  if (threadIdx.x == 0) DT_STAMP(0);   // CTA start
+
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t* smem = smem_raw + (base - raw);
-
-  const uint32_t xs = base;                          // NT token slices (1024-aligned for the swizzle)
-  const uint32_t ws = xs + NT * C::kXStage;          // NW weight tiles
-  const uint32_t bar_wfull = ws + NW * kTileBytes;   // [NW] weight tile landed
-  const uint32_t bar_wfree = bar_wfull + NW * 8;     // [NW] a dequant set holds the tile in registers
-  const uint32_t bar_aready = bar_wfree + NW * 8;    // [NT] dequantised operand and token slice are in place
-  const uint32_t bar_afree = bar_aready + NT * 8;    // [NT] the MMAs that read operand and token slice are done
-  const uint32_t bar_accfull = bar_afree + NT * 8;   // [2] the accumulator's segment is final
-  const uint32_t bar_accfree = bar_accfull + 16;     // [2] the accumulator has been read
-  const uint32_t tmem_slot = bar_accfree + 16;
+  const Layout lay = layout(BN, (kt_total + S - 1) / S, NW, S);
+  const uint32_t xs = base;                              // token slices of the whole k-range (1024-aligned for the swizzle)
+  const uint32_t ws = base + lay.ws;                     // weight ring
+  const uint32_t join = base + lay.join;                 // [splits][BN / 4][join_rows_max][4] int32
+  const uint32_t bar_wfull = base + lay.bars;            // [ring] weight tile landed
+  const uint32_t bar_wfree = bar_wfull + kMaxRing * 8;   // [ring] a dequant set holds the tile in registers
+  const uint32_t bar_aready = bar_wfree + kMaxRing * 8;  // [NT] unpacked operand in place
+  const uint32_t bar_afree = bar_aready + 8 * 8;         // [NT] the MMAs that read the operand are done
+  const uint32_t bar_x = bar_afree + 8 * 8;              // the tokens are in place
+  const uint32_t bar_acc = bar_x + 8;                    // the accumulator is final
+  const uint32_t bar_join = bar_acc + 8;                 // the cluster's sums for this CTA's rows have landed
+  const uint32_t bar_amax = bar_join + 8;                // the cluster's row maxima have landed
+  const uint32_t tmem_slot = bar_amax + 8;
   volatile uint32_t* tmem_slot_p = reinterpret_cast<volatile uint32_t*>(smem + (tmem_slot - base));
-  float* tok_scale = reinterpret_cast<float*>(smem + (tmem_slot + 16 - base));   // [2 sets][BN] token scales
+  float* tok_scale = reinterpret_cast<float*>(smem + lay.small);   // [32]
+  float* chan_scale = tok_scale + 32;                              // [128] of the rows this CTA stores
+  float* chan_bias = chan_scale + 128;
+  const uint32_t parts = base + lay.small + (32 + 2 * 128) * 4;    // [M][splits * wpr] 16 bytes: bits of a part's maximum
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int fb = join_first_block(rank, S);
+  const int rows_own = (join_first_block(rank + 1, S) - fb) * 8;
+  const int rows_max = join_rows_max(S);
+  const int groups = (M + 3) >> 2;   // of four tokens
+  // warps of a token row while the maxima are taken (QUANT)
+  const int wpr = M > 4 ? 1 : M > 2 ? 2 : M == 2 ? 4 : 8;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < NW; ++s) {
@@ -148,46 +183,42 @@ w4a8_decode_tc_kernel(const Args args, const std::conditional_t<MULTI, MultiOut,
       ptx::mbar_init(bar_aready + 8 * t, 128);
       ptx::mbar_init(bar_afree + 8 * t, 1);
     }
-    for (int p = 0; p < 2; ++p) {
-      ptx::mbar_init(bar_accfull + 8 * p, 1);
-      ptx::mbar_init(bar_accfree + 8 * p, 128);
-    }
+    ptx::mbar_init(bar_x, kDequant);
+    ptx::mbar_init(bar_acc, 1);
+    ptx::mbar_init(bar_join, 1);
+    ptx::mbar_init(bar_amax, 1);
     ptx::fence_mbar_init();
+    ptx::mbar_expect_tx(bar_join, (uint32_t)(S * rows_own * groups * 16));
+    if (QUANT) ptx::mbar_expect_tx(bar_amax, (uint32_t)(S * wpr * M * 16));
+    // Weight tiles do not depend on the previous kernel of the stream, so they are requested at once.
+    ptx::mbar_expect_tx(bar_wfull, kTileBytes);
+    ptx::bulk_load(ws, args.blob + ((size_t)tile * kt_total + kb) * kTileBytes, kTileBytes, bar_wfull);
   }
   __syncthreads();
-  allow_dependents();   // the next kernel of the stream may start prefetching its weights
-
-  const SchedArgs sched{kt_total, (args.N + 127) >> 7, 1, args.fixed_split};
-  SegmentWalk walk(sched, blockIdx.x, gridDim.x);
-  Segment sg;
+  allow_dependents();         // the next kernel of the stream may start prefetching its weights
+  if (S > 1) ptx::cluster_sync_all();   // every CTA's barriers are initialised
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer
     if (lane == 0) {
-      Ring<NW> ring;
-      int issued = 0;
+      const uint8_t* src = args.blob + ((size_t)tile * kt_total + kb + 1) * kTileBytes;
+      int s = 1, issued = 1;   // the first tile is under way
+      uint32_t ph = 0;
       bool ok = true;
-      TR_VAR(tr_idle);
-      const long long tr_p0 = TR_NOW();
-      // Weight tiles do not depend on the previous kernel of the stream, so they are requested at once.
-      while (ok && walk.next(sg)) {
-        const uint8_t* src = args.blob + ((size_t)sg.tile * kt_total + sg.kb) * kTileBytes;
-        for (int kt = sg.kb; kt < sg.ke; ++kt, src += kTileBytes) {
-          const long long tr_i0 = TR_NOW();
-          if (!ptx::mbar_wait_bounded(bar_wfree + 8 * ring.s, ring.ph ^ 1u, kWaitLimitNs)) {
-            atomicExch(args.status, 401);
-            ok = false;
-            break;
-          }
-          TR_ADD(tr_idle, tr_i0);
-          ptx::mbar_expect_tx(bar_wfull + 8 * ring.s, kTileBytes);
-          ptx::bulk_load(ws + ring.s * kTileBytes, src, kTileBytes, bar_wfull + 8 * ring.s);
-          ring.advance();
-          ++issued;
+      for (int i = 1; i < nk; ++i, src += kTileBytes) {
+        if (i >= NW && !ptx::mbar_wait_bounded(bar_wfree + 8 * s, ph ^ 1u, kWaitLimitNs)) {
+          atomicExch(args.status, 401);
+          ok = false;
+          break;
+        }
+        ptx::mbar_expect_tx(bar_wfull + 8 * s, kTileBytes);
+        ptx::bulk_load(ws + s * kTileBytes, src, kTileBytes, bar_wfull + 8 * s);
+        ++issued;
+        if (++s == NW) {
+          s = 0;
+          ph ^= 1u;
         }
       }
-      TR_SET(0, tr_idle);
-      TR_SET(1, TR_NOW() - tr_p0);
       if (!ok) {
         // Copies in flight write shared memory: they must have landed before the CTA may exit.  (On the
         // normal path the dequant sets have waited for every one of them.)
@@ -197,336 +228,431 @@ w4a8_decode_tc_kernel(const Args args, const std::conditional_t<MULTI, MultiOut,
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ tensor memory + MMA issue
-    ptx::tmem_alloc(tmem_slot, C::kTmemCols);
+    ptx::tmem_alloc(tmem_slot, kTmemCols);
     ptx::tmem_relinquish();
     ptx::tc_fence_before();
     asm volatile("bar.sync 2, %0;" ::"n"(32 + kDequant) : "memory");   // publishes the allocation to the dequant warps
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot_p;
-    const uint32_t tmem_a = tmem_base + C::kAccCols;
     {
       // The whole warp walks the loop; one elected lane issues (see ptx::elect_one).
       const bool leader = ptx::elect_one();
       constexpr uint32_t idesc = ptx::idesc_i8(BN);
-      Ring<NT> ring;
       bool ok = true;
-      uint32_t seg = 0;
-      TR_VAR(tr_wa);
-      TR_VAR(tr_issue);
-      TR_VAR(tr_commit);
-      const long long tr_m0 = TR_NOW();
-      while (walk.next(sg)) {
-        const uint32_t p = seg & 1u;
-        // the accumulator's previous segment (two back) must have been read out by its set
-        if (seg >= 2 && ok && !ptx::mbar_wait_bounded(bar_accfree + 8 * p, ((seg >> 1) - 1u) & 1u, kWaitLimitNs)) {
-          if (leader) atomicExch(args.status, 402);
-          ok = false;
-        }
-        const uint32_t tmem_acc = tmem_base + p * BN;
-        for (int kt = sg.kb; kt < sg.ke; ++kt) {
-          const long long tr_a1 = TR_NOW();
-          if (ok && !ptx::mbar_wait_bounded(bar_aready + 8 * ring.s, ring.ph, kWaitLimitNs)) {
-            if (leader) atomicExch(args.status, 403);
-            ok = false;
-          }
-          TR_ADD(tr_wa, tr_a1);
-          __syncwarp();
-          ptx::tc_fence_after();
-          const long long tr_i1 = TR_NOW();
-          const uint32_t xb = xs + ring.s * C::kXStage;
-          const uint32_t ab = tmem_a + ring.s * 32;
-          if (leader) {
+      // The operands that were unpacked ahead of the tokens: once the tokens are there their MMAs go out back to back.
+      // (With a wait and a commit around each k-tile's four MMAs a k-tile takes the issuing warp 350 cycles instead of
+      // about 110.)
+      const int pre = min(nk, NT);
+      for (int t = 0; t < pre; ++t) ok = ok && ptx::mbar_wait_bounded(bar_aready + 8 * t, 0u, kWaitLimitNs);
+      ok = ok && ptx::mbar_wait_bounded(bar_x, 0u, kWaitLimitNs);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok && leader) atomicExch(args.status, 402);
+      ptx::tc_fence_after();
+      if (leader) {
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+          if (t < pre) {
 #pragma unroll
             for (int j = 0; j < 4; ++j)
-              ptx::mma_i8_ts(tmem_acc, ab + j * 8, ptx::smem_desc_sw128(xb + j * 32), idesc, (kt > sg.kb || j > 0) ? 1u : 0u);
+              ptx::mma_i8_ts(tmem_base, tmem_base + Cfg<BN>::kACol + t * 32 + j * 8,
+                             ptx::smem_desc_sw128(xs + t * kXStage + j * 32), idesc, (t > 0 || j > 0) ? 1u : 0u);
+            if (t + NT < nk) ptx::tc_commit(bar_afree + 8 * t);   // a later k-tile takes this stage
           }
-          TR_ADD(tr_issue, tr_i1);
-          const long long tr_i2 = TR_NOW();
-          if (leader) ptx::tc_commit(bar_afree + 8 * ring.s);   // frees the operand stage and its token slice
-          TR_ADD(tr_commit, tr_i2);
-          ring.advance();
         }
-        if (leader) ptx::tc_commit(bar_accfull + 8 * p);
-        ++seg;
       }
-      if (leader) {
-        TR_SET(3, tr_wa);
-        TR_SET(4, TR_NOW() - tr_m0);
-        TR_SET(10, tr_issue);
-        TR_SET(11, tr_commit);
+      __syncwarp();
+      int t = 0;
+      uint32_t ph = 1;
+      for (int i = NT; i < nk; ++i) {
+        if (ok && !ptx::mbar_wait_bounded(bar_aready + 8 * t, ph, kWaitLimitNs)) {
+          if (leader) atomicExch(args.status, 403);
+          ok = false;
+        }
+        __syncwarp();
+        ptx::tc_fence_after();
+        if (leader) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            ptx::mma_i8_ts(tmem_base, tmem_base + Cfg<BN>::kACol + t * 32 + j * 8,
+                           ptx::smem_desc_sw128(xs + i * kXStage + j * 32), idesc, 1u);
+          if (i + NT < nk) ptx::tc_commit(bar_afree + 8 * t);
+        }
+        if (++t == NT) {
+          t = 0;
+          ph ^= 1u;
+        }
       }
+      if (leader) ptx::tc_commit(bar_acc);
     }
     __syncwarp();
-    // tensor memory is released after every role is done
-    ptx::tc_fence_before();
-    __syncthreads();
+    // Tensor memory is released as soon as the accumulator has been read, ahead of the join.
+    asm volatile("bar.sync 4, %0;" ::"n"(32 + kDequant) : "memory");
     ptx::tc_fence_after();
-    ptx::tmem_dealloc(tmem_base, C::kTmemCols);
-    return;
+    ptx::tmem_dealloc(tmem_base, kTmemCols);
   } else {
-    // ------------------------------------------------------------------ dequant sets, then epilogues
+    // ------------------------------------------------------------------ dequant sets: unpack, tokens, join
     const int d = threadIdx.x - 64;
-    const int set = d >> 7;                   // takes the k-tiles whose running index is set (mod 2); owns accumulator `set`
+    const int set = d >> 7;                   // takes k-tiles set, set + 2, ...
     const int quad = warp & 3;                // tensor-memory lane quadrant this warp may access
     const int row = quad * 32 + lane;         // weight row inside the tile == tensor-memory lane
     const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
+    const bool scaled = args.out_mode != kOutI32;
+    const bool has_bias = scaled && args.bias != nullptr;
+    auto all_sets = []() { asm volatile("bar.sync 3, %0;" ::"n"(kDequant) : "memory"); };
+    // Token rows past M are zero; channel scales and bias are weights.
+    if (M < BN) {
+      const int chunks = (BN - M) * 8;
+      for (int i = d; i < nk * chunks; i += kDequant)
+        *reinterpret_cast<uint4*>(smem + (i / chunks) * kXStage + M * 128 + (i % chunks) * 16) = make_uint4(0u, 0u, 0u, 0u);
+    }
+    if (d < rows_own) {
+      const long n = (long)tile * 128 + fb * 8 + d;
+      chan_scale[d] = (scaled && n < args.N) ? __ldg(args.s1 + n) : 0.f;
+      chan_bias[d] = (has_bias && n < args.N) ? load_bias(args.bias, n, args.out_mode) : 0.f;
+    }
     asm volatile("bar.sync 2, %0;" ::"n"(32 + kDequant) : "memory");
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot_p;
-    const uint32_t tmem_a = tmem_base + C::kAccCols + lane_addr;
-    // Token slice of a k-tile: BN rows of 128 bytes.  Thread j of the owning set moves 16-byte chunk
-    // (j & 7) of token rows (j >> 3) + 16 q; in the 128-byte swizzle chunk c of row r sits at chunk
-    // c ^ (r & 7) of that row.  Rows past M are zero.
-    const int jx = d & 127;
-    const int x_row = jx >> 3;
-    const uint32_t x_off = (uint32_t)(x_row * 128 + (((jx & 7) ^ (x_row & 7)) << 4));
-    const int8_t* x_src = args.x + (size_t)x_row * args.K + (jx & 7) * 16;
-    Ring<NW> rw;   // weight ring position
-    Ring<NT> rt;   // operand ring position
+    const uint32_t tmem_a = tmem_base + Cfg<BN>::kACol + lane_addr;
     bool ok = true;
-    TR_VAR(tr_wfull);
-    TR_VAR(tr_flush);
-    TR_VAR(tr_unpack);
-    TR_VAR(tr_afree);
-    TR_VAR(tr_st);
-    TR_VAR(tr_epi);
-    const long long tr_d0 = TR_NOW();
-    if (d == 0) {
-      TR_SET(13, ptx::globaltimer_ns());
-      uint32_t smid;
-      asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
-      TR_SET(15, smid);
-    }
-    uint32_t step = 0;   // running k-tile index of this CTA
-    uint32_t seg = 0;
-    bool waited_dependency = false;
-    SegInfo mine = {0, 0, 0, true, 0.f, 0.f};   // the last segment that went into this set's accumulator
-    const bool scaled = args.out_mode != kOutI32;
-    const bool has_bias = scaled && args.bias != nullptr;
-
-    // Epilogue of segment number `s` (accumulator s & 1 == set), described by `si`.
-    auto epilogue = [&](const SegInfo& si, uint32_t s) {
-      const uint32_t p = s & 1u;
-      if (ok && !ptx::mbar_wait_bounded(bar_accfull + 8 * p, (s >> 1) & 1u, kWaitLimitNs)) {
-        atomicExch(args.status, 405);
+    int i = set;                                  // k-tile
+    uint32_t stage = (uint32_t)(set % NW), ph = (uint32_t)(set / NW) & 1u;   // its ring stage and the pass over the ring
+    uint32_t t = (uint32_t)set, tph = 1u;         // its operand stage
+    const uint8_t* const my_row = smem + lay.ws + row * 16;
+    const uint8_t* const my_meta = smem + lay.ws + 8192 + row * 4;
+    // One k-tile of this thread's weight row: nibbles and (step, offset) -> 128 INT8 ...
+    uint32_t v[32];
+    auto unpack = [&]() {
+      if (ok && !ptx::mbar_wait_bounded(bar_wfull + 8 * stage, ph, kWaitLimitNs)) {
+        atomicExch(args.status, 404);
         ok = false;
       }
-      __syncwarp();
-      ptx::tc_fence_after();
-      if (!waited_dependency) {
-        dependency_wait();   // token scales, outputs and the reduction workspace belong to earlier kernels until here
-        waited_dependency = true;
+      const uint8_t* p = my_row + stage * kTileBytes;
+      uint4 ch[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) ch[c] = *reinterpret_cast<const uint4*>(p + c * 2048);
+      const uint32_t meta = *reinterpret_cast<const uint32_t*>(my_meta + stage * kTileBytes);
+      ptx::mbar_arrive(bar_wfree + 8 * stage);   // the tile is in registers: its stage may be refilled
+      stage += kSets;
+      if (stage >= (uint32_t)NW) {
+        stage -= (uint32_t)NW;
+        ph ^= 1u;
       }
-      const long n = (long)si.tile * 128 + row;
-      const bool n_ok = n < args.N;
-      const float w_scale = si.w_scale, bias = si.bias;
-      unsigned long long* slot = args.slots + (size_t)si.slot * (BN * 128);
-      const long long nk = si.nk;
-      const uint32_t tmem_acc = tmem_base + p * BN + lane_addr;
-#pragma unroll 1
-      for (int c0 = 0; c0 < BN; c0 += 16) {
-        if (c0 >= args.M) break;   // uniform over the warp
-        int v[16];
-        ptx::tmem_ld16(tmem_acc + c0, v);
-        ptx::tc_wait_ld();
-        if (c0 + 16 >= BN || c0 + 16 >= args.M) {   // last chunk: the accumulator may be reused
-          __syncwarp();
-          ptx::tc_fence_before();
-          ptx::mbar_arrive(bar_accfree + 8 * p);
-        }
-        if (!n_ok) continue;
-        float sc[16];
+      const uint32_t step0 = meta & 0xffu, a0 = __byte_perm(meta, 0u, 0x1111);
+      const uint32_t step1 = __byte_perm(meta, 0u, 0x4442), a1 = __byte_perm(meta, 0u, 0x3333);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) sc[j] = tok_scale[set * BN + c0 + j];   // staged at the set's first k-tile
-        if (!si.whole) {
-          // One returning 64-bit atomic per element does the cross-CTA reduction: the word holds the
-          // k-tiles added so far (bits 40..) and the sum of the contributions, each biased by 2^21 per
-          // k-tile so that it is non-negative and never borrows from the count.  The thread whose add
-          // completes the tile's count holds the full sum in the value it got back: it stores the
-          // output and re-zeroes the word.  No fence, no counter, no read-back.
-          unsigned long long old[16];
+      for (int c = 0; c < 4; ++c) {
+        const uint32_t st = c < 2 ? step0 : step1;
+        const uint32_t ab = c < 2 ? a0 : a1;
+        const uint32_t pk[4] = {ch[c].x, ch[c].y, ch[c].z, ch[c].w};
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const unsigned long long add = (unsigned long long)((long long)v[j] + (nk << 21)) |
-                                           ((unsigned long long)nk << 40);
-            old[j] = (c0 + j < args.M) ? atomicAdd(slot + (c0 + j) * 128 + row, add) : 0ull;
-          }
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const bool done = (c0 + j < args.M) && ((long long)(old[j] >> 40) + nk == (long long)kt_total);
-            if (done) {
-              __stcg(slot + (c0 + j) * 128 + row, 0ull);
-              v[j] = (int)((long long)(old[j] & ((1ull << 40) - 1)) + (long long)v[j] + (nk << 21) -
-                           ((long long)kt_total << 21));
-            } else {
-              sc[j] = __int_as_float(0x7fc00000);   // marks "not finished here"
-            }
-          }
-        }
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          if (c0 + j < args.M && (si.whole || sc[j] == sc[j])) {
-            if (!scaled) {
-              reinterpret_cast<int32_t*>(args.out)[(size_t)(c0 + j) * args.N + n] = v[j];
-            } else {
-              const float y = lqq_scale(v[j], sc[j], w_scale);
-              if constexpr (MULTI) store_out_all(multi.out, c0 + j, n, y, bias, has_bias, args.out_mode);
-              else store_out_bias(args.out, (size_t)(c0 + j) * args.N + n, y, bias, has_bias, args.out_mode);
-            }
-          }
+        for (int h = 0; h < 4; ++h) {
+          v[8 * c + 2 * h] = lqq_dequant4(pk[h] & 0x0F0F0F0Fu, st, ab);
+          v[8 * c + 2 * h + 1] = lqq_dequant4((pk[h] >> 4) & 0x0F0F0F0Fu, st, ab);
         }
       }
     };
+    // ... -> tensor memory: the operand of k-tile i.
+    auto store_operand = [&]() {
+      if (i >= NT && ok && !ptx::mbar_wait_bounded(bar_afree + 8 * t, tph, kWaitLimitNs)) {
+        atomicExch(args.status, 406);
+        ok = false;
+      }
+      __syncwarp();
+      if (i >= NT) ptx::tc_fence_after();
+      ptx::tmem_st32(tmem_a + t * 32, v);
+      ptx::tc_wait_st();
+      ptx::tc_fence_before();
+      ptx::mbar_arrive(bar_aready + 8 * t);
+      i += kSets;
+      t += kSets;
+      if (t >= (uint32_t)NT) {
+        t -= NT;
+        tph ^= 1u;
+      }
+    };
 
-    for (;;) {
-      const bool more = walk.next(sg);
-      // One place decides which finished segment this set reads out now.  While the stream runs: the
-      // segment two back, just before its accumulator (this set's) takes a new one.  After the last
-      // segment: whichever of the last two segments sits in this set's accumulator -- the two sets
-      // finish the CTA's last two segments side by side.
-      uint32_t epi = 0xffffffffu;
-      if (more) {
-        if (seg >= 2 && (int)(seg & 1u) == set) epi = seg - 2;
-      } else if (seg >= 1 && (int)((seg - 1u) & 1u) == set) {
-        epi = seg - 1;
-      } else if (seg >= 2) {
-        epi = seg - 2;
-      }
-      if (epi != 0xffffffffu) {
-        const long long tr_e1 = TR_NOW();
-        epilogue(mine, epi);
-        TR_ADD(tr_epi, tr_e1);
-      }
-      if (!more) break;
-      if ((int)(seg & 1u) == set) {
-        // channel scale and bias are weights: fetched here, far from the epilogue that needs them
-        const long n = (long)sg.tile * 128 + row;
-        const bool n_ok = n < args.N;
-        mine = SegInfo{sg.tile, sg.ke - sg.kb, sg.slot, sg.whole, (n_ok && scaled) ? __ldg(args.s1 + n) : 0.f,
-                       (n_ok && has_bias) ? load_bias(args.bias, n, args.out_mode) : 0.f};
-      }
+    // ---- before the wait for the previous kernel: operands of the first NT k-tiles, and one more in the set's registers
 #pragma unroll 1
-      for (int kt = sg.kb; kt < sg.ke; ++kt, ++step, rw.advance(), rt.advance()) {
-        if ((int)(step & 1u) != set) continue;
-        if (!waited_dependency) {
-          dependency_wait();   // the tokens (and later the outputs) belong to earlier kernels until here
-          waited_dependency = true;
-          // Token scales (an earlier kernel's output) go to shared memory once per set; the epilogue, which
-          // this set runs much later and under time pressure, reads them from there.
-          if (jx < BN) tok_scale[set * BN + jx] = (scaled && jx < args.M) ? __ldg(args.ascale + jx) : 0.f;
-          if (set == 0) asm volatile("bar.sync 5, 128;" ::: "memory");
-          else asm volatile("bar.sync 6, 128;" ::: "memory");
-          if constexpr (MULTI) {
-            // tokens gathered from peer GPUs: one thread waits for their flags on behalf of its set
-            if ((d & 127) == 0 && !peer_wait(multi.sync, kPeerWaitLimitNs)) atomicExch(args.status, 409);
-            if (set == 0) asm volatile("bar.sync 3, 128;" ::: "memory");
-            else asm volatile("bar.sync 4, 128;" ::: "memory");
-          }
-        }
-        // request this k-tile's tokens now (L2 hits); they are stored after the unpack
-        uint4 xv[BN / 16];
-#pragma unroll
-        for (int q = 0; q < BN / 16; ++q)
-          xv[q] = (x_row + 16 * q < args.M) ? ldg_stream_v4(x_src + (size_t)(16 * q) * args.K + (size_t)kt * 128)
-                                            : make_uint4(0u, 0u, 0u, 0u);
-        const long long tr_w0 = TR_NOW();
-        if (ok && !ptx::mbar_wait_bounded(bar_wfull + 8 * rw.s, rw.ph, kWaitLimitNs)) {
-          atomicExch(args.status, 404);
-          ok = false;
-        }
-        TR_ADD(tr_wfull, tr_w0);
-        const long long tr_u0 = TR_NOW();
-        const uint8_t* wst = smem + (ws - base) + rw.s * kTileBytes;
-        uint4 ch[4];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) ch[c] = *reinterpret_cast<const uint4*>(wst + (c * 128 + row) * 16);
-        const uint32_t meta = *reinterpret_cast<const uint32_t*>(wst + 8192 + row * 4);
-        ptx::mbar_arrive(bar_wfree + 8 * rw.s);   // the tile is in registers: its stage may be refilled
-        // unpack into registers first, wait for the operand stage afterwards
-        const uint32_t step0 = meta & 0xffu, a0 = ((meta >> 8) & 0xffu) * 0x01010101u;
-        const uint32_t step1 = (meta >> 16) & 0xffu, a1 = (meta >> 24) * 0x01010101u;
-        uint32_t v[32];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const uint32_t st = c < 2 ? step0 : step1;
-          const uint32_t ab = c < 2 ? a0 : a1;
-          const uint32_t pk[4] = {ch[c].x, ch[c].y, ch[c].z, ch[c].w};
-#pragma unroll
-          for (int h = 0; h < 4; ++h) {
-            v[8 * c + 2 * h] = lqq_dequant4(pk[h] & 0x0F0F0F0Fu, st, ab);
-            v[8 * c + 2 * h + 1] = lqq_dequant4((pk[h] >> 4) & 0x0F0F0F0Fu, st, ab);
-          }
-        }
-#ifdef LQ_PIPELINE_TRACE
-        if (v[0] == 0x12345678u && v[31] == 0x9abcdef0u) TR_SET(8, 1);   // pins the arithmetic before the timer
-#endif
-        TR_ADD(tr_unpack, tr_u0);
-        const long long tr_f0 = TR_NOW();
-        if (ok && !ptx::mbar_wait_bounded(bar_afree + 8 * rt.s, rt.ph ^ 1u, kWaitLimitNs)) {
-          atomicExch(args.status, 406);
-          ok = false;
-        }
-        TR_ADD(tr_afree, tr_f0);
-        __syncwarp();
-        ptx::tc_fence_after();
-        const long long tr_s0 = TR_NOW();
-        ptx::tmem_st32(tmem_a + rt.s * 32, v);   // one store instruction for the whole operand stage row
-#pragma unroll
-        for (int q = 0; q < BN / 16; ++q)
-          *reinterpret_cast<uint4*>(smem + rt.s * C::kXStage + x_off + q * 2048) = xv[q];
-        // Wait for the operand store at once.  (Leaving it in flight during the next unpack and arriving
-        // afterwards was measured: 1-3 % slower here, 10-30 % slower in the prefill kernel -- "operand ready"
-        // one unpack later starves the MMAs more than the store's latency costs the thread.)
-        ptx::tc_wait_st();
-        TR_ADD(tr_st, tr_s0);
-        const long long tr_s2 = TR_NOW();
-        // the token slice was written with ordinary stores: make it visible to the tensor core's reads
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        ptx::tc_fence_before();
-        ptx::mbar_arrive(bar_aready + 8 * rt.s);
-        TR_ADD(tr_flush, tr_s2);
-      }
-      ++seg;
+    while (i < min(nk, NT)) {
+      unpack();
+      store_operand();
     }
+    if (i < nk) unpack();
 
-    if (d == 0) {
-      TR_SET(2, tr_flush);
-      TR_SET(12, tr_unpack);
-      TR_SET(5, tr_wfull);
-      TR_SET(6, tr_afree);
-      TR_SET(7, tr_st);
-      TR_SET(8, TR_NOW() - tr_d0);
-      TR_SET(9, tr_epi);
-      TR_SET(14, ptx::globaltimer_ns());
+    // ---- the previous kernel is done: the tokens of the whole k-range
+    if (d == 0) DT_STAMP(1);   // operands of the first stages done
+    dependency_wait();   // tokens, token scales and outputs belong to earlier kernels until here
+    if (d == 0) DT_STAMP(2);
+    if constexpr (MULTI) {
+      // tokens gathered from peer GPUs: one thread waits for their flags on behalf of the others
+      if (d == 0 && !peer_wait(multi.sync, kPeerWaitLimitNs)) atomicExch(args.status, 409);
+      all_sets();
+    }
+    // In the 128-byte swizzle chunk c (16 bytes) of token row r sits at chunk c ^ (r & 7) of that row.
+    if constexpr (!QUANT) {
+      const int jx = d & 127;
+      const int x_row = jx >> 3;
+      const uint32_t x_off = (uint32_t)(x_row * 128 + (((jx & 7) ^ (x_row & 7)) << 4));
+      const int8_t* src = static_cast<const int8_t*>(args.x) + (size_t)x_row * args.K + (size_t)kb * 128 + (jx & 7) * 16;
+      if (d < M) tok_scale[d] = scaled ? __ldg(args.ascale + d) : 0.f;
+      constexpr int Q = BN / 16, U = Q == 1 ? 8 : 4;
+#pragma unroll 1
+      for (int j0 = set; j0 < nk; j0 += kSets * U) {
+        uint4 xv[U][Q];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+          for (int q = 0; q < Q; ++q)
+            if (j0 + kSets * u < nk && x_row + 16 * q < M)
+              xv[u][q] = ldg_stream_v4(src + (size_t)(16 * q) * args.K + (size_t)(j0 + kSets * u) * 128);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+          for (int q = 0; q < Q; ++q)
+            if (j0 + kSets * u < nk && x_row + 16 * q < M)
+              *reinterpret_cast<uint4*>(smem + (j0 + kSets * u) * kXStage + x_off + q * 2048) = xv[u][q];
+      }
+    } else {
+      // Up to eight tokens, one or more warps a row (wpr); a lane takes every 32 * wpr-th chunk of sixteen activations of
+      // the CTA's k-range and keeps the first H of them in registers until the row's scale is known.
+      constexpr int H = sizeof(XT) == 4 ? 2 : 4;
+      const int m = (d >> 5) / wpr, part = (d >> 5) % wpr;
+      const int c0 = part * 32 + lane, cstep = 32 * wpr, nch = m < M ? nk * 8 : 0;
+      const XT* x = static_cast<const XT*>(args.x) + (size_t)m * args.K + (size_t)kb * 128;
+      Chunk<XT> held[H];
+#pragma unroll
+      for (int h = 0; h < H; ++h) {
+        const int c = c0 + h * cstep;
+        if (c < nch) held[h].load(x + (size_t)c * 16);
+        else held[h].clear();
+      }
+      RowMax<XT> rm;
+#pragma unroll
+      for (int h = 0; h < H; ++h)
+#pragma unroll
+        for (int k = 0; k < (int)sizeof(XT); ++k) rm.take(held[h].r[k]);
+#pragma unroll 2
+      for (int c = c0 + H * cstep; c < nch; c += cstep) {
+        Chunk<XT> ck;
+        ck.load(x + (size_t)c * 16);
+#pragma unroll
+        for (int k = 0; k < (int)sizeof(XT); ++k) rm.take(ck.r[k]);
+      }
+      // The maxima of the row's parts (warps of all CTAs of the cluster) go to every CTA; non-negative floats are ordered
+      // like their bits.
+      const uint32_t top = __reduce_max_sync(0xffffffffu, __float_as_uint(rm.value()));
+      const int np = S * wpr;
+      if (m < M && lane < S) {
+        const uint32_t slot = parts + (uint32_t)((m * np + rank * wpr + part) * 16);
+        if (S == 1) asm volatile("st.shared.b32 [%0], %1;" ::"r"(slot), "r"(top) : "memory");
+        else ptx::st_async_v4(ptx::map_to_cta(slot, (uint32_t)lane), (int)top, 0, 0, 0, ptx::map_to_cta(bar_amax, (uint32_t)lane));
+      }
+      if (S == 1) {
+        all_sets();
+      } else if (ok && !ptx::mbar_wait_bounded_cluster(bar_amax, 0u, kWaitLimitNs)) {
+        atomicExch(args.status, 407);
+        ok = false;
+      }
+      if (m < M) {   // uniform over the warp
+        uint32_t mine = 0u;
+        for (int k = lane; k < np; k += 32) {
+          uint32_t t;
+          asm volatile("ld.shared.b32 %0, [%1];" : "=r"(t) : "r"(parts + (uint32_t)((m * np + k) * 16)) : "memory");
+          mine = max(mine, t);
+        }
+        const float scale = token_scale(__uint_as_float(__reduce_max_sync(0xffffffffu, mine)));
+        const float inv = __frcp_rn(scale);
+        if (c0 == 0) tok_scale[m] = scale;
+        uint8_t* dst = smem + m * 128;
+        auto put = [&](int c, uint4 q) {
+          *reinterpret_cast<uint4*>(dst + (c >> 3) * kXStage + (((c & 7) ^ (m & 7)) << 4)) = q;
+        };
+#pragma unroll
+        for (int h = 0; h < H; ++h)
+          if (c0 + h * cstep < nch) put(c0 + h * cstep, held[h].quantised(scale, inv));
+#pragma unroll 2
+        for (int c = c0 + H * cstep; c < nch; c += cstep) {
+          Chunk<XT> ck;
+          ck.load(x + (size_t)c * 16);
+          put(c, ck.quantised(scale, inv));
+        }
+      }
+    }
+    // written with ordinary stores: make the tokens visible to the tensor core's reads
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    ptx::mbar_arrive(bar_x);
+    if (d == 0) DT_STAMP(3);   // tokens in place
+#pragma unroll 1
+    while (i < nk) {
+      store_operand();
+      if (i < nk) unpack();
+    }
+    all_sets();   // token scales (and everything above) before the epilogue of any thread
+
+    // ---- epilogue: a set takes every other eight columns (tokens)
+    const int units = rows_own * groups;       // (four tokens, channel) sums that this CTA joins
+    int g = d / rows_own, r = d - g * rows_own;
+    const int owner = ((row >> 3) * S) >> 4;   // the CTA that joins this thread's channel
+    const uint32_t peer_bar = ptx::map_to_cta(bar_join, (uint32_t)owner);
+    const uint32_t peer_row = ptx::map_to_cta(join, (uint32_t)owner) +
+                              (uint32_t)((rank * (BN / 4) * rows_max + row - 8 * join_first_block(owner, S)) * 16);
+    if (ok && !ptx::mbar_wait_bounded(bar_acc, 0u, kWaitLimitNs)) {
+      atomicExch(args.status, 405);
+      ok = false;
+    }
+    __syncwarp();
+    ptx::tc_fence_after();
+    if (d == 0) DT_STAMP(4);   // accumulator final
+    // One channel of four consecutive tokens: scale (or not) and store.
+    auto emit4 = [&](int r, int m0, int4 sum) {
+      const long n = (long)tile * 128 + fb * 8 + r;
+      if (n >= args.N) return;
+      const float w_scale = chan_scale[r], bias = chan_bias[r];
+      const int v[4] = {sum.x, sum.y, sum.z, sum.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (m0 + j >= M) break;
+        if (!scaled) {
+          reinterpret_cast<int32_t*>(args.out)[(size_t)(m0 + j) * args.N + n] = v[j];
+        } else {
+          const float y = lqq_scale(v[j], tok_scale[m0 + j], w_scale);
+          if constexpr (MULTI) store_out_all(multi.out, m0 + j, n, y, bias, has_bias, args.out_mode);
+          else store_out_bias(args.out, (size_t)(m0 + j) * args.N + n, y, bias, has_bias, args.out_mode);
+        }
+      }
+    };
+#pragma unroll 1
+    for (int c0 = 8 * set; c0 < BN; c0 += 8 * kSets) {
+      if (c0 >= M) break;   // uniform over the set
+      int v[8];
+      __syncwarp();
+      ptx::tmem_ld8(tmem_base + lane_addr + c0, v);
+      ptx::tc_wait_ld();
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        if (c0 + 4 * h >= M) break;
+        if (S == 1) emit4(row, c0 + 4 * h, make_int4(v[4 * h], v[4 * h + 1], v[4 * h + 2], v[4 * h + 3]));
+        else
+          ptx::st_async_v4(peer_row + (uint32_t)((c0 / 4 + h) * rows_max * 16), v[4 * h], v[4 * h + 1], v[4 * h + 2],
+                           v[4 * h + 3], peer_bar);
+      }
+    }
+    __syncwarp();
+    ptx::tc_fence_before();
+    asm volatile("bar.arrive 4, %0;" ::"n"(32 + kDequant) : "memory");
+    if (S > 1) {
+      if (ok && !ptx::mbar_wait_bounded_cluster(bar_join, 0u, kWaitLimitNs)) {
+        atomicExch(args.status, 408);
+        ok = false;
+      }
+      if (d == 0) DT_STAMP(5);   // sums landed
+      for (int u = d; u < units; u += kDequant) {
+        if (u != d) {
+          g = u / rows_own;
+          r = u - g * rows_own;
+        }
+        const int4* p = reinterpret_cast<const int4*>(smem + lay.join) + g * rows_max + r;
+        int4 sum = p[0];
+#pragma unroll 4
+        for (int k = 1; k < S; ++k) {
+          const int4 w = p[k * (BN / 4) * rows_max];
+          sum.x += w.x; sum.y += w.y; sum.z += w.z; sum.w += w.w;
+        }
+        emit4(r, 4 * g, sum);
+      }
     }
     if constexpr (MULTI) {
       // Every output store of this CTA, including those into peer memory, is ordered before the flags:
       // the barrier makes the other threads' stores visible to thread 0 (CTA scope), and the release of
       // its system-scope reduction is cumulative over them.
-      asm volatile("bar.sync 1, %0;" ::"n"(kDequant) : "memory");
-      if (d == 0) {
-        peer_signal(multi.sync);   // red.release.sys: ordered after everything the barrier made visible
-      }
+      all_sets();
+      if (d == 0) peer_signal(multi.sync);   // red.release.sys: ordered after everything the barrier made visible
+    }
+    if (d == 0) DT_STAMP(6);   // outputs stored
+    // Whoever has waited for the cluster's sums has nothing of its shared memory accessed any more and may exit.  A thread
+    // whose wait expired stays until the other CTAs' threads have done the same or exited.
+    if (S > 1 && !ok) {
+      ptx::cluster_arrive();
+      ptx::cluster_wait();
     }
   }
-  ptx::tc_fence_before();
-  __syncthreads();
 }
 
-template <int BN, int NW, int NT, bool MULTI>
-static int launch(const Args& a, const MultiOut* multi, int grid, cudaStream_t st) {
-  using C = Cfg<BN, NW, NT>;
-  auto kern = &w4a8_decode_tc_kernel<BN, NW, NT, MULTI>;
+struct Plan {
+  int tiles, splits, nk, ring, smem;   // ring 0: not a shape for this kernel
+};
+// Which shapes the kernel takes and how it cuts them.  Two launches have to fit the machine side by side (one CTA of each
+// per SM), or the second loses the head start that the design lives from: at most one CTA per SM, and at most 128
+// where clusters of three and more leave slots of a GPC empty (6144 x 4096 at 8 tokens: 2 / 3 / 4 / 6 k-ranges a tile
+// = 96 / 144 / 192 / 288 CTAs 6.0 / 6.8 / 6.5 / 10.4 us).  Within that as many k-ranges as there is room for (4096 x 4096: 3 / 4 ranges
+// 4.8 / 4.4; 2048 x 8192: 4 / 5 / 8 6.0 / 5.4 / 4.9).  A k-range is at most 16 k-tiles (8 above 16 tokens): the tokens of the
+// range stay in shared memory, and k-tiles beyond those unpacked ahead cost 0.2 us each behind the tokens (4096 x 14336 in 28s:
+// 9.8 us against the tile kernel's 9.9 with its finish pass; 7168 x 8192 in 32s 12.2 against 9.7).
+static Plan plan_for(int M, int N, int K) {
+  const int bn = M <= 16 ? 16 : 32;
+  const int kt = K / 128;
+  Plan p = {};
+  p.tiles = (N + 127) / 128;
+  const int sms = sm_count();
+  int S = sms / p.tiles;
+  if (S >= 3) S = (sms - sms / 8) / p.tiles > 2 ? (sms - sms / 8) / p.tiles : 2;
+  if (S > kMaxSplits) S = kMaxSplits;
+  if (S > kt / 4) S = kt / 4 > 1 ? kt / 4 : 1;
+  if (S == 1 && kt > 16 && p.tiles <= sms && bn == 16) S = 2;
+  if (S < 1) return p;
+  p.splits = S;
+  p.nk = (kt + S - 1) / S;
+  if (p.nk > (bn == 16 ? 16 : 8)) return p;
+  // The ring holds the whole k-range, or an even number of stages: a stage then always belongs to the same dequant set.
+  // (Otherwise a set could meet a stage whose previous tile, the other set's, has not landed yet, and the parity of
+  // the pass before would let it through.)
+  for (int ring = p.nk <= kMaxRing ? p.nk : kMaxRing; ring >= 1; --ring) {
+    if (ring < p.nk && (ring & 1)) continue;
+    p.smem = layout(bn, p.nk, ring, S).total + 1024;
+    if (p.smem <= kSmemLimit) {
+      p.ring = ring;
+      break;
+    }
+  }
+  // more than a third of the SM's shared memory, so that never three CTAs (of this and of the next kernels, under
+  // programmatic dependent launch) share an SM: the third would wait for tensor memory
+  if (p.smem < 78 * 1024) p.smem = 78 * 1024;
+  return p;
+}
+
+template <int BN, bool MULTI, typename XT>
+static int launch(const Args& a, const MultiOut* multi, const Plan& p, cudaStream_t st) {
+  auto kern = &w4a8_decode_tc_kernel<BN, MULTI, XT>;
   static std::once_flag once[64];
   int dev = 0;
   cudaGetDevice(&dev);
   cudaError_t e = cudaSuccess;
   std::call_once(once[dev & 63], [&]() {
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
   });
   if (e == cudaSuccess) {
-    if constexpr (MULTI) e = launch_overlapped(kern, dim3(grid), dim3(kThreads), (size_t)C::kSmemBytes, st, a, *multi);
-    else e = launch_overlapped(kern, dim3(grid), dim3(kThreads), (size_t)C::kSmemBytes, st, a, NoMultiOut{});
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(p.tiles * p.splits);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = (size_t)p.smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (p.splits > 1) {
+      attr[n].id = cudaLaunchAttributeClusterDimension;
+      attr[n].val.clusterDim.x = p.splits;
+      attr[n].val.clusterDim.y = 1;
+      attr[n++].val.clusterDim.z = 1;
+    }
+    if (pdl_enabled()) {
+      attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    if constexpr (MULTI) e = cudaLaunchKernelEx(&cfg, kern, a, *multi);
+    else e = cudaLaunchKernelEx(&cfg, kern, a, NoMultiOut{});
   }
   if (e != cudaSuccess) {
     record_cuda_error(e, "w4a8_decode_tc_kernel launch");
@@ -535,32 +661,42 @@ static int launch(const Args& a, const MultiOut* multi, int grid, cudaStream_t s
   return check_launch("w4a8_decode_tc_kernel");
 }
 
-static int bn_for(int M) { return M <= 16 ? 16 : 32; }
-
-static DecodePlan plan_for(int N, int K) { return decode_plan((N + 127) / 128, K / 128, 2 * sm_count(), false); }
-
 }  // namespace dtc
+
+bool decode_tc_serves(int M, int N, int K) {
+  return M >= 1 && M <= 32 && N >= 1 && K >= 128 && K % 128 == 0 && dtc::plan_for(M, N, K).ring > 0;
+}
+
+// Whether it also quantises its tokens: three to eight, one CTA per SM at most.  Below, the quantising GEMV is ahead (two
+// tokens 1280 x 8192 5.0 against 5.1 us, 6144 x 4096 6.8 against 6.8, one token 4096 x 4096 4.8 against 5.2); above, the pass over the
+// activations costs more than the quantiser's launch (4096 x 4096 at 16 tokens 6.2 us behind the quantiser, 7.6 here; at eight 6.1 and
+// 5.7), and so it does where two CTAs share an SM (12800 x 2560 at eight tokens 8.1 and 9.0).
+bool decode_tc_quantises(int M, int N, int K) {
+  if (M < 3 || M > dtc::kQuantTokens || !decode_tc_serves(M, N, K)) return false;
+  const dtc::Plan p = dtc::plan_for(M, N, K);
+  return p.tiles * p.splits <= sm_count();
+}
+
+// What callers are told to bring for this kernel (all zero, left all zero).  It is not used: the join stays inside the
+// cluster.  The size and the check of it are those of the kernel that joined through global memory.
+size_t decode_tc_workspace_bytes(int M) { return (size_t)(2 * sm_count()) * (size_t)((M <= 16 ? 16 : 32) * 128 * 8); }
 
 // CTAs a launch of this shape uses: what a consumer of the gather-by-stores epilogue must see arrive
 // from every rank.
-int decode_tc_grid(int N, int K) { return dtc::plan_for(N, K).grid; }
-
-size_t decode_tc_workspace_bytes(int M, int N, int K) {
-  (void)N;
-  (void)K;
-  return (size_t)(2 * sm_count()) * (size_t)(dtc::bn_for(M) * 128 * 8);   // one slot per resident CTA
+int decode_tc_grid(int M, int N, int K) {
+  const dtc::Plan p = dtc::plan_for(M, N, K);
+  return p.tiles * p.splits;
 }
 
-// out_mode: LQ_DT_* or 3 (raw int32).  M <= 32.  `ws`: decode_tc_workspace_bytes(), all zero, left all zero.
-int run_decode_tc(const int8_t* x, const uint8_t* blob, const float* ascale, const float* s1, const void* bias,
-                  const OutSpec& out, const PeerSync* sync, int out_mode, int M, int N, int K, void* ws,
-                  size_t ws_bytes, cudaStream_t st) {
+// x_dtype: LQ_DT_* of activations to quantise, or -1 for int8 tokens with their scales.  out_mode: LQ_DT_* or 3 (raw int32).
+int run_decode_tc(const void* x, int x_dtype, const uint8_t* blob, const float* ascale, const float* s1, const void* bias,
+                  const OutSpec& out, const PeerSync* sync, int out_mode, int M, int N, int K, void* ws, size_t ws_bytes,
+                  cudaStream_t st) {
   using namespace dtc;
-  if (M < 1 || M > 32) return LQ_ERR_SHAPE;
-  if (!ws || ws_bytes < decode_tc_workspace_bytes(M, N, K)) return LQ_ERR_WORKSPACE;
-  const int bn = bn_for(M);
-  const DecodePlan plan = plan_for(N, K);
-  const int grid = plan.grid;
+  if (M < 1 || M > (x_dtype >= 0 ? kQuantTokens : 32)) return LQ_ERR_SHAPE;
+  if (!ws || ws_bytes < decode_tc_workspace_bytes(M)) return LQ_ERR_WORKSPACE;
+  const Plan plan = plan_for(M, N, K);
+  if (plan.ring == 0) return LQ_ERR_SHAPE;
   Args a;
   a.blob = blob;
   a.x = x;
@@ -569,32 +705,35 @@ int run_decode_tc(const int8_t* x, const uint8_t* blob, const float* ascale, con
   a.bias = bias;
   // one plain destination with nothing to signal or wait for: the small-parameter kernels
   const bool multi = out.n != 1 || out.ld != N || out.col0 != 0 || (sync && (sync->n_signal > 0 || sync->wait));
-  if (multi && out_mode == kOutI32) return LQ_ERR_BAD_ARG;
+  if (multi && (out_mode == kOutI32 || x_dtype >= 0)) return LQ_ERR_BAD_ARG;
   a.out = out.ptr[0];
-  a.slots = static_cast<unsigned long long*>(ws);
   a.status = status_word();
   a.out_mode = out_mode;
   a.M = M;
   a.N = N;
   a.K = K;
-  a.fixed_split = plan.fixed_split;
+  a.splits = plan.splits;
+  a.ring = plan.ring;
   if (!a.status) return LQ_ERR_CUDA;
+  if (x_dtype == LQ_DT_BF16) return launch<16, false, __nv_bfloat16>(a, nullptr, plan, st);
+  if (x_dtype == LQ_DT_F16) return launch<16, false, __half>(a, nullptr, plan, st);
+  if (x_dtype == LQ_DT_F32) return launch<16, false, float>(a, nullptr, plan, st);
   if (!multi) {
-    if (bn == 16) return launch<16, 8, 7, false>(a, nullptr, grid, st);
-    return launch<32, 8, 6, false>(a, nullptr, grid, st);
+    if (M <= 16) return launch<16, false, int8_t>(a, nullptr, plan, st);
+    return launch<32, false, int8_t>(a, nullptr, plan, st);
   }
   MultiOut mo;
   mo.out = out;
   mo.sync = sync ? *sync : PeerSync{};
-  if (bn == 16) return launch<16, 8, 7, true>(a, &mo, grid, st);
-  return launch<32, 8, 6, true>(a, &mo, grid, st);
+  if (M <= 16) return launch<16, true, int8_t>(a, &mo, plan, st);
+  return launch<32, true, int8_t>(a, &mo, plan, st);
 }
 
 }  // namespace lq
 
 #ifdef LQ_PIPELINE_TRACE
-// Copies the per-CTA counters of the last launches (1024 CTAs x 16 slots of int64) to host memory.
+// Copies the per-CTA stamps of the last launch (1024 CTAs x 8 slots of int64) to host memory.
 extern "C" LQ_API int lq_debug_read_decode_trace(long long* host_dst) {
-  return cudaMemcpyFromSymbol(host_dst, lq::dtc::g_trace, sizeof(long long) * 1024 * 16) == cudaSuccess ? 0 : -4;
+  return cudaMemcpyFromSymbol(host_dst, lq::dtc::g_trace, sizeof(long long) * 1024 * 8) == cudaSuccess ? 0 : -4;
 }
 #endif

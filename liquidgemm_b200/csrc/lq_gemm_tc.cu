@@ -58,10 +58,12 @@ int run_tile_gemm(const int8_t* x, const uint8_t* blob, const float* ascale, con
                   const OutSpec& out, const PeerSync* sync, int out_mode, int M, int N, int K, int splits, void* ws,
                   size_t ws_bytes, cudaStream_t st);  // lq_gemm_tile.cu
 int tile_output_grid(int M, int N, int K, int splits);                            // lq_gemm_tile.cu
-size_t decode_tc_workspace_bytes(int M, int N, int K);                       // lq_decode_tc.cu
-int run_decode_tc(const int8_t* x, const uint8_t* blob, const float* ascale, const float* s1, const void* bias,
-                  const OutSpec& out, const PeerSync* sync, int out_mode, int M, int N, int K, void* ws,
-                  size_t ws_bytes, cudaStream_t st);  // lq_decode_tc.cu
+bool decode_tc_serves(int M, int N, int K);                                  // lq_decode_tc.cu
+bool decode_tc_quantises(int M, int N, int K);                               // lq_decode_tc.cu
+size_t decode_tc_workspace_bytes(int M);                                     // lq_decode_tc.cu
+int run_decode_tc(const void* x, int x_dtype, const uint8_t* blob, const float* ascale, const float* s1, const void* bias,
+                  const OutSpec& out, const PeerSync* sync, int out_mode, int M, int N, int K, void* ws, size_t ws_bytes,
+                  cudaStream_t st);  // lq_decode_tc.cu
 size_t gemv_blob_workspace_bytes(int N, int K);                              // lq_gemv_blob.cu
 int run_gemv_blob_ws(const int8_t* x, const uint8_t* blob, const float* ascale, const float* s1, const void* bias,
                      const OutSpec& out, const PeerSync* sync, int out_dtype, int M, int N, int K, void* ws,
@@ -69,7 +71,7 @@ int run_gemv_blob_ws(const int8_t* x, const uint8_t* blob, const float* ascale, 
 bool gemv_quant_serves(int M, int N, int K);                                 // lq_gemv_blob.cu
 int run_gemv_quant(const void* x, int x_dtype, const uint8_t* blob, const float* s1, const void* bias, void* out,
                    int out_dtype, int M, int N, int K, void* ws, size_t ws_bytes, cudaStream_t st);   // lq_gemv_blob.cu
-int decode_tc_grid(int N, int K);                                            // lq_decode_tc.cu
+int decode_tc_grid(int M, int N, int K);                                      // lq_decode_tc.cu
 bool pair_serves(int M, int N, int K);                                       // lq_gemm_pair.cu
 bool i8_pair_serves(int M, int N, int K);                                    // lq_i8_pair.cu
 int run_i8_pair_gemm(const int8_t* x, const int8_t* w, const float* ascale, const float* s1, const void* bias, void* out,
@@ -682,13 +684,11 @@ struct Route {
 // uses tensor cores.
 constexpr int kGemvBlobMaxM = 4;
 
-// Largest decode batch of the single-launch streaming tensor-core kernel: its one-atomic-per-element
-// join is cheap only while a CTA holds few tokens.  LQ_DECODE_TC_MAX_M (16 or 32) moves the limit for
-// measurements.
+// Largest batch of the single-launch decode kernel; LQ_DECODE_TC_MAX_M (16 or 32; 0: none) lowers it for measurements.
 static int decode_tc_max_m() {
   static const int v = []() {
     const char* e = getenv("LQ_DECODE_TC_MAX_M");
-    const int n = e ? atoi(e) : 16;
+    const int n = e ? atoi(e) : 32;
     return n <= 0 ? 0 : n >= 32 ? 32 : 16;
   }();
   return v;
@@ -719,10 +719,12 @@ static int gemv_max_m() {   // LQ_GEMV_MAX_M (0..4) lowers the limit of both for
   return cap;
 }
 
+static bool decode_serves(int M, int N, int K) { return M <= decode_tc_max_m() && decode_tc_serves(M, N, K); }
+
 static bool gemv_serves(int M, int N, int K) {
   if (M > gemv_max_m()) return false;
   const long w = (long)N * K;
-  return M == 1 || (M == 2 && w <= (1L << 26)) || (M <= kGemvBlobMaxM && w <= (1L << 24));
+  return M == 1 || (M == 2 && w <= (1L << 26)) || (M <= kGemvBlobMaxM && w <= (1L << 24) && !decode_serves(M, N, K));
 }
 
 // Large token counts on layers the INT8 pair kernel serves: unpacking the whole blob to INT8 once (a pass over
@@ -751,10 +753,9 @@ static Route route_for(int M, int N, int K, int splitk, bool scaled, bool single
   if (M <= 128) {
     if (splitk == 0) {
       if (scaled && gemv_serves(M, N, K)) return {kRouteGemv, 0};
-      // Small matrices (up to 32 M weights) only: on larger ones the tile kernel's whole tiles (or its planes
-      // and finish pass) are ahead since the MMA issue became cheap (28672 x 4096 at 8 tokens: 14.7 vs 16.7 us,
-      // 4096 x 14336: 10.4 vs 10.8 us; 6144 x 4096: 7.3 vs 7.0 us, 4096 x 4096: 6.6 vs 6.0 us).
-      if (M <= decode_tc_max_m() && (long)N * K <= (1L << 25)) return {kRouteDecodeTc, 0};
+      // What fits one CTA per SM (lq_decode_tc.cu); larger matrices are ahead on the tile kernel's whole tiles (or its
+      // planes and finish pass).
+      if (decode_serves(M, N, K)) return {kRouteDecodeTc, 0};
     }
     // int32 outputs where the scaled call takes the GEMV: callers are told one kind of workspace for both, the all-zero
     // buffer, so the tile kernel must not write its planes there.
@@ -777,7 +778,7 @@ static Route route_for(int M, int N, int K, int splitk, bool scaled, bool single
 static size_t route_ws_bytes(const Route& r, int M, int N, int K) {
   switch (r.kind) {
     case kRouteGemv: return gemv_blob_workspace_bytes(N, K);
-    case kRouteDecodeTc: return decode_tc_workspace_bytes(M, N, K);
+    case kRouteDecodeTc: return decode_tc_workspace_bytes(M);
     case kRouteTile: return tile_workspace_bytes(M, N, r.splits);
     case kRoutePair: return pair_workspace_bytes(M, N, K);
     case kRouteUnpackI8: return (size_t)N * K;   // scratch: the INT8 weights
@@ -822,7 +823,7 @@ static int blob_gemm(const int8_t* x, const uint8_t* blob, const float* ascale, 
     case kRouteGemv:
       return run_gemv_blob_ws(x, blob, ascale, s1, bias, single_out(out, N), nullptr, out_mode, M, N, K, ws, ws_bytes, st);
     case kRouteDecodeTc:
-      return run_decode_tc(x, blob, ascale, s1, bias, single_out(out, N), nullptr, out_mode, M, N, K, ws, ws_bytes, st);
+      return run_decode_tc(x, -1, blob, ascale, s1, bias, single_out(out, N), nullptr, out_mode, M, N, K, ws, ws_bytes, st);
     case kRouteTile:
       return run_tile_gemm(x, blob, ascale, s1, bias, single_out(out, N), nullptr, out_mode, M, N, K, r.splits, ws,
                            ws_bytes, st);
@@ -870,6 +871,10 @@ static bool quantises_in_gemv(const void* x, int M, int N, int K, int splitk) {
 
 static size_t token_scratch_bytes(int M, int K) { return (((size_t)M * K + 255) & ~(size_t)255) + (size_t)M * 4; }
 
+static bool quantises_in_decode(const void* x, int M, int N, int K, int splitk) {
+  return splitk == 0 && M <= decode_tc_max_m() && decode_tc_quantises(M, N, K) && reinterpret_cast<uintptr_t>(x) % 16 == 0;
+}
+
 int lq_linear_plan(const void* x, int M, int N, int K, int splitk, size_t* plan) {
   if (!plan || M <= 0 || N <= 0) return LQ_ERR_BAD_ARG;
   if (K < 128 || K % 128) return LQ_ERR_SHAPE;
@@ -893,6 +898,12 @@ static int linear_impl(const void* x, int x_dtype, const uint8_t* blob, const fl
     return run_gemv_quant(x, x_dtype, blob, s1, bias, y, out_dtype, M, N, K, workspace, workspace_bytes, as_stream(stream));
   }
   if (!scratch || reinterpret_cast<uintptr_t>(scratch) % 16 || scratch_bytes < token_scratch_bytes(M, K)) return LQ_ERR_WORKSPACE;
+  // One kernel again, without need of the scratch and workspace that the two launches take: callers are told the same sizes.
+  if (quantises_in_decode(x, M, N, K, splitk)) {
+    if (!workspace || workspace_bytes < decode_tc_workspace_bytes(M)) return LQ_ERR_WORKSPACE;
+    if (int rc = lq_check_device()) return rc;
+    return run_decode_tc(x, x_dtype, blob, nullptr, s1, bias, single_out(y, N), nullptr, out_dtype, M, N, K, workspace, workspace_bytes, as_stream(stream));
+  }
   int8_t* xq = static_cast<int8_t*>(scratch);
   float* ascale = reinterpret_cast<float*>(xq + (((size_t)M * K + 255) & ~(size_t)255));
   if (int rc = lq_quant_per_token(x, x_dtype, xq, ascale, M, K, stream)) return rc;
@@ -953,7 +964,7 @@ int lq_w4a8_gemm_fused_scatter_sync(const int8_t* x_i8, const uint8_t* blob, con
       return run_gemv_blob_ws(x_i8, blob, ascale, s1, nullptr, o, &ps, out_dtype, M, N, K, workspace, workspace_bytes,
                               as_stream(stream));
     case kRouteDecodeTc:
-      return run_decode_tc(x_i8, blob, ascale, s1, nullptr, o, &ps, out_dtype, M, N, K, workspace, workspace_bytes,
+      return run_decode_tc(x_i8, -1, blob, ascale, s1, nullptr, o, &ps, out_dtype, M, N, K, workspace, workspace_bytes,
                            as_stream(stream));
     case kRoutePair:
       return run_pair_gemm(x_i8, blob, ascale, s1, nullptr, o, &ps, out_dtype, M, N, K, workspace, workspace_bytes,
@@ -986,7 +997,7 @@ int lq_decode_grid(int M, int N, int K) {
   const Route r = route_for(M, N, K, 0, true, false);
   switch (r.kind) {
     case kRouteGemv: return gemv_blob_grid(N, K);
-    case kRouteDecodeTc: return decode_tc_grid(N, K);
+    case kRouteDecodeTc: return decode_tc_grid(M, N, K);
     case kRoutePair: return pair_grid(M, N, K);
     default: return tile_output_grid(M, N, K, r.splits);
   }

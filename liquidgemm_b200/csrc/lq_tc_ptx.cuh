@@ -169,6 +169,13 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, int (&v)[16]) {
       : "r"(taddr)
       : "memory");
 }
+// The same for 8 columns.
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, int (&v)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "r"(taddr)
+               : "memory");
+}
 
 // ---- issuing thread -------------------------------------------------------------------------------
 // One lane of the converged warp (the same one every time it is asked).  The MMA-issuing role runs its loop
@@ -259,6 +266,9 @@ __device__ __forceinline__ uint32_t cluster_id_x() {
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// The two halves of a cluster barrier for threads that need not be converged; each thread arrives once per phase.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 // Address of the same shared-memory location in CTA `rank` of the cluster (shared::cluster window).
 __device__ __forceinline__ uint32_t map_to_cta(uint32_t saddr, uint32_t rank) {
   uint32_t r;
@@ -274,6 +284,14 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
 // (The cluster-scope release costs the arriving thread about 1000 cycles.)
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// Sixteen bytes to shared memory of any CTA of the cluster, counted, in bytes, on a barrier of that
+// same CTA (addresses from map_to_cta); visible to whoever waits for that barrier with acquire at cluster scope.
+__device__ __forceinline__ void st_async_v4(uint32_t cluster_addr, int a, int b, int c, int d, uint32_t cluster_bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(
+                   cluster_addr),
+               "r"(a), "r"(b), "r"(c), "r"(d), "r"(cluster_bar)
+               : "memory");
 }
 // Bounded wait on a barrier of this CTA whose arrivals may come from the peer CTA (acquire at cluster scope).
 __device__ __forceinline__ bool mbar_wait_bounded_cluster(uint32_t bar, uint32_t parity, uint64_t limit_ns) {

@@ -11,7 +11,7 @@
     python -m liquidgemm_b200.microbench tma_rows     # the same with one bulk copy per weight row
 
     python -m liquidgemm_b200.build --trace           # once: the product sources with -DLQ_PIPELINE_TRACE
-    python -m liquidgemm_b200.microbench decode_trace gate_up 8   # per-CTA cycle counters of the decode kernel
+    python -m liquidgemm_b200.microbench decode_trace o 8         # time stamps of every CTA of the decode kernel
     python -m liquidgemm_b200.microbench pair_trace gate_up 8192  # the same for the CTA-pair prefill kernel
     python -m liquidgemm_b200.microbench tile_trace gate_up 8     # time stamps of every CTA of the tile kernel
 
@@ -266,10 +266,10 @@ def tma_rows(total_bytes: int = 400_000_000) -> None:
               f"cycles/stage {float(np.median(cyc.cpu().numpy())) / steps:7.1f}", flush=True)
 
 
-def decode_trace(shape: str = "gate_up", M: int = 8) -> None:
-    """Per-CTA cycle counters of ``w4a8_decode_tc_kernel`` on one Llama-3.1-8B shape (trace build of the
-    library): median / 10th / 90th percentile over the CTAs of the last launch of a graph of back-to-back
-    launches over rotating weight copies.  Counters are sums over the k-tiles a role handled."""
+def decode_trace(shape: str = "o", M: int = 8) -> None:
+    """%globaltimer stamps of every CTA of ``w4a8_decode_tc_kernel`` on one Llama-3.1-8B shape (trace build of the
+    library) for the last launch of a graph of back-to-back launches over rotating weight copies: nanoseconds
+    around the return of the wait for the previous kernel."""
     if os.environ.get("LIQUIDGEMM_B200_TRACE") != "1":
         import subprocess
         env = dict(os.environ, LIQUIDGEMM_B200_TRACE="1")
@@ -282,26 +282,18 @@ def decode_trace(shape: str = "gate_up", M: int = 8) -> None:
     layers = [B.device_lqq(N, K, seed=31 * c + 1, want_gp=False) for c in range(C)]
     x, sc = B.device_tokens(M, K, seed=M)
     t = B.graph_time_us(lambda i: B.linear_call(layers[i % C], x, sc, M), C, 3)
-    buf = (ctypes.c_longlong * (1024 * 16))()
+    buf = (ctypes.c_longlong * (1024 * 8))()
     plib.lq_debug_read_decode_trace.argtypes = [ctypes.c_void_p]
     assert plib.lq_debug_read_decode_trace(buf) == 0
-    a = np.frombuffer(buf, dtype=np.int64).reshape(1024, 16)[:plib.lq_decode_grid(M, N, K)]
-    names = {0: "producer: waiting for a free weight stage", 1: "producer: whole loop",
-             3: "MMA thread: waiting for operands", 4: "MMA thread: whole loop", 10: "MMA thread: issuing 4 MMAs",
-             11: "MMA thread: commit", 5: "dequant thread: waiting for the weight tile",
-             12: "dequant thread: shared loads + unpack", 7: "dequant thread: tcgen05.st + token store + wait::st",
-             2: "dequant thread: proxy fence + arrive", 6: "dequant thread: waiting for the operand stage",
-             9: "dequant thread: epilogues", 8: "dequant thread: whole role (incl. wait for the previous kernel)"}
-    print(f"{shape} {N}x{K}, M = {M}: {t:.2f} us per launch (trace build), {len(a)} CTAs; cycles per CTA")
+    a = np.frombuffer(buf, dtype=np.int64).reshape(1024, 8)[:plib.lq_decode_grid(M, N, K)]
+    t0 = a[:, 2].min()
+    names = {0: "CTA start", 1: "operands of the first k-tiles unpacked",
+             2: "previous kernel complete (griddepcontrol.wait returned)", 3: "tokens in place", 4: "accumulator final",
+             5: "the cluster's sums landed", 6: "outputs stored"}
+    print(f"{shape} {N}x{K}, M = {M}: {t:.2f} us per launch (trace build), {len(a)} CTAs; ns after the first CTA's wait")
     for slot, label in names.items():
-        col = a[:, slot]
-        print(f"  {label:62s} median {int(np.median(col)):7d}   p10 {int(np.percentile(col, 10)):7d}   "
-              f"p90 {int(np.percentile(col, 90)):7d}")
-    t0 = a[:, 13].min()
-    for label, col in (("CTA start", a[:, 13]), ("CTA end", a[:, 14])):
-        c = col - t0
-        print(f"  {label:10s} ns after the first CTA's start: min {int(c.min())}  median {int(np.median(c))}  "
-              f"max {int(c.max())}")
+        col = a[:, slot] - t0
+        print(f"  {label:58s} min {int(col.min()):6d}   median {int(np.median(col)):6d}   max {int(col.max()):6d}")
 
 
 def tile_trace(shape: str = "gate_up", M: int = 8) -> None:
@@ -394,7 +386,7 @@ if __name__ == "__main__":
     torch.cuda.set_device(0)
     if len(sys.argv) > 1 and sys.argv[1] in ("decode_trace", "pair_trace", "tile_trace"):
         fn = {"decode_trace": decode_trace, "pair_trace": pair_trace, "tile_trace": tile_trace}[sys.argv[1]]
-        fn(*(sys.argv[2:3] or ["gate_up"]), *(int(v) for v in sys.argv[3:4]))
+        fn(*sys.argv[2:3], *(int(v) for v in sys.argv[3:4]))
         sys.exit(0)
     which = sys.argv[1:] or list(_CASES)
     for name in which:

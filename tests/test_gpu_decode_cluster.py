@@ -1,0 +1,68 @@
+"""The decode tensor-core kernel whose k-ranges meet inside a thread-block cluster: int8 tokens against the oracle, and its
+quantising form against the token quantiser followed by the same operator.  Tolerance: none (exact integer sums)."""
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import lqq_oracle as O
+from tests.helpers import assert_bits_equal, random_lqq, random_tokens, to_torch_qw, with_bias_f32
+
+pytestmark = pytest.mark.gpu
+
+# k-tiles x k-ranges: one k-tile; fewer k-tiles than operand stages, as many and one more; every cluster size up to eight
+# with even and odd ranges; a ring shorter than the range; ragged N; whole tiles up to one per SM; two CTAs per SM
+SHAPES = [(128, 128), (64, 896), (200, 1024), (320, 2176), (1000, 1920), (2048, 2048), (3072, 4224), (3840, 3072), (6144, 640),
+          (512, 14336), (6144, 4096), (8960, 2048), (9600, 1152), (18944, 512), (12800, 2560)]
+TOKENS = [3, 8, 9, 16, 17, 32]
+
+
+@pytest.mark.parametrize("N,K", SHAPES)
+def test_int8_tokens_match_the_oracle(N, K):
+    from liquidgemm_b200 import ops
+    qw = random_lqq(N, K, seed=N + K)
+    tq = to_torch_qw(qw)
+    blob = ops._repack_device(tq.qweight_u4, 0, tq.s_u8, tq.offset_a, N, K, 64).reshape(-1)
+    w = (qw.qweight_u4.astype(np.int32) * np.repeat(qw.s_u8, 64, 1) + np.repeat(qw.offset_a, 64, 1).astype(np.int32) - 128)
+    rng = np.random.default_rng(N)
+    for M in TOKENS:
+        x, sc = random_tokens(M, K, seed=M)
+        acc = (x.astype(np.float64) @ w.astype(np.float64).T).astype(np.int64).astype(np.int32)   # below 2^53: exact
+        xt, st = torch.from_numpy(x).cuda(), torch.from_numpy(sc).cuda()
+        assert np.array_equal(ops.gemm_i32(xt, blob, N, K).cpu().numpy(), acc), M
+        y = O.scale_f32(acc, sc, qw.s1)
+        for code in (0, 1, 2):
+            assert_bits_equal(ops.gemm_fused(xt, blob, st, tq.s1, N, K, code), y, code, f"{M}x{N}x{K}")
+        bias = torch.from_numpy(rng.standard_normal(N).astype(np.float32)).cuda().to(torch.bfloat16)
+        got = ops.linear_bias(xt, blob, st, tq.s1, bias, N, K, 0)
+        assert_bits_equal(got, with_bias_f32(y, bias.cpu().view(torch.int16).numpy().view(np.uint16), 0), 0, f"bias {M}x{N}x{K}")
+    ops.poll_status()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("N,K", SHAPES)
+def test_quantising_form_equals_two_launches(N, K, dtype):
+    """Maxima in every part of the cluster's k-range, a zero row, infinities, NaN and halves between two integers."""
+    from liquidgemm_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    qw, blob = ops.quantize_weight_cuda(torch.randn(N, K, generator=g, device="cuda") * 0.03, 64, want_codes=False, want_blob=True)
+    L = {"s1": qw.s1, "s_u8": qw.s_u8, "offset_a": qw.offset_a, "N": N, "K": K, "rs": blob.reshape(-1)}
+    code = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}[dtype]
+    raw = torch.int32 if dtype == torch.float32 else torch.int16
+    for M in (3, 4, 5, 7, 8):
+        x = torch.randn(M, K, generator=g, device="cuda")
+        for m in range(M):
+            x[m, (m * K) // M] = 9.0 + m
+        x[0] = torch.arange(K, device="cuda").remainder(255) / 2 - 63.5   # scale 1/2 exactly: halves everywhere
+        x[1] = 0.0
+        x[2, K // 2], x[2, 3] = float("inf"), float("nan")
+        x = x.to(dtype)
+        xq, sc = torch.ops.liquidgemm.quant_per_token(x)
+        want = torch.ops.liquidgemm.w4a8_wgmma_rs_fused(xq, L["rs"], L["s_u8"], L["offset_a"], sc, L["s1"], N, K, 64, code) \
+            if N % 64 == 0 else ops.gemm_fused(xq, L["rs"], sc, L["s1"], N, K, code)
+        bias = torch.randn(N, device="cuda").to(dtype)
+        if N % 64 == 0:
+            assert torch.equal(ops.w4a8_linear(x, L).view(raw), want.view(raw)), M
+        got = torch.ops.liquidgemm.w4a8_linear(x, L["rs"], L["s_u8"], L["offset_a"], L["s1"], bias, N, K, 64, code)
+        assert torch.equal(got.view(raw), (want + bias).view(raw)), M
+    ops.poll_status()
