@@ -5,7 +5,7 @@
 // gather for the prepack (liquidgemm/ops.py:118-150).
 //
 // Rows that a CTA can hold (aligned, up to 65536 elements; float32 32768) take quantise_rows_kernel, one pass over the
-// weights: 28672 x 4096 bf16 481 -> 83 us, 4096 x 14336 273 -> 51 us against the two passes below, which serve the rest:
+// weights: 28672 x 4096 bf16 481 -> 80 us, 4096 x 14336 273 -> 51 us against the two passes below, which serve the rest:
 //   pass 1  row_amax_kernel      one warp per row: s1 = max(amax, 1e-12) / 119 (IEEE division)
 //   pass 2  quantise_tiles_kernel one CTA per 128 x 128 tile of the weight matrix, thread = (row, 64-wide half):
 //             q    = clamp(rint(w / s1[row]), -119, 119)                       (level 1, :70-72)
@@ -103,9 +103,11 @@ quantise_rows_kernel(const T* __restrict__ w, float* __restrict__ s1, uint8_t* _
       }
       if (!round_quotients(x, inv, t[o])) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          t[o][j].x = kRoundMagic + (float)max(-119, min(119, __float2int_rn(__fdiv_rn(x[j].x, scale))));
-          t[o][j].y = kRoundMagic + (float)max(-119, min(119, __float2int_rn(__fdiv_rn(x[j].y, scale))));
+        for (int j = 0; j < 4; ++j) {   // one element, nearly always
+          if (!near_integer(x[j].x, inv))
+            t[o][j].x = kRoundMagic + (float)max(-119, min(119, __float2int_rn(__fdiv_rn(x[j].x, scale))));
+          if (!near_integer(x[j].y, inv))
+            t[o][j].y = kRoundMagic + (float)max(-119, min(119, __float2int_rn(__fdiv_rn(x[j].y, scale))));
         }
       }
 #pragma unroll
