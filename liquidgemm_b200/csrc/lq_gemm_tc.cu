@@ -530,36 +530,15 @@ int make_byte_matrix_map(CUtensorMap* map, const void* ptr, long rows, long row_
   return LQ_OK;
 }
 
-// Tensor map over tokens [M, K] as [K / 128][M][128] with a box of `box_kts` k-tiles x box_rows tokens x 128 bytes: one copy
-// brings the slices of several k-tiles, each with the 128-byte swizzle; tokens and k-tiles out of range read as zero.
-int make_token_map(CUtensorMap* map, const void* ptr, long M, long K, int box_rows, int box_kts) {
-  EncodeTiledFn fn = encode_fn();
-  if (!fn) {
-    record_cuda_error(cudaErrorUnknown, "cuTensorMapEncodeTiled entry point not found");
-    return LQ_ERR_CUDA;
-  }
-  const cuuint64_t dims[3] = {128u, (cuuint64_t)M, (cuuint64_t)(K / 128)};
-  const cuuint64_t strides[2] = {(cuuint64_t)K, 128u};
-  const cuuint32_t box[3] = {128u, (cuuint32_t)box_rows, (cuuint32_t)box_kts};
-  const cuuint32_t estr[3] = {1u, 1u, 1u};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(ptr), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    record_cuda_error(cudaErrorInvalidValue, "cuTensorMapEncodeTiled failed");
-    return LQ_ERR_CUDA;
-  }
-  return LQ_OK;
-}
-
 static int pick_bn(int M, int K = 0) {
   (void)K;
   if (M <= 16) return 16;
   if (M <= 32) return 32;
   if (M <= 64) return 64;
   if (M <= 128) return 128;
-  // Two 192-token accumulators.  (A single 256-token accumulator with five stages raised launch failures: an odd ring with
-  // two dequant sets, whose waits can pass on a stage that has not landed.)
+  // Two 192-token accumulators.  A single 256-token accumulator (5 stages) measured 20-40 % faster
+  // on long-K shapes but produced intermittent launch failures on a 8192 x 28672 layer; it stays
+  // off until the cause is understood.
   return 192;
 }
 
@@ -690,7 +669,7 @@ enum RouteKind {
   kRoutePersistent,   // one CTA per SM, stream-K or a fixed split (explicit requests above 128 tokens, splitk -1)
   kRouteTile,         // two CTAs per SM, one tile each, `splits` int32 planes + finish pass when splits > 1
   kRouteGemv,         // streaming dp4a GEMV over the blob (scaled outputs only)
-  kRouteDecodeTc,     // small matrices: k-ranges of a tile in a thread-block cluster, one launch
+  kRouteDecodeTc,     // streaming tensor-core kernel, one launch, atomic join
   kRoutePair,         // CTA pairs, 256 channels x 192 tokens per tile (prefill)
   kRouteUnpackI8,     // very large token counts: unpack the blob to INT8 once, then the INT8 x INT8 pair kernel
 };

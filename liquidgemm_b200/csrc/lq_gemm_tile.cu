@@ -12,14 +12,12 @@
 // (float)acc * ascale[m] * s1[n] (the reference's design, csrc/liquid_gemm/w4a8_wgmma.cu:39-56,
 // 523-534); with one split the epilogue is fused in the GEMM kernel.
 //
-// Per CTA: warp 0 = weight producer (8704-byte bulk copies), warp 10 = token producer (boxes of BN x 128 tokens of two or
-// four k-tiles; a box per k-tile queued behind the weights in the copy engine, 28672 x 4096 at 16 tokens 15.8 -> 15.0 us),
-// warp 1 = TMEM allocation and tcgen05.mma issue (the warp walks the loop, one elected lane issues; A operand from tensor
-// memory), warps 2..5 and 6..9 = two dequant sets taking alternate k-tiles (thread r of a set owns weight row r -> TMEM lane
-// r; one set alone needs ~800 cycles per k-tile, more than the MMAs of two CTAs), then epilogue, the sets sharing the
-// accumulator's columns.  The weights run ahead of the tokens: they are unpacked into up to six operand stages before the
-// previous kernel has ended.  All waits are bounded.  Behind the token quantiser, us before -> now at 32 / 64 / 128 tokens:
-// 28672 x 4096 16.2 / 18.1 / 22.6 -> 15.1 / 16.3 / 19.3, 4096 x 14336 12.9 / 14.9 / 17.3 -> 12.5 / 14.6 / 16.6.
+// Per CTA: warp 0 = TMA producer (8704-byte bulk copy of the weight tile + BN x 128 token box per
+// k-step), warp 1 = TMEM allocation and tcgen05.mma issue (the warp walks the loop, one elected lane issues; A
+// operand from tensor memory), warps
+// 2..5 and 6..9 = two dequant sets taking alternate k-steps (thread r of a set owns weight row r ->
+// TMEM lane r; one set alone needs ~800 cycles per k-step, more than the MMAs of two CTAs), then
+// epilogue, the sets sharing the accumulator's columns.  All waits are bounded.
 #include <cuda.h>
 
 #include <cstdlib>
@@ -33,14 +31,19 @@ namespace lq {
 
 int launch_finish(const int32_t* acc, const float* ascale, const float* s1, const void* bias, const OutSpec& out,
                   const PeerSync* sync, int out_dtype, int planes, int M, int N, cudaStream_t st);  // lq_elementwise.cu
-int make_token_map(CUtensorMap* map, const void* ptr, long M, long K, int box_rows, int box_kts);  // lq_gemm_tc.cu
+int make_byte_matrix_map(CUtensorMap* map, const void* ptr, long rows, long row_bytes, int box_rows,
+                         int box_bytes);  // lq_gemm_tc.cu
 
 namespace tile {
 
 constexpr int kTileBytes = 8704;
-// Dequant sets of 128 threads, taking k-tiles round-robin.  Two keep up with the MMAs of two CTAs per SM.
+constexpr int kI8TileBytes = 16384;
+// Dequant sets of 128 threads, taking k-tiles round-robin.  Two keep up with the MMAs of two CTAs per
+// SM.  A build with three (448 threads per CTA) ended its first benchmark run with an unspecified launch
+// failure whose cause reading the code did not show; it is not used and must not be tried again
+// without an explanation.
 constexpr int kSets = 2;
-constexpr int kThreads = 64 + 128 * kSets + 32;
+constexpr int kThreads = 64 + 128 * kSets;
 constexpr uint64_t kWaitLimitNs = 2000000000ull;
 constexpr int kOutI32 = kEpiI32;
 
@@ -70,50 +73,47 @@ struct GemmArgs {
   int vec_out;           // 2-byte outputs whose rows allow 16-byte stores: stage the tile through shared memory
 };
 
-// NW weight stages, NX token stages of G k-tiles each, NP pairs of operand stages in tensor memory (one of either set).
-template <int BN, int NW, int NX, int G, int NP>
+template <int BN, int NS, int NT, bool W4>
 struct TcCfg {
-  static constexpr int kXTile = BN * 128;
-  static constexpr int kXStage = G * kXTile;
-  static constexpr int kACol = BN < 32 ? 32 : BN;   // operand stages behind the accumulator
-  static constexpr int kTmemCols = 256;
-  static constexpr int kNumBars = 2 * NW + 2 * NX + 2 * NP + 1;
-  static constexpr int kBarBytes = kNumBars * 8 + 8;
+  static constexpr int kXStage = BN * 128;
+  static constexpr int kWStage = W4 ? kTileBytes : kI8TileBytes;
+  static constexpr int kAccCols = BN;
+  static constexpr int kACols = W4 ? 32 * NT : 0;
+  static constexpr int kColsNeeded = kAccCols + kACols;
+  static constexpr int kTmemCols = kColsNeeded <= 32 ? 32 : kColsNeeded <= 64 ? 64 : kColsNeeded <= 128 ? 128
+                                   : kColsNeeded <= 256 ? 256 : 512;
+  static constexpr int kBarBytes = (2 * NS + 2 * NT + 1) * 8 + 8;
   static constexpr int kOutStage = 16 * 128 * 2;   // per dequant set: 16 tokens x 128 channels of 2-byte outputs
-  static constexpr int kSmemBytes = 1024 /* alignment slack */ + NX * kXStage + NW * kTileBytes + kBarBytes + 16 +
+  static constexpr int kSmemBytes = 1024 /* alignment slack */ + NS * (kXStage + kWStage) + kBarBytes + 16 +
                                     kSets * kOutStage;
-  static_assert(G % kSets == 0, "a pair of k-tiles shares a token stage");
-  static_assert(kACol + 64 * NP <= kTmemCols, "two CTAs per SM share the tensor memory");
-  static_assert(kSmemBytes <= 113 * 1024, "two CTAs per SM share the shared memory");
-  // A stage always belongs to the same dequant set.  Otherwise a set could meet a stage whose previous tile, another
-  // set's, has not landed yet, and the parity of the pass before would let it through.
-  static_assert(NW % kSets == 0, "stages are tied to sets");
+  static_assert(kColsNeeded <= 512, "tensor memory budget exceeded");
 };
 
-template <int BN, int NW, int NX, int G, int NP, bool MULTI>
-__global__ void __launch_bounds__(kThreads, 2)
+template <int BN, int NS, int NT, bool W4, bool MULTI>
+__global__ void __launch_bounds__(kThreads, 1)
 w4a8_tile_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmArgs args,
                  const std::conditional_t<MULTI, MultiOut, NoMultiOut> multi) {
-  using Cfg = TcCfg<BN, NW, NX, G, NP>;
+  // Only the blob-fed form exists, so the kernel takes one tensor map (the tokens).
+  static_assert(W4, "the tile kernel reads its weights from the tile blob");
+  using Cfg = TcCfg<BN, NS, NT, W4>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   const uint32_t base = (raw_addr + 1023u) & ~1023u;
   uint8_t* smem = smem_raw + (base - raw_addr);
 
-  const uint32_t xs = base;                                  // NX token stages (1024-aligned)
-  const uint32_t ws = xs + NX * Cfg::kXStage;                // NW weight stages
-  const uint32_t bars = ws + NW * kTileBytes;                // barriers
-  const uint32_t bar_wfull = bars;                           // [NW] weight tile landed
-  const uint32_t bar_wfree = bar_wfull + NW * 8;             // [NW] the dequant set holds the tile in registers
-  const uint32_t bar_xfull = bar_wfree + NW * 8;             // [NX] token box landed
-  const uint32_t bar_xfree = bar_xfull + NX * 8;             // [NX] the MMAs that read it are done
-  const uint32_t bar_aready = bar_xfree + NX * 8;            // [NP] a pair of unpacked operands in tensor memory
-  const uint32_t bar_afree = bar_aready + NP * 8;            // [NP] the MMAs that read it are done
-  const uint32_t bar_acc = bar_afree + NP * 8;               // accumulators final
+  const uint32_t xs = base;                                  // NS activation stages (1024-aligned)
+  const uint32_t ws = xs + NS * Cfg::kXStage;                // NS weight stages
+  const uint32_t bars = ws + NS * Cfg::kWStage;              // barriers
+  const uint32_t bar_full = bars;                            // [NS] TMA landed
+  const uint32_t bar_empty = bars + NS * 8;                  // [NS] stage may be overwritten
+  const uint32_t bar_aready = bars + 2 * NS * 8;             // [NT] dequantised operand in TMEM
+  const uint32_t bar_afree = bars + (2 * NS + NT) * 8;       // [NT] MMAs that read the operand are done
+  const uint32_t bar_acc = bars + (2 * NS + 2 * NT) * 8;     // accumulators final
   const uint32_t tmem_slot = bar_acc + 8;
   uint8_t* gen = smem + (bars - base);
-  volatile uint32_t* tmem_slot_p = reinterpret_cast<volatile uint32_t*>(gen + Cfg::kNumBars * 8);
+  volatile uint32_t* tmem_slot_p = reinterpret_cast<volatile uint32_t*>(gen + (2 * NS + 2 * NT + 1) * 8);
   uint8_t* out_stage = gen + ((Cfg::kBarBytes + 15) & ~15);   // 16-byte aligned (`bars` is)
+
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nt = blockIdx.x, mt = blockIdx.y, z = blockIdx.z, splits = gridDim.z;
@@ -124,17 +124,13 @@ w4a8_tile_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmArgs args
   const int m0 = mt * BN;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < NW; ++s) {
-      ptx::mbar_init(bar_wfull + 8 * s, 1);
-      ptx::mbar_init(bar_wfree + 8 * s, 128);
+    for (int s = 0; s < NS; ++s) {
+      ptx::mbar_init(bar_full + 8 * s, 1);
+      ptx::mbar_init(bar_empty + 8 * s, W4 ? 129 : 1);
     }
-    for (int s = 0; s < NX; ++s) {
-      ptx::mbar_init(bar_xfull + 8 * s, 1);
-      ptx::mbar_init(bar_xfree + 8 * s, 1);
-    }
-    for (int p = 0; p < NP; ++p) {
-      ptx::mbar_init(bar_aready + 8 * p, 128 * kSets);
-      ptx::mbar_init(bar_afree + 8 * p, 1);
+    for (int t = 0; t < NT; ++t) {
+      ptx::mbar_init(bar_aready + 8 * t, 128);
+      ptx::mbar_init(bar_afree + 8 * t, 1);
     }
     ptx::mbar_init(bar_acc, 1);
     ptx::fence_mbar_init();
@@ -149,105 +145,86 @@ w4a8_tile_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmArgs args
   ptx::tc_fence_after();
   allow_dependents();   // the next kernel of the stream may start prefetching its weights
   const uint32_t tmem_base = *tmem_slot_p;
-  const uint32_t tmem_acc = tmem_base;                   // columns [0, BN)
-  const uint32_t tmem_a = tmem_base + Cfg::kACol;        // 2 NP operand stages of 32 columns
+  const uint32_t tmem_acc = tmem_base;             // columns [0, BN)
+  const uint32_t tmem_a = tmem_base + BN;          // NT operand stages of 32 columns
 
   if (warp == 0) {
-    // ------------------------------------------------------------------ weight producer
-    // Weight tiles never depend on the previous kernel of the stream: they are requested at once, and as stages are
-    // unpacked.
+    // ------------------------------------------------------------------ producer
     if (lane == 0) {
+      constexpr uint32_t kTx = Cfg::kXStage + Cfg::kWStage;
       int issued = 0;
       bool ok = true;
-      const uint8_t* src = args.blob + ((size_t)nt * args.kt_total + kt_begin) * kTileBytes;
-      for (int i = 0; i < nk; ++i, src += kTileBytes) {
-        const int s = i % NW;
-        if (i >= NW && !ptx::mbar_wait_bounded(bar_wfree + 8 * s, ((uint32_t)(i / NW) & 1u) ^ 1u, kWaitLimitNs)) {
-          atomicExch(args.status, 101);
-          ok = false;
-          break;
-        }
-        ptx::mbar_expect_tx(bar_wfull + 8 * s, kTileBytes);
-        ptx::bulk_load(ws + s * kTileBytes, src, kTileBytes, bar_wfull + 8 * s);
-        ++issued;
-        if (i == 0) TT_STAMP(1);   // first weight copy issued
+      // Weight tiles never depend on the previous kernel of the stream, the tokens do: the first NS
+      // weight tiles are requested at once, then comes the wait for that kernel, then the token boxes.
+      const int early = nk < NS ? nk : NS;
+      for (int i = 0; i < early; ++i) {
+        ptx::mbar_expect_tx(bar_full + 8 * i, kTx);
+        const uint8_t* src = args.blob + ((size_t)nt * args.kt_total + kt_begin + i) * kTileBytes;
+        ptx::bulk_load(ws + i * Cfg::kWStage, src, kTileBytes, bar_full + 8 * i);
       }
-      if (!ok) {
-        // copies already issued still write shared memory: let them land before the CTA exits
-        for (int i = issued > NW ? issued - NW : 0; i < issued; ++i)
-          ptx::mbar_wait_bounded(bar_wfull + 8 * (i % NW), (uint32_t)(i / NW) & 1u, kWaitLimitNs);
-      }
-    }
-  } else if (warp == 2 + 4 * kSets) {
-    // ------------------------------------------------------------------ token producer
-    if (lane == 0) {
+      TT_STAMP(1);   // first weight copies issued
       dependency_wait();
       TT_STAMP(2);   // the previous kernel is complete
       if constexpr (MULTI) {
         if (!peer_wait(multi.sync, 1000000000ull)) atomicExch(args.status, 109);   // tokens gathered from peers
       }
-      int issued = 0;
-      bool ok = true;
-      const int groups = (nk + G - 1) / G;   // the last box may reach into the next k-range (unused) or past K (zeros)
-      for (int i = 0; i < groups; ++i) {
-        const int s = i % NX;
-        if (i >= NX && !ptx::mbar_wait_bounded(bar_xfree + 8 * s, ((uint32_t)(i / NX) & 1u) ^ 1u, kWaitLimitNs)) {
-          atomicExch(args.status, 106);
+      for (int i = 0; i < early; ++i)
+        ptx::tensor_load_2d(xs + i * Cfg::kXStage, &tmap_x, (kt_begin + i) * 128, m0, bar_full + 8 * i);
+      issued = early;
+      for (int i = early; i < nk; ++i) {
+        const int s = i % NS;
+        const uint32_t ph = (uint32_t)(i / NS) & 1u;
+        if (!ptx::mbar_wait_bounded(bar_empty + 8 * s, ph ^ 1u, kWaitLimitNs)) {
+          atomicExch(args.status, 101);
           ok = false;
           break;
         }
-        ptx::mbar_expect_tx(bar_xfull + 8 * s, Cfg::kXStage);
-        ptx::tensor_load_3d(xs + s * Cfg::kXStage, &tmap_x, 0, m0, kt_begin + i * G, bar_xfull + 8 * s);
+        ptx::mbar_expect_tx(bar_full + 8 * s, kTx);
+        const int kt = kt_begin + i;
+        const uint8_t* src = args.blob + ((size_t)nt * args.kt_total + kt) * kTileBytes;
+        ptx::bulk_load(ws + s * Cfg::kWStage, src, kTileBytes, bar_full + 8 * s);
+        ptx::tensor_load_2d(xs + s * Cfg::kXStage, &tmap_x, kt * 128, m0, bar_full + 8 * s);
         ++issued;
       }
       if (!ok) {
-        for (int i = issued > NX ? issued - NX : 0; i < issued; ++i)
-          ptx::mbar_wait_bounded(bar_xfull + 8 * (i % NX), (uint32_t)(i / NX) & 1u, kWaitLimitNs);
+        // copies already issued still write shared memory: let them land before the CTA exits
+        for (int i = issued > NS ? issued - NS : 0; i < issued; ++i)
+          ptx::mbar_wait_bounded(bar_full + 8 * (i % NS), (uint32_t)(i / NS) & 1u, kWaitLimitNs);
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issue
-    // The whole warp walks the loop; one elected lane issues (see ptx::elect_one).  Two k-tiles a step, one of either
-    // dequant set: what a step costs is the scalar code around the MMAs (two satisfied waits, the branch, the commits and
-    // the stage arithmetic: 480 of a k-tile's 560 cycles when every k-tile was a step), and it bounded the stream.
+    // The whole warp walks the loop; one elected lane issues (see ptx::elect_one).
     {
       const bool leader = ptx::elect_one();
       constexpr uint32_t idesc = ptx::idesc_i8(BN);
       bool ok = true;
-      int p = 0, s = 0, in_stage = 0;   // operand pair, token stage, k-tile of the token stage
-      uint32_t pph = 0, sph = 0;
-#pragma unroll 1
-      for (int i = 0; i < nk; i += kSets) {
-        if (in_stage == 0) ok = ptx::mbar_wait_bounded(bar_xfull + 8 * s, sph, kWaitLimitNs);
-        if (ok) ok = ptx::mbar_wait_bounded(bar_aready + 8 * p, pph, kWaitLimitNs);
+      for (int i = 0; i < nk; ++i) {
+        const int s = i % NS;
+        const uint32_t ph = (uint32_t)(i / NS) & 1u;
+        const int t = i % NT;
+        const uint32_t pht = (uint32_t)(i / NT) & 1u;
+        ok = ptx::mbar_wait_bounded(bar_full + 8 * s, ph, kWaitLimitNs);
+        if (ok && W4) ok = ptx::mbar_wait_bounded(bar_aready + 8 * t, pht, kWaitLimitNs);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) {
           if (leader) atomicExch(args.status, 102);
           break;
         }
         ptx::tc_fence_after();
-        const uint32_t xb = xs + s * Cfg::kXStage + in_stage * Cfg::kXTile;
-        const uint32_t ab = tmem_a + p * 64;
-        in_stage += kSets;
+        const uint32_t xb = xs + s * Cfg::kXStage;
+        const uint32_t ab = tmem_a + t * 32;
+        const uint32_t wb = ws + s * Cfg::kWStage;
         if (leader) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j)
-            if (j < 4 || i + 1 < nk)
-              ptx::mma_i8_ts(tmem_acc, ab + j * 8, ptx::smem_desc_sw128(xb + (j >> 2) * Cfg::kXTile + (j & 3) * 32), idesc,
-                             (i > 0 || j > 0) ? 1u : 0u);
-          ptx::tc_commit(bar_afree + 8 * p);
-          if (in_stage == G) ptx::tc_commit(bar_xfree + 8 * s);
-        }
-        if (in_stage == G) {
-          in_stage = 0;
-          if (++s == NX) {
-            s = 0;
-            sph ^= 1u;
+          for (int j = 0; j < 4; ++j) {
+            const uint64_t bdesc = ptx::smem_desc_sw128(xb + j * 32);
+            const uint32_t accumulate = (i > 0 || j > 0) ? 1u : 0u;
+            if (W4) ptx::mma_i8_ts(tmem_acc, ab + j * 8, bdesc, idesc, accumulate);
+            else ptx::mma_i8_ss(tmem_acc, ptx::smem_desc_sw128(wb + j * 32), bdesc, idesc, accumulate);
           }
-        }
-        if (++p == NP) {
-          p = 0;
-          pph ^= 1u;
+          ptx::tc_commit(bar_empty + 8 * s);
+          if (W4) ptx::tc_commit(bar_afree + 8 * t);
         }
       }
       if (ok && leader) ptx::tc_commit(bar_acc);
@@ -259,66 +236,56 @@ w4a8_tile_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmArgs args
     const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
     const int set = (threadIdx.x - 64) >> 7;
     bool ok = true;
-    int p = 0;              // operand pair
-    uint32_t pph = 1u;      // parity of the pass before
-#pragma unroll 1
-    for (int i = set; i < nk; i += kSets) {
-      const int s = i % NW;
-      if (!ptx::mbar_wait_bounded(bar_wfull + 8 * s, (uint32_t)(i / NW) & 1u, kWaitLimitNs)) {
-        atomicExch(args.status, 103);
-        ok = false;
-        break;
-      }
-      if (i == 0 && threadIdx.x == 64) TT_STAMP(3);   // first weight tile landed
-      if (i + kSets >= nk && (threadIdx.x & 127) == 64 % 128 && set == ((nk - 1) % kSets)) TT_STAMP(4);   // last one landed
-      const uint8_t* wst = smem + (ws - base) + s * kTileBytes;
-      uint4 ch[4];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) ch[c] = *reinterpret_cast<const uint4*>(wst + (c * 128 + row) * 16);
-      const uint32_t meta = *reinterpret_cast<const uint32_t*>(wst + 8192 + row * 4);
-      ptx::mbar_arrive(bar_wfree + 8 * s);
-
-      // Unpack into registers first, wait for the operand stage afterwards: the arithmetic of this k-step
-      // overlaps the MMAs that still read the stage.  (Leaving the operand store in flight during the NEXT
-      // unpack was measured here and lost 10-30 % at prefill sizes: the MMAs of
-      // a 128-token tile are long enough to starve when "operand ready" comes one unpack later.)
-      const uint32_t step0 = meta & 0xffu, a0 = ((meta >> 8) & 0xffu) * 0x01010101u;
-      const uint32_t step1 = (meta >> 16) & 0xffu, a1 = (meta >> 24) * 0x01010101u;
-      uint32_t v[32];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const uint32_t step = c < 2 ? step0 : step1;
-        const uint32_t ab = c < 2 ? a0 : a1;
-        const uint32_t pk[4] = {ch[c].x, ch[c].y, ch[c].z, ch[c].w};
-#pragma unroll
-        for (int h = 0; h < 4; ++h) {
-          v[8 * c + 2 * h] = lqq_dequant4(pk[h] & 0x0F0F0F0Fu, step, ab);
-          v[8 * c + 2 * h + 1] = lqq_dequant4((pk[h] >> 4) & 0x0F0F0F0Fu, step, ab);
+    if (W4) {
+      for (int i = set; i < nk; i += kSets) {
+        const int s = i % NS;
+        const uint32_t ph = (uint32_t)(i / NS) & 1u;
+        const int t = i % NT;
+        const uint32_t pht = (uint32_t)(i / NT) & 1u;
+        if (!ptx::mbar_wait_bounded(bar_full + 8 * s, ph, kWaitLimitNs)) {
+          atomicExch(args.status, 103);
+          ok = false;
+          break;
         }
-      }
-      if (i >= kSets * NP && !ptx::mbar_wait_bounded(bar_afree + 8 * p, pph, kWaitLimitNs)) {
-        atomicExch(args.status, 104);
-        ok = false;
-        break;
-      }
-      __syncwarp();   // lanes leave the poll loops one by one; tcgen05.st / wait::st need the warp converged
-      ptx::tc_fence_after();
-      ptx::tmem_st32(tmem_a + lane_addr + p * 64 + set * 32, v);   // one store: four of 8 columns took 300 cycles longer
-      ptx::tc_wait_st();
-      ptx::tc_fence_before();
-      ptx::mbar_arrive(bar_aready + 8 * p);
-      if (++p == NP) {
-        p = 0;
-        pph ^= 1u;
-      }
-    }
-    // An odd range's last pair has no second k-tile: the second set completes the pair's barrier all the same.
-    if ((nk & 1) && set == 1 && ok) {
-      if (nk > kSets * NP && !ptx::mbar_wait_bounded(bar_afree + 8 * p, pph, kWaitLimitNs)) {
-        atomicExch(args.status, 104);
-        ok = false;
-      } else {
-        ptx::mbar_arrive(bar_aready + 8 * p);
+        if (i == 0 && threadIdx.x == 64) TT_STAMP(3);   // first stage (weights and tokens) landed
+        if (i + kSets >= nk && (threadIdx.x & 127) == 64 % 128 && set == ((nk - 1) % kSets)) TT_STAMP(4);   // last stage landed
+        const uint8_t* wst = smem + (ws - base) + s * Cfg::kWStage;
+        uint4 ch[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) ch[c] = *reinterpret_cast<const uint4*>(wst + (c * 128 + row) * 16);
+        const uint32_t meta = *reinterpret_cast<const uint32_t*>(wst + 8192 + row * 4);
+        ptx::mbar_arrive(bar_empty + 8 * s);
+
+        // Unpack into registers first, wait for the operand stage afterwards: the arithmetic of this k-step
+        // overlaps the MMAs that still read the stage.  (Leaving the operand store in flight during the NEXT
+        // unpack, as the decode kernel does, was measured here and lost 10-30 % at prefill sizes: the MMAs of
+        // a 128-token tile are long enough to starve when "operand ready" comes one unpack later.)
+        const uint32_t step0 = meta & 0xffu, a0 = ((meta >> 8) & 0xffu) * 0x01010101u;
+        const uint32_t step1 = (meta >> 16) & 0xffu, a1 = (meta >> 24) * 0x01010101u;
+        uint32_t v[4][8];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const uint32_t step = c < 2 ? step0 : step1;
+          const uint32_t ab = c < 2 ? a0 : a1;
+          const uint32_t pk[4] = {ch[c].x, ch[c].y, ch[c].z, ch[c].w};
+#pragma unroll
+          for (int h = 0; h < 4; ++h) {
+            v[c][2 * h] = lqq_dequant4(pk[h] & 0x0F0F0F0Fu, step, ab);
+            v[c][2 * h + 1] = lqq_dequant4((pk[h] >> 4) & 0x0F0F0F0Fu, step, ab);
+          }
+        }
+        if (!ptx::mbar_wait_bounded(bar_afree + 8 * t, pht ^ 1u, kWaitLimitNs)) {
+          atomicExch(args.status, 104);
+          ok = false;
+          break;
+        }
+        __syncwarp();   // lanes leave the poll loops one by one; tcgen05.st / wait::st need the warp converged
+        ptx::tc_fence_after();
+#pragma unroll
+        for (int c = 0; c < 4; ++c) ptx::tmem_st8(tmem_a + lane_addr + t * 32 + c * 8, v[c]);
+        ptx::tc_wait_st();
+        ptx::tc_fence_before();
+        ptx::mbar_arrive(bar_aready + 8 * t);
       }
     }
     if (ok && !ptx::mbar_wait_bounded(bar_acc, 0u, kWaitLimitNs)) {
@@ -423,10 +390,10 @@ w4a8_tile_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmArgs args
   }
 }
 
-template <int BN, int NW, int NX, int G, int NP, bool MULTI>
+template <int BN, int NS, int NT, bool W4, bool MULTI>
 static int launch_one(const CUtensorMap& tx, const GemmArgs& a, const MultiOut* multi, int splits, cudaStream_t st) {
-  using Cfg = TcCfg<BN, NW, NX, G, NP>;
-  auto kern = &w4a8_tile_kernel<BN, NW, NX, G, NP, MULTI>;
+  using Cfg = TcCfg<BN, NS, NT, W4>;
+  auto kern = &w4a8_tile_kernel<BN, NS, NT, W4, MULTI>;
   static std::once_flag once[64];
   int dev = 0;
   cudaGetDevice(&dev);
@@ -449,13 +416,18 @@ static int launch_one(const CUtensorMap& tx, const GemmArgs& a, const MultiOut* 
   return check_launch("w4a8_tile_kernel");
 }
 
-template <int BN, int NW, int NX, int G, int NP>
+template <int BN, int NS, int NT, bool W4>
 static int launch_cfg(const CUtensorMap& tx, const GemmArgs& a, const MultiOut* multi, int splits, cudaStream_t st) {
-  if (multi) return launch_one<BN, NW, NX, G, NP, true>(tx, a, multi, splits, st);
-  return launch_one<BN, NW, NX, G, NP, false>(tx, a, nullptr, splits, st);
+  if (multi) return launch_one<BN, NS, NT, W4, true>(tx, a, multi, splits, st);
+  return launch_one<BN, NS, NT, W4, false>(tx, a, nullptr, splits, st);
 }
 
-// Token-tile widths: the smallest that holds a decode batch, 128 tokens for prefill.
+// Token-tile widths: the smallest that holds a decode batch, 128 tokens for prefill.  A 192-token
+// configuration (three shared-memory stages, two operand stages, otherwise this kernel) would do 1.5x the
+// tensor-core work per unpacked weight byte; it passed the parity tests on three full-size shapes and then
+// raised an unspecified launch failure on a fourth (28672 x 4096, 8192 tokens) and in back-to-back graph
+// replays.  Reading the index arithmetic, the barrier counts and the tensor-memory budget (192 + 2 x 32 =
+// 256 columns, two CTAs per SM) did not show the cause, so the configuration is not built.
 // Between 65 and 128 tokens a small matrix (up to 32 M weights: the qkv and o projections of an 8B model)
 // takes 64-token tiles: twice the CTAs, so the split factor halves and so do the int32 planes each CTA
 // writes (measured at 128 tokens: 6144 x 4096 15.7 -> 14.4 us, 4096 x 4096 13.5 -> 11.7 us; 28672 x 4096
@@ -472,9 +444,6 @@ static int tile_bn(int M, int N, int K) {
   }
   return M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
 }
-
-// k-tiles of a token box.
-static int tile_group(int bn) { return bn <= 32 ? 4 : 2; }
 
 }  // namespace tile
 
@@ -516,7 +485,7 @@ int run_tile_gemm(const int8_t* x, const uint8_t* blob, const float* ascale, con
   if (splits > 1 && (!ws || ws_bytes < tile_workspace_bytes(M, N, splits))) return LQ_ERR_WORKSPACE;
   const int bn = tile_bn(M, N, K);
   CUtensorMap tx;
-  int rc = make_token_map(&tx, x, M, K, bn, tile_group(bn));
+  int rc = make_byte_matrix_map(&tx, x, M, K, bn, 128);
   if (rc) return rc;
   const bool multi = out.n != 1 || out.ld != N || out.col0 != 0 || (sync && (sync->n_signal > 0 || sync->wait));
   if (multi && out_mode == kOutI32) return LQ_ERR_BAD_ARG;
@@ -555,10 +524,10 @@ int run_tile_gemm(const int8_t* x, const uint8_t* blob, const float* ascale, con
     // 16 tokens: 8 stages, 4 operand stages (95 KB, two CTAs per SM).  Five stages and two operand stages, so
     // that three CTAs fit an SM and the next launch's CTAs can start beside this one's, measured 30 % slower
     // on 28672 x 4096 (19.2 vs 14.8 us) and 9 % slower on 4096 x 14336.
-    case 16: rc = launch_cfg<16, 8, 3, 4, 3>(tx, a, mop, splits, st); break;
-    case 32: rc = launch_cfg<32, 6, 3, 4, 3>(tx, a, mop, splits, st); break;
-    case 64: rc = launch_cfg<64, 6, 3, 2, 3>(tx, a, mop, splits, st); break;
-    default: rc = launch_cfg<128, 4, 2, 2, 2>(tx, a, mop, splits, st); break;
+    case 16: rc = launch_cfg<16, 8, 4, true>(tx, a, mop, splits, st); break;
+    case 32: rc = launch_cfg<32, 8, 4, true>(tx, a, mop, splits, st); break;
+    case 64: rc = launch_cfg<64, 6, 4, true>(tx, a, mop, splits, st); break;
+    default: rc = launch_cfg<128, 4, 4, true>(tx, a, mop, splits, st); break;
   }
   if (rc || splits <= 1) return rc;
   PeerSync fsync = {};

@@ -113,15 +113,7 @@ __device__ __forceinline__ void tensor_load_2d(uint32_t dst_smem, const void* tm
       "l"(tmap), "r"(bar), "r"(x), "r"(y)
       : "memory");
 }
-// 3-D tiled load; x innermost.
-__device__ __forceinline__ void tensor_load_3d(uint32_t dst_smem, const void* tmap, int x, int y, int z, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(
-          dst_smem),
-      "l"(tmap), "r"(bar), "r"(x), "r"(y), "r"(z)
-      : "memory");
-}
-// A 2-D box fetched into L2 only: a hint, without effect on what any later access reads.
+// The same box fetched into L2 only: a hint, without effect on what any later access reads.
 __device__ __forceinline__ void tensor_prefetch_2d(const void* tmap, int x, int y) {
   asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(tmap), "r"(x), "r"(y) : "memory");
 }
