@@ -171,6 +171,8 @@ w4a8_decode_tc_kernel(const Args args, const std::conditional_t<MULTI, MultiOut,
   const int rows_own = (join_first_block(rank + 1, S) - fb) * 8;
   const int rows_max = join_rows_max(S);
   const int groups = (M + 3) >> 2;   // of four tokens
+  const bool scaled = args.out_mode != kOutI32;
+  const bool has_bias = scaled && args.bias != nullptr;
   // warps of a token row while the maxima are taken (QUANT)
   const int wpr = M > 4 ? 1 : M > 2 ? 2 : M == 2 ? 4 : 8;
 
@@ -239,6 +241,24 @@ w4a8_decode_tc_kernel(const Args args, const std::conditional_t<MULTI, MultiOut,
       const bool leader = ptx::elect_one();
       constexpr uint32_t idesc = ptx::idesc_i8(BN);
       bool ok = true;
+      // Scales and bias of the CTA's channels, in the MMA warp's registers (the dequant threads have none to spare).  A hint to
+      // L2 ahead of the wait, which has no effect on what is read; read only behind it, since the kernel before may be their
+      // writer (a copy that made them contiguous, a linear whose output is this one's bias).
+      float w_scale[4], w_bias[4];
+      const long n0 = (long)tile * 128 + fb * 8 + lane;
+      auto chan_ok = [&](int q) { return scaled && lane + 32 * q < rows_own && n0 + 32 * q < args.N; };
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (!chan_ok(q)) continue;
+        ptx::prefetch_l2(args.s1 + n0 + 32 * q);
+        if (has_bias) ptx::prefetch_l2(static_cast<const char*>(args.bias) + (n0 + 32 * q) * (args.out_mode == LQ_DT_F32 ? 4 : 2));
+      }
+      dependency_wait();
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        w_scale[q] = chan_ok(q) ? args.s1[n0 + 32 * q] : 0.f;
+        w_bias[q] = (chan_ok(q) && has_bias) ? load_bias(args.bias, n0 + 32 * q, args.out_mode) : 0.f;
+      }
       // The operands that were unpacked ahead of the tokens: once the tokens are there their MMAs go out back to back.
       // (With a wait and a commit around each k-tile's four MMAs a k-tile takes the issuing warp 350 cycles instead of
       // about 110.)
@@ -283,8 +303,15 @@ w4a8_decode_tc_kernel(const Args args, const std::conditional_t<MULTI, MultiOut,
         }
       }
       if (leader) ptx::tc_commit(bar_acc);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (lane + 32 * q >= rows_own) continue;
+        chan_scale[lane + 32 * q] = w_scale[q];
+        chan_bias[lane + 32 * q] = w_bias[q];
+      }
     }
     __syncwarp();
+    asm volatile("bar.arrive 5, %0;" ::"n"(32 + kDequant) : "memory");
     // Tensor memory is released as soon as the accumulator has been read, ahead of the join.
     asm volatile("bar.sync 4, %0;" ::"n"(32 + kDequant) : "memory");
     ptx::tc_fence_after();
@@ -296,19 +323,12 @@ w4a8_decode_tc_kernel(const Args args, const std::conditional_t<MULTI, MultiOut,
     const int quad = warp & 3;                // tensor-memory lane quadrant this warp may access
     const int row = quad * 32 + lane;         // weight row inside the tile == tensor-memory lane
     const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
-    const bool scaled = args.out_mode != kOutI32;
-    const bool has_bias = scaled && args.bias != nullptr;
     auto all_sets = []() { asm volatile("bar.sync 3, %0;" ::"n"(kDequant) : "memory"); };
-    // Token rows past M are zero; channel scales and bias are weights.
+    // Token rows past M are zero.
     if (M < BN) {
       const int chunks = (BN - M) * 8;
       for (int i = d; i < nk * chunks; i += kDequant)
         *reinterpret_cast<uint4*>(smem + (i / chunks) * kXStage + M * 128 + (i % chunks) * 16) = make_uint4(0u, 0u, 0u, 0u);
-    }
-    if (d < rows_own) {
-      const long n = (long)tile * 128 + fb * 8 + d;
-      chan_scale[d] = (scaled && n < args.N) ? __ldg(args.s1 + n) : 0.f;
-      chan_bias[d] = (has_bias && n < args.N) ? load_bias(args.bias, n, args.out_mode) : 0.f;
     }
     asm volatile("bar.sync 2, %0;" ::"n"(32 + kDequant) : "memory");
     ptx::tc_fence_after();
@@ -382,7 +402,7 @@ w4a8_decode_tc_kernel(const Args args, const std::conditional_t<MULTI, MultiOut,
 
     // ---- the previous kernel is done: the tokens of the whole k-range
     if (d == 0) DT_STAMP(1);   // operands of the first stages done
-    dependency_wait();   // tokens, token scales and outputs belong to earlier kernels until here
+    dependency_wait();   // tokens, scales, bias and outputs belong to earlier kernels until here
     if (d == 0) DT_STAMP(2);
     if constexpr (MULTI) {
       // tokens gathered from peer GPUs: one thread waits for their flags on behalf of the others
@@ -488,7 +508,8 @@ w4a8_decode_tc_kernel(const Args args, const std::conditional_t<MULTI, MultiOut,
       store_operand();
       if (i < nk) unpack();
     }
-    all_sets();   // token scales (and everything above) before the epilogue of any thread
+    // token scales (and everything above), channel scales and bias before the epilogue of any thread
+    asm volatile("bar.sync 5, %0;" ::"n"(32 + kDequant) : "memory");
 
     // ---- epilogue: a set takes every other eight columns (tokens)
     const int units = rows_own * groups;       // (four tokens, channel) sums that this CTA joins

@@ -109,3 +109,70 @@ def test_blob_written_just_before(M, N, K, writer):
         y = ops.gemm_fused(x8, blob.reshape(-1), sx, qw.s1, N, K, 0)
         assert torch.equal(y, want[i & 1]), i
     ops.poll_status()
+
+
+def _w4_layer(n, k, g):
+    from liquidgemm_b200 import ops
+    qw, blob = ops.quantize_weight_cuda(torch.randn(n, k, device="cuda", generator=g) * 0.05, 64, want_codes=False, want_blob=True)
+    return {"s1": qw.s1, "s_u8": qw.s_u8, "offset_a": qw.offset_a, "N": n, "K": k, "rs": blob.reshape(-1)}
+
+
+def _linear_into(y, x, layer, code, s1=None, bias=None):
+    """``lq_w4a8_linear`` of activations ``x`` into the given buffer, with the sizes that it reports."""
+    from liquidgemm_b200 import ops
+    from liquidgemm_b200._lib import lib, check
+    M, N, K = x.shape[0], layer["N"], layer["K"]
+    nscratch, nws, kind = ops._linear_sizes(x.data_ptr(), M, N, K, 0)
+    scratch = torch.empty(max(nscratch, 1), dtype=torch.uint8, device="cuda")
+    ws = ops._workspace(nws, x.device) if kind == 2 else torch.empty(max(nws, 1), dtype=torch.uint8, device="cuda")
+    check(lib.lq_w4a8_linear(x.data_ptr(), {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}[x.dtype], layer["rs"].data_ptr(),
+                             (layer["s1"] if s1 is None else s1).data_ptr(), None if bias is None else bias.data_ptr(),
+                             y.data_ptr(), code, M, N, K, 0, scratch.data_ptr(), nscratch,
+                             None if ws is None else ws.data_ptr(), 0 if ws is None else ws.numel(),
+                             torch.cuda.current_stream().cuda_stream), "w4a8_linear")
+
+
+@pytest.mark.parametrize("M", [1, 2, 3, 4, 8, 16, 24, 32, 64])
+@pytest.mark.parametrize("N,K", [(4096, 4096), (1000, 1920), (18944, 512), (2048, 14336)])
+@pytest.mark.parametrize("what", ["bias", "s1", "copies"])
+def test_scales_and_bias_written_just_before(M, N, K, what):
+    """The channel scales or the bias are the output of the one-token linear directly before (the same buffer in every
+    pass, with other contents), or the operator itself makes them contiguous.  At 1 to 8 tokens the operator that takes
+    activations has no quantiser launch in between."""
+    from liquidgemm_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    layer, writer = _w4_layer(N, K, g), _w4_layer(N, 512, g)
+    x = torch.randn(M, K, device="cuda", generator=g, dtype=torch.bfloat16)
+    x8, sx = torch.ops.liquidgemm.quant_per_token(x)
+    conds = [torch.randn(1, 512, device="cuda", generator=g, dtype=torch.float32) for _ in range(2)]
+    code = 2 if what == "s1" else 0
+    vec = torch.zeros(1, N, device="cuda", dtype=torch.float32 if code == 2 else torch.bfloat16)
+    plain = torch.randn(N, device="cuda", generator=g).to(torch.bfloat16)
+
+    def args(i):
+        if what == "copies":
+            s1, b = (layer["s1"], plain) if i == 0 else (layer["s1"] * 2, plain + 1)
+            return [t.repeat_interleave(2)[::2] for t in (s1, b)]
+        return (vec.view(-1), plain) if what == "s1" else (layer["s1"], vec.view(-1))
+
+    def both(i, settle):
+        out = []
+        for op in range(2):
+            s1, b = args(i)
+            if what != "copies":
+                _linear_into(vec, conds[1 - i], writer, code)   # the other contents, then at once these
+                _linear_into(vec, conds[i], writer, code)
+            if settle:
+                torch.cuda.synchronize()
+            if op:
+                out.append(torch.ops.liquidgemm.w4a8_linear(x, layer["rs"], layer["s_u8"], layer["offset_a"], s1, b, N, K, 64, 0))
+            else:
+                out.append(ops.linear_bias(x8, layer["rs"], sx, s1, b, N, K, 0))
+        return out
+    want = [both(i, True) for i in range(2)]
+    assert not torch.equal(want[0][0], want[1][0])
+    got = [both(i & 1, False) for i in range(12)]
+    for i, ys in enumerate(got):
+        for y, w in zip(ys, want[i & 1]):
+            assert torch.equal(y.view(torch.int16), w.view(torch.int16)), i
+    ops.poll_status()
