@@ -461,6 +461,19 @@ __device__ __forceinline__ uint4 ldg_stream_v4(const void* p) {
   return r;
 }
 
+// Data that an earlier kernel of the stream may still be writing while this one is resident already (programmatic launch): a
+// coherent load, for use behind dependency_wait().  ld.global.nc (which __ldg, and const __restrict__ parameters, stand for as well)
+// is defined only for data that nobody writes during the kernel's life: its lines may be in the SM's L1 from a
+// kernel that read the same addresses before they were written again.  Tile blobs, whose writers settle, take the one above.
+__device__ __forceinline__ uint4 ld_stream_v4(const void* p) {
+  uint4 r;
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
+               : "l"(p)
+               : "memory");
+  return r;
+}
+
 // Programmatic dependent launch, device side.  allow_dependents(): the next kernel of the stream may be
 // scheduled once every CTA of this grid has executed it.  dependency_wait(): returns when all earlier
 // kernels of the stream have completed and their writes are visible (no-op for an ordinary launch).

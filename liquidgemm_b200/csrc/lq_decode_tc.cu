@@ -111,7 +111,7 @@ struct Chunk {
   uint4 r[sizeof(XT)];
   __device__ __forceinline__ void load(const XT* p) {
 #pragma unroll
-    for (int i = 0; i < (int)sizeof(XT); ++i) r[i] = __ldg(reinterpret_cast<const uint4*>(p) + i);
+    for (int i = 0; i < (int)sizeof(XT); ++i) r[i] = reinterpret_cast<const uint4*>(p)[i];
   }
   __device__ __forceinline__ void clear() {
 #pragma unroll
@@ -415,7 +415,7 @@ w4a8_decode_tc_kernel(const Args args, const std::conditional_t<MULTI, MultiOut,
       const int x_row = jx >> 3;
       const uint32_t x_off = (uint32_t)(x_row * 128 + (((jx & 7) ^ (x_row & 7)) << 4));
       const int8_t* src = static_cast<const int8_t*>(args.x) + (size_t)x_row * args.K + (size_t)kb * 128 + (jx & 7) * 16;
-      if (d < M) tok_scale[d] = scaled ? __ldg(args.ascale + d) : 0.f;
+      if (d < M) tok_scale[d] = scaled ? args.ascale[d] : 0.f;
       constexpr int Q = BN / 16, U = Q == 1 ? 8 : 4;
 #pragma unroll 1
       for (int j0 = set; j0 < nk; j0 += kSets * U) {
@@ -425,7 +425,7 @@ w4a8_decode_tc_kernel(const Args args, const std::conditional_t<MULTI, MultiOut,
 #pragma unroll
           for (int q = 0; q < Q; ++q)
             if (j0 + kSets * u < nk && x_row + 16 * q < M)
-              xv[u][q] = ldg_stream_v4(src + (size_t)(16 * q) * args.K + (size_t)(j0 + kSets * u) * 128);
+              xv[u][q] = ld_stream_v4(src + (size_t)(16 * q) * args.K + (size_t)(j0 + kSets * u) * 128);
 #pragma unroll
         for (int u = 0; u < U; ++u)
 #pragma unroll

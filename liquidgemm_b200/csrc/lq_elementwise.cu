@@ -52,7 +52,7 @@ dequant_weight_kernel(const uint32_t* __restrict__ q, const uint8_t* __restrict_
 // tokens 30.5 / 95.8 / 190 -> 20.5 / 66 / 137 us (5.0 / 5.4 / 5.2 TB/s of the 6.5 a copy reaches).
 template <typename T, int NV>
 __global__ void __launch_bounds__(1024)
-quant_row_kernel(const T* __restrict__ x, int8_t* __restrict__ xq, float* __restrict__ ascale, int K) {
+quant_row_kernel(const T* x, int8_t* __restrict__ xq, float* __restrict__ ascale, int K) {
   __shared__ float red[32];
   constexpr int VEC = 16 / sizeof(T);
   allow_dependents();   // as in quant_per_token_kernel below
@@ -90,7 +90,7 @@ quant_row_kernel(const T* __restrict__ x, int8_t* __restrict__ xq, float* __rest
 // (amax, then quantise) and the second visit is served by L1/L2.
 template <typename T>
 __global__ void __launch_bounds__(256)
-quant_per_token_kernel(const T* __restrict__ x, int8_t* __restrict__ xq, float* __restrict__ ascale,
+quant_per_token_kernel(const T* x, int8_t* __restrict__ xq, float* __restrict__ ascale,
                        int K) {
   __shared__ float red[32];
   // The linear that consumes these tokens is launched with programmatic stream serialisation: let it
@@ -186,13 +186,14 @@ int run_unpack_blob_i8(const uint8_t* blob, int8_t* w, int N, int K, cudaStream_
 // planes == 1: plain epilogue.  planes > 1: sum of `planes` int32 partial planes [planes][M][N]
 // first (exact in any order), then the same formula
 // (reference csrc/liquid_gemm/w4a8_wgmma.cu:39-56).
+// The parameters are not __restrict__: planes, scales and bias come from kernels that may still be writing them when this one
+// becomes resident, so they must not be read through the non-coherent path (see ld_stream_v4).
 // MULTI: the outputs go to several row-major matrices with their own row stride and column offset (gather by
 // stores over NVLink, see OutSpec), element by element, and every CTA signals the peers' flags at its end.
 template <bool MULTI>
 __global__ void __launch_bounds__(256)
-finish_kernel(const int32_t* __restrict__ acc, const float* __restrict__ ascale,
-              const float* __restrict__ s1, const void* __restrict__ bias, void* __restrict__ y, int out_dtype,
-              int planes, int M, int N, bool vec, const std::conditional_t<MULTI, MultiOut, NoMultiOut> multi) {
+finish_kernel(const int32_t* acc, const float* ascale, const float* s1, const void* bias, void* y, int out_dtype, int planes,
+              int M, int N, bool vec, const std::conditional_t<MULTI, MultiOut, NoMultiOut> multi) {
   // Launched with programmatic stream serialisation behind the kernel that writes the planes: let the
   // kernel after this one start (it prefetches weights, and waits for this grid before it touches
   // tokens, planes or outputs), then wait for the planes to be complete.

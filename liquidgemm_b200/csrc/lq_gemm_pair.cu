@@ -419,7 +419,7 @@ w4a8_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const Args args,
         const long n = (long)(2 * n2 + (int)rank) * 128 + row;
         const int cols = (args.M - m0) < kBN ? (args.M - m0) : kBN;
         const uint32_t tmem_acc = tmem_base + b * kBN + lane_addr;
-        const float w_scale = raw ? 0.f : __ldg(args.s1 + n);
+        const float w_scale = raw ? 0.f : args.s1[n];
         const float bias = has_bias ? load_bias(args.bias, n, args.out_mode) : 0.f;
 #pragma unroll 1
         for (int c0 = 16 * (2 + my_set); c0 < cols; c0 += 16 * kGroupsLast) {
@@ -427,7 +427,7 @@ w4a8_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const Args args,
           ptx::tmem_ld16(tmem_acc + c0, v);
           float sc[16];
 #pragma unroll
-          for (int j = 0; j < 16; ++j) sc[j] = (!raw && c0 + j < cols) ? __ldg(args.ascale + m0 + c0 + j) : 0.f;
+          for (int j = 0; j < 16; ++j) sc[j] = (!raw && c0 + j < cols) ? args.ascale[m0 + c0 + j] : 0.f;
           ptx::tc_wait_ld();
           if (completes) add_planes(v, planes, 2 * kPlane4, S - 1, c0, cols, row);
           epi_store_cols(args.out, args.out_mode, (size_t)(m0 + c0) * args.N + n, args.N, v, sc, w_scale, bias, has_bias,
@@ -504,7 +504,7 @@ w4a8_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const Args args,
       const bool n_ok = n < args.N;
       const int cols = (args.M - m0) < kBN ? (args.M - m0) : kBN;   // valid token columns of this tile
       const uint32_t tmem_acc = tmem_base + b * kBN + lane_addr;
-      const float w_scale = (n_ok && !raw) ? __ldg(args.s1 + n) : 0.f;
+      const float w_scale = (n_ok && !raw) ? args.s1[n] : 0.f;
       const float bias = (has_bias && n_ok) ? load_bias(args.bias, n, args.out_mode) : 0.f;
       // A tile cut along k between S pairs: every pair but the one with the last k-range writes its sums to a
       // plane of its own in the workspace (plain 16-byte stores; int32 atomics on whole tiles from every pair at
@@ -522,7 +522,7 @@ w4a8_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const Args args,
         float* tsc = tok_scale + (2 * g + fslot) * kBN;
         const long long tr_t0 = TR_NOW();
         if (!raw) {
-          for (int i = et; i < kBN; i += 128) tsc[i] = (i < cols) ? __ldg(args.ascale + m0 + i) : 0.f;
+          for (int i = et; i < kBN; i += 128) tsc[i] = (i < cols) ? args.ascale[m0 + i] : 0.f;
         }
         if (completes && et == 0) {
           // the other pairs took their k-ranges first of all: their sums have been there for a long time

@@ -321,12 +321,12 @@ w4a8_tile_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmArgs args
           const float4* sp = reinterpret_cast<const float4*>(args.ascale + m0 + c0);
 #pragma unroll
           for (int q4 = 0; q4 < 4; ++q4) {
-            const float4 f = __ldg(sp + q4);
+            const float4 f = sp[q4];
             sc[4 * q4] = f.x; sc[4 * q4 + 1] = f.y; sc[4 * q4 + 2] = f.z; sc[4 * q4 + 3] = f.w;
           }
         } else {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) sc[j] = (m0 + c0 + j < args.M) ? __ldg(args.ascale + m0 + c0 + j) : 0.f;
+          for (int j = 0; j < 16; ++j) sc[j] = (m0 + c0 + j < args.M) ? args.ascale[m0 + c0 + j] : 0.f;
         }
         ptx::tc_wait_ld();
         if (vec) {

@@ -263,7 +263,7 @@ gemv_blob_kernel(const Args args, const std::conditional_t<MULTI, MultiOut, NoMu
     [[maybe_unused]] int x_tile = 0, x_tiles = 0;   // QUANT: position in, and number of, the CTA's token tiles
     if constexpr (!QUANT) {
 #pragma unroll
-      for (int m = 0; m < MT; ++m) a_scale[m] = (m < M) ? __ldg(args.ascale + m) : 0.f;
+      for (int m = 0; m < MT; ++m) a_scale[m] = (m < M) ? args.ascale[m] : 0.f;
     } else {
       const XT* x = static_cast<const XT*>(args.x);
       float inv[MT];
@@ -321,7 +321,7 @@ gemv_blob_kernel(const Args args, const std::conditional_t<MULTI, MultiOut, NoMu
 
     while (walk.next(sg)) {
       const long n = (long)sg.tile * 128 + row;
-      const float w_scale = (n < args.N) ? __ldg(args.s1 + n) : 0.f;   // a weight: fetched ahead of the loop
+      const float w_scale = (n < args.N) ? args.s1[n] : 0.f;   // a weight: fetched ahead of the loop
       int acc[MT];
 #pragma unroll
       for (int m = 0; m < MT; ++m) acc[m] = 0;

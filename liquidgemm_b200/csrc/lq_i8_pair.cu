@@ -263,7 +263,7 @@ i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
       const int cols = (args.M - m0) < args.bn ? (args.M - m0) : args.bn;   // valid token columns of this tile
       float* tsc = tok_scale + (2 * g + fslot) * kMaxBN;
       if (!raw) {
-        for (int i = et; i < kMaxBN; i += 128) tsc[i] = (i < cols) ? __ldg(args.ascale + m0 + i) : 0.f;
+        for (int i = et; i < kMaxBN; i += 128) tsc[i] = (i < cols) ? args.ascale[m0 + i] : 0.f;
       }
       group_bar(g);
       if (wflag[fslot] == 0) {
@@ -272,7 +272,7 @@ i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
       }
       ptx::tc_fence_after();
       const uint32_t tmem_acc = tmem_base + b * kMaxBN + lane_addr;
-      const float w_scale = raw ? 0.f : __ldg(args.s1 + n);
+      const float w_scale = raw ? 0.f : args.s1[n];
       const float bias = has_bias ? load_bias(args.bias, n, args.out_mode) : 0.f;
 #pragma unroll 1
       for (int c0 = 16 * g; c0 < cols; c0 += 16 * kGroups) {

@@ -169,7 +169,7 @@ i8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const Args args) {
       uint4 xv[BN / 16];
 #pragma unroll
       for (int q = 0; q < BN / 16; ++q)
-        xv[q] = (m0 + x_row + 16 * q < args.M) ? ldg_stream_v4(x_src + (size_t)(16 * q) * args.K + (size_t)i * 128)
+        xv[q] = (m0 + x_row + 16 * q < args.M) ? ld_stream_v4(x_src + (size_t)(16 * q) * args.K + (size_t)i * 128)
                                                : make_uint4(0u, 0u, 0u, 0u);
       if (i >= NS && !ptx::mbar_wait_bounded(bar_empty + 8 * s, ((uint32_t)(i / NS) & 1u) ^ 1u, kWaitLimitNs)) {
         atomicExch(args.status, 153);
@@ -192,7 +192,7 @@ i8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const Args args) {
       const long n = (long)nt * 128 + row;
       const bool n_ok = n < args.N;
       const bool raw = args.out_mode == kEpiI32;
-      const float w_scale = (n_ok && !raw) ? __ldg(args.s1 + n) : 0.f;
+      const float w_scale = (n_ok && !raw) ? args.s1[n] : 0.f;
       char* out = static_cast<char*>(args.out) + (raw ? (size_t)z * args.M * args.N * 4 : 0);
 #pragma unroll 1
       for (int c0 = 16 * set; c0 < BN; c0 += 16 * kSets) {   // the sets share the accumulator's columns
@@ -201,7 +201,7 @@ i8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const Args args) {
         ptx::tmem_ld16(tmem_acc + lane_addr + c0, v);
         float sc[16];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) sc[j] = (!raw && m0 + c0 + j < args.M) ? __ldg(args.ascale + m0 + c0 + j) : 0.f;
+        for (int j = 0; j < 16; ++j) sc[j] = (!raw && m0 + c0 + j < args.M) ? args.ascale[m0 + c0 + j] : 0.f;
         ptx::tc_wait_ld();
         if (n_ok)
           epi_store_cols(out, args.out_mode, (size_t)(m0 + c0) * args.N + n, args.N, v, sc, w_scale, 0.f, false,

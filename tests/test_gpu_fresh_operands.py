@@ -176,3 +176,72 @@ def test_scales_and_bias_written_just_before(M, N, K, what):
         for y, w in zip(ys, want[i & 1]):
             assert torch.equal(y.view(torch.int16), w.view(torch.int16)), i
     ops.poll_status()
+
+
+@pytest.mark.parametrize("M", [1, 2, 3, 5, 8, 16, 32, 64, 200])
+@pytest.mark.parametrize("widths", [(2048, 4096), (1024, 14336)])
+def test_chains_reuse_every_buffer(M, widths):
+    """Eight linears in a graph, each reading what the one before wrote, through two activation buffers and the same
+    scratch (tokens, scales, planes): every address is written anew while the next reader is resident already.  New
+    contents in every replay, without synchronising in between."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    n, k = widths
+    down, up = _w4_layer(n, k, g), _w4_layer(k, n, g)
+    a, b = (torch.zeros(M, w, device="cuda", dtype=torch.bfloat16) for w in (k, n))
+
+    def chain(settle=False):
+        for _ in range(4):
+            for y, x, layer in ((b, a, down), (a, b, up)):
+                _linear_into(y, x, layer, 0)
+                if settle:
+                    torch.cuda.synchronize()
+    xs = [torch.randn(M, k, device="cuda", generator=g, dtype=torch.bfloat16) for _ in range(5)]
+    want = []
+    for x in xs:
+        a.copy_(x)
+        chain(settle=True)
+        want.append(a.clone())
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        chain()
+        stream.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            chain()
+        wrong = torch.zeros((), dtype=torch.int64, device="cuda")
+        for i in range(200):
+            a.copy_(xs[i % 5])
+            graph.replay()
+            wrong += (a.view(torch.int16) != want[i % 5].view(torch.int16)).sum()
+        stream.synchronize()
+    assert int(wrong) == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(8, 4096, 4096), (33, 1024, 14336), (200, 1024, 4096), (300, 16384, 512)])
+def test_int8_layers_reuse_every_buffer(M, N, K):
+    """The same for the INT8-weights mode: tokens, token scales and planes at the same addresses, layer after layer."""
+    from liquidgemm_b200 import ops
+    from liquidgemm_b200._lib import lib, check
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    w8 = torch.randint(-127, 128, (N, K), device="cuda", dtype=torch.int8, generator=g)
+    sw = torch.rand(N, device="cuda", generator=g)
+    xs = [torch.randn(M, K, device="cuda", generator=g, dtype=torch.bfloat16) for _ in range(4)]
+    want = [torch.ops.liquidgemm.i8_gemm_scaled(q, w8, s, sw, 0) for q, s in (torch.ops.liquidgemm.quant_per_token(x) for x in xs)]
+    torch.cuda.synchronize()
+    x8, sx = torch.empty(M, K, device="cuda", dtype=torch.int8), torch.empty(M, device="cuda")
+    nb = lib.lq_i8_workspace_bytes(M, N, K)
+    ws = torch.empty(max(nb, 1), dtype=torch.uint8, device="cuda")
+    ys = [torch.empty(M, N, device="cuda", dtype=torch.bfloat16) for _ in xs]
+    st = torch.cuda.current_stream().cuda_stream
+    wrong = torch.zeros((), dtype=torch.int64, device="cuda")
+    for _ in range(50):
+        for x, y in zip(xs, ys):
+            check(lib.lq_quant_per_token(x.data_ptr(), 0, x8.data_ptr(), sx.data_ptr(), M, K, st), "quant_per_token")
+            check(lib.lq_i8_gemm_scaled_ws(x8.data_ptr(), w8.data_ptr(), sx.data_ptr(), sw.data_ptr(), y.data_ptr(), 0, M, N, K,
+                                           ws.data_ptr() if nb else None, nb, st), "i8_gemm_scaled")
+        for y, w in zip(ys, want):
+            wrong += (y.view(torch.int16) != w.view(torch.int16)).sum()
+            y.zero_()
+    assert int(wrong) == 0
+    ops.poll_status()
