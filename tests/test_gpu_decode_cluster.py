@@ -66,3 +66,47 @@ def test_quantising_form_equals_two_launches(N, K, dtype):
         got = torch.ops.liquidgemm.w4a8_linear(x, L["rs"], L["s_u8"], L["offset_a"], L["s1"], bias, N, K, 64, code)
         assert torch.equal(got.view(raw), (want + bias).view(raw)), M
     ops.poll_status()
+
+
+def test_several_streams_at_once():
+    """Four streams replay graphs of this kernel side by side (int8 tokens and the quantising form, k-ranges longer than
+    the seven operands unpacked ahead and longer than the ring), beside the tile kernel's planes and finish pass on 4096 x 14336.
+    Every output of every replay is compared, in the stream, with the persistent kernel's."""
+    from liquidgemm_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(5)
+    layers = []
+    for N, K in [(4096, 4096), (6144, 4096), (2048, 14336), (1024, 7680), (4096, 14336)]:
+        qw, blob = ops.quantize_weight_cuda(torch.randn(N, K, generator=g, device="cuda") * 0.03, 64, want_codes=False, want_blob=True)
+        layers.append({"s1": qw.s1, "s_u8": qw.s_u8, "offset_a": qw.offset_a, "N": N, "K": K, "rs": blob.reshape(-1)})
+    runs = []
+    for M in (3, 8, 16, 32):
+        cases = []
+        for L in layers:
+            x = torch.randn(M, L["K"], generator=g, device="cuda", dtype=torch.bfloat16)
+            x8, sx = torch.ops.liquidgemm.quant_per_token(x)
+            cases.append((L, x, x8, sx, ops.gemm_fused(x8, L["rs"], sx, L["s1"], L["N"], L["K"], 0, splitk=-1)))
+        torch.cuda.synchronize()
+        stream, wrong = torch.cuda.Stream(), torch.zeros((), dtype=torch.int64, device="cuda")
+
+        def step():
+            out = []
+            for L, x, x8, sx, want in cases:
+                out.append((ops.w4a8_linear(x, L), want))
+                out.append((ops.gemm_fused(x8, L["rs"], sx, L["s1"], L["N"], L["K"], 0), want))
+            for y, want in out:
+                wrong.add_((y.view(torch.int16) != want.view(torch.int16)).sum())
+        with torch.cuda.stream(stream):
+            step()
+            stream.synchronize()
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=stream):
+                step()
+        runs.append((M, stream, graph, wrong, cases))
+    for _ in range(1500):
+        for _, stream, graph, *_ in runs:
+            with torch.cuda.stream(stream):
+                graph.replay()
+    torch.cuda.synchronize()
+    for M, _, _, wrong, _ in runs:
+        assert int(wrong) == 0, M
+    ops.poll_status()

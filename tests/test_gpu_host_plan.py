@@ -128,3 +128,24 @@ def test_a_dropped_plan_keeps_its_buffers_until_its_replays_end():
     main.synchronize()
     assert all(torch.equal(y, e) for (_, _, y), e in zip(req, want))
     del junk
+
+
+def test_many_replays_of_a_decode_step():
+    """Two decoder layers' linears at four tokens, several streams at once, some thousand replays: every output of every
+    replay is compared."""
+    from liquidgemm_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(23)
+    req, want = [], []
+    for n, k in [(6144, 4096), (4096, 4096), (28672, 4096), (4096, 14336)] * 2:
+        req.append((torch.randn(4, k).half().pin_memory(), _layer(n, k, g), _pinned(4, n)))
+        x8, sx = torch.ops.liquidgemm.quant_per_token(req[-1][0].cuda())
+        L = req[-1][1]
+        want.append(ops.gemm_fused(x8, L["rs"], sx, L["s1"], n, k, 1, splitk=-1).cpu())
+    plan = ops.HostStepPlan(req)
+    for i in range(3000):
+        plan.run()
+        plan.synchronize()
+        for (_, _, y), w in zip(req, want):
+            assert torch.equal(y.view(torch.int16), w.view(torch.int16)), i
+            y.zero_()
+    ops.poll_status()
