@@ -335,11 +335,11 @@ __device__ __forceinline__ void quant_vec(const uint4& raw, float scale, float i
     q[2 * i] = __float_as_uint(t[i].x);
     q[2 * i + 1] = __float_as_uint(t[i].y);
   }
-  if (!safe) {   // one element, nearly always
+  if (!safe) {
 #pragma unroll
     for (int i = 0; i < VEC / 2; ++i) {
-      if (!near_integer(x[i].x, inv)) q[2 * i] = (uint32_t)quant1(x[i].x, scale);
-      if (!near_integer(x[i].y, inv)) q[2 * i + 1] = (uint32_t)quant1(x[i].y, scale);
+      q[2 * i] = (uint32_t)quant1(x[i].x, scale);
+      q[2 * i + 1] = (uint32_t)quant1(x[i].y, scale);
     }
   }
 #pragma unroll
