@@ -5,7 +5,7 @@
 // gather for the prepack (liquidgemm/ops.py:118-150).
 //
 // Rows that a CTA can hold (aligned, up to 65536 elements; float32 32768) take quantise_rows_kernel, one pass over the
-// weights: 28672 x 4096 bf16 481 -> 80 us, 4096 x 14336 273 -> 51 us against the two passes below, which serve the rest:
+// weights: 28672 x 4096 bf16 481 -> 82 us, 4096 x 14336 273 -> 51 us against the two passes below, which serve the rest:
 //   pass 1  row_amax_kernel      one warp per row: s1 = max(amax, 1e-12) / 119 (IEEE division)
 //   pass 2  quantise_tiles_kernel one CTA per 128 x 128 tile of the weight matrix, thread = (row, 64-wide half):
 //             q    = clamp(rint(w / s1[row]), -119, 119)                       (level 1, :70-72)
