@@ -272,7 +272,8 @@ LQ_API int lq_w4a8_linear_bias(const int8_t* x_i8, const uint8_t* blob, const fl
 
 /* One W4A8 linear from activations to outputs: lq_quant_per_token followed by lq_w4a8_gemm_fused (with `bias`, or null:
  * lq_w4a8_linear_bias), bit for bit.  For a few tokens it is ONE kernel, which quantises the tokens itself; otherwise
- * the quantised tokens go through `scratch`.
+ * the quantised tokens go through `scratch`.  y may overlap x from three tokens on (then it is always the two); at one
+ * and two tokens it must not.
  * lq_linear_plan() fills plan[0] = scratch bytes (any content, 16-byte aligned), plan[1] = workspace bytes and
  * plan[2] = workspace kind (as lq_gemm_workspace_kind) for the same x (its alignment matters), M, N, K and splitk. */
 LQ_API int lq_linear_plan(const void* x, int M, int N, int K, int splitk, size_t* plan);

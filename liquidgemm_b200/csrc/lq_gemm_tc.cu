@@ -875,6 +875,11 @@ static bool quantises_in_decode(const void* x, int M, int N, int K, int splitk) 
   return splitk == 0 && M <= decode_tc_max_m() && decode_tc_quantises(M, N, K) && reinterpret_cast<uintptr_t>(x) % 16 == 0;
 }
 
+static bool ranges_overlap(const void* a, size_t a_bytes, const void* b, size_t b_bytes) {
+  const uintptr_t p = reinterpret_cast<uintptr_t>(a), q = reinterpret_cast<uintptr_t>(b);
+  return p < q + b_bytes && q < p + a_bytes;
+}
+
 int lq_linear_plan(const void* x, int M, int N, int K, int splitk, size_t* plan) {
   if (!plan || M <= 0 || N <= 0) return LQ_ERR_BAD_ARG;
   if (K < 128 || K % 128) return LQ_ERR_SHAPE;
@@ -898,8 +903,10 @@ static int linear_impl(const void* x, int x_dtype, const uint8_t* blob, const fl
     return run_gemv_quant(x, x_dtype, blob, s1, bias, y, out_dtype, M, N, K, workspace, workspace_bytes, as_stream(stream));
   }
   if (!scratch || reinterpret_cast<uintptr_t>(scratch) % 16 || scratch_bytes < token_scratch_bytes(M, K)) return LQ_ERR_WORKSPACE;
-  // One kernel again, without need of the scratch and workspace that the two launches take: callers are told the same sizes.
-  if (quantises_in_decode(x, M, N, K, splitk)) {
+  // One kernel again, without need of the scratch that the two launches take.  It is asked for all the same: outputs that
+  // overlap the activations, which that kernel still reads when its first CTAs store, take the two launches.
+  const size_t x_bytes = (size_t)M * K * (x_dtype == LQ_DT_F32 ? 4 : 2), y_bytes = (size_t)M * N * (out_dtype == LQ_DT_F32 ? 4 : 2);
+  if (quantises_in_decode(x, M, N, K, splitk) && !ranges_overlap(x, x_bytes, y, y_bytes)) {
     if (!workspace || workspace_bytes < decode_tc_workspace_bytes(M)) return LQ_ERR_WORKSPACE;
     if (int rc = lq_check_device()) return rc;
     return run_decode_tc(x, x_dtype, blob, nullptr, s1, bias, single_out(y, N), nullptr, out_dtype, M, N, K, workspace, workspace_bytes, as_stream(stream));

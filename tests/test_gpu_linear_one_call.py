@@ -112,3 +112,26 @@ def test_refusals_stay(ops):
         ops.w4a8_linear(good, {**L, "s1": L["s1"][:-1]})
     assert ops.w4a8_linear(good[:0], L).shape == (0, 128)
     assert torch.equal(ops.w4a8_linear(good.t().contiguous().t(), L), ops.w4a8_linear(good, L))
+
+
+@pytest.mark.parametrize("M", [3, 5, 8, 9, 32, 64])
+@pytest.mark.parametrize("shift", [0, 1024, -1024])
+def test_outputs_over_the_activations(ops, M, shift):
+    """From three tokens on the outputs may lie over the activations (here at the same address, or some elements before or
+    behind it): the tokens are quantised into the scratch first."""
+    from liquidgemm_b200._lib import lib, check
+    N = K = 4096
+    L, x = _layer(ops, N, K, 1), _tokens(M, K, torch.bfloat16, M)
+    want = _two_calls(x, L, None, 0)
+    buf = torch.empty(M * K + 2048, dtype=torch.bfloat16, device="cuda")
+    src, dst = buf[1024:1024 + M * K], buf[1024 + shift:1024 + shift + M * N]
+    nscratch, nws, kind = ops._linear_sizes(src.data_ptr(), M, N, K, 0)
+    scratch = torch.empty(nscratch, dtype=torch.uint8, device="cuda")
+    ws = ops._workspace(nws, x.device) if kind != 1 else torch.empty(nws, dtype=torch.uint8, device="cuda")
+    for _ in range(20):
+        src.copy_(x.view(-1))
+        check(lib.lq_w4a8_linear(src.data_ptr(), 0, L["rs"].data_ptr(), L["s1"].data_ptr(), None, dst.data_ptr(), 0, M, N, K, 0,
+                                 scratch.data_ptr(), nscratch, None if ws is None else ws.data_ptr(),
+                                 0 if ws is None else ws.numel(), torch.cuda.current_stream().cuda_stream), "w4a8_linear")
+        assert torch.equal(dst.view(M, N), want)
+    ops.poll_status()
