@@ -698,9 +698,16 @@ bool decode_tc_quantises(int M, int N, int K) {
   return p.tiles * p.splits <= sm_count();
 }
 
-// What callers are told to bring for this kernel (all zero, left all zero).  It is not used: the join stays inside the
-// cluster.  The size and the check of it are those of the kernel that joined through global memory.
-size_t decode_tc_workspace_bytes(int M) { return (size_t)(2 * sm_count()) * (size_t)((M <= 16 ? 16 : 32) * 128 * 8); }
+// What callers are told to bring for this kernel: nothing, since the join stays inside the cluster.  Only where a kernel that
+// joined through global memory served before (up to 16 tokens on matrices up to 32 M weights) the all-zero buffer that
+// callers were told of, and without which the call is refused, is kept; it is not touched.
+size_t decode_tc_workspace_bytes(int M, int N, int K) {
+  return M <= 16 && (long)N * K <= (1L << 25) ? (size_t)(2 * sm_count()) * (size_t)(16 * 128 * 8) : 0;
+}
+bool decode_tc_workspace_ok(int M, int N, int K, const void* ws, size_t ws_bytes) {
+  const size_t need = decode_tc_workspace_bytes(M, N, K);
+  return need == 0 || (ws && ws_bytes >= need);
+}
 
 // CTAs a launch of this shape uses: what a consumer of the gather-by-stores epilogue must see arrive
 // from every rank.
@@ -715,7 +722,7 @@ int run_decode_tc(const void* x, int x_dtype, const uint8_t* blob, const float* 
                   cudaStream_t st) {
   using namespace dtc;
   if (M < 1 || M > (x_dtype >= 0 ? kQuantTokens : 32)) return LQ_ERR_SHAPE;
-  if (!ws || ws_bytes < decode_tc_workspace_bytes(M)) return LQ_ERR_WORKSPACE;
+  if (!decode_tc_workspace_ok(M, N, K, ws, ws_bytes)) return LQ_ERR_WORKSPACE;
   const Plan plan = plan_for(M, N, K);
   if (plan.ring == 0) return LQ_ERR_SHAPE;
   Args a;

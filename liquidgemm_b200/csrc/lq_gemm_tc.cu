@@ -60,7 +60,8 @@ int run_tile_gemm(const int8_t* x, const uint8_t* blob, const float* ascale, con
 int tile_output_grid(int M, int N, int K, int splits);                            // lq_gemm_tile.cu
 bool decode_tc_serves(int M, int N, int K);                                  // lq_decode_tc.cu
 bool decode_tc_quantises(int M, int N, int K);                               // lq_decode_tc.cu
-size_t decode_tc_workspace_bytes(int M);                                     // lq_decode_tc.cu
+size_t decode_tc_workspace_bytes(int M, int N, int K);                       // lq_decode_tc.cu
+bool decode_tc_workspace_ok(int M, int N, int K, const void* ws, size_t ws_bytes);   // lq_decode_tc.cu
 int run_decode_tc(const void* x, int x_dtype, const uint8_t* blob, const float* ascale, const float* s1, const void* bias,
                   const OutSpec& out, const PeerSync* sync, int out_mode, int M, int N, int K, void* ws, size_t ws_bytes,
                   cudaStream_t st);  // lq_decode_tc.cu
@@ -778,7 +779,7 @@ static Route route_for(int M, int N, int K, int splitk, bool scaled, bool single
 static size_t route_ws_bytes(const Route& r, int M, int N, int K) {
   switch (r.kind) {
     case kRouteGemv: return gemv_blob_workspace_bytes(N, K);
-    case kRouteDecodeTc: return decode_tc_workspace_bytes(M);
+    case kRouteDecodeTc: return decode_tc_workspace_bytes(M, N, K);
     case kRouteTile: return tile_workspace_bytes(M, N, r.splits);
     case kRoutePair: return pair_workspace_bytes(M, N, K);
     case kRouteUnpackI8: return (size_t)N * K;   // scratch: the INT8 weights
@@ -907,7 +908,7 @@ static int linear_impl(const void* x, int x_dtype, const uint8_t* blob, const fl
   // overlap the activations, which that kernel still reads when its first CTAs store, take the two launches.
   const size_t x_bytes = (size_t)M * K * (x_dtype == LQ_DT_F32 ? 4 : 2), y_bytes = (size_t)M * N * (out_dtype == LQ_DT_F32 ? 4 : 2);
   if (quantises_in_decode(x, M, N, K, splitk) && !ranges_overlap(x, x_bytes, y, y_bytes)) {
-    if (!workspace || workspace_bytes < decode_tc_workspace_bytes(M)) return LQ_ERR_WORKSPACE;
+    if (!decode_tc_workspace_ok(M, N, K, workspace, workspace_bytes)) return LQ_ERR_WORKSPACE;
     if (int rc = lq_check_device()) return rc;
     return run_decode_tc(x, x_dtype, blob, nullptr, s1, bias, single_out(y, N), nullptr, out_dtype, M, N, K, workspace, workspace_bytes, as_stream(stream));
   }

@@ -110,3 +110,28 @@ def test_several_streams_at_once():
     for M, _, _, wrong, _ in runs:
         assert int(wrong) == 0, M
     ops.poll_status()
+
+
+@pytest.mark.parametrize("M,N,K", [(17, 4096, 4096), (32, 6144, 2048), (24, 18944, 512), (8, 18944, 4096)])
+def test_calls_without_a_workspace(M, N, K):
+    """Where callers are told that none is needed, none is asked for, with int8 tokens and with activations."""
+    from liquidgemm_b200 import ops
+    from liquidgemm_b200._lib import lib, check
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    qw, blob = ops.quantize_weight_cuda(torch.randn(N, K, generator=g, device="cuda") * 0.03, 64, want_codes=False, want_blob=True)
+    x = torch.randn(M, K, generator=g, device="cuda", dtype=torch.bfloat16)
+    x8, sx = torch.ops.liquidgemm.quant_per_token(x)
+    want = ops.gemm_fused(x8, blob.reshape(-1), sx, qw.s1, N, K, 0, splitk=-1)
+    st = torch.cuda.current_stream().cuda_stream
+    y = torch.empty_like(want)
+    check(lib.lq_w4a8_gemm_fused(x8.data_ptr(), blob.data_ptr(), sx.data_ptr(), qw.s1.data_ptr(), y.data_ptr(), 0, M, N, K, 0,
+                                 None, 0, st), "w4a8_gemm_fused")
+    assert torch.equal(y, want)
+    y.zero_()
+    nscratch, nws, kind = ops._linear_sizes(x.data_ptr(), M, N, K, 0)
+    assert nws == kind == 0
+    scratch = torch.empty(nscratch, dtype=torch.uint8, device="cuda")
+    check(lib.lq_w4a8_linear(x.data_ptr(), 0, blob.data_ptr(), qw.s1.data_ptr(), None, y.data_ptr(), 0, M, N, K, 0,
+                             scratch.data_ptr(), nscratch, None, 0, st), "w4a8_linear")
+    assert torch.equal(y, want)
+    ops.poll_status()
