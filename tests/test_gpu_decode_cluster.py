@@ -112,6 +112,35 @@ def test_several_streams_at_once():
     ops.poll_status()
 
 
+@pytest.mark.parametrize("M", [8, 17, 32])
+@pytest.mark.parametrize("N,K", [(384, 2048), (200, 7680), (18944, 512)])   # K cut evenly, unevenly, not at all
+def test_several_destinations(M, N, K):
+    """The multi-destination form: two wider matrices, then a sequence in which each launch waits for the flags that the
+    one before has raised, one count per CTA."""
+    from liquidgemm_b200 import ops
+    qw = random_lqq(N, K, seed=N + M)
+    tq = to_torch_qw(qw)
+    blob = ops._repack_device(tq.qweight_u4, 0, tq.s_u8, tq.offset_a, N, K, 64).reshape(-1)
+    x, sc = random_tokens(M, K, seed=M)
+    xt, st = torch.from_numpy(x).cuda(), torch.from_numpy(sc).cuda()
+    want = O.w4a8_matmul(x, sc, qw)
+    ld, col = N + 616, 256
+    outs = [torch.full((M, ld), -7.0, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    ops.gemm_fused_scatter(xt, blob, st, tq.s1, [o.data_ptr() for o in outs], ld, col, N, K, 0)
+    for o in outs:
+        assert_bits_equal(o[:, col:col + N].contiguous(), want, 0, "destinations")
+        assert bool((o[:, :col] == -7.0).all()) and bool((o[:, col + N:] == -7.0).all())
+    grid, flags = ops.decode_grid(M, N, K), torch.zeros(4, dtype=torch.int32, device="cuda")
+    outs = [torch.zeros((M, N), dtype=torch.float16, device="cuda") for _ in range(3)]
+    for k, o in enumerate(outs):
+        ops.gemm_fused_scatter(xt, blob, st, tq.s1, [o.data_ptr()], N, 0, N, K, 1, flag_ptrs=[flags.data_ptr()], flag_index=k,
+                               wait_ptr=(flags.data_ptr() + 4 * (k - 1)) if k else None, wait_value=grid if k else 0)
+    for o in outs:
+        assert_bits_equal(o, want, 1, "flags")
+    assert flags.tolist() == [grid] * 3 + [0]
+    ops.poll_status()
+
+
 @pytest.mark.parametrize("M,N,K", [(17, 4096, 4096), (32, 6144, 2048), (24, 18944, 512), (8, 18944, 4096)])
 def test_calls_without_a_workspace(M, N, K):
     """Where callers are told that none is needed, none is asked for, with int8 tokens and with activations."""
