@@ -164,3 +164,20 @@ def test_calls_without_a_workspace(M, N, K):
                              scratch.data_ptr(), nscratch, None, 0, st), "w4a8_linear")
     assert torch.equal(y, want)
     ops.poll_status()
+
+
+def test_token_scales_over_the_range():
+    """The quantising form's own division by 127 against the token quantiser's, over the exponents of float32."""
+    from liquidgemm_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(9)
+    N, K = 64, 128
+    qw, blob = ops.quantize_weight_cuda(torch.randn(N, K, generator=g, device="cuda"), 64, want_codes=False, want_blob=True)
+    L = {"s1": qw.s1, "s_u8": qw.s_u8, "offset_a": qw.offset_a, "N": N, "K": K, "rs": blob.reshape(-1)}
+    for i in range(300):
+        x = torch.randn(8, K, generator=g, device="cuda") * torch.exp2(torch.rand(8, 1, generator=g, device="cuda") * 160 - 40)
+        if i == 0:
+            x[:, 0] = torch.tensor([3e38, 3.1e38, torch.finfo(torch.float32).max, 1e-12, 0.9e-12, 1.1e-12, 0.0, 127.0], device="cuda")
+        xq, sc = torch.ops.liquidgemm.quant_per_token(x)
+        want = torch.ops.liquidgemm.w4a8_wgmma_rs_fused(xq, L["rs"], L["s_u8"], L["offset_a"], sc, L["s1"], N, K, 64, 2)
+        assert torch.equal(ops.w4a8_linear(x, L).view(torch.int32), want.view(torch.int32)), i
+    ops.poll_status()

@@ -31,3 +31,27 @@ def test_safe_distance_covers_both_roundings():
         safe = np.abs(prod - near).astype(np.float32) < np.float32(0.5 - 2.0 ** -14)
         assert np.array_equal(near[safe], np.rint(x / scale)[safe])
         assert safe.any() and not safe.all()
+
+
+def _fma(a, b, c):
+    """float32 fused multiply-add: the exact sum rounded to odd in float64, then to float32."""
+    p, c = a.astype(np.float64) * np.float64(b), c.astype(np.float64)      # 24 x 24 bits: exact
+    hi = p + c
+    t = hi - p
+    err = (p - (hi - t)) + (c - t)
+    bits = hi.view(np.int64)
+    odd = np.where((err > 0) == (hi > 0), bits | 1, bits - 1)
+    return np.where((err != 0) & (bits & 1 == 0), odd, bits).view(np.float64).astype(np.float32)
+
+
+def test_token_scale_is_the_rounded_quotient():
+    """max(amax, 1e-12) / 127 by the residual of the product with fl(1 / 127): every mantissa of a binade, and the ends of
+    the range of exponents (above 3e38, infinity and NaN are divided)."""
+    inv = np.float32(1) / np.float32(127)
+    one = (np.arange(1 << 23, dtype=np.uint32) | np.uint32(0x3F800000)).view(np.float32)
+    for scale in (1.0, 2.0 ** -39, 2.0 ** 126):
+        a = one[:: 1 if scale == 1.0 else 97] * np.float32(scale)
+        a = np.maximum(a[a < np.float32(3e38)], np.float32(1e-12))
+        q = a * inv
+        r = _fma(q, np.float32(-127), a)
+        assert np.array_equal(_fma(r, inv, q), a / np.float32(127)), scale
