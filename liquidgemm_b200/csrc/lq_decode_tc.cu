@@ -603,13 +603,19 @@ w4a8_decode_tc_kernel(const Args args, const std::conditional_t<MULTI, MultiOut,
 struct Plan {
   int tiles, splits, nk, ring, smem;   // ring 0: not a shape for this kernel
 };
-// Which shapes the kernel takes and how it cuts them.  Two launches have to fit the machine side by side (one CTA of each
-// per SM), or the second loses the head start that the design lives from: at most one CTA per SM, and at most 128
-// where clusters of three and more leave slots of a GPC empty (6144 x 4096 at 8 tokens: 2 / 3 / 4 / 6 k-ranges a tile
+// Which shapes the kernel takes and how it cuts them.  Two launches should fit the machine side by side (one CTA of each
+// per SM), or the second loses the head start that the design lives from: up to 74 tiles at most one CTA per SM, and at most
+// 130 where clusters of three and more leave slots of a GPC empty (6144 x 4096 at 8 tokens: 2 / 3 / 4 / 6 k-ranges a tile
 // = 96 / 144 / 192 / 288 CTAs 6.0 / 6.8 / 6.5 / 10.4 us).  Within that as many k-ranges as there is room for (4096 x 4096: 3 / 4 ranges
 // 4.8 / 4.4; 2048 x 8192: 4 / 5 / 8 6.0 / 5.4 / 4.9).  A k-range is at most 16 k-tiles (8 above 16 tokens): the tokens of the
 // range stay in shared memory, and k-tiles beyond those unpacked ahead cost 0.2 us each behind the tokens (4096 x 14336 in 28s:
 // 9.8 us against the tile kernel's 9.9 with its finish pass; 7168 x 8192 in 32s 12.2 against 9.7).
+// From 75 tiles on a k longer than that is cut in two all the same, with two CTAs on most SMs (here and below in us with the
+// quantiser at 8 tokens, weights from HBM, this kernel / the tile kernel: 9728 x 4096 9.3 / 10.0, 12800 x 4096 10.1 / 11.7, 17408 x
+// 4096 12.1 / 12.7).  With a tile on nearly every SM only one range of 9..16 k-tiles is left (148 tiles: K = 512 5.6 / 4.8, 1024 6.1 /
+// 6.0, 2048 8.8 / 10.3, 4096 in two 13.8 / 13.3).  Above 16 tokens the tile kernel's whole tiles are ahead on short
+// k and on many tiles (24 tokens: 4096 x 512 and its like 5.2 / 5.0, 12800 x 1024 6.1 / 5.9, 16384 x 1024 6.4 / 6.0; 8192 x 1024
+// 6.0 / 6.6, 9728 x 1024 6.2 / 6.4).
 static Plan plan_for(int M, int N, int K) {
   const int bn = M <= 16 ? 16 : 32;
   const int kt = K / 128;
@@ -622,6 +628,8 @@ static Plan plan_for(int M, int N, int K) {
   if (S > kt / 4) S = kt / 4 > 1 ? kt / 4 : 1;
   if (S == 1 && kt > 16 && p.tiles <= sms && bn == 16) S = 2;
   if (S < 1) return p;
+  if (p.tiles > sms - sms / 16 && (kt <= 8 || S > 1)) return p;
+  if (bn == 32 && (kt < 8 || p.tiles > sms * 5 / 8)) return p;
   p.splits = S;
   p.nk = (kt + S - 1) / S;
   if (p.nk > (bn == 16 ? 16 : 8)) return p;

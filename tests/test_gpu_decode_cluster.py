@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 # k-tiles x k-ranges: one k-tile; fewer k-tiles than operand stages, as many and one more; every cluster size up to eight
 # with even and odd ranges; a ring shorter than the range; ragged N; whole tiles up to one per SM; two CTAs per SM
 SHAPES = [(128, 128), (64, 896), (200, 1024), (320, 2176), (1000, 1920), (2048, 2048), (3072, 4224), (3840, 3072), (6144, 640),
-          (512, 14336), (6144, 4096), (8960, 2048), (9600, 1152), (18944, 512), (12800, 2560)]
+          (512, 14336), (6144, 4096), (8960, 2048), (9600, 1152), (18944, 512), (18944, 1152), (12800, 2560)]
 TOKENS = [3, 8, 9, 16, 17, 32]
 
 
@@ -113,7 +113,7 @@ def test_several_streams_at_once():
 
 
 @pytest.mark.parametrize("M", [8, 17, 32])
-@pytest.mark.parametrize("N,K", [(384, 2048), (200, 7680), (18944, 512)])   # K cut evenly, unevenly, not at all
+@pytest.mark.parametrize("N,K", [(384, 2048), (200, 7680), (9728, 1024)])   # K cut evenly, unevenly, not at all
 def test_several_destinations(M, N, K):
     """The multi-destination form: two wider matrices, then a sequence in which each launch waits for the flags that the
     one before has raised, one count per CTA."""
@@ -141,7 +141,7 @@ def test_several_destinations(M, N, K):
     ops.poll_status()
 
 
-@pytest.mark.parametrize("M,N,K", [(17, 4096, 4096), (32, 6144, 2048), (24, 18944, 512), (8, 18944, 4096)])
+@pytest.mark.parametrize("M,N,K", [(17, 4096, 4096), (32, 6144, 2048), (24, 9728, 1024), (8, 17408, 4096)])
 def test_calls_without_a_workspace(M, N, K):
     """Where callers are told that none is needed, none is asked for, with int8 tokens and with activations."""
     from liquidgemm_b200 import ops

@@ -47,9 +47,11 @@ def test_size_helpers_without_gpu():
     assert lib.lq_gemm_workspace_kind(2, 4096, 14336, 0) == 2        # streaming decode kernels
     assert lib.lq_gemm_workspace_kind(8, 6144, 4096, 0) == 2         # streaming tensor-core kernel, atomic join
     assert lib.lq_gemm_workspace_bytes(16, 4096, 4096, 0) == lib.lq_gemm_workspace_bytes(5, 4096, 4096, 0) > 0
-    for m, n, k in [(17, 4096, 4096), (32, 6144, 2048), (24, 18944, 512), (8, 18944, 4096)]:   # one launch, joined in clusters
+    for m, n, k in [(17, 4096, 4096), (32, 6144, 2048), (24, 9728, 1024), (8, 17408, 4096)]:   # one launch, joined in clusters
         assert lib.lq_gemm_workspace_bytes(m, n, k, 0) == lib.lq_gemm_workspace_kind(m, n, k, 0) == 0
         assert lib.lq_scatter_workspace_bytes(m, n, k) == lib.lq_scatter_workspace_kind(m, n, k) == 0
+    assert lib.lq_gemm_launches(8, 17408, 4096, 0) == 1 and lib.lq_decode_grid(8, 17408, 4096) == 2 * 136
+    assert lib.lq_gemm_launches(8, 18944, 4096, 0) == 2              # a tile on every SM: k-ranges by the tile kernel
     assert lib.lq_gemm_workspace_kind(8, 4096, 14336, 0) == 1        # larger matrix: tile kernel with split-K planes
     assert lib.lq_gemm_workspace_kind(64, 4096, 14336, 0) == 1       # tile kernel with split-K planes
     assert lib.lq_gemm_workspace_kind(4096, 28672, 4096, 0) == 2     # pair kernel, last wave split along k
