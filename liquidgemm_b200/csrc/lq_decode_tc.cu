@@ -84,6 +84,8 @@ struct Cfg {
   static constexpr int kNT = (kTmemCols - kACol) / 32;
 };
 constexpr int kQuantTokens = 8;              // limit of the quantising form: a warp per row
+constexpr int kQuantChunks = 2;              // chunks of sixteen activations that a lane of it holds
+__host__ __device__ inline int quant_warps(int M) { return M > 4 ? 1 : 2; }   // warps of a token row
 constexpr int kMaxParts = 8 * kMaxSplits;    // parts of the row maxima: one per warp and CTA of the cluster
 constexpr int kNumBars = 2 * kMaxRing + 2 * 8 + 4;
 
@@ -173,8 +175,7 @@ w4a8_decode_tc_kernel(const Args args, const std::conditional_t<MULTI, MultiOut,
   const int groups = (M + 3) >> 2;   // of four tokens
   const bool scaled = args.out_mode != kOutI32;
   const bool has_bias = scaled && args.bias != nullptr;
-  // warps of a token row while the maxima are taken (QUANT)
-  const int wpr = M > 4 ? 1 : M > 2 ? 2 : M == 2 ? 4 : 8;
+  const int wpr = quant_warps(M);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < NW; ++s) {
@@ -434,9 +435,9 @@ w4a8_decode_tc_kernel(const Args args, const std::conditional_t<MULTI, MultiOut,
               *reinterpret_cast<uint4*>(smem + (j0 + kSets * u) * kXStage + x_off + q * 2048) = xv[u][q];
       }
     } else {
-      // Up to eight tokens, one or more warps a row (wpr); a lane takes every 32 * wpr-th chunk of sixteen activations of
-      // the CTA's k-range and keeps the first H of them in registers until the row's scale is known.
-      constexpr int H = sizeof(XT) == 4 ? 2 : 4;
+      // Up to eight tokens, one or two warps a row (wpr); a lane holds every 32 * wpr-th chunk of sixteen activations of
+      // the CTA's k-range in registers until the row's scale is known (decode_tc_quantises() keeps them to H).
+      constexpr int H = kQuantChunks;
       const int m = (d >> 5) / wpr, part = (d >> 5) % wpr;
       const int c0 = part * 32 + lane, cstep = 32 * wpr, nch = m < M ? nk * 8 : 0;
       const XT* x = static_cast<const XT*>(args.x) + (size_t)m * args.K + (size_t)kb * 128;
@@ -452,13 +453,6 @@ w4a8_decode_tc_kernel(const Args args, const std::conditional_t<MULTI, MultiOut,
       for (int h = 0; h < H; ++h)
 #pragma unroll
         for (int k = 0; k < (int)sizeof(XT); ++k) rm.take(held[h].r[k]);
-#pragma unroll 2
-      for (int c = c0 + H * cstep; c < nch; c += cstep) {
-        Chunk<XT> ck;
-        ck.load(x + (size_t)c * 16);
-#pragma unroll
-        for (int k = 0; k < (int)sizeof(XT); ++k) rm.take(ck.r[k]);
-      }
       // The maxima of the row's parts (warps of all CTAs of the cluster) go to every CTA; non-negative floats are ordered
       // like their bits.
       const uint32_t top = __reduce_max_sync(0xffffffffu, __float_as_uint(rm.value()));
@@ -491,12 +485,6 @@ w4a8_decode_tc_kernel(const Args args, const std::conditional_t<MULTI, MultiOut,
 #pragma unroll
         for (int h = 0; h < H; ++h)
           if (c0 + h * cstep < nch) put(c0 + h * cstep, held[h].quantised(scale, inv));
-#pragma unroll 2
-        for (int c = c0 + H * cstep; c < nch; c += cstep) {
-          Chunk<XT> ck;
-          ck.load(x + (size_t)c * 16);
-          put(c, ck.quantised(scale, inv));
-        }
       }
     }
     // written with ordinary stores: make the tokens visible to the tensor core's reads
@@ -698,12 +686,17 @@ bool decode_tc_serves(int M, int N, int K) {
 
 // Whether it also quantises its tokens: three to eight, one CTA per SM at most.  Below, the quantising GEMV is ahead (two
 // tokens 1280 x 8192 5.0 against 5.1 us, 6144 x 4096 6.8 against 6.8, one token 4096 x 4096 4.8 against 5.2); above, the pass over the
-// activations costs more than the quantiser's launch (4096 x 4096 at 16 tokens 6.2 us behind the quantiser, 7.6 here; at eight 6.1 and
-// 5.7), and so it does where two CTAs share an SM (12800 x 2560 at eight tokens 8.1 and 9.0).
+// activations costs more than the quantiser's launch (4096 x 4096 at 16 tokens 6.2 us behind the quantiser, 7.6 here), and so it does
+// where two CTAs share an SM (12800 x 2560 at eight tokens 8.1 and 9.0).  A lane holds two chunks of activations: with two warps a
+// row (up to four tokens) any range that the plan cuts, with one up to eight k-tiles.  Four chunks a lane spilled registers and
+// lengthened every such launch by 8 to 11 %, and ranges above eight k-tiles at five to eight tokens lost to the quantiser's launch
+// (6144 x 4096 at eight tokens 9.6 us against 8.2).  us at four and eight tokens, weights from HBM, in the kernel / behind the
+// quantiser: 1024 x 4096 4.1 / 5.2 and 4.3 / 5.4; 1280 x 8192 4.9 / 6.2 and 5.6 / 6.6; 6144 x 2048 4.8 / 5.6 and 5.4 / 5.7; 4096 x 4096
+// 5.3 / 6.2 and 6.0 / 6.3; 6144 x 4096 7.4 / 7.9 at four.
 bool decode_tc_quantises(int M, int N, int K) {
   if (M < 3 || M > dtc::kQuantTokens || !decode_tc_serves(M, N, K)) return false;
   const dtc::Plan p = dtc::plan_for(M, N, K);
-  return p.tiles * p.splits <= sm_count();
+  return p.tiles * p.splits <= sm_count() && p.nk * 8 <= dtc::kQuantChunks * 32 * dtc::quant_warps(M);
 }
 
 // What callers are told to bring for this kernel: nothing, since the join stays inside the cluster.  Only where a kernel that
@@ -729,7 +722,7 @@ int run_decode_tc(const void* x, int x_dtype, const uint8_t* blob, const float* 
                   const OutSpec& out, const PeerSync* sync, int out_mode, int M, int N, int K, void* ws, size_t ws_bytes,
                   cudaStream_t st) {
   using namespace dtc;
-  if (M < 1 || M > (x_dtype >= 0 ? kQuantTokens : 32)) return LQ_ERR_SHAPE;
+  if (M < 1 || M > 32 || (x_dtype >= 0 && !decode_tc_quantises(M, N, K))) return LQ_ERR_SHAPE;
   if (!decode_tc_workspace_ok(M, N, K, ws, ws_bytes)) return LQ_ERR_WORKSPACE;
   const Plan plan = plan_for(M, N, K);
   if (plan.ring == 0) return LQ_ERR_SHAPE;
