@@ -190,7 +190,8 @@ int run_unpack_blob_i8(const uint8_t* blob, int8_t* w, int N, int K, cudaStream_
 // becomes resident, so they must not be read through the non-coherent path (see ld_stream_v4).
 // MULTI: the outputs go to several row-major matrices with their own row stride and column offset (gather by
 // stores over NVLink, see OutSpec), element by element, and every CTA signals the peers' flags at its end.
-template <bool MULTI>
+// CLEAR: the planes lie in the buffer that is all zero between calls and are left zero (int32 outputs at a few tokens).
+template <bool MULTI, bool CLEAR>
 __global__ void __launch_bounds__(256)
 finish_kernel(const int32_t* acc, const float* ascale, const float* s1, const void* bias, void* y, int out_dtype, int planes,
               int M, int N, bool vec, const std::conditional_t<MULTI, MultiOut, NoMultiOut> multi) {
@@ -211,6 +212,10 @@ finish_kernel(const int32_t* acc, const float* ascale, const float* s1, const vo
       for (int p = 1; p < planes; ++p) {
         const int4 w = *reinterpret_cast<const int4*>(acc + (long)p * total + idx);
         v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w;
+      }
+      if constexpr (CLEAR) {
+        for (int p = 0; p < planes; ++p)
+          *reinterpret_cast<int4*>(const_cast<int32_t*>(acc) + (long)p * total + idx) = make_int4(0, 0, 0, 0);
       }
       if (out_dtype == 3) {  // exact int32 sum, no scaling
         *reinterpret_cast<int4*>(reinterpret_cast<int32_t*>(y) + idx) = v;
@@ -259,6 +264,9 @@ finish_kernel(const int32_t* acc, const float* ascale, const float* s1, const vo
       const int n = (int)(idx - (long)m * N);
       int v = acc[idx];
       for (int p = 1; p < planes; ++p) v += acc[(long)p * total + idx];
+      if constexpr (CLEAR) {
+        for (int p = 0; p < planes; ++p) const_cast<int32_t*>(acc)[(long)p * total + idx] = 0;
+      }
       if (out_dtype == 3) reinterpret_cast<int32_t*>(y)[idx] = v;
       else if constexpr (MULTI)
         store_out_all(multi.out, m, n, lqq_scale(v, ascale[m], s1[n]), bias ? load_bias(bias, n, out_dtype) : 0.f,
@@ -394,7 +402,7 @@ static long finish_items(int M, int N, bool vec) { return vec ? ((long)M * N) >>
 int finish_grid(int M, int N) { return grid_for(finish_items(M, N, false), 256, 8); }
 
 int launch_finish(const int32_t* acc, const float* ascale, const float* s1, const void* bias, const OutSpec& out,
-                  const PeerSync* sync, int out_dtype, int planes, int M, int N, cudaStream_t st) {
+                  const PeerSync* sync, int out_dtype, int planes, bool clear_planes, int M, int N, cudaStream_t st) {
   const bool multi = out.n != 1 || out.ld != N || out.col0 != 0 || (sync && (sync->n_signal > 0 || sync->wait));
   void* y = out.ptr[0];
   // four outputs per thread when every row start stays 16-byte aligned (single destination only)
@@ -407,11 +415,11 @@ int launch_finish(const int32_t* acc, const float* ascale, const float* s1, cons
     MultiOut mo;
     mo.out = out;
     mo.sync = sync ? *sync : PeerSync{};
-    e = launch_overlapped(finish_kernel<true>, dim3(grid), dim3(256), (size_t)0, st, acc, ascale, s1, bias, y, out_dtype,
+    e = launch_overlapped(finish_kernel<true, false>, dim3(grid), dim3(256), (size_t)0, st, acc, ascale, s1, bias, y, out_dtype,
                           planes, M, N, vec, mo);
   } else {
-    e = launch_overlapped(finish_kernel<false>, dim3(grid), dim3(256), (size_t)0, st, acc, ascale, s1, bias, y,
-                          out_dtype, planes, M, N, vec, NoMultiOut{});
+    e = launch_overlapped(clear_planes ? finish_kernel<false, true> : finish_kernel<false, false>, dim3(grid), dim3(256),
+                          (size_t)0, st, acc, ascale, s1, bias, y, out_dtype, planes, M, N, vec, NoMultiOut{});
   }
   if (e != cudaSuccess) {
     record_cuda_error(e, "finish_kernel launch");
@@ -472,7 +480,7 @@ int lq_scale_epilogue(const int32_t* acc, const float* ascale, const float* s1, 
   if (!acc || !ascale || !s1 || !y || M < 0 || N <= 0) return LQ_ERR_BAD_ARG;
   if (out_dtype < 0 || out_dtype > 2) return LQ_ERR_BAD_ARG;
   if (M == 0) return LQ_OK;
-  return launch_finish(acc, ascale, s1, nullptr, single_out(y, N), nullptr, out_dtype, 1, M, N, as_stream(stream));
+  return launch_finish(acc, ascale, s1, nullptr, single_out(y, N), nullptr, out_dtype, 1, false, M, N, as_stream(stream));
 }
 
 size_t lq_tile_blob_bytes(int N, int K) {

@@ -56,7 +56,7 @@ int tile_pick_splits(int M, int N, int K);                                   // 
 size_t tile_workspace_bytes(int M, int N, int splits);                       // lq_gemm_tile.cu
 int run_tile_gemm(const int8_t* x, const uint8_t* blob, const float* ascale, const float* s1, const void* bias,
                   const OutSpec& out, const PeerSync* sync, int out_mode, int M, int N, int K, int splits, void* ws,
-                  size_t ws_bytes, cudaStream_t st);  // lq_gemm_tile.cu
+                  size_t ws_bytes, bool clear_planes, cudaStream_t st);  // lq_gemm_tile.cu
 int tile_output_grid(int M, int N, int K, int splits);                            // lq_gemm_tile.cu
 bool decode_tc_serves(int M, int N, int K);                                  // lq_decode_tc.cu
 bool decode_tc_quantises(int M, int N, int K);                               // lq_decode_tc.cu
@@ -758,9 +758,6 @@ static Route route_for(int M, int N, int K, int splitk, bool scaled, bool single
       // planes and finish pass).
       if (decode_serves(M, N, K)) return {kRouteDecodeTc, 0};
     }
-    // int32 outputs where the scaled call takes the GEMV: callers are told one kind of workspace for both, the all-zero
-    // buffer, so the tile kernel must not write its planes there.
-    if (splitk == 0 && !scaled && gemv_serves(M, N, K)) return {kRoutePersistent, 0};
     int S = splitk > 0 ? splitk : tile_pick_splits(M, N, K);
     if (S > kt) S = kt;
     return {kRouteTile, S < 1 ? 1 : S};
@@ -774,6 +771,14 @@ static Route route_for(int M, int N, int K, int splitk, bool scaled, bool single
     return {kRouteTile, tile_pick_splits(M, N, K)};
   }
   return {kRoutePersistent, splitk};
+}
+
+// int32 outputs where the scaled call takes the GEMV: callers are told one kind of workspace for both, the all-zero buffer.
+// The tile kernel's planes then lie in it, and the finish pass clears what it has read.  (The persistent kernel, which joins
+// through the buffer as it is, costs more; us at one token, tile kernel / persistent: 24000 x 512 3.4 / 9.0, 28672 x 4096 14.5 /
+// 19.3, 4096 x 14336 9.6 / 13.4, 7168 x 8192 9.0 / 13.6, 256 x 28672 7.6 / 8.0.)
+static bool planes_in_zeroed_buffer(int M, int N, int K, int splitk, bool scaled) {
+  return splitk == 0 && !scaled && gemv_serves(M, N, K);
 }
 
 static size_t route_ws_bytes(const Route& r, int M, int N, int K) {
@@ -827,7 +832,7 @@ static int blob_gemm(const int8_t* x, const uint8_t* blob, const float* ascale, 
       return run_decode_tc(x, -1, blob, ascale, s1, bias, single_out(out, N), nullptr, out_mode, M, N, K, ws, ws_bytes, st);
     case kRouteTile:
       return run_tile_gemm(x, blob, ascale, s1, bias, single_out(out, N), nullptr, out_mode, M, N, K, r.splits, ws,
-                           ws_bytes, st);
+                           ws_bytes, planes_in_zeroed_buffer(M, N, K, splitk, out_mode != kOutI32), st);
     case kRoutePair:
       return run_pair_gemm(x, blob, ascale, s1, bias, single_out(out, N), nullptr, out_mode, M, N, K, ws, ws_bytes, st);
     case kRouteUnpackI8: {
@@ -979,7 +984,7 @@ int lq_w4a8_gemm_fused_scatter_sync(const int8_t* x_i8, const uint8_t* blob, con
                            as_stream(stream));
     default:
       return run_tile_gemm(x_i8, blob, ascale, s1, nullptr, o, &ps, out_dtype, M, N, K, r.splits, workspace,
-                           workspace_bytes, as_stream(stream));
+                           workspace_bytes, false, as_stream(stream));
   }
 }
 

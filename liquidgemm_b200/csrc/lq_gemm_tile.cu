@@ -30,7 +30,7 @@
 namespace lq {
 
 int launch_finish(const int32_t* acc, const float* ascale, const float* s1, const void* bias, const OutSpec& out,
-                  const PeerSync* sync, int out_dtype, int planes, int M, int N, cudaStream_t st);  // lq_elementwise.cu
+                  const PeerSync* sync, int out_dtype, int planes, bool clear_planes, int M, int N, cudaStream_t st);  // lq_elementwise.cu
 int make_byte_matrix_map(CUtensorMap* map, const void* ptr, long rows, long row_bytes, int box_rows,
                          int box_bytes);  // lq_gemm_tc.cu
 
@@ -476,11 +476,12 @@ int tile_output_grid(int M, int N, int K, int splits) {
   return ((N + 127) / 128) * ((M + bn - 1) / bn);
 }
 
-// out_mode: LQ_DT_* or 3 (raw int32).  Any M.  `ws` holds `splits` int32 planes (need not be zeroed).
+// out_mode: LQ_DT_* or 3 (raw int32).  Any M.  `ws` holds `splits` int32 planes (need not be zeroed;
+// clear_planes: left zero, one destination only).
 // `out`: one or several destinations (gather by stores); `sync`: optional cross-GPU flags.
 int run_tile_gemm(const int8_t* x, const uint8_t* blob, const float* ascale, const float* s1, const void* bias,
                   const OutSpec& out, const PeerSync* sync, int out_mode, int M, int N, int K, int splits, void* ws,
-                  size_t ws_bytes, cudaStream_t st) {
+                  size_t ws_bytes, bool clear_planes, cudaStream_t st) {
   using namespace tile;
   if (splits > 1 && (!ws || ws_bytes < tile_workspace_bytes(M, N, splits))) return LQ_ERR_WORKSPACE;
   const int bn = tile_bn(M, N, K);
@@ -536,7 +537,7 @@ int run_tile_gemm(const int8_t* x, const uint8_t* blob, const float* ascale, con
     fsync.wait = nullptr;   // the planes kernel already waited
   }
   return launch_finish(static_cast<const int32_t*>(ws), ascale, s1, bias, out, sync ? &fsync : nullptr, out_mode, splits,
-                       M, N, st);
+                       clear_planes, M, N, st);
 }
 
 }  // namespace lq

@@ -28,7 +28,7 @@
 namespace lq {
 
 int launch_finish(const int32_t* acc, const float* ascale, const float* s1, const void* bias, const OutSpec& out,
-                  const PeerSync* sync, int out_dtype, int planes, int M, int N, cudaStream_t st);  // lq_elementwise.cu
+                  const PeerSync* sync, int out_dtype, int planes, bool clear_planes, int M, int N, cudaStream_t st);  // lq_elementwise.cu
 int make_byte_matrix_map(CUtensorMap* map, const void* ptr, long rows, long row_bytes, int box_rows,
                          int box_bytes);  // lq_gemm_tc.cu
 
@@ -303,8 +303,8 @@ int run_i8_stream(const int8_t* x, const int8_t* w, const float* ascale, const f
     default: rc = launch<128, 3>(tw, a, S, st); break;
   }
   if (rc || S <= 1) return rc;
-  return launch_finish(static_cast<const int32_t*>(ws), ascale, s1, nullptr, single_out(out, N), nullptr, out_mode, S, M, N,
-                       st);
+  return launch_finish(static_cast<const int32_t*>(ws), ascale, s1, nullptr, single_out(out, N), nullptr, out_mode, S, false,
+                       M, N, st);
 }
 
 }  // namespace lq
