@@ -277,7 +277,7 @@ def parity_gate(torch, sets, acts, launches, run_linear):
 # DRAM read+write bytes per launch / algorithmic bytes per launch, mean over the ncu captures of the decode
 # kernels summarised under profiles/ (taken on single launches of the same shapes; the benchmark itself
 # never runs under a profiler, so `roofline.traffic` is that measured ratio times the step's algorithmic bytes).
-NCU_TRAFFIC_RATIO = 1.007
+NCU_TRAFFIC_RATIO = 1.002
 
 
 def main():

@@ -124,7 +124,7 @@ LQ_API int lq_w4a8_gemv_blob_static(const void* x_i8, const void* blob, const vo
                                     void* stream);
 LQ_API int lq_w4a8_gemv_blob_static_reset(void* stream);
 
-/* lq_w4a8_gemm_fused for a decode batch (M <= 16) whose output block [M, N] is written into n_outs
+/* lq_w4a8_gemm_fused (any M) whose output block [M, N] is written into n_outs
  * (1..8) row-major matrices with row stride ld_out elements at column col0: with the full-width
  * outputs of this GPU and of its peers as destinations (peer memory mapped into this process), the
  * epilogue performs the all-gather of an N-sharded layer with plain stores over NVLink.  `outs` is
@@ -200,7 +200,8 @@ LQ_API int lq_repack_tiles(const uint8_t* src, int src_layout, const uint8_t* s_
 /* The W4A8 calls request the first tiles of their blob while the kernel before them on the stream may still run, so a
  * blob must be settled by then.  lq_repack_tiles and lq_quantize_weight see to that themselves; a caller whose own
  * kernel writes a blob and that wants to use it without synchronising calls lq_settle_blob() on the stream in between
- * (one empty kernel). */
+ * (one empty kernel).  Everything else a call reads (activations, tokens, scales, bias) may be the output of the work
+ * directly before. */
 LQ_API int lq_settle_blob(void* stream);
 
 /* LiquidQuant weight quantiser on the device: w [N, K] (w_dtype: LQ_DT_*) -> s1 [N] float32, s_u8 and
@@ -217,10 +218,10 @@ LQ_API int lq_quantize_weight(const void* w, int w_dtype, int N, int K, int grou
 
 /* Scheduling of the tensor-core GEMM, selected by the `splitk` argument of the calls below.
  *   splitk = 0 (automatic):
- *     one token, two tokens on matrices up to 64 M weights, three or four on matrices up to 16 M weights
- *              (scaled outputs only): streaming dp4a GEMV over the tile blob;
- *     up to 16 tokens on matrices up to 32 M weights: the streaming tensor-core kernel, ONE launch:
- *              stream-K over two CTAs per SM, one 64-bit atomic per element joins cut tiles;
+ *     one token, two tokens on matrices up to 64 M weights, and three or four on matrices up to 16 M weights that
+ *              the next kernel does not take (scaled outputs only): streaming dp4a GEMV over the tile blob;
+ *     up to 32 tokens on matrices whose 128-channel tiles and k-ranges of at most 16 x 128 (8 above 16 tokens)
+ *              fit the SMs: the decode kernel, ONE launch, the k-ranges of a tile joined in a thread-block cluster;
  *     3072 tokens and more (5120 on matrices above 32 M weights) on layers with K < 8192, whole 256-channel
  *              blocks and at most 256 M weights, one destination: the blob is unpacked to INT8 in the workspace
  *              (scratch, N x K bytes) and the INT8 x INT8 CTA-pair kernel does the GEMM, TWO launches

@@ -48,8 +48,8 @@ TRACE_LIB_PATH = os.path.join(HERE, "_lq_b200_trace.so")
 
 def build(force: bool = False, verbose: bool = False, debug: bool = False, trace: bool = False) -> str:
     """Compile every .cu of the product (or, with ``debug``, the measurement kernels) into one shared
-    library; returns its path.  ``trace`` builds the product sources with -DLQ_PIPELINE_TRACE (per-CTA cycle
-    counters in the decode kernel) into a library of its own, which ``LIQUIDGEMM_B200_TRACE=1`` makes
+    library; returns its path.  ``trace`` builds the product sources with -DLQ_PIPELINE_TRACE (per-CTA time stamps
+    and cycle counters) into a library of its own, which ``LIQUIDGEMM_B200_TRACE=1`` makes
     :mod:`liquidgemm_b200._lib` load instead."""
     lib_path, sources = (DEBUG_LIB_PATH, DEBUG_SOURCES) if debug else (LIB_PATH, SOURCES)
     if trace:

@@ -537,9 +537,8 @@ static int pick_bn(int M, int K = 0) {
   if (M <= 32) return 32;
   if (M <= 64) return 64;
   if (M <= 128) return 128;
-  // Two 192-token accumulators.  A single 256-token accumulator (5 stages) measured 20-40 % faster
-  // on long-K shapes but produced intermittent launch failures on a 8192 x 28672 layer; it stays
-  // off until the cause is understood.
+  // Two 192-token accumulators.  (A single 256-token accumulator with five stages raised launch failures on a 8192 x 28672
+  // layer: with an odd ring and two dequant sets a set's wait can pass on a stage that has not landed.)
   return 192;
 }
 
@@ -670,7 +669,7 @@ enum RouteKind {
   kRoutePersistent,   // one CTA per SM, stream-K or a fixed split (explicit requests above 128 tokens, splitk -1)
   kRouteTile,         // two CTAs per SM, one tile each, `splits` int32 planes + finish pass when splits > 1
   kRouteGemv,         // streaming dp4a GEMV over the blob (scaled outputs only)
-  kRouteDecodeTc,     // streaming tensor-core kernel, one launch, atomic join
+  kRouteDecodeTc,     // small matrices: k-ranges of a tile joined in a thread-block cluster, one launch
   kRoutePair,         // CTA pairs, 256 channels x 192 tokens per tile (prefill)
   kRouteUnpackI8,     // very large token counts: unpack the blob to INT8 once, then the INT8 x INT8 pair kernel
 };
@@ -679,10 +678,10 @@ struct Route {
   int splits;
 };
 // The dp4a streaming GEMV over the blob serves one token, two on matrices up to 64 M weights (28672 x 4096 at two
-// tokens: 15.7 us against the tile kernel's 14.8) and three or four on matrices up to 16 M weights (measured on
-// the Llama-3.1-8B shapes against the tensor-core decode kernel: 4096 x 4096 5.2 vs 5.7 us at three tokens;
-// 6144 x 4096 equal; 4096 x 14336 11.2 vs 10.5 us); it only produces scaled outputs, the int32 entry point always
-// uses tensor cores.
+// tokens: 15.7 us against the tile kernel's 14.8) and three or four on matrices up to 16 M weights that the decode kernel does not
+// take (with the quantiser 4096 x 14336, larger, 11.2 us against the tile kernel's 10.5; where the decode kernel serves it is ahead
+// at three tokens too: 4096 x 4096 5.9 against 7.1, 1024 x 4096 4.5 against 5.1); it only produces scaled outputs, the int32
+// entry point always uses tensor cores.
 constexpr int kGemvBlobMaxM = 4;
 
 // Largest batch of the single-launch decode kernel; LQ_DECODE_TC_MAX_M (16 or 32; 0: none) lowers it for measurements.

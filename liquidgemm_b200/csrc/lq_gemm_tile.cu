@@ -422,12 +422,8 @@ static int launch_cfg(const CUtensorMap& tx, const GemmArgs& a, const MultiOut* 
   return launch_one<BN, NS, NT, W4, false>(tx, a, nullptr, splits, st);
 }
 
-// Token-tile widths: the smallest that holds a decode batch, 128 tokens for prefill.  A 192-token
-// configuration (three shared-memory stages, two operand stages, otherwise this kernel) would do 1.5x the
-// tensor-core work per unpacked weight byte; it passed the parity tests on three full-size shapes and then
-// raised an unspecified launch failure on a fourth (28672 x 4096, 8192 tokens) and in back-to-back graph
-// replays.  Reading the index arithmetic, the barrier counts and the tensor-memory budget (192 + 2 x 32 =
-// 256 columns, two CTAs per SM) did not show the cause, so the configuration is not built.
+// Token-tile widths: the smallest that holds a decode batch, 128 tokens for prefill.  (A 192-token configuration with three
+// stages raised launch failures: an odd ring and two dequant sets, whose waits can pass on a stage that has not landed.)
 // Between 65 and 128 tokens a small matrix (up to 32 M weights: the qkv and o projections of an 8B model)
 // takes 64-token tiles: twice the CTAs, so the split factor halves and so do the int32 planes each CTA
 // writes (measured at 128 tokens: 6144 x 4096 15.7 -> 14.4 us, 4096 x 4096 13.5 -> 11.7 us; 28672 x 4096
