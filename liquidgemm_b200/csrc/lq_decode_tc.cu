@@ -353,7 +353,7 @@ w4a8_decode_tc_kernel(const Args args, const std::conditional_t<MULTI, MultiOut,
 #pragma unroll
       for (int c = 0; c < 4; ++c) ch[c] = *reinterpret_cast<const uint4*>(p + c * 2048);
       const uint32_t meta = *reinterpret_cast<const uint32_t*>(my_meta + stage * kTileBytes);
-      ptx::mbar_arrive(bar_wfree + 8 * stage);   // the tile is in registers: its stage may be refilled
+      if (i + NW < nk) ptx::mbar_arrive_reader(bar_wfree + 8 * stage);   // the tile is in registers: its stage is refilled
       stage += kSets;
       if (stage >= (uint32_t)NW) {
         stage -= (uint32_t)NW;

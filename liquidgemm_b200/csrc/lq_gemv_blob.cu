@@ -361,7 +361,7 @@ gemv_blob_kernel(const Args args, const std::conditional_t<MULTI, MultiOut, NoMu
           }
           acc[m] = a + b;
         }
-        ptx::mbar_arrive(bar_empty + 8 * ring.s);
+        ptx::mbar_arrive_reader(bar_empty + 8 * ring.s);
         ring.advance();
       }
 

@@ -69,9 +69,10 @@ def test_quantising_form_equals_two_launches(N, K, dtype):
 
 
 def test_several_streams_at_once():
-    """Four streams replay graphs of this kernel side by side (int8 tokens and the quantising form, k-ranges longer than
-    the seven operands unpacked ahead and longer than the ring), beside the tile kernel's planes and finish pass on 4096 x 14336.
-    Every output of every replay is compared, in the stream, with the persistent kernel's."""
+    """Six streams replay graphs of this kernel side by side (int8 tokens and the quantising form, k-ranges longer than
+    the seven operands unpacked ahead and longer than the ring), beside the GEMV and the tile kernel's planes and finish pass.  A
+    thread that handed a ring stage back too early would meet the next tile's bytes.  Every output of every replay is compared, in
+    the stream, with the persistent kernel's."""
     from liquidgemm_b200 import ops
     g = torch.Generator(device="cuda").manual_seed(5)
     layers = []
@@ -79,7 +80,7 @@ def test_several_streams_at_once():
         qw, blob = ops.quantize_weight_cuda(torch.randn(N, K, generator=g, device="cuda") * 0.03, 64, want_codes=False, want_blob=True)
         layers.append({"s1": qw.s1, "s_u8": qw.s_u8, "offset_a": qw.offset_a, "N": N, "K": K, "rs": blob.reshape(-1)})
     runs = []
-    for M in (3, 8, 16, 32):
+    for M in (1, 2, 3, 8, 16, 32):
         cases = []
         for L in layers:
             x = torch.randn(M, L["K"], generator=g, device="cuda", dtype=torch.bfloat16)
