@@ -221,7 +221,10 @@ LQ_API int lq_quantize_weight(const void* w, int w_dtype, int N, int K, int grou
  *     one token, two tokens on matrices up to 64 M weights, and three or four on matrices up to 16 M weights that
  *              the next kernel does not take (scaled outputs only): streaming dp4a GEMV over the tile blob;
  *     up to 32 tokens on matrices whose 128-channel tiles and k-ranges of at most 16 x 128 (8 above 16 tokens)
- *              fit the SMs: the decode kernel, ONE launch, the k-ranges of a tile joined in a thread-block cluster;
+ *              fit the SMs: the decode kernel, ONE launch, the k-ranges of a tile joined in a thread-block cluster
+ *              (up to 16 tokens on matrices up to 32 M weights in at most four k-ranges of more than 8 x 128, for example
+ *              6144 x 4096, only behind lq_w4a8_linear's own quantiser; given int8 tokens the tile kernel, its planes in
+ *              the all-zero buffer and cleared again);
  *     3072 tokens and more (5120 on matrices above 32 M weights) on layers with K < 8192, whole 256-channel
  *              blocks and at most 256 M weights, one destination: the blob is unpacked to INT8 in the workspace
  *              (scratch, N x K bytes) and the INT8 x INT8 CTA-pair kernel does the GEMM, TWO launches
@@ -240,7 +243,7 @@ LQ_API int lq_quantize_weight(const void* w, int w_dtype, int N, int K, int grou
  * the reference the override only applies to M <= 128 and is clamped to K/128; otherwise 0. */
 LQ_API int lq_gemm_pick_splitk(int M, int N, int K, int env_override);
 /* Workspace bytes for (M,N,K,splitk) and its kind: 0 = none, 1 = scratch (any contents; the
- * tile kernel's planes, or the INT8 weights of the unpack route: 16-byte aligned), 2 = reduction buffer of the streaming, pair and persistent kernels, which must be ALL ZERO when
+ * tile kernel's planes, or the INT8 weights of the unpack route: 16-byte aligned), 2 = reduction buffer, which must be ALL ZERO when
  * a call starts and is all zero again when its kernel ends (the kernel cleans up after itself), so
  * one zero-filled buffer serves any number of successive calls on a stream; calls that overlap on
  * the GPU need separate buffers, and after a LQ_ERR_TIMEOUT the caller must clear it. */

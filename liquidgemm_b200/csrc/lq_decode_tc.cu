@@ -710,6 +710,13 @@ bool decode_tc_workspace_ok(int M, int N, int K, const void* ws, size_t ws_bytes
   return need == 0 || (ws && ws_bytes >= need);
 }
 
+// Ranges of more than eight k-tiles on wide matrices (at most four ranges a tile; 6144 x 4096, 4096 x 7680): more than half of a
+// launch lies behind the wait, and on a part of the SMs only.
+bool decode_tc_long_ranges(int M, int N, int K) {
+  const dtc::Plan p = dtc::plan_for(M, N, K);
+  return p.ring > 0 && p.nk > 8 && p.splits <= 4;
+}
+
 // CTAs a launch of this shape uses: what a consumer of the gather-by-stores epilogue must see arrive
 // from every rank.
 int decode_tc_grid(int M, int N, int K) {

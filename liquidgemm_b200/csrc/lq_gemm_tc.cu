@@ -60,6 +60,7 @@ int run_tile_gemm(const int8_t* x, const uint8_t* blob, const float* ascale, con
 int tile_output_grid(int M, int N, int K, int splits);                            // lq_gemm_tile.cu
 bool decode_tc_serves(int M, int N, int K);                                  // lq_decode_tc.cu
 bool decode_tc_quantises(int M, int N, int K);                               // lq_decode_tc.cu
+bool decode_tc_long_ranges(int M, int N, int K);                             // lq_decode_tc.cu
 size_t decode_tc_workspace_bytes(int M, int N, int K);                       // lq_decode_tc.cu
 bool decode_tc_workspace_ok(int M, int N, int K, const void* ws, size_t ws_bytes);   // lq_decode_tc.cu
 int run_decode_tc(const void* x, int x_dtype, const uint8_t* blob, const float* ascale, const float* s1, const void* bias,
@@ -747,7 +748,17 @@ static bool unpack_i8_serves(int M, int N, int K) {
   return lim > 0 && M >= lim && K < 8192 && (size_t)N * K <= ((size_t)256 << 20) && i8_pair_serves(M, N, K);
 }
 
-static Route route_for(int M, int N, int K, int splitk, bool scaled, bool single_dest = true) {
+// Calls with int8 tokens, one destination and a workspace of the all-zero kind, whose k-ranges would be long: the tile kernel, its planes
+// in that buffer.  Which of the two is ahead depends on the neighbours in the stream.  us of a launch on 6144 x 4096 at 4 / 16 tokens,
+// decode / tile kernel: in a chain of its like 6.2 / 6.4 and 6.5 / 6.4; in front of 28672 x 4096 8.2 / 6.9 and 8.7 / 6.8; behind an
+// ordinary kernel 11.6 / 9.9 and 11.6 / 10.3 (with that kernel).  Behind the token quantiser of the same call (lq_w4a8_linear) the decode
+// kernel stays: the four linears of a decoder layer 43.8 / 47.3 / 45.3 us at 4 / 8 / 16 tokens, 45.4 / 46.4 / 45.7 without it here.
+static bool long_decode_ranges(int M, int N, int K) {
+  return M <= 16 && (long)N * K <= (1L << 25) && decode_serves(M, N, K) && decode_tc_long_ranges(M, N, K);
+}
+
+// behind_quantiser: the tokens come from the same call's quantiser.
+static Route route_for(int M, int N, int K, int splitk, bool scaled, bool single_dest = true, bool behind_quantiser = false) {
   const int kt = K / 128;
   if (splitk == -1) return {kRoutePersistent, 0};
   if (M <= 128) {
@@ -755,7 +766,7 @@ static Route route_for(int M, int N, int K, int splitk, bool scaled, bool single
       if (scaled && gemv_serves(M, N, K)) return {kRouteGemv, 0};
       // What fits one CTA per SM (lq_decode_tc.cu); larger matrices are ahead on the tile kernel's whole tiles (or its
       // planes and finish pass).
-      if (decode_serves(M, N, K)) return {kRouteDecodeTc, 0};
+      if (decode_serves(M, N, K) && !(single_dest && !behind_quantiser && long_decode_ranges(M, N, K))) return {kRouteDecodeTc, 0};
     }
     int S = splitk > 0 ? splitk : tile_pick_splits(M, N, K);
     if (S > kt) S = kt;
@@ -777,7 +788,7 @@ static Route route_for(int M, int N, int K, int splitk, bool scaled, bool single
 // through the buffer as it is, costs more; us at one token, tile kernel / persistent: 24000 x 512 3.4 / 9.0, 28672 x 4096 14.5 /
 // 19.3, 4096 x 14336 9.6 / 13.4, 7168 x 8192 9.0 / 13.6, 256 x 28672 7.6 / 8.0.)
 static bool planes_in_zeroed_buffer(int M, int N, int K, int splitk, bool scaled) {
-  return splitk == 0 && !scaled && gemv_serves(M, N, K);
+  return splitk == 0 && M <= 128 && ((!scaled && gemv_serves(M, N, K)) || long_decode_ranges(M, N, K));
 }
 
 static size_t route_ws_bytes(const Route& r, int M, int N, int K) {
@@ -795,7 +806,9 @@ static size_t route_ws_bytes(const Route& r, int M, int N, int K) {
 size_t lq_gemm_workspace_bytes(int M, int N, int K, int splitk) {
   if (M <= 0 || N <= 0 || K < 128) return 0;
   const size_t a = route_ws_bytes(route_for(M, N, K, splitk, true), M, N, K);
-  const size_t b = route_ws_bytes(route_for(M, N, K, splitk, false), M, N, K);
+  size_t b = route_ws_bytes(route_for(M, N, K, splitk, false), M, N, K);
+  // (what both kernels of such a shape are told of)
+  if (splitk == 0 && long_decode_ranges(M, N, K)) b = b > decode_tc_workspace_bytes(M, N, K) ? b : decode_tc_workspace_bytes(M, N, K);
   return a > b ? a : b;
 }
 
@@ -803,6 +816,7 @@ size_t lq_gemm_workspace_bytes(int M, int N, int K, int splitk) {
 int lq_gemm_workspace_kind(int M, int N, int K, int splitk) {
   if (lq_gemm_workspace_bytes(M, N, K, splitk) == 0) return 0;
   const RouteKind k = route_for(M, N, K, splitk, true).kind;
+  if (k == kRouteTile && planes_in_zeroed_buffer(M, N, K, splitk, true)) return 2;
   return (k == kRouteTile || k == kRouteUnpackI8) ? 1 : 2;   // 1: scratch, 2: all-zero reduction buffer
 }
 
@@ -815,12 +829,12 @@ int lq_gemm_launches(int M, int N, int K, int splitk) {
 
 static int blob_gemm(const int8_t* x, const uint8_t* blob, const float* ascale, const float* s1, const void* bias,
                      void* out, int out_mode, int M, int N, int K, int splitk, void* ws, size_t ws_bytes,
-                     cudaStream_t st) {
+                     cudaStream_t st, bool behind_quantiser = false) {
   if (!x || !blob || !out || M < 0 || N <= 0 || K <= 0) return LQ_ERR_BAD_ARG;
   if (K % 128) return LQ_ERR_SHAPE;
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(blob)) % 16) return LQ_ERR_BAD_ARG;
   if (M == 0) return LQ_OK;
-  const Route r = route_for(M, N, K, splitk, out_mode != kOutI32);
+  const Route r = route_for(M, N, K, splitk, out_mode != kOutI32, true, behind_quantiser);
   if (r.kind != kRoutePersistent) {
     if (int rc = lq_check_device()) return rc;
   }
@@ -830,6 +844,7 @@ static int blob_gemm(const int8_t* x, const uint8_t* blob, const float* ascale, 
     case kRouteDecodeTc:
       return run_decode_tc(x, -1, blob, ascale, s1, bias, single_out(out, N), nullptr, out_mode, M, N, K, ws, ws_bytes, st);
     case kRouteTile:
+      if (splitk == 0 && long_decode_ranges(M, N, K) && !decode_tc_workspace_ok(M, N, K, ws, ws_bytes)) return LQ_ERR_WORKSPACE;
       return run_tile_gemm(x, blob, ascale, s1, bias, single_out(out, N), nullptr, out_mode, M, N, K, r.splits, ws,
                            ws_bytes, planes_in_zeroed_buffer(M, N, K, splitk, out_mode != kOutI32), st);
     case kRoutePair:
@@ -919,7 +934,7 @@ static int linear_impl(const void* x, int x_dtype, const uint8_t* blob, const fl
   int8_t* xq = static_cast<int8_t*>(scratch);
   float* ascale = reinterpret_cast<float*>(xq + (((size_t)M * K + 255) & ~(size_t)255));
   if (int rc = lq_quant_per_token(x, x_dtype, xq, ascale, M, K, stream)) return rc;
-  return blob_gemm(xq, blob, ascale, s1, bias, y, out_dtype, M, N, K, splitk, workspace, workspace_bytes, as_stream(stream));
+  return blob_gemm(xq, blob, ascale, s1, bias, y, out_dtype, M, N, K, splitk, workspace, workspace_bytes, as_stream(stream), true);
 }
 
 int lq_w4a8_linear(const void* x, int x_dtype, const uint8_t* blob, const float* s1, const void* bias, void* y,

@@ -29,3 +29,30 @@ def test_buffer_stays_zero(M, N, K):
         assert_bits_equal(ops.gemm_fused(xt, blob, st, tq.s1, N, K, 0), O.scale_f32(acc, sc, qw.s1), 0, f"{M}x{N}x{K}")
     assert ops._WORKSPACES and all(int(ws.max()) == 0 for ws in ops._WORKSPACES.values())
     ops.poll_status()
+
+
+@pytest.mark.parametrize("M", [3, 8, 16])
+@pytest.mark.parametrize("N,K", [(6144, 4096), (4096, 7680), (4998, 4096)])
+def test_scaled_planes_are_cleared(M, N, K):
+    """int8 tokens on shapes whose k-ranges are too long for the decode kernel: callers bring the all-zero buffer, the tile
+    kernel writes its planes into it, the finish pass clears them; too small a buffer stays refused."""
+    from liquidgemm_b200 import ops
+    from liquidgemm_b200._lib import lib
+    assert lib.lq_gemm_workspace_kind(M, N, K, 0) == 2 and lib.lq_gemm_launches(M, N, K, 0) == 2
+    qw = random_lqq(N, K, seed=M + N)
+    tq = to_torch_qw(qw)
+    blob = ops._repack_device(tq.qweight_u4, 0, tq.s_u8, tq.offset_a, N, K, 64).reshape(-1)
+    x, sc = random_tokens(M, K, seed=M)
+    xt, st = torch.from_numpy(x).cuda(), torch.from_numpy(sc).cuda()
+    want = ops.gemm_fused(xt, blob, st, tq.s1, N, K, 0, splitk=-1)
+    bias = torch.randn(N, device="cuda").to(torch.bfloat16)
+    for _ in range(3):
+        assert torch.equal(ops.gemm_fused(xt, blob, st, tq.s1, N, K, 0), want)
+        assert torch.equal(ops.linear_bias(xt, blob, st, tq.s1, bias, N, K, 0), want + bias)
+        assert torch.equal(ops.gemm_i32(xt, blob, N, K), ops.gemm_i32(xt, blob, N, K, splitk=1))
+    assert ops._WORKSPACES and all(int(ws.max()) == 0 for ws in ops._WORKSPACES.values())
+    y, nb = torch.empty_like(want), lib.lq_gemm_workspace_bytes(M, N, K, 0)
+    ws = torch.zeros(nb, dtype=torch.uint8, device="cuda")
+    assert lib.lq_w4a8_gemm_fused(xt.data_ptr(), blob.data_ptr(), st.data_ptr(), tq.s1.data_ptr(), y.data_ptr(), 0, M, N, K, 0,
+                                  ws.data_ptr(), nb - 1, None) == -3
+    ops.poll_status()
