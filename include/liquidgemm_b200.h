@@ -222,7 +222,7 @@ LQ_API int lq_quantize_weight(const void* w, int w_dtype, int N, int K, int grou
  *              the next kernel does not take (scaled outputs only): streaming dp4a GEMV over the tile blob;
  *     up to 32 tokens on matrices whose 128-channel tiles and k-ranges of at most 16 x 128 (8 above 16 tokens)
  *              fit the SMs: the decode kernel, ONE launch, the k-ranges of a tile joined in a thread-block cluster
- *              (up to 16 tokens on matrices up to 32 M weights in at most four k-ranges of more than 8 x 128, for example
+ *              (9 to 16 tokens on matrices up to 32 M weights in at most four k-ranges of more than 8 x 128, for example
  *              6144 x 4096, only behind lq_w4a8_linear's own quantiser; given int8 tokens the tile kernel, its planes in
  *              the all-zero buffer and cleared again);
  *     3072 tokens and more (5120 on matrices above 32 M weights) on layers with K < 8192, whole 256-channel

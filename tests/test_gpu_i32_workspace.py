@@ -31,7 +31,7 @@ def test_buffer_stays_zero(M, N, K):
     ops.poll_status()
 
 
-@pytest.mark.parametrize("M", [3, 8, 16])
+@pytest.mark.parametrize("M", [9, 13, 16])
 @pytest.mark.parametrize("N,K", [(6144, 4096), (4096, 7680), (4998, 4096)])
 def test_scaled_planes_are_cleared(M, N, K):
     """int8 tokens on shapes whose k-ranges are too long for the decode kernel: callers bring the all-zero buffer, the tile
