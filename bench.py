@@ -489,7 +489,7 @@ def main():
                          "of": peaks["source"], "traffic_source": f"ncu DRAM bytes / algorithmic bytes = {NCU_TRAFFIC_RATIO} on single launches "
                                            "(profiles/decode_kernels_ncu_full.md) x this step's algorithmic bytes",
                          "kernel": "w4a8_tile_kernel (gate_up and down at M = 4, 8, 16; down with finish_kernel), "
-                                   "w4a8_decode_tc_kernel (qkv at M = 4, 8, 16), gemv_blob_kernel (M = 1): the 12-op sweep",
+                                   "w4a8_decode_tc_kernel (qkv at M = 4, 8; tile kernel at 16), gemv_blob_kernel (M = 1): the 12-op sweep",
                          "algorithmic_bytes_per_step": abytes},
             "cpu_baseline": cpu,
             "e2e": {"value": e2e_value, "unit": UNIT,

@@ -751,7 +751,7 @@ static bool unpack_i8_serves(int M, int N, int K) {
 // Calls with nine to sixteen int8 tokens, one destination and a workspace of the all-zero kind, whose k-ranges would be long: the tile
 // kernel, its planes in that buffer.  Which of the two is ahead depends on the neighbours in the stream; up to eight tokens callers
 // know it as one launch, and it is ahead in a chain of its like.  us of a launch on 6144 x 4096 at 4 / 16 tokens,
-// decode / tile kernel: in such a chain 6.2 / 6.4 and 6.5 / 6.4; in front of 28672 x 4096 8.2 / 6.9 and 8.7 / 6.8; behind an
+// decode / tile kernel: in such a chain 6.2 / 6.4 and 6.4 / 7.3 (behind quantisers 8.5 / 8.3); in front of 28672 x 4096 8.2 / 6.9 and 8.7 / 6.8; behind an
 // ordinary kernel 11.6 / 9.9 and 11.6 / 10.3 (with that kernel).  Behind the token quantiser of the same call (lq_w4a8_linear) the decode
 // kernel stays: the four linears of a decoder layer 43.8 / 47.3 / 45.3 us at 4 / 8 / 16 tokens, 45.4 / 46.4 / 45.7 without it here.
 static bool long_decode_ranges(int M, int N, int K) {
